@@ -18,6 +18,11 @@ so that one text compiles as
   * host C++ over a counting number type (K<sq_count,..>), which gives the algorithmic flop count of
     the double path per point for each SQ_AB (+ - * / each 1, as in scripts/plot5_cost.py:11).
 
+An integrand that is a scan over its axes (axis_plan: a product or sum accumulated axis by axis of functions
+of one coordinate each, then a function of the accumulated values) is also emitted in that form, as a second
+class template KA: the functions of one coordinate become columns of a table over (axis, k), evaluated once per
+lattice instead of once per point.
+
 The graph descriptor `const graph_t G_<g>={name,volkov,L,D,weight,n,fixed,...}` (driver/common.h:38)
 and the Gauss-Legendre tables are carried over as data.
 
@@ -181,6 +186,204 @@ def split_plan(k, max_parts=12):
     return groups, '\n'.join(out)
 
 
+# ---------------------------------------- the axis form ---------------------------------------------
+_TOK = re.compile(r'\s*(?:([A-Za-z_]\w*)|(\d+\.?\d*(?:[eE][+-]?\d+)?|\.\d+(?:[eE][+-]?\d+)?)|([-+*/()\[\],]))')
+
+
+class _Expr:
+    """An expression of the kernel sources: identifiers, numbers, + - * /, unary minus, calls, indexing."""
+
+    def __init__(self, op, text, args=()):
+        self.op, self.text, self.args = op, text, args
+
+
+def _parse(text):
+    """The expression's tree, left-associative as C reads it; ValueError outside the subset."""
+    toks, p = [], 0
+    text = text.strip()
+    while p < len(text):
+        m = _TOK.match(text, p)
+        if not m:
+            raise ValueError(text)
+        toks.append(m.group(1) or m.group(2) or m.group(3))
+        p = m.end()
+    pos = [0]
+
+    def peek():
+        return toks[pos[0]] if pos[0] < len(toks) else None
+
+    def take(want=None):
+        t = peek()
+        if t is None or (want and t != want):
+            raise ValueError(text)
+        pos[0] += 1
+        return t
+
+    def atom():
+        t = take()
+        if t == '-':
+            e = atom()
+            return _Expr('neg', '-' + e.text, (e,))
+        if t == '(':
+            e = add()
+            take(')')
+            return _Expr('par', '(' + e.text + ')', (e,))
+        if re.match(r'[A-Za-z_]', t):
+            if peek() == '(':
+                take()
+                args = [add()]
+                while peek() == ',':
+                    take()
+                    args.append(add())
+                take(')')
+                return _Expr('call', '%s(%s)' % (t, ','.join(a.text for a in args)), (t,) + tuple(args))
+            if peek() == '[':
+                take()
+                e = add()
+                take(']')
+                return _Expr('idx', '%s[%s]' % (t, e.text), (t, e))
+            return _Expr('id', t)
+        if re.match(r'[\d.]', t):
+            return _Expr('num', t)
+        raise ValueError(text)
+
+    def chain(sub, ops):
+        e = sub()
+        while peek() in ops:
+            o = take()
+            f = sub()
+            e = _Expr(o, e.text + o + f.text, (e, f))
+        return e
+
+    def mul():
+        return chain(atom, ('*', '/'))
+
+    def add():
+        return chain(mul, ('+', '-'))
+
+    e = add()
+    if pos[0] != len(toks):
+        raise ValueError(text)
+    return e
+
+
+_LOOP = re.compile(r'^\s*REAL ([^;]*);\s*for\(int i=0;i<(\d+);i\+\+\)\{(.*?)\n  \}\n(.*)$', re.S)
+
+
+def axis_plan(k):
+    """The axis form of f_<g>, or None.
+
+    f_ must be: scalar accumulators with literal starts; one loop over all D axes whose body defines constants
+    from sf[i] (and constant tables at i) alone and updates the accumulators; a tail that uses the
+    accumulators only.  In the updates every largest subexpression that depends on sf[i] alone and is more than
+    sf[i] itself becomes a table column; a division of an accumulated value by a column carries the column's
+    reciprocal along (sq_divu: the same rounded quotient).  Every remaining operation and its order are those
+    of f_, so the values are the same bit for bit.
+
+    Returns the text of the class template KA: NU columns and NR reciprocals per (axis, k) entry; axis() fills
+    an entry's columns; rc(n) is the column of reciprocal n; init/step/fin are the scan."""
+    m = re.search(r'^static REAL FN\(f_%s\)\(const REAL \*sf, REAL \*ab\)\{\n(.*?)\n\}$' % re.escape(k.name), k.qhalf, re.M | re.S)
+    lm = _LOOP.match(m.group(1)) if m else None
+    if not lm or int(lm.group(2)) != k.D or k.D < 4:
+        return None
+    decl, body, tail = lm.group(1), lm.group(3), lm.group(4)
+    carried = {}
+    for d in decl.split(','):
+        dm = re.match(r'^\s*([A-Za-z_]\w*)\s*=\s*(\d+(?:\.\d*)?)\s*$', d)
+        if not dm:
+            return None
+        carried[dm.group(1)] = dm.group(2)
+    if re.search(r'\b(sf|i)\b|\bfor\b|\bstatic\b|\bFN\b', tail) or 'return' not in tail:
+        return None
+    tables, uni, consts, cols, recip, steps = {t[0] for t in k.gl}, set(), [], [], [], []
+
+    def kind(e):
+        """0: no coordinate, 1: a function of sf[i], 2: uses an accumulator; ValueError for anything else"""
+        if e.op == 'num':
+            return 0
+        if e.op == 'id':
+            if e.text in carried:
+                return 2
+            if e.text in uni:
+                return 1
+            raise ValueError(e.text)
+        if e.op == 'idx':
+            if e.args[1].text != 'i' or (e.args[0] != 'sf' and e.args[0] not in tables):
+                raise ValueError(e.text)
+            return 1
+        if e.op == 'call':
+            if e.args[0] not in ('SQ_EXP', 'SQ_LOG', 'RABS'):
+                raise ValueError(e.text)
+            return max(kind(a) for a in e.args[1:])
+        return max(kind(a) for a in e.args)
+
+    def column(e):
+        if e.text == 'sf[i]':
+            return 'si', None
+        if e.text not in cols:
+            cols.append(e.text)
+        return 'u[%d]' % cols.index(e.text), cols.index(e.text)
+
+    def rewrite(e, term=False):
+        kd = kind(e)
+        if kd == 0:
+            return e.text
+        if kd == 1:
+            # a product that is added to an accumulated value keeps its factors apart, so that the contracted
+            # build fuses it as it fuses f_'s own
+            if term and e.op == '*':
+                return rewrite(e.args[0]) + '*' + rewrite(e.args[1])
+            if term and e.op in ('par', 'neg'):
+                return ('(%s)' if e.op == 'par' else '-%s') % rewrite(e.args[0], True)
+            return column(e)[0]
+        if e.op == 'id':
+            return 'S.' + e.text
+        if e.op == 'neg':
+            return '-' + rewrite(e.args[0])
+        if e.op == 'par':
+            return '(' + rewrite(e.args[0]) + ')'
+        if e.op == 'call':
+            return '%s(%s)' % (e.args[0], ','.join(rewrite(a) for a in e.args[1:]))
+        a, b = e.args
+        if e.op == '/' and kind(a) == 2 and kind(b) == 1:
+            name, c = column(b)
+            if c is not None:
+                if c not in recip:
+                    recip.append(c)
+                return 'sq_divu(%s,%s,r[%d])' % (rewrite(a), name, recip.index(c))
+        return rewrite(a, e.op in '+-') + e.op + rewrite(b, e.op in '+-')
+
+    try:
+        for stmt in [x.strip() for x in body.split(';') if x.strip()]:
+            cm = re.match(r'^const REAL ([A-Za-z_]\w*)=(.*)$', stmt, re.S)
+            am = re.match(r'^([A-Za-z_]\w*)=(.*)$', stmt, re.S)
+            if cm:
+                if cm.group(1) in carried or cm.group(1) in uni or cm.group(1) in ('si', 'u', 'r', 'S') or kind(_parse(cm.group(2))) == 2:
+                    return None
+                consts.append('    const REAL %s=%s;' % (cm.group(1), re.sub(r'\bsf\[i\]', 'si', cm.group(2))))
+                uni.add(cm.group(1))
+            elif am and am.group(1) in carried:
+                steps.append('    S.%s=%s;' % (am.group(1), rewrite(_parse(am.group(2)))))
+            else:
+                return None
+    except ValueError:
+        return None
+    if not any(re.search(r'SQ_(EXP|LOG)|/', c) for c in cols + consts):
+        return None
+    out = ['template<class SqReal_, int SQ_AB> struct KA {',
+           '  enum { NU = %d, NR = %d };' % (len(cols), len(recip)),
+           '  static SQ_FUNC constexpr int rc(int n){ const int c[%d]={%s}; return c[n]; }'
+           % (max(1, len(recip)), ','.join(str(c) for c in recip) or '0'),
+           '  struct st { REAL %s; };' % ', '.join(carried),
+           '  static SQ_FUNC_K void init(st &S){ %s }' % ' '.join('S.%s=%s;' % c for c in carried.items()),
+           '  static SQ_FUNC_K void axis(int i, const REAL si, REAL *u){'] + consts
+    out += ['    u[%d]=%s;' % (n, re.sub(r'\bsf\[i\]', 'si', c)) for n, c in enumerate(cols)]
+    out += ['  }', '  static SQ_FUNC_K void step(st &S, const REAL si, const REAL *u, const double *r){'] + steps
+    out += ['  }', '  static SQ_FUNC_K REAL fin(const st &S, REAL *ab){',
+            '    const REAL %s;' % ', '.join('%s=S.%s' % (c, c) for c in carried), tail.rstrip(), '  }', '};']
+    return '\n'.join(out)
+
+
 def emit(src):
     """Header text for one graph: namespace SQG_NS(<name>) (a macro of the including unit, normally
     sqg_<name>) with the tables and two copies of the class
@@ -209,13 +412,16 @@ def emit(src):
                 '};']
     else:
         out += ['template<class SqReal_, int SQ_AB> using KD = K<SqReal_, SQ_AB>;']
+    axis = None if plan else axis_plan(k)
+    if axis:
+        out += ['#ifdef SQ_AXIS_FORM', '/* the same function as a scan over the axes (kgen.axis_plan) */', axis, '#endif']
     out += ['#undef REAL', '#undef FN', '}']
     if plan:
         out.append('SQ_GRAPH_SPLIT(%s, "%s", %d, %d, %d, %d, %d, %d)' % (k.name, k.volkov.replace('"', '\\"'),
                                                                     k.L, k.D, k.weight, k.n, k.fixed, len(plan[0])))
     else:
-        out.append('SQ_GRAPH(%s, "%s", %d, %d, %d, %d, %d)' % (k.name, k.volkov.replace('"', '\\"'),
-                                                            k.L, k.D, k.weight, k.n, k.fixed))
+        line = '(%s, "%s", %d, %d, %d, %d, %d)' % (k.name, k.volkov.replace('"', '\\"'), k.L, k.D, k.weight, k.n, k.fixed)
+        out += ['#ifdef SQ_AXIS_FORM', 'SQ_GRAPH_AXIS' + line, '#else', 'SQ_GRAPH' + line, '#endif'] if axis else ['SQ_GRAPH' + line]
     if k.has_ptq:
         out.append('SQ_SCALE(%s)' % k.name)
     return k, '\n'.join(out) + '\n'

@@ -291,11 +291,12 @@ struct Integral {
             if(R.g->zlattice){ R.X[k + K] = k*h; R.Wt[k + K] = h; }
             else { R.X[k + K] = exp(k*h); R.Wt[k + K] = R.X[k + K]*h; }
         }
-        if(sqb_dev_tables(R.X.data(), R.Wt.data(), K)) FAIL("device: %s", sqb_last_error());
+        if(sqb_dev_tables(R.X.data(), R.Wt.data(), K) || sqb_dev_axis(R.g, R.o.fma)) FAIL("device: %s", sqb_last_error());
         if(tables){
-            dtab = (double*)sqb_dev_alloc(2*(2*K + 1)*sizeof(double));
+            dtab = (double*)sqb_dev_alloc((2*(2*K + 1) + sqb_dev_axis_words(R.g, K))*sizeof(double));
             if(!dtab || sqb_dev_upload(dtab, R.X.data(), (2*K + 1)*sizeof(double)) ||
-               sqb_dev_upload(dtab + 2*K + 1, R.Wt.data(), (2*K + 1)*sizeof(double))) FAIL("device copy of the lattice tables failed");
+               sqb_dev_upload(dtab + 2*K + 1, R.Wt.data(), (2*K + 1)*sizeof(double)) ||
+               sqb_dev_axis_fill(R.g, R.o.fma, dtab, K, dtab + 2*(2*K + 1))) FAIL("device copy of the lattice tables failed");
         }
         /* the symmetry fold's group (driver/sum.c:566-592), before the run's clock starts as there */
         sym.n = 1;

@@ -92,6 +92,7 @@ struct Dev {
     cudaStream_t s;
     cudaEvent_t e0, e1;
     double *X, *Wt; int tabcap, K;
+    double *axb; long axcap; const double *U, *Ud;   /* axis tables of the current lattice and graph (NULL: none) */
     long cap;                      /* points per batch */
     double *v, *uu; unsigned char *stt, *cfl, *cw; long *fb; unsigned long long *nfb;
     unsigned long long *sel, *nsel;   /* list mode: the children to evaluate and their number */
@@ -168,7 +169,37 @@ extern "C" int sqb_dev_tables(const double *X, const double *Wt, int K){
     CKR(cudaMemcpy(G.X, X, nt*sizeof(double), cudaMemcpyHostToDevice));
     CKR(cudaMemcpy(G.Wt, Wt, nt*sizeof(double), cudaMemcpyHostToDevice));
     H2D += 2*nt*sizeof(double);
-    G.K = K;
+    G.K = K; G.U = G.Ud = NULL;
+    return 0;
+}
+
+/* doubles of a graph's two axis tables over a lattice (0: the integrand has no axis form); FP64 first */
+static long axis_words(const sqb_graph_t *g, int K, int which){ return g->axis ? (long)g->D*(2*K + 1)*g->axw[which] : 0; }
+extern "C" long sqb_dev_axis_words(const sqb_graph_t *g, int K){ return axis_words(g, K, 0) + axis_words(g, K, 1); }
+/* fills the tables of the lattice X (device) for the FP64 build fma at T (device), on the thread's stream */
+extern "C" int sqb_dev_axis_fill(const sqb_graph_t *g, int fma, const double *X, int K, double *T){
+    if(!g->axis) return 0;
+    g->axis(fma && g->f64_fma ? 2 : 0, X, K, T, G.s);
+    g->axis(1, X, K, T + axis_words(g, K, 0), G.s);
+    CKR(cudaGetLastError());
+    G.launches += 2;
+    return 0;
+}
+/* the axis tables of graph g on the thread's current lattice (sqb_dev_tables), used by the evaluations that
+ * follow until the lattice changes */
+extern "C" int sqb_dev_axis(const sqb_graph_t *g, int fma){
+    G.U = G.Ud = NULL;
+    const long n = sqb_dev_axis_words(g, G.K);
+    if(!n) return 0;
+    if(n > G.axcap){
+        if(G.axb) cudaFree(G.axb);
+        G.axb = NULL; G.axcap = 0;
+        long c = 1L << 13; while(c < n) c <<= 1;
+        CKR(cudaMalloc(&G.axb, c*sizeof(double)));
+        G.axcap = c;
+    }
+    if(sqb_dev_axis_fill(g, fma, G.X, G.K, G.axb)) return -1;
+    G.U = G.axb; G.Ud = G.axb + axis_words(g, G.K, 0);
     return 0;
 }
 
@@ -213,11 +244,14 @@ static int grid_for(const sqb_graph_t *g, int which, long npts, size_t smem){
 }
 
 static void fill_eval(sqb_eval_t *a, const sqb_test_t *t){
-    a->X = G.X; a->Wt = G.Wt; a->K = G.K; a->H = 0; a->raw = 0;
+    a->X = G.X; a->Wt = G.Wt; a->K = G.K; a->H = 0; a->raw = 0; a->U = G.U; a->Ud = G.Ud;
     a->abskip = t->abskip; a->abcheck = t->abcheck;
     a->abserr = t->abserr; a->near_thr = t->nearf*t->abserr; a->ddslack = t->ddslack;
     a->v = G.v; a->ab = NULL; a->stt = G.stt; a->fb = G.fb; a->nfb = G.nfb; a->fbcap = G.cap;
 }
+
+/* work items per tile of an axis-form level launch whose tiles the reduce kernel sums: 1024 children each */
+#define SQB_SUB 4
 
 /* whether a batch's FP64 pass runs in passes (the graph has them, they are asked for, a level batch) */
 static inline bool use_split(const sqb_graph_t *g, const sqb_eval_t *a, const sqb_test_t *t){
@@ -277,7 +311,8 @@ static int eval_batch(const sqb_graph_t *g, sqb_eval_t *a, const sqb_test_t *t, 
             CKR(cudaMemsetAsync(a->queue, 0, sizeof(unsigned long long), G.s));
             int sw = 1;
             const long cap = grid_cap(g, w | (sqb_level_launch(a) ? SQB_ATTR_LEVEL : 0), smem, NULL, &sw);
-            const long items = a->ntile*sw;       /* the level kernel may take every tile twice */
+            const long items = sqb_axis_launch(a) && a->sub > 1 ? a->ntile*a->sub : a->ntile*sw;   /* the level kernel may
+                                                                                  take every tile twice */
             launch_f64(g, w, a, (int)(items < cap ? items : cap), smem, G.s);
         } else launch_f64(g, w, a, grid_for(g, w, npts, smem), smem, G.s);
         CKR(cudaGetLastError());
@@ -706,7 +741,8 @@ extern "C" int sqb_dev_level(const sqb_level_t *L, sqb_acc_t *acc, long *next_n,
             sqb_inst_t &I = a.inst[0];
             I.pts = cells; I.n = nc; I.child0 = 0; I.st = L->st; I.K = G.K; I.toff = 0; I.fused = fused;
             I.last = L->last; I.pw = L->pw; I.thr = L->thr; I.abserr = L->t.abserr; I.near_thr = L->t.nearf*L->t.abserr;
-            I.X = G.X; I.Wt = G.Wt;
+            I.X = G.X; I.Wt = G.Wt; I.U = G.U; I.Ud = G.Ud;
+            a.sub = fused ? 1 : SQB_SUB;
         }
         lvl_t r; memset(&r, 0, sizeof r);
         r.cells = (const signed char*)cells; r.n = nch; r.D = D; r.st = L->st; r.last = L->last;
@@ -755,6 +791,12 @@ extern "C" int sqb_dev_level(const sqb_level_t *L, sqb_acc_t *acc, long *next_n,
     return 0;
 }
 
+/* an integral's axis tables: they follow X and Wt (sqb_level_t) when the graph has the axis form */
+static const double *level_axis(const sqb_level_t &L, int dd){
+    if(!L.X || !L.g->axis) return NULL;
+    return L.X + 2*(2*L.K + 1) + (dd ? axis_words(L.g, L.K, 0) : 0);
+}
+
 /* A level of several integrals of one graph at once (see sqb_rt.h).  Each integral keeps the batches,
  * tiles and fused/unfused choice that sqb_dev_level would give it alone; round r launches batch r of every
  * integral that has one, its children numbered integral after integral from tile boundaries. */
@@ -774,13 +816,16 @@ extern "C" int sqb_dev_level_multi(const sqb_level_t *Ls, int n, sqb_acc_t *accs
     if(one_by_one){
         /* each integral on its own tables: the thread's current ones are lent the integral's device copy */
         double tot = 0; int rc = 0;
-        double *sx = G.X, *sw = G.Wt; const int sk = G.K;
+        double *sx = G.X, *sw = G.Wt; const int sk = G.K; const double *su = G.U, *sd = G.Ud;
         for(int k = 0; k < n && !rc; k++){
-            if(Ls[k].X){ G.X = (double*)Ls[k].X; G.Wt = (double*)Ls[k].Wt; G.K = Ls[k].K; }
+            if(Ls[k].X){
+                G.X = (double*)Ls[k].X; G.Wt = (double*)Ls[k].Wt; G.K = Ls[k].K;
+                G.U = level_axis(Ls[k], 0); G.Ud = level_axis(Ls[k], 1);
+            }
             double m = 0;
             rc = sqb_dev_level(&Ls[k], &accs[k], &next_n[k], &m);
             tot += m;
-            G.X = sx; G.Wt = sw; G.K = sk;
+            G.X = sx; G.Wt = sw; G.K = sk; G.U = su; G.Ud = sd;
         }
         if(ms) *ms = tot;
         return rc;
@@ -829,6 +874,7 @@ extern "C" int sqb_dev_level_multi(const sqb_level_t *Ls, int n, sqb_acc_t *accs
         lvl_t rl; memset(&rl, 0, sizeof rl);
         rl.D = D; rl.abskip = L0.t.abskip; rl.v = G.v; rl.uu = G.uu; rl.stt = G.stt; rl.sym = a.sym;
         long child0 = 0; int m = 0, toff = 0, last = 0, kof[SQB_MAXINST];
+        a.sub = SQB_SUB;
         for(int k = 0; k < n; k++){
             if(r >= nbat[k]) continue;
             const sqb_level_t &L = Ls[k];
@@ -837,7 +883,8 @@ extern "C" int sqb_dev_level_multi(const sqb_level_t *Ls, int n, sqb_acc_t *accs
             I.pts = L.cells + c0; I.n = nc; I.child0 = child0; I.st = L.st; I.K = L.K; I.toff = toff;
             I.fused = tile_sums() && cank[k] && nch >= 2*SQB_TILE*capk[k];
             I.last = L.last; I.pw = L.pw; I.thr = L.thr; I.abserr = L.t.abserr; I.near_thr = L.t.nearf*L.t.abserr;
-            I.X = L.X; I.Wt = L.Wt;
+            I.X = L.X; I.Wt = L.Wt; I.U = level_axis(L, 0); I.Ud = level_axis(L, 1);
+            if(I.fused) a.sub = 1;
             lvi_t &V = rl.inst[m];
             V.cells = (const signed char*)(L.cells + c0); V.n = nch; V.child0 = child0; V.st = L.st; V.last = L.last;
             V.pw = L.pw; V.thr = L.thr; V.next = L.next; V.cap = L.next_cap; V.acc = G.accm + k; V.base = G.basem + k;

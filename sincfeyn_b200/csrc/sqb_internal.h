@@ -59,6 +59,7 @@ typedef struct {
     double pw, thr;               /* its level's weight step^D and keep threshold */
     double abserr, near_thr;      /* its per-point test thresholds (ABSERR depends on the integral's Ref) */
     const double *X, *Wt;         /* its tables (device, 2K+1 each) */
+    const double *U, *Ud;         /* its axis tables (device; NULL: none), FP64 and double-double */
 } sqb_inst_t;
 
 typedef struct {
@@ -68,6 +69,8 @@ typedef struct {
     int cells, st;                /* cells: child b of cell c is k_d - st*bit_d(b) (driver/sum.c:407) */
     const double *X, *Wt;         /* 2K+1 entries: integration variable and weight factor per k;
                                      Wt == NULL: the factor is X*H (driver/lattice.c:33) */
+    const double *U, *Ud;         /* axis form: the columns of every (axis, k), entry axis (2K+1) + k + K, for the FP64
+                                     pass and the double-double pass (sqb_graph_t axis); NULL: evaluate them */
     int K;
     double H;
     int raw;                      /* 1: plain form, v = f w and ab = ab w, no tests */
@@ -104,6 +107,8 @@ typedef struct {
      * others; the FP64 kernel walks the list (tiles of SQB_TILE entries from the queue) and leaves every
      * tile's sums to the reduce kernel */
     const unsigned long long *sel, *nsel;
+    int sub;                      /* level launch of the axis form: work items per tile (1, or 4 when the reduce kernel sums
+                                     every tile, so that a small batch fills the device) */
 } sqb_eval_t;
 #define SQB_SEL_SHIFT 56
 
@@ -143,6 +148,13 @@ typedef struct {
 static inline bool sqb_level_launch(const sqb_eval_t *a){
     return a->ninst > 0 && a->cells && a->esize == 1 && a->part && !a->sel && !a->sfin && !a->raw;
 }
+/* a level launch that the axis form's level kernel runs: every integral has its table, and neither a fold nor
+ * the predictor chooses among a cell's children */
+static inline bool sqb_axis_launch(const sqb_eval_t *a){
+    if(!sqb_level_launch(a) || a->sym.n > 1 || a->cfl) return false;
+    for(int q = 0; q < a->ninst; q++) if(!a->inst[q].U) return false;
+    return true;
+}
 
 typedef struct {
     const char *name, *volkov;
@@ -166,6 +178,10 @@ typedef struct {
     int (*split_attr)(int P, int fma, int block, size_t smem, sqb_kattr_t *out);
     /* the scaling test on the raw double-double point function ptq; NULL for graphs without one (VP) */
     void (*scale)(const sqb_scale_t *a, int grid, int block, void *stream);
+    /* the axis form (kgen.axis_plan; axis NULL: the integrand has none): fills the table T of one lattice,
+     * D (2K+1) entries of axw[which] doubles, which as attr (0 as written, 1 double-double, 2 contracted) */
+    void (*axis)(int which, const double *X, int K, double *T, void *stream);
+    int axw[3];
 } sqb_graph_t;
 
 #ifdef __cplusplus

@@ -57,6 +57,11 @@ const char *sqb_dev_info(void);
 const char *sqb_last_error(void);
 /* tables X[k+K], Wt[k+K] for the current graph (2K+1 entries each) */
 int  sqb_dev_tables(const double *X, const double *Wt, int K);
+/* the axis form (sqb_graph_t axis): the tables of graph g on the thread's current lattice; or, for a caller's own
+ * lattice X on the device, their size in doubles (0: no axis form) and their filling, FP64 then double-double */
+int  sqb_dev_axis(const sqb_graph_t *g, int fma);
+long sqb_dev_axis_words(const sqb_graph_t *g, int K);
+int  sqb_dev_axis_fill(const sqb_graph_t *g, int fma, const double *X, int K, double *T);
 
 /* n nodes (host pt_t list, flags ignored) evaluated with the tests and the fallback: values v, near
  * flags (may be NULL); skip (host, may be NULL) per node; counters added to *nq, *u, *unres */
@@ -79,8 +84,8 @@ typedef struct {
      * the last level = leave out the children whose predicted mean is below predict*thr (esok: and cap
      * their tiers) */
     sqb_vtab_t *vt; int vput; double predict; int esok;
-    /* the integral's lattice tables on the device (2K+1 each), for sqb_dev_level_multi; sqb_dev_level uses
-     * the thread's current tables (sqb_dev_tables) */
+    /* the integral's lattice tables on the device (2K+1 each, X then Wt, then the axis tables of a graph that has
+     * the axis form), for sqb_dev_level_multi; sqb_dev_level uses the thread's current tables (sqb_dev_tables) */
     const double *X, *Wt; int K;
 } sqb_level_t;
 int  sqb_dev_level(const sqb_level_t *L, sqb_acc_t *acc, long *next_n, double *ms);

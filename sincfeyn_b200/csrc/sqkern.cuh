@@ -36,6 +36,7 @@
 #define RABS(x) sq_rabs(x)
 #define SQ_EXP(x) sq_exp(x)
 #define SQ_LOG(x) sq_log(x)
+#define SQ_AXIS_FORM                             /* the axis form of the integrands that have one is compiled */
 
 #ifndef SQB_BLOCK
 #define SQB_BLOCK 128
@@ -78,7 +79,7 @@
 __device__ __forceinline__ void sqb_inst_of(const sqb_eval_t &a, sqb_inst_t *I){
     I->pts = a.pts; I->n = a.n; I->child0 = 0; I->st = a.st; I->K = a.K; I->toff = 0; I->fused = 1;
     I->last = a.last; I->pw = a.pw; I->thr = a.thr; I->abserr = a.abserr; I->near_thr = a.near_thr;
-    I->X = a.X; I->Wt = a.Wt;
+    I->X = a.X; I->Wt = a.Wt; I->U = a.U; I->Ud = a.Ud;
 }
 /* the instance of global child index i (ninst >= 1): the last one whose range starts at or before i */
 __device__ __forceinline__ int sqb_inst_at(const sqb_eval_t &a, long i){
@@ -100,7 +101,7 @@ __host__ __device__ __forceinline__ int sqb_table_words(const sqb_eval_t &a){
  * size; 1 without a fold) */
 template<int D, bool ORB = true, int LV = 0>
 __device__ __forceinline__ int sqb_point(const sqb_eval_t &a, const sqb_inst_t &I, const double *sX, const double *sW,
-                                         long il, long ig, long *cell, double *sf, double *w){
+                                         long il, long ig, long *cell, double *sf, double *w, int *ko = NULL){
     long c; int b;
     const bool cells = LV || a.cells;           /* the level kernel: cells of int8 coordinates */
     if(cells){ c = il >> D; b = (int)(il & ((1L << D) - 1)); } else { c = il; b = 0; }
@@ -121,6 +122,7 @@ __device__ __forceinline__ int sqb_point(const sqb_eval_t &a, const sqb_inst_t &
             int kd = p[d] - (((b >> d) & 1) ? st : 0);
             kk[d] = kd;
             if(kd < -K){ in = false; kd = -K; }
+            if(ko) ko[d] = kd;
             sf[d] = SQB_TAB(sX, kd + K); ww = ww*SQB_TAB(sW, kd + K);
         }
     } else {
@@ -130,6 +132,7 @@ __device__ __forceinline__ int sqb_point(const sqb_eval_t &a, const sqb_inst_t &
             int kd = p[d] - (((b >> d) & 1) ? st : 0);
             kk[d] = kd;
             if(kd < -K){ in = false; kd = -K; }
+            if(ko) ko[d] = kd;
             sf[d] = SQB_TAB(sX, kd + K); ww = ww*SQB_TAB(sW, kd + K);
         }
     }
@@ -247,6 +250,59 @@ __device__ __noinline__ sqb_fab sqb_fcall(const sqb_pt<D> p){
     return r;
 }
 
+/* ------------------------------------- the axis form --------------------------------------------------
+ * An integrand that is a scan over its axes (kgen.axis_plan: class template KA) reads its functions of one
+ * coordinate from a table over (axis, k) instead of evaluating them at every point: NU columns and the
+ * reciprocals of the NR columns it divides by.  Entries in FP64: u then r; in double-double: (hi, lo) of
+ * every column, then r. */
+template<class R> struct sqb_axrow;
+template<> struct sqb_axrow<double> {
+    static __device__ __forceinline__ void put(double *e, int c, double x){ e[c] = x; }
+    static __device__ __forceinline__ double get(const double *e, int c){ return __ldg(e + c); }
+    enum { W = 1 };
+};
+template<> struct sqb_axrow<sqdd> {
+    static __device__ __forceinline__ void put(double *e, int c, const sqdd &x){ e[2*c] = x.hi; e[2*c + 1] = x.lo; }
+    static __device__ __forceinline__ sqdd get(const double *e, int c){ return sqdd(__ldg(e + 2*c), __ldg(e + 2*c + 1)); }
+    enum { W = 2 };
+};
+template<class A, class R> struct sqb_axw { enum { N = A::NU*sqb_axrow<R>::W + A::NR }; };
+
+/* the table of one lattice: one thread per (axis, k) */
+template<class A, class R, int D>
+__global__ void sqb_k_axis(const double *X, int K, double *T){
+    const int nt = 2*K + 1;
+    for(int j = blockIdx.x*blockDim.x + threadIdx.x; j < D*nt; j += gridDim.x*blockDim.x){
+        R u[A::NU > 0 ? A::NU : 1];
+        A::axis(j/nt, R(X[j % nt]), u);
+        double *e = T + (long)j*sqb_axw<A, R>::N;
+#pragma unroll
+        for(int c = 0; c < A::NU; c++) sqb_axrow<R>::put(e, c, u[c]);
+#pragma unroll
+        for(int n = 0; n < A::NR; n++) e[A::NU*sqb_axrow<R>::W + n] = sqdd_rcp(u[A::rc(n)]);
+    }
+}
+/* one step of the scan from table entry e */
+template<class A, class R>
+__device__ __forceinline__ void sqb_axstep(typename A::st &S, double si, const double *e){
+    R u[A::NU > 0 ? A::NU : 1]; double r[A::NR > 0 ? A::NR : 1];
+#pragma unroll
+    for(int c = 0; c < A::NU; c++) u[c] = sqb_axrow<R>::get(e, c);
+#pragma unroll
+    for(int n = 0; n < A::NR; n++) r[n] = __ldg(e + A::NU*sqb_axrow<R>::W + n);
+    A::step(S, R(si), u, r);
+}
+/* the integrand at one point k (inside the box) from its table */
+template<class A, class R, int D>
+__device__ __forceinline__ R sqb_axeval(const double *T, int K, const double *sf, const int *k, R *ab){
+    typename A::st S;
+    A::init(S);
+    const int nt = 2*K + 1;
+#pragma unroll
+    for(int d = 0; d < D; d++) sqb_axstep<A, R>(S, sf[d], T + (d*nt + k[d] + K)*(int)sqb_axw<A, R>::N);
+    return A::fin(S, ab);
+}
+
 /* The FP64 pass.  The CTAs take tiles of consecutive points in turn: tile b, b + gridDim.x, ... of one
  * batch, or, in a multi-instance launch, the next tile of the device counter queue (the tile's integral
  * from its position); SQB_TILE points per tile in level mode and in multi-instance launches, SQB_BLOCK
@@ -313,19 +369,22 @@ __global__ void __launch_bounds__(SQB_BLOCK, SQB_MINB) sqb_k_f64(const __grid_co
         for(int j = 0; j < tl/SQB_BLOCK; j++){
             long il, i; int mw;
             long c; double sf[D], w;
+            [[maybe_unused]] int kk[D];
+            constexpr bool AX = F::template AX<double, 0>::NU > 0;
+            int *const ko = AX ? kk : NULL;
             if(list){
                 const long e_ = tile*tl + (long)j*SQB_BLOCK + t;
                 if(e_ >= nsel) break;
                 const unsigned long long e = a.sel[e_];
                 il = i = (long)(e & ((1ULL << SQB_SEL_SHIFT) - 1));
-                sqb_point<D, false, LV>(a, I, sX, sW, il, i, &c, sf, &w);
+                sqb_point<D, false, LV>(a, I, sX, sW, il, i, &c, sf, &w, ko);
                 mw = (int)(e >> SQB_SEL_SHIFT);
             } else {
                 il = base + (long)j*SQB_BLOCK + t; i = il + off;
                 if(il >= n) break;
                 /* two sweeps: this child only in its cell's sweep (0: skips the |.| sums, 1: the others) */
                 if(NSW > 1 && (sqb_skip<D>(a, I, il >> D) ? 0 : 1) != sweep) continue;
-                mw = sqb_point<D, true, LV>(a, I, sX, sW, il, i, &c, sf, &w);
+                mw = sqb_point<D, true, LV>(a, I, sX, sW, il, i, &c, sf, &w, ko);
             }
             if(!mw){
                 a.v[i] = 0;
@@ -335,8 +394,14 @@ __global__ void __launch_bounds__(SQB_BLOCK, SQB_MINB) sqb_k_f64(const __grid_co
             const int sk = sqb_skip<D>(a, I, c);
             const bool noab = sk && !a.abcheck;
             double ab = 0, f;
+            bool tab = false;
+            if constexpr(AX) if(I.U){
+                tab = true;
+                if(noab) f = sqb_axeval<typename F::template AX<double, 0>, double, D>(I.U, I.K, sf, kk, &ab);
+                else     f = sqb_axeval<typename F::template AX<double, 1>, double, D>(I.U, I.K, sf, kk, &ab);
+            }
 #if SQB_LEVEL_KERNEL
-            {
+            if(!AX || !tab){
                 sqb_pt<D> p;
 #pragma unroll
                 for(int d = 0; d < D; d++) p.s[d] = sf[d];
@@ -344,7 +409,8 @@ __global__ void __launch_bounds__(SQB_BLOCK, SQB_MINB) sqb_k_f64(const __grid_co
                 f = r.f; ab = r.ab;
             }
 #else
-            if(noab) f = F::template f<double, 0>(sf, &ab);
+            if(AX && tab);
+            else if(noab) f = F::template f<double, 0>(sf, &ab);
             else     f = F::template f<double, 1>(sf, &ab);
 #endif
             const double fw = f*w;
@@ -387,6 +453,149 @@ __global__ void __launch_bounds__(SQB_BLOCK, SQB_MINB) sqb_k_f64(const __grid_co
     }
 }
 
+/* The axis form's level kernel (sqb_axis_launch).  The general kernel is bound by the FP64 pipe with the
+ * integrand's exponentials and logarithms (syn_d8: 25 a point, 710 FP64 instructions); here one exponential a
+ * point is left.  A thread takes the eight children of a cell that agree in
+ * the first D - 3 axes: it scans those axes once, then the last three as a binary tree, so that a child costs
+ * under two and a half steps of the scan instead of D.  Thread t of a tile takes groups t, t + SQB_BLOCK, ... in
+ * order of (cell, first axes): a warp's writes for one choice of the last axes are 2^(D-3) consecutive
+ * children.  The thread's sums stay in registers.  Every child's value is the general kernel's bit for bit; the
+ * tile sums add the same values in another fixed order.  Measured on the B200, whole last level against the
+ * general kernel: syn_d8 at h = 0.7 (1.18e9 children) 125.4 -> 21.8 ms, syn_d11 at h = 2 (9.2e8) 93.6 -> 16.9 ms,
+ * syn_d5 at h = 1 (2.7e6) 0.40 -> 0.12 ms. */
+#define SQB_AXG 8
+#ifndef SQB_AX_MINB
+#define SQB_AX_MINB 5
+#endif
+struct sqb_ax_acc { sqdd S, b1, b2; double A, dr; unsigned ne, nsk, keep; bool fb; };
+
+template<class F, int D, int AB>
+__device__ __forceinline__ void sqb_ax_group(const sqb_eval_t &a, const sqb_inst_t &I, const double *sX, const double *sW,
+                                             const int *k, int low, int sk, int tier, long i0, bool tsum, sqb_ax_acc &t){
+    using A = typename F::template AX<double, AB>;
+    constexpr int M = D - 3, EW = sqb_axw<A, double>::N;
+    const int K = I.K, st = I.st, nt = 2*K + 1;
+    const double *U = I.U + K*EW;
+    typename A::st S0;
+    A::init(S0);
+    double w0 = 1.0; bool in0 = true;
+#pragma unroll
+    for(int d = 0; d < M; d++){
+        int kd = k[d] - (((low >> d) & 1) ? st : 0);
+        if(kd < -K){ in0 = false; kd = -K; }
+        sqb_axstep<A, double>(S0, sX[kd + K], U + (d*nt + kd)*EW);
+        w0 = w0*sW[kd + K];
+    }
+#pragma unroll 1
+    for(int h = 0; h < 4; h++){
+        typename A::st S1 = S0; double w1 = w0; bool in1 = in0;
+#pragma unroll
+        for(int q = 0; q < 2; q++){
+            int kd = k[M + q] - (((h >> q) & 1) ? st : 0);
+            if(kd < -K){ in1 = false; kd = -K; }
+            sqb_axstep<A, double>(S1, sX[kd + K], U + ((M + q)*nt + kd)*EW);
+            w1 = w1*sW[kd + K];
+        }
+#pragma unroll
+        for(int b = 0; b < 2; b++){
+            const long i = i0 + ((long)(h + 4*b) << M);
+            int kd = k[D - 1] - (b ? st : 0);
+            if(!in1 || kd < -K){ a.v[i] = 0; a.stt[i] = 0; continue; }
+            typename A::st S2 = S1;
+            sqb_axstep<A, double>(S2, sX[kd + K], U + ((D - 1)*nt + kd)*EW);
+            const double w = w1*sW[kd + K];
+            double ab = 0;
+            const double f = A::fin(S2, &ab);
+            bool fallback;
+            const double v = sqb_point_test(a, I, i, sk, AB == 0, f*w, ab*w, &fallback);
+            if(!tsum) continue;
+            if(fallback){ t.fb = true; continue; }
+            const double vp = v*I.pw, av = fabs(v);
+            t.S = sqdd_add_d(t.S, vp); t.A += av; t.ne++; t.nsk += sk ? 1 : 0;
+            if(I.last){
+                if(tier >= 1) t.b1 = sqdd_add_d(t.b1, vp);
+                if(tier >= 2) t.b2 = sqdd_add_d(t.b2, vp);
+            } else if(av >= I.thr) t.keep++;
+            else t.dr += av*I.pw;
+        }
+    }
+}
+
+template<class F, int D>
+__global__ void __launch_bounds__(SQB_BLOCK, SQB_AX_MINB) sqb_k_lvax(const __grid_constant__ sqb_eval_t a){
+    extern __shared__ double sqb_sm[];
+    __shared__ sqb_inst_t sI[SQB_MAXINST];
+    __shared__ long s_item;
+    __shared__ double wd[SQB_BLOCK/32][10];
+    __shared__ unsigned wc[SQB_BLOCK/32][3];
+    constexpr int M = D - 3;
+    sqb_tables(a, sqb_sm, sI);
+    const int t = threadIdx.x, sub = a.sub > 1 ? a.sub : 1;
+    const int gper = SQB_TILE/SQB_AXG/sub;                     /* groups per work item */
+    for(;;){
+        __syncthreads();                                       /* every thread has read s_item, wd, wc */
+        if(t == 0) s_item = (long)atomicAdd(a.queue, 1ULL);
+        __syncthreads();
+        const long item = s_item;
+        if(item >= a.ntile*sub) break;
+        const long tile = item/sub;
+        const int ki = sqb_inst_at(a, tile*SQB_TILE);
+        const sqb_inst_t &I = sI[ki];
+        const double *sX = sqb_sm + I.toff, *sW = sX + (2*I.K + 1);
+        const bool tsum = I.fused != 0;
+        const long g0 = (tile*SQB_TILE - I.child0)/SQB_AXG + (item - tile*sub)*gper;
+        sqb_ax_acc ac; ac.A = ac.dr = 0; ac.ne = ac.nsk = ac.keep = 0; ac.fb = false;
+        for(int j = t; j < gper; j += SQB_BLOCK){
+            const long gi = g0 + j, c = gi >> M;
+            if(c >= I.n) break;
+            const int low = (int)(gi & ((1 << M) - 1));
+            union { int w[3]; signed char k[12]; } p;
+            const int *src = (const int*)((const signed char*)I.pts + c*12);
+            p.w[0] = src[0]; p.w[1] = src[1]; p.w[2] = src[2];
+            int k[D];
+#pragma unroll
+            for(int d = 0; d < D; d++) k[d] = (int)(signed char)(p.w[d >> 2] >> (8*(d & 3)));
+            const int fl = (int)(signed char)(p.w[2] >> 24);
+            const int sk = a.abskip && (fl & 1);
+            const long i0 = (c << D) + low + I.child0;
+            if(sk && !a.abcheck) sqb_ax_group<F, D, 0>(a, I, sX, sW, k, low, sk, (fl >> 1) & 3, i0, tsum, ac);
+            else                 sqb_ax_group<F, D, 1>(a, I, sX, sW, k, low, sk, (fl >> 1) & 3, i0, tsum, ac);
+        }
+        const int fb = __syncthreads_or(tsum && ac.fb);
+        if(!tsum || fb){ if(t == 0) a.tfb[tile] = 1; continue; }       /* summed by the reduce kernel */
+        sqdd Ad(ac.A), dd(ac.dr);
+        for(int off = 16; off; off >>= 1){
+            ac.S = ac.S + sqdd(__shfl_down_sync(0xffffffffu, ac.S.hi, off), __shfl_down_sync(0xffffffffu, ac.S.lo, off));
+            Ad = Ad + sqdd(__shfl_down_sync(0xffffffffu, Ad.hi, off), __shfl_down_sync(0xffffffffu, Ad.lo, off));
+            dd = dd + sqdd(__shfl_down_sync(0xffffffffu, dd.hi, off), __shfl_down_sync(0xffffffffu, dd.lo, off));
+            ac.b1 = ac.b1 + sqdd(__shfl_down_sync(0xffffffffu, ac.b1.hi, off), __shfl_down_sync(0xffffffffu, ac.b1.lo, off));
+            ac.b2 = ac.b2 + sqdd(__shfl_down_sync(0xffffffffu, ac.b2.hi, off), __shfl_down_sync(0xffffffffu, ac.b2.lo, off));
+            ac.ne += __shfl_down_sync(0xffffffffu, ac.ne, off); ac.nsk += __shfl_down_sync(0xffffffffu, ac.nsk, off);
+            ac.keep += __shfl_down_sync(0xffffffffu, ac.keep, off);
+        }
+        if((t & 31) == 0){
+            double *x = wd[t >> 5];
+            x[0] = ac.S.hi; x[1] = ac.S.lo; x[2] = Ad.hi; x[3] = Ad.lo; x[4] = dd.hi; x[5] = dd.lo;
+            x[6] = ac.b1.hi; x[7] = ac.b1.lo; x[8] = ac.b2.hi; x[9] = ac.b2.lo;
+            wc[t >> 5][0] = ac.ne; wc[t >> 5][1] = ac.nsk; wc[t >> 5][2] = ac.keep;
+        }
+        __syncthreads();
+        if(t < 5){                                              /* sum t of the five over the warps, in warp order */
+            sqdd z(wd[0][2*t], wd[0][2*t + 1]);
+            for(int w = 1; w < SQB_BLOCK/32; w++) z = z + sqdd(wd[w][2*t], wd[w][2*t + 1]);
+            sqb_part_t &P = a.part[tile];
+            double *dst = t == 0 ? P.S : t == 1 ? P.A : t == 2 ? P.drop : t == 3 ? P.b1 : P.b2;
+            dst[0] = z.hi; dst[1] = z.lo;
+        } else if(t == 5){
+            unsigned ne = 0, nsk = 0, keep = 0;
+            for(int w = 0; w < SQB_BLOCK/32; w++){ ne += wc[w][0]; nsk += wc[w][1]; keep += wc[w][2]; }
+            sqb_part_t &P = a.part[tile];
+            P.u[0] = P.u[1] = 0; P.ne = ne; P.nq = 0; P.unres = 0; P.skipped = nsk;
+            a.tkeep[tile] = keep; a.tfb[tile] = 0;
+        }
+    }
+}
+
 template<class F, int D>
 __global__ void __launch_bounds__(SQB_BLOCK) sqb_k_dd(const __grid_constant__ sqb_dd_t a){
     extern __shared__ double sqb_sm[];
@@ -405,11 +614,18 @@ __global__ void __launch_bounds__(SQB_BLOCK) sqb_k_dd(const __grid_constant__ sq
         const long il = i - I.child0;
         if(multi && il >= (e.cells ? (I.n << D) : I.n)) continue;    /* a tile's padding: no point */
         long c; double sf[D], w;
-        if(!sqb_point<D>(e, I, sX, sW, il, i, &c, sf, &w)){ e.v[i] = 0; e.stt[i] = 0; a.uu[i] = 0; continue; }
-        sqdd sq[D], abq;
+        using A = typename F::template AX<sqdd, 1>;
+        [[maybe_unused]] int kk[D];
+        if(!sqb_point<D>(e, I, sX, sW, il, i, &c, sf, &w, A::NU > 0 ? kk : NULL)){ e.v[i] = 0; e.stt[i] = 0; a.uu[i] = 0; continue; }
+        sqdd abq, vq;
+        bool tab = false;
+        if constexpr(A::NU > 0) if(I.Ud){ tab = true; vq = sqb_axeval<A, sqdd, D>(I.Ud, I.K, sf, kk, &abq); }
+        if(!tab){
+            sqdd sq[D];
 #pragma unroll
-        for(int d = 0; d < D; d++) sq[d] = sqdd(sf[d]);
-        const sqdd vq = F::template f<sqdd, 1>(sq, &abq);
+            for(int d = 0; d < D; d++) sq[d] = sqdd(sf[d]);
+            vq = F::template f<sqdd, 1>(sq, &abq);
+        }
         if(e.raw){ e.v[i] = vq.hi; e.vlo[i] = vq.lo; e.ab[i] = abq.hi; e.ablo[i] = abq.lo; continue; }
         const double vqd = vq.value(), abqd = abq.value();
         /* qvalue(), driver/eval.c:25-30 */
@@ -510,6 +726,34 @@ static int sqb_split_attr(int P, int block, size_t smem, sqb_kattr_t *o){
     return sqb_attr_of(sqb_k_fin<F, D>, block, smem, o);
 }
 
+/* the axis form's launchers, empty for an integrand without one */
+template<class R, int AB> struct sqb_noaxis { enum { NU = 0, NR = 0 }; };
+template<class F, int D>
+static bool sqb_ax_level(const sqb_eval_t *a, int grid, int block, size_t smem, cudaStream_t st){
+    if constexpr(F::template AX<double, 0>::NU > 0) if(sqb_axis_launch(a)){
+        sqb_k_lvax<F, D><<<grid, block, smem, st>>>(*a);
+        return true;
+    }
+    return false;
+}
+template<class F, int D>
+static bool sqb_ax_attr(int block, size_t smem, sqb_kattr_t *o, int *ok){
+    if constexpr(F::template AX<double, 0>::NU > 0){
+        *ok = sqb_attr_of(sqb_k_lvax<F, D>, block, smem, o);
+        o->fused = 1; o->sweeps = 1;
+        return true;
+    }
+    return false;
+}
+template<class F, class R, int AB, int D>
+static void sqb_ax_table(const double *X, int K, double *T, cudaStream_t st){
+    if constexpr(F::template AX<double, 0>::NU > 0){
+        const int n = D*(2*K + 1);
+        sqb_k_axis<typename F::template AX<R, AB>, R, D><<<(n + 31)/32, 32, 0, st>>>(X, K, T);
+    }
+}
+template<class F, class R> struct sqb_ax_words { enum { N = F::template AX<R, 0>::NU > 0 ? (int)sqb_axw<typename F::template AX<R, 0>, R>::N : 0 }; };
+
 /* the scaling test (sqb_scale_t): one thread per (direction, q); P::pt is the graph's raw double-double
  * point function (pt_<name> of the QREAL half, SQ_AB = 1 as the reference's default) */
 template<class P>
@@ -536,19 +780,27 @@ struct FS {                                                                     
         return K<double, AB>::ffin_##NAME(sf, T, A, ab); }                                         \
 };                                                                                                 \
 }
+/* an integrand without the axis form */
+#define SQ_NOAXIS(NAME) namespace SQG_NS(NAME) { template<class R, int AB> using KA = sqb_noaxis<R, AB>; }
+#define SQ_GRAPH(NAME, VOLKOV, L, D, W, NP, FIX) SQ_NOAXIS(NAME) SQ_GRAPH_AXIS(NAME, VOLKOV, L, D, W, NP, FIX)
 #if defined(SQB_FMA_TU)
 #define SQ_SCALE(NAME)
-#define SQ_GRAPH(NAME, VOLKOV, L, D, W, NP, FIX)                                                    \
+#define SQ_GRAPH_AXIS(NAME, VOLKOV, L, D, W, NP, FIX)                                               \
 namespace SQG_NS(NAME) {                                                                           \
 struct F {                                                                                         \
+    template<class R, int AB> using AX = KA<R, AB>;                                                \
     template<class R, int AB> static __device__ __forceinline__ R f(const R *sf, R *ab){           \
         return K<R, AB>::f_##NAME(sf, ab); }                                                       \
 };                                                                                                 \
 }                                                                                                  \
+extern "C" void SQB_##NAME##_axisfma(const double *X, int K, double *T, void *st){                 \
+    sqb_ax_table<SQG_NS(NAME)::F, double, 0, D>(X, K, T, (cudaStream_t)st); }                       \
 extern "C" void SQB_##NAME##_f64fma(const sqb_eval_t *a, int grid, int block, size_t smem, void *st){ \
+    if(sqb_ax_level<SQG_NS(NAME)::F, D>(a, grid, block, smem, (cudaStream_t)st)) return;            \
     if(sqb_level_launch(a)) sqb_k_f64<SQG_NS(NAME)::F, D, 1><<<grid, block, smem, (cudaStream_t)st>>>(*a); \
     else sqb_k_f64<SQG_NS(NAME)::F, D, 0><<<grid, block, smem, (cudaStream_t)st>>>(*a); }           \
 extern "C" int SQB_##NAME##_attrfma(int lv, int block, size_t smem, sqb_kattr_t *o){               \
+    int ok; if(lv && sqb_ax_attr<SQG_NS(NAME)::F, D>(block, smem, o, &ok)) return ok;               \
     return lv ? sqb_f64_attr(sqb_k_f64<SQG_NS(NAME)::F, D, 1>, 1, block, smem, o)                  \
               : sqb_f64_attr(sqb_k_f64<SQG_NS(NAME)::F, D, 0>, 0, block, smem, o); }
 #define SQ_GRAPH_SPLIT(NAME, VOLKOV, L, D, W, NP, FIX, NPARTS)                                      \
@@ -572,34 +824,46 @@ extern "C" void SQB_##NAME##_scale(const sqb_scale_t *a, int grid, int block, vo
     sqb_k_scale<SQG_NS(NAME)::PT><<<grid, block, 0, (cudaStream_t)st>>>(*a); }
 #define SQ_GRAPH_CORE(NAME, D)                                                                      \
 extern "C" void SQB_##NAME##_f64fma(const sqb_eval_t *, int, int, size_t, void *) __attribute__((weak)); \
+extern "C" void SQB_##NAME##_axisfma(const double *, int, double *, void *) __attribute__((weak)); \
 extern "C" void SQB_##NAME##_scale(const sqb_scale_t *, int, int, void *) __attribute__((weak));   \
 extern "C" int SQB_##NAME##_attrfma(int, int, size_t, sqb_kattr_t *) __attribute__((weak));        \
 namespace SQG_NS(NAME) {                                                                           \
 struct F {                                                                                         \
+    template<class R, int AB> using AX = KA<R, AB>;                                                \
     template<class R, int AB> static __device__ __forceinline__ R f(const R *sf, R *ab){           \
         return K<R, AB>::f_##NAME(sf, ab); }                                                       \
 };                                                                                                 \
 template<> __device__ __forceinline__ sqdd F::f<sqdd, 1>(const sqdd *sf, sqdd *ab){                \
     return KD<sqdd, 1>::f_##NAME(sf, ab); }                                                        \
 static void f64(const sqb_eval_t *a, int grid, int block, size_t smem, void *st){                  \
+    if(sqb_ax_level<F, D>(a, grid, block, smem, (cudaStream_t)st)) return;                         \
     if(SQB_LEVEL_KERNEL && sqb_level_launch(a))                                                    \
         sqb_k_f64<F, D, SQB_LEVEL_KERNEL><<<grid, block, smem, (cudaStream_t)st>>>(*a);            \
     else sqb_k_f64<F, D, 0><<<grid, block, smem, (cudaStream_t)st>>>(*a); }                        \
 static void dd(const sqb_dd_t *a, int grid, int block, size_t smem, void *st){                     \
     sqb_k_dd<F, D><<<grid, block, smem, (cudaStream_t)st>>>(*a); }                                 \
+static void axis(int which, const double *X, int K, double *T, void *st){                          \
+    if(which == 2){ if(SQB_##NAME##_axisfma) SQB_##NAME##_axisfma(X, K, T, st); }                   \
+    else if(which == 1) sqb_ax_table<F, sqdd, 1, D>(X, K, T, (cudaStream_t)st);                     \
+    else sqb_ax_table<F, double, 0, D>(X, K, T, (cudaStream_t)st); }                               \
 static int attr(int which, int block, size_t smem, sqb_kattr_t *o){                                \
     const int lv = (which & SQB_ATTR_LEVEL) != 0; which &= ~SQB_ATTR_LEVEL;                        \
     if(which == 2) return SQB_##NAME##_attrfma ? SQB_##NAME##_attrfma(lv, block, smem, o) : 0;      \
     if(which == 1) return sqb_f64_attr(sqb_k_dd<F, D>, 0, block, smem, o);                         \
+    int ok; if(lv && sqb_ax_attr<F, D>(block, smem, o, &ok)) return ok;                             \
     return SQB_LEVEL_KERNEL && lv ? sqb_f64_attr(sqb_k_f64<F, D, SQB_LEVEL_KERNEL>, 1, block, smem, o) \
                                   : sqb_f64_attr(sqb_k_f64<F, D, 0>, 0, block, smem, o); }         \
 }
-#define SQ_GRAPH(NAME, VOLKOV, L, D, W, NP, FIX)                                                    \
+#define SQ_AXIS_ENTRY(NAME) sqb_ax_words<SQG_NS(NAME)::F, double>::N ? SQG_NS(NAME)::axis : NULL,    \
+    {sqb_ax_words<SQG_NS(NAME)::F, double>::N, sqb_ax_words<SQG_NS(NAME)::F, sqdd>::N,              \
+     sqb_ax_words<SQG_NS(NAME)::F, double>::N}
+#define SQ_GRAPH_AXIS(NAME, VOLKOV, L, D, W, NP, FIX)                                               \
 SQ_GRAPH_CORE(NAME, D)                                                                             \
 extern "C" const sqb_graph_t SQB_##NAME = {#NAME, VOLKOV, L, D, W, NP, FIX, 0,                     \
     SQG_NS(NAME)::f64, SQG_NS(NAME)::dd, SQG_NS(NAME)::attr, SQB_##NAME##_f64fma, 0, NULL, NULL,     \
-    SQB_##NAME##_scale};
+    SQB_##NAME##_scale, SQ_AXIS_ENTRY(NAME)};
 #define SQ_GRAPH_SPLIT(NAME, VOLKOV, L, D, W, NP, FIX, NPARTS)                                      \
+SQ_NOAXIS(NAME)                                                                                    \
 SQ_GRAPH_CORE(NAME, D)                                                                             \
 SQ_SPLIT_F(NAME)                                                                                   \
 extern "C" void SQB_##NAME##_splitfma(int, const sqb_eval_t *, double *, double *, int, int, size_t, void *) \
@@ -616,5 +880,5 @@ static int split_attr(int P, int fma, int block, size_t smem, sqb_kattr_t *o){  
 }                                                                                                  \
 extern "C" const sqb_graph_t SQB_##NAME = {#NAME, VOLKOV, L, D, W, NP, FIX, 0,                     \
     SQG_NS(NAME)::f64, SQG_NS(NAME)::dd, SQG_NS(NAME)::attr, SQB_##NAME##_f64fma, NPARTS,           \
-    SQG_NS(NAME)::split, SQG_NS(NAME)::split_attr, SQB_##NAME##_scale};
+    SQG_NS(NAME)::split, SQG_NS(NAME)::split_attr, SQB_##NAME##_scale, NULL, {0, 0, 0}};
 #endif
