@@ -9,8 +9,9 @@ files its tools/gpugen.py reads): DIR is that kernels/ directory, given by --ker
   sincfeyn_b200/lib/libsqb200.so   the C ABI (include/sincfeyn_b200.h), every graph's sm_100a kernels;
   sincfeyn_b200/bin/sincqed        the command line;
   sincfeyn_b200/lib/flops.json     algorithmic FP64 flops per point of every graph (SQ_AB = 1 and 0).
-A step is redone only when one of its inputs is newer than its output.  Without a kernel tree (e.g. on
-a host that only runs the prebuilt library) the build keeps what is there.
+A step is redone only when one of its inputs is newer than its output.  Without a kernel tree the build keeps a
+prebuilt library of the reference's graphs as it is (e.g. on a host that only runs it); where there is none it
+builds the library of the synthetic integrands, whose sources are in the package.
 """
 import argparse
 import concurrent.futures as cf
@@ -139,17 +140,26 @@ def _compile_graph(tu, o, tuf, of, name, do_exact, do_fma, sweeps=1):
 
 
 def kernel_sources(kdir, classes):
-    """the reference's kernels of these classes, then the synthetic integrands of sincfeyn_b200/synth"""
+    """the reference's kernels of these classes, then the synthetic integrands of sincfeyn_b200/synth; without
+    any of the former, nothing if a library of other graphs is already built, else the synthetic ones alone"""
     out = []
-    if not kdir:
-        return out
-    for c in classes.split():
+    for c in classes.split() if kdir else ():
         d = os.path.join(kdir, c)
         if os.path.isdir(d):
             out += sorted(os.path.join(d, f) for f in os.listdir(d) if f.endswith('.c'))
-    if out:
-        out += sorted(os.path.join(SYNTH, f) for f in os.listdir(SYNTH) if f.endswith('.c'))
-    return out
+    synth = sorted(os.path.join(SYNTH, f) for f in os.listdir(SYNTH) if f.endswith('.c'))
+    if not out and os.path.exists(LIBSO) and not _synthetic_only(synth):
+        return out
+    return out + synth
+
+
+def _synthetic_only(synth):
+    """whether the built library holds the synthetic integrands and nothing else (its flop record)"""
+    names = {os.path.splitext(os.path.basename(f))[0] for f in synth}
+    if not os.path.exists(FLOPS):
+        return False
+    with open(FLOPS) as f:
+        return set(json.load(f)) <= names
 
 
 def generate(srcs):
