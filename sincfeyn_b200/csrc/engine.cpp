@@ -6,13 +6,13 @@
  *   box_zero     4097 fixed probe nodes; an integrand that is 0 at all of them is reported as zero
  *                (driver/sum.c:346-359);
  *   grow         the support-following top level (driver/sumkey.h:126-461): breadth-first from z = 0
- *                over axis neighbours at step 2^top h; a frontier is evaluated as one device batch,
- *                its values come to the host for the order-dependent sums (Neumaier S, the running
- *                sum|f w| whose threshold eps_rel * a decides what is kept, the outer shells, the
- *                dropped weight), and the device builds the next frontier: every not-yet-seen
+ *                over axis neighbours at step 2^top h; a frontier is evaluated as one device batch and
+ *                stays on the device: its sums (the running sum|f w| whose threshold eps_rel * a decides
+ *                what is kept added in point order as the reference adds it; S, the outer shells and the
+ *                dropped weight in double-double) and the next frontier, every not-yet-seen
  *                neighbour of a kept point, in (kept point, axis, sign) order -- the order the
  *                reference's parallel lowest-id claims produce (topgrid.cu); then the final
- *                re-threshold and the shadow-tier flood fill on the device.  One table holds every
+ *                re-threshold and the shadow-tier flood fill.  One table holds every
  *                evaluated point, which is the reference's result whenever it reports no candidate
  *                below its freed boundary tables (BTUNS = 0, driver/sum.c:631);
  *   dilate       on the device: the kept cells and their axis neighbours, deduplicated (skip bit AND,
@@ -20,18 +20,15 @@
  *                (driver/sumkey.h:20-90);
  *   levels       sqb_dev_level() for lev = top-1 .. 0 (driver/sum.c:652-799), the cell lists staying
  *                in device memory.
- * Sums of the grow are Neumaier sums in point order as the reference's kadd (driver/sum.c:18-20);
- * the levels' sums are double-double on the device. */
+ * The grow's S is a double-double sum on the device, where the reference's is a Neumaier sum (driver/sum.c:18-20); the
+ * levels' sums are double-double too. */
 #include <stdio.h>
 #include <stdlib.h>
 #include <string.h>
 #include <math.h>
 #include <stdint.h>
 #include <vector>
-#include <algorithm>
-#include <omp.h>
 #include <chrono>
-#include <future>
 #include "sqb_rt.h"
 #include "sincfeyn_b200.h"
 
@@ -74,11 +71,6 @@ extern "C" int sqb_graph_info(const char *name, int *info){
 }
 extern "C" const char *sqb_device_info(void){ return sqb_dev_info(); }
 
-/* Neumaier sum, driver/sum.c:18-20 */
-struct ksum { double s = 0, c = 0;
-    void add(double x){ double t = s + x; if(fabs(s) >= fabs(x)) c += (s - t) + x; else c += (x - t) + s; s = t; }
-    double val() const { return s + c; } };
-
 /* ---------------------------------------------------------------------------------------------- */
 /* the run of one graph */
 struct Run {
@@ -105,34 +97,6 @@ static void set_test(Run &R, double abserr){
     R.t.fma = R.o.fma; R.t.split = R.o.split;
 }
 
-static int eval(Run &R, const std::vector<sqb_pt_t> &p, const unsigned char *skip, std::vector<double> &v, std::vector<unsigned char> &nr){
-    v.resize(p.size()); nr.resize(p.size());
-    if(p.empty()) return 0;
-    if(sqb_dev_eval_nodes(R.g, (long)p.size(), p.data(), skip, &R.t, v.data(), nr.data(), &R.nq, &R.u, &R.unresdrop))
-        FAIL("device: %s", sqb_last_error());
-    return 0;
-}
-
-/* driver/sum.c:346-359 */
-static int box_zero(Run &R, int lev, long *nev, int *zero){
-    const int st = 1 << lev, W = 2*(R.K/st) + 1, NP = 4096;
-    std::vector<sqb_pt_t> p(NP + 1);
-    for(long i = 0; i <= NP; i++){
-        memset(&p[i], 0, sizeof p[i]);
-        unsigned long long y = 0x9E3779B97F4A7C15ULL*(unsigned long long)(i + 1);
-        if(i) for(int d = 0; d < R.D; d++){ y ^= y >> 29; y *= 0xBF58476D1CE4E5B9ULL; y ^= y >> 32; p[i].k[d] = (signed char)(((int)(y % (unsigned long long)W) - R.K/st)*st); }
-    }
-    std::vector<double> v; std::vector<unsigned char> nr;
-    long nq0 = R.nq; double u0 = R.u;
-    if(eval(R, p, NULL, v, nr)) return -1;
-    R.nq = nq0; R.u = u0;        /* the probe's fallback count and round column are its own; its
-                                    unresolved points are counted, as the global UNRESDROP does */
-    *zero = 1;
-    for(double x : v) if(x != 0){ *zero = 0; break; }
-    if(*zero) *nev += NP + 1;
-    return 0;
-}
-
 /* mixed-radix key (driver/sumkey.h:7-18): 1 c_0 ... c_{D-1} in base W, c_i = k_i/st + K/st; W = 0 if
  * the keys would not fit 63 bits; *nbits = bit length of the largest key */
 static int keyradix(const Run &R, int st, uint64_t *P, int *nbits){
@@ -142,98 +106,64 @@ static int keyradix(const Run &R, int st, uint64_t *P, int *nbits){
     return (int)W;
 }
 
-struct GrowOut { double S, A, e1, e2, drop, gshs; long gshn, nev; };
+struct GrowOut { double S, A, e1, e2, drop, gshs; long gshn, nev; int zero; };
 
-/* driver/sumkey.h:126-461 (see the file comment); the kept cells, dilated at the same step when
- * dilate_out is given, stay on the device */
+/* the zero probe (driver/sum.c:346-359) and the grow (driver/sumkey.h:126-461, see the file comment); the kept
+ * cells, dilated at the same step for lev > 0, stay on the device.  go->zero: the integrand vanished at every
+ * probe node */
 static int grow(Run &R, int lev, double eps_rel, GrowOut *go, sqb_pt_t **dilated, long *ndil){
-    const int st = 1 << lev; uint64_t P[SQB_MAXD]; int nbits = 0;
+    const int st = 1 << lev; uint64_t P[SQB_MAXD] = {0}; int nbits = 0;
     const int W = keyradix(R, st, P, &nbits);
-    if(!W) FAIL("lattice too wide for 64-bit grid keys (D=%d, N=%d, step %dh)", R.D, 2*R.K + 1, st);
-    const double pw = pow(st, R.D);
     const int store = lev > 0, gs = lev == 0 && R.o.abskip ? R.o.growskip : 0;
-    if(sqb_grow_begin(R.D, R.K, st, W, (const unsigned long long*)P, gs, R.o.abskip, sqb_dev_stream()))
-        FAIL("device grow: %s", sqb_top_error());
+    const double t0 = now();
+    *dilated = NULL; *ndil = 0; memset(go, 0, sizeof *go);
     /* the grow's device tables are released on every return, an error included, so that a failed
      * integral leaves its memory to the next one */
     struct End { ~End(){ sqb_grow_end(); } } end_of_grow;
-    std::vector<unsigned char> stt;
-    ksum ks; double a = 0, x1 = 0, x2 = 0, dr = 0, gshs = 0; long ne = 0, gshn = 0, nkeep = 0;
-    double te = 0, th = 0, tx = 0; int nfr = 0; const double tg0 = now();    /* phase times (verbose) */
-    /* A frontier's order-dependent sums that its expansion does not need (the Neumaier S, the shell, drop
-     * and shadow sums) run on a helper task while the device expands the frontier and evaluates the next;
-     * the tasks run one frontier after another (each waits for its predecessor), each over its frontier in
-     * point order, so every sum is the in-line one bit for bit.  Only the |v| sum that sets the threshold
-     * stays in line.  Values and shell classes alternate between two buffers; every return joins the
-     * tasks first. */
-    std::vector<double> vb[2]; std::vector<unsigned char> cb[2];
-    std::shared_future<void> fut[2], last;
-    struct Join { std::shared_future<void> &f; ~Join(){ if(f.valid()) f.wait(); } } join{last};
+    const sqb_pt_t *pts; const unsigned char *skip, *sd; const double *vd, *ud; long n = 0, nfr = 0, nn = 0;
+    if(sqb_grow_begin(R.D, R.K, st, W ? W : 1, (const unsigned long long*)P, gs, R.o.abskip, eps_rel, pow(st, R.D), sqb_dev_stream(), &pts, &n))
+        FAIL("device grow: %s", sqb_top_error());
+    if(sqb_dev_eval_resident(R.g, pts, n, NULL, &R.t, &vd, &sd, &ud)) FAIL("device: %s", sqb_last_error());
+    if(sqb_grow_probe(vd, sd)) FAIL("device grow: %s", sqb_top_error());
+    const long nprobe = n;
+    sqb_grow_sums_t s;
+    if(!W && (sqb_grow_sums(&s) || !sqb_grow_probe_zero(&nn)))
+        FAIL("lattice too wide for 64-bit grid keys (D=%d, N=%d, step %dh)", R.D, 2*R.K + 1, st);
     for(;;){
-        const sqb_pt_t *pts; const unsigned char *skip;
-        const long n = sqb_grow_frontier(&pts, &skip);
+        n = sqb_grow_frontier(&pts, &skip);
         if(n <= 0) break;
-        const int b = nfr & 1;
-        if(fut[b].valid()) fut[b].wait();          /* the task two frontiers back read this buffer */
-        std::vector<double> &v = vb[b]; std::vector<unsigned char> &cls = cb[b];
-        v.resize(n); stt.resize(n); cls.resize(n);
-        const double *vd; const unsigned char *sd;
-        const double t0 = now();
-        if(sqb_grow_shells_async()) FAIL("device grow: %s", sqb_top_error());
-        if(sqb_dev_eval_resident(R.g, pts, n, skip, &R.t, v.data(), stt.data(), &R.nq, &R.u, &R.unresdrop, &vd, &sd))
-            FAIL("device: %s", sqb_last_error());
-        sqb_grow_shells_take(cls.data());
+        if(sqb_dev_eval_resident(R.g, pts, n, skip, &R.t, &vd, &sd, &ud)) FAIL("device: %s", sqb_last_error());
         /* the predictor stores every grow value (driver/sumkey.h:219-222) */
         if(R.vt && (sqb_vtab_reserve(R.vt, n, sqb_dev_stream()) || sqb_vtab_put_nodes(R.vt, pts, vd, n, R.D, sqb_dev_stream())))
             FAIL("predictor: %s", sqb_vtab_error());
-        const double t1 = now(); te += t1 - t0; nfr++;
-        ne += n;
-        /* the frontier's sums in point order, then its threshold (driver/sumkey.h:225-245) */
-        for(long i = 0; i < n; i++) a += fabs(v[i])*pw;
-        const double thr = eps_rel*a;
-        {
-            const std::shared_future<void> prev = last;
-            last = fut[b] = std::async(std::launch::async, [&, b, n, thr, prev]{
-                if(prev.valid()) prev.wait();
-                const double *vv = vb[b].data(); const unsigned char *cc = cb[b].data();
-                for(long i = 0; i < n; i++) ks.add(vv[i]*pw);
-                for(long i = 0; i < n; i++){
-                    const double w = fabs(vv[i])*pw;
-                    if(cc[i] & 2) x1 += w; else if(cc[i] & 4) x2 += w;
-                    if(!(fabs(vv[i]) >= thr)){ dr += w; gshs += vv[i]*pw; gshn++; }
-                }
-            }).share();
+        if(sqb_grow_expand(vd, sd, ud, &nn)) FAIL("device grow: %s", sqb_top_error());
+        go->nev += n;
+        if(!nfr++){
+            /* the first wait has brought the probe's answer; its fallback count and round column are its own, its
+             * unresolved points are counted, as the global UNRESDROP does */
+            long un = 0;
+            go->zero = sqb_grow_probe_zero(&un);
+            R.unresdrop += un;
+            if(go->zero){ go->nev = nprobe; return 0; }
         }
-        long nk = 0, nn = 0;
-        const double t2 = now(); th += t2 - t1;
-        if(sqb_grow_expand(vd, sd, thr, &nk, &nn)) FAIL("device grow: %s", sqb_top_error());
-        tx += now() - t2;
-        nkeep += nk;
     }
-    if(last.valid()) last.wait();                  /* every frontier's sums are in */
-    const double tg1 = now();
-    /* the final threshold, driver/sumkey.h:399-401 */
-    const double thr = eps_rel*a;
-    { std::vector<double> kv(nkeep);
-      if(nkeep && sqb_grow_kv(kv.data(), nkeep)) FAIL("device grow: %s", sqb_top_error());
-      for(long i = 0; i < nkeep; i++) if(!(kv[i] >= thr)) dr += kv[i]*pw; }
-    long m = 0;
-    if(sqb_grow_finish(thr, store && R.D < SQB_MAXD, &m)) FAIL("device grow: %s", sqb_top_error());
-    /* ... and what the eps*10^t grows evaluated (driver/sumkey.h:445-451) */
-    if(R.vt && store && R.D < SQB_MAXD && m){
+    const double t1 = now();
+    if(sqb_grow_finish(store && R.D < SQB_MAXD)) FAIL("device grow: %s", sqb_top_error());
+    /* the final threshold, driver/sumkey.h:399-401 ... and what the eps*10^t grows evaluated (driver/sumkey.h:445-451) */
+    if(R.vt && store && R.D < SQB_MAXD){
         const sqb_pt_t *kp; long km;
+        if(sqb_grow_sums(&s)) FAIL("device grow: %s", sqb_top_error());
         sqb_grow_kept(&kp, &km);
-        if(sqb_vtab_raise_kept(R.vt, kp, km, R.D, st, R.K, sqb_dev_stream())) FAIL("predictor: %s", sqb_vtab_error());
+        if(km && sqb_vtab_raise_kept(R.vt, kp, km, R.D, st, R.K, sqb_dev_stream())) FAIL("predictor: %s", sqb_vtab_error());
     }
-    const double tg2 = now();
-    *dilated = NULL; *ndil = 0;
-    if(store && sqb_grow_dilate(nbits, dilated, ndil)) FAIL("device dilate: %s", sqb_top_error());
+    if(store && sqb_grow_dilate(nbits, dilated)) FAIL("device dilate: %s", sqb_top_error());
+    if(sqb_grow_sums(&s)){ sqb_dev_free(*dilated); *dilated = NULL; FAIL("device grow: %s", sqb_top_error()); }
+    *ndil = s.cells;
+    R.nq += s.nq; R.u += s.u; R.unresdrop += s.unres;
+    go->S = s.S; go->A = s.a; go->e1 = s.x1; go->e2 = s.x2; go->drop = s.drop; go->gshs = s.gshs; go->gshn = s.gshn;
     if(R.o.verbose)
-        fprintf(stderr, "# %s grow: %d frontiers, %ld points, %ld kept: eval %.1f ms, host sums %.1f ms, expand %.1f ms; "
-                "final threshold + tiers %.1f ms; dilate %.1f ms (%ld cells)\n", R.g->name, nfr, ne, nkeep,
-                1e3*te, 1e3*th, 1e3*tx, 1e3*(tg2 - tg1), 1e3*(now() - tg2), *ndil);
-    (void)tg0;
-    go->S = ks.val(); go->A = a; go->e1 = x1; go->e2 = x2; go->drop = dr; go->gshs = gshs; go->gshn = gshn; go->nev = ne;
+        fprintf(stderr, "# %s grow: %ld frontiers, %ld points, %ld kept, %ld dilated cells: frontiers %.2f ms; final threshold, "
+                "tiers and dilation %.2f ms\n", R.g->name, nfr, go->nev, s.kept, s.cells, 1e3*(t1 - t0), 1e3*(now() - t1));
     return 0;
 }
 
@@ -347,11 +277,9 @@ struct Integral {
             res->t_top = 0;
         } else {
             set_test(R, R.o.abserr0);
-            int zero = 0;
-            if(box_zero(R, top, &res->nev, &zero)) return -1;
-            if(zero){ res->zero = 1; res->t = now() - t0; return 1; }
             GrowOut go;
             if(grow(R, top, eps*1e-3, &go, &dcur, &ncur)) return -1;
+            if(go.zero){ res->nev += go.nev; res->zero = 1; res->t = now() - t0; return 1; }
             if(vt_check(R, E_, sizeof E_)) return -1;
             res->nev += go.nev; res->ref = go.A; res->prune = go.drop;
             if(top == 0 && go.gshn) res->prune = fabs(go.gshs);

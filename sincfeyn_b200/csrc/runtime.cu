@@ -100,8 +100,6 @@ struct Dev {
     long ttcap; double *tt, *ta;   /* split FP64 pass: running sums per point */
     sqb_acc_t *acc; unsigned long long *base;
     sqb_acc_t *accm; unsigned long long *basem, *queue;   /* multi-instance levels: per integral, tile queue */
-    long dcap; sqb_pt_t *dpts; unsigned char *dskip;
-    long hcap; sqb_pt_t *hpts; unsigned char *hskip, *hst; double *hv, *huu;
 };
 static thread_local Dev G;
 static int KTIME;                  /* sqb_kernel_timing(): all threads */
@@ -327,79 +325,18 @@ static int eval_batch(const sqb_graph_t *g, sqb_eval_t *a, const sqb_test_t *t, 
     return 0;
 }
 
-extern "C" int sqb_dev_eval_nodes(const sqb_graph_t *g, long n, const sqb_pt_t *pts, const unsigned char *skip,
-                                  const sqb_test_t *t, double *v, unsigned char *near, long *nq, double *u, long *unres){
-    if(n <= 0) return 0;
-    const long CH = 1L << 22;
-    long m0 = n < CH ? n : CH;
-    if(reserve_points(m0)) return -1;
-    if(m0 > G.dcap){
-        if(G.dpts){ cudaFree(G.dpts); cudaFree(G.dskip); cudaFreeHost(G.hpts); cudaFreeHost(G.hskip); cudaFreeHost(G.hv); cudaFreeHost(G.hst); cudaFreeHost(G.huu); }
-        long c = 1L << 16; while(c < m0) c <<= 1;
-        CKR(cudaMalloc(&G.dpts, c*sizeof(sqb_pt_t))); CKR(cudaMalloc(&G.dskip, c));
-        CKR(cudaMallocHost(&G.hpts, c*sizeof(sqb_pt_t))); CKR(cudaMallocHost(&G.hskip, c));
-        CKR(cudaMallocHost(&G.hv, c*sizeof(double))); CKR(cudaMallocHost(&G.hst, c)); CKR(cudaMallocHost(&G.huu, c*sizeof(double)));
-        G.dcap = c; G.hcap = c;
-    }
-    long q = 0, nd = 0; double uu = 0;
-    for(long i0 = 0; i0 < n; i0 += CH){
-        long m = n - i0 < CH ? n - i0 : CH;
-        memcpy(G.hpts, pts + i0, m*sizeof(sqb_pt_t));
-        CKR(cudaMemcpyAsync(G.dpts, G.hpts, m*sizeof(sqb_pt_t), cudaMemcpyHostToDevice, G.s));
-        if(skip){ memcpy(G.hskip, skip + i0, m); CKR(cudaMemcpyAsync(G.dskip, G.hskip, m, cudaMemcpyHostToDevice, G.s)); }
-        H2D += m*sizeof(sqb_pt_t) + (skip ? m : 0); D2H += m*(2*sizeof(double) + 1);
-        sqb_eval_t a; memset(&a, 0, sizeof a); fill_eval(&a, t);
-        a.pts = G.dpts; a.n = m; a.esize = 1; a.stride = SQB_MAXD; a.flag_at = -1; a.cells = 0; a.st = 0;
-        a.skip = skip ? G.dskip : NULL;
-        if(eval_batch(g, &a, t, m)) return -1;
-        CKR(cudaMemcpyAsync(G.hv, G.v, m*sizeof(double), cudaMemcpyDeviceToHost, G.s));
-        CKR(cudaMemcpyAsync(G.hst, G.stt, m, cudaMemcpyDeviceToHost, G.s));
-        CKR(cudaMemcpyAsync(G.huu, G.uu, m*sizeof(double), cudaMemcpyDeviceToHost, G.s));
-        CKR(cudaStreamSynchronize(G.s));
-        for(long i = 0; i < m; i++){
-            unsigned char s = G.hst[i];
-            v[i0 + i] = G.hv[i];
-            if(near) near[i0 + i] = (s & SQB_NEAR) ? 1 : 0;
-            if(s & SQB_FALLBACK){ q++; uu += G.huu[i]; }
-            if(s & SQB_UNRES) nd++;
-        }
-    }
-    *nq += q; *u += uu; *unres += nd;
-    return 0;
-}
-
-/* n device-resident nodes (pt_t, flags ignored; skip per node on the device or NULL): values and status
- * to the host; the device copies stay valid until the next evaluation (*v_dev, *stt_dev) */
-extern "C" int sqb_dev_eval_resident(const sqb_graph_t *g, const sqb_pt_t *pts, long n, const unsigned char *skip,
-                                     const sqb_test_t *t, double *v, unsigned char *stt, long *nq, double *u, long *unres,
-                                     const double **v_dev, const unsigned char **stt_dev){
-    *v_dev = NULL; *stt_dev = NULL;
+/* n device-resident nodes (pt_t, flags ignored; skip per node on the device or NULL) evaluated with the tests and the
+ * fallback; the values, status and round column stay on the device until the next evaluation.  Queued on the
+ * thread's stream, no wait */
+extern "C" int sqb_dev_eval_resident(const sqb_graph_t *g, const sqb_pt_t *pts, long n, const unsigned char *skip, const sqb_test_t *t,
+                                     const double **v_dev, const unsigned char **stt_dev, const double **uu_dev){
+    *v_dev = *uu_dev = NULL; *stt_dev = NULL;
     if(n <= 0) return 0;
     if(reserve_points(n)) return -1;
-    if(n > G.hcap){
-        if(G.hv){ cudaFreeHost(G.hv); cudaFreeHost(G.hst); cudaFreeHost(G.huu); cudaFreeHost(G.hpts); cudaFreeHost(G.hskip); }
-        long c = 1L << 16; while(c < n) c <<= 1;
-        CKR(cudaMallocHost(&G.hv, c*sizeof(double))); CKR(cudaMallocHost(&G.hst, c)); CKR(cudaMallocHost(&G.huu, c*sizeof(double)));
-        CKR(cudaMallocHost(&G.hpts, c*sizeof(sqb_pt_t))); CKR(cudaMallocHost(&G.hskip, c));
-        G.hcap = c;
-    }
     sqb_eval_t a; memset(&a, 0, sizeof a); fill_eval(&a, t);
     a.pts = pts; a.n = n; a.esize = 1; a.stride = SQB_MAXD; a.flag_at = -1; a.cells = 0; a.st = 0; a.skip = skip;
     if(eval_batch(g, &a, t, n)) return -1;
-    CKR(cudaMemcpyAsync(G.hv, G.v, n*sizeof(double), cudaMemcpyDeviceToHost, G.s));
-    CKR(cudaMemcpyAsync(G.hst, G.stt, n, cudaMemcpyDeviceToHost, G.s));
-    CKR(cudaMemcpyAsync(G.huu, G.uu, n*sizeof(double), cudaMemcpyDeviceToHost, G.s));
-    CKR(cudaStreamSynchronize(G.s));
-    D2H += n*(2*sizeof(double) + 1);
-    long q = 0, nd = 0; double uu = 0;
-    memcpy(v, G.hv, n*sizeof(double)); memcpy(stt, G.hst, n);
-    for(long i = 0; i < n; i++){
-        const unsigned char s = G.hst[i];
-        if(s & SQB_FALLBACK){ q++; uu += G.huu[i]; }
-        if(s & SQB_UNRES) nd++;
-    }
-    *nq += q; *u += uu; *unres += nd;
-    *v_dev = G.v; *stt_dev = G.stt;
+    *v_dev = G.v; *stt_dev = G.stt; *uu_dev = G.uu;
     return 0;
 }
 extern "C" void *sqb_dev_stream(void){ return (void*)G.s; }

@@ -63,11 +63,6 @@ int  sqb_dev_axis(const sqb_graph_t *g, int fma);
 long sqb_dev_axis_words(const sqb_graph_t *g, int K);
 int  sqb_dev_axis_fill(const sqb_graph_t *g, int fma, const double *X, int K, double *T);
 
-/* n nodes (host pt_t list, flags ignored) evaluated with the tests and the fallback: values v, near
- * flags (may be NULL); skip (host, may be NULL) per node; counters added to *nq, *u, *unres */
-int  sqb_dev_eval_nodes(const sqb_graph_t *g, long n, const sqb_pt_t *pts, const unsigned char *skip,
-                        const sqb_test_t *t, double *v, unsigned char *near, long *nq, double *u, long *unres);
-
 /* one refinement level on the device: the children (step st) of the ncell cells in the device list,
  * summed with weight pw; kept children (|v| >= thr, not last) appended to the device list next.
  * Accumulators are added into *acc.  Returns 0, or an error; *next_n is the length of next. */
@@ -97,22 +92,24 @@ int  sqb_dev_level(const sqb_level_t *L, sqb_acc_t *acc, long *next_n, double *m
  * or the pass split run one after another through sqb_dev_level. */
 int  sqb_dev_level_multi(const sqb_level_t *L, int n, sqb_acc_t *acc, long *next_n, double *ms);
 
-/* the same for n nodes already on the device (pts, skip device pointers); the values and status come
- * back to the host (v, stt) and stay on the device until the next evaluation (*v_dev, *stt_dev) */
-int  sqb_dev_eval_resident(const sqb_graph_t *g, const sqb_pt_t *pts, long n, const unsigned char *skip,
-                           const sqb_test_t *t, double *v, unsigned char *stt, long *nq, double *u, long *unres,
-                           const double **v_dev, const unsigned char **stt_dev);
+/* n nodes on the device (pts, skip device pointers) evaluated with the tests and the fallback, queued on the thread's
+ * stream; the values, status and round column stay on the device until the next evaluation */
+int  sqb_dev_eval_resident(const sqb_graph_t *g, const sqb_pt_t *pts, long n, const unsigned char *skip, const sqb_test_t *t,
+                           const double **v_dev, const unsigned char **stt_dev, const double **uu_dev);
 void *sqb_dev_stream(void);
 
-/* the top level on the device (topgrid.cu): grow frontiers, final threshold, tiers, dilation */
-int  sqb_grow_begin(int D, int K, int st, int W, const unsigned long long *P, int gs, int abskip, void *stream);
+/* the top level on the device (topgrid.cu): the zero probe, grow frontiers, final threshold, tiers, dilation.  Calls
+ * in this order: begin, probe, (frontier, expand)..., finish, dilate, sums, end */
+typedef struct { double S, a, x1, x2, drop, gshs, u; long gshn, nq, unres, kept, cells; } sqb_grow_sums_t;
+int  sqb_grow_begin(int D, int K, int st, int W, const unsigned long long *P, int gs, int abskip, double eps, double pw, void *stream,
+                    const sqb_pt_t **probe, long *nprobe);
+int  sqb_grow_probe(const double *v_dev, const unsigned char *stt_dev);
+int  sqb_grow_probe_zero(long *unres);
 long sqb_grow_frontier(const sqb_pt_t **pts, const unsigned char **skip);
-int  sqb_grow_shells_async(void);
-void sqb_grow_shells_take(unsigned char *cls_host);
-int  sqb_grow_expand(const double *v_dev, const unsigned char *stt_dev, double thr, long *nkept, long *nnext);
-int  sqb_grow_kv(double *kv_host, long n);
-int  sqb_grow_finish(double thr, int tiers, long *m);
-int  sqb_grow_dilate(int nbits, sqb_pt_t **out, long *n);
+int  sqb_grow_expand(const double *v_dev, const unsigned char *stt_dev, const double *uu_dev, long *nnext);
+int  sqb_grow_finish(int tiers);
+int  sqb_grow_dilate(int nbits, sqb_pt_t **out);
+int  sqb_grow_sums(sqb_grow_sums_t *r);
 void sqb_grow_kept(const sqb_pt_t **keep, long *m);
 void sqb_grow_end(void);
 const char *sqb_top_error(void);

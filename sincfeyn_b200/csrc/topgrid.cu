@@ -1,5 +1,5 @@
-/* topgrid.cu -- the top level of the hierarchical sum on the device: the support-following grow's
- * bookkeeping, the shadow-tier flood fill and the dilation (driver/sumkey.h:20-461).
+/* topgrid.cu -- the top level of the hierarchical sum on the device: the support-following grow, the
+ * shadow-tier flood fill and the dilation (driver/sumkey.h:20-461).
  *
  * Points of the top grid (step st) are identified by the reference's mixed-radix key
  * 1 c_0 ... c_{D-1} in base W = 2(K/st)+1, c_i = k_i/st + K/st (driver/sumkey.h:7-18): numeric order is
@@ -11,20 +11,33 @@
  * driver/sumkey.h:288-374).  The winners, compacted in id order, are the next frontier: exactly the
  * not-yet-seen neighbours of the kept points in (kept point, axis, sign) order.
  *
- * Order-preserving compactions (kept points, winners, re-threshold) use per-tile counts, one exclusive
- * scan and a per-tile ranked scatter.  The dilation inserts every cell and its in-box axis neighbours
- * into a hash table merging the flags (skip bit AND, tier max, driver/sumkey.h:41-44), collects the
- * distinct keys and sorts them with a stable LSD radix sort (8-bit digits), the reference's summation
- * order.  Every probe loop is bounded by the table size and reports overflow instead of spinning. */
+ * A frontier's values never leave the device.  The running sum a of |f w| whose threshold eps a decides what is
+ * kept is a sequence of rounded additions in point order, and it is replayed exactly in parallel (seq_sum): while
+ * a stays in one binade with unit u every addition adds RN(x/u) units, so a chunk's additions are one integer sum;
+ * the element that leaves the binade, or that lies half-way between units, is added by itself.  The sums
+ * that decide nothing (S, the shells, the dropped weight, the round column) are double-double in a fixed order.
+ * The host waits once per frontier, for the next one's size.  Waits, launches and the host's sums bound the grow
+ * before (three waits and about 19 operations a frontier, 17 bytes a point to the host), launches now: d = 5, h = 1.5
+ * (10 frontiers, 8816 points) 2.1 -> 0.66 ms; d = 8, h = 1 (17 frontiers, 4.06e6 points) 37 -> 3.5 ms.
+ *
+ * After the grow the table's claim words, all SEEN by then, serve the tiers (the index of a kept point) and the
+ * dilation (the merged flags of a cell): every neighbour of a kept point was a candidate and is in the table.
+ * (A table of its own, sized for four cells a kept point, overflowed at D = 11 and was probed from end to end before
+ * it was enlarged: 26.4 s at h = 1, eps = 1e-8, 3.3 ms with the tiers now.)  The dilation's cells are the marked slots'
+ * keys, sorted with a stable LSD radix sort (8-bit digits), the
+ * reference's summation order.  Every probe loop is bounded by the table size and reports overflow instead of
+ * spinning. */
 #include <cuda_runtime.h>
 #include <stdio.h>
 #include <stdlib.h>
 #include <string.h>
 #include "sqb_rt.h"
+#include "sqdd.cuh"
 
 #define TG_T 256                 /* threads per CTA of the compaction kernels */
-#define TG_I 8                   /* items per thread */
-#define TG_TILE (TG_T*TG_I)
+#define GT 1024                  /* threads of the one-CTA kernels */
+#define GS_SMALL 4096            /* frontiers up to this size: sums, threshold and kept points in one CTA */
+#define GS_TILE 2048             /* points per tile of a larger frontier's sums */
 #define SEEN 0xFFFFFFFFu
 #define CLAIM(id) (0xFFFFFFFEu - (unsigned)(id))
 
@@ -34,17 +47,19 @@ static thread_local char terr[512];   /* the state of this file is per host thre
     return (int)e_; } } while(0)
 extern "C" const char *sqb_top_error(void){ return terr; }
 
-__device__ __forceinline__ unsigned long long hslot(unsigned long long y, unsigned long long mask){
+typedef unsigned long long u64;
+
+__device__ __forceinline__ u64 hslot(u64 y, u64 mask){
     return ((y*0x9E3779B97F4A7C15ULL) >> 21) & mask;
 }
 /* slot of key y, inserting it if absent (*isnew = 1); -1 if the table is full */
-__device__ long h_insert(unsigned long long *key, unsigned long long mask, unsigned long long y, int *isnew){
-    unsigned long long i = hslot(y, mask);
-    for(unsigned long long p = 0; p <= mask; p++){
-        unsigned long long c = key[i];
+__device__ long h_insert(u64 *key, u64 mask, u64 y, int *isnew){
+    u64 i = hslot(y, mask);
+    for(u64 p = 0; p <= mask; p++){
+        u64 c = key[i];
         if(c == y){ *isnew = 0; return (long)i; }
         if(c == 0){
-            unsigned long long o = atomicCAS(&key[i], 0ULL, y);
+            u64 o = atomicCAS(&key[i], 0ULL, y);
             if(o == 0){ *isnew = 1; return (long)i; }
             if(o == y){ *isnew = 0; return (long)i; }
         }
@@ -52,10 +67,10 @@ __device__ long h_insert(unsigned long long *key, unsigned long long mask, unsig
     }
     return -1;
 }
-__device__ long h_find(const unsigned long long *key, unsigned long long mask, unsigned long long y){
-    unsigned long long i = hslot(y, mask);
-    for(unsigned long long p = 0; p <= mask; p++){
-        unsigned long long c = key[i];
+__device__ long h_find(const u64 *key, u64 mask, u64 y){
+    u64 i = hslot(y, mask);
+    for(u64 p = 0; p <= mask; p++){
+        u64 c = key[i];
         if(c == y) return (long)i;
         if(c == 0) return -1;
         i = (i + 1) & mask;
@@ -63,116 +78,306 @@ __device__ long h_find(const unsigned long long *key, unsigned long long mask, u
     return -1;
 }
 
-struct geom_t { int D, K, st, W; unsigned long long P[SQB_MAXD]; };
+/* sh: log2 of the step */
+struct geom_t { int D, K, st, sh, W; u64 P[SQB_MAXD]; };
 
-__device__ __forceinline__ unsigned long long key_of(const geom_t &g, const signed char *k){
-    unsigned long long y = 1;
-    for(int i = 0; i < g.D; i++) y = y*g.W + (unsigned long long)(k[i]/g.st + g.K/g.st);
+__device__ __forceinline__ u64 key_of(const geom_t &g, const signed char *k){
+    u64 y = 1;
+    for(int i = 0; i < g.D; i++) y = y*g.W + (u64)((k[i] + g.K) >> g.sh);
     return y;
 }
 
-/* --------------------------------- generic ordered compaction ----------------------------------- */
-/* Op: __device__ bool pred(long i); __device__ void emit(long i, unsigned long long rank) */
-template<class Op>
-__global__ void __launch_bounds__(TG_T) k_count(Op op, long n, unsigned *bcnt){
-    const long t0 = blockIdx.x*(long)TG_TILE + threadIdx.x*(long)TG_I;
-    unsigned c = 0;
-    for(int j = 0; j < TG_I; j++){ long i = t0 + j; if(i < n && op.pred(i)) c++; }
-    for(int off = 16; off; off >>= 1) c += __shfl_down_sync(0xffffffffu, c, off);
-    __shared__ unsigned ws[TG_T/32];
-    if((threadIdx.x & 31) == 0) ws[threadIdx.x >> 5] = c;
-    __syncthreads();
-    if(threadIdx.x == 0){ unsigned s = 0; for(int w = 0; w < TG_T/32; w++) s += ws[w]; bcnt[blockIdx.x] = s; }
+/* the grow's counters and sums, in device memory and, after each wait, in pinned host memory */
+struct gacc_t {
+    double a, thr, eps, pw;                 /* running sum of |f w|, its threshold eps a, the weight step^D */
+    double S[2], x1[2], x2[2], dr[2], gs[2], u[2];   /* sum f w; outer shells; dropped weight; its signed sum; round column */
+    u64 ngs, nq, unres;                     /* points below the threshold; fallback and unresolved points */
+    u64 nk, nn, nkeep;                      /* this frontier's kept points, the next frontier, kept so far */
+    u64 m, ncell, err;                      /* kept after the final threshold; dilated cells; full-table inserts */
+    u64 nz, punres;                         /* the zero probe: any value not 0; its unresolved points */
+};
+
+/* ------------------------------------- block sums and scans ------------------------------------------ */
+__device__ __forceinline__ sqdd dd_shfl(const sqdd &a, int off){
+    return sqdd(__shfl_down_sync(0xffffffffu, a.hi, off), __shfl_down_sync(0xffffffffu, a.lo, off));
 }
-/* one CTA: exclusive scan of nb counts; total into *tot */
-__global__ void __launch_bounds__(256) k_scan(const unsigned *bcnt, long nb, unsigned long long *boff, unsigned long long *tot){
-    __shared__ unsigned long long pre[256];
-    const int t = threadIdx.x; const long ch = (nb + 255)/256, j0 = t*ch, j1 = j0 + ch < nb ? j0 + ch : nb;
-    unsigned long long s = 0; for(long j = j0; j < j1; j++) s += bcnt[j];
-    pre[t] = s; __syncthreads();
-    if(t == 0){ unsigned long long x = 0; for(int j = 0; j < 256; j++){ unsigned long long y = pre[j]; pre[j] = x; x += y; } *tot = x; }
+/* the CTA's sum of x in a fixed order, in thread 0; sh: T/32 entries; ends with a barrier */
+template<int T> __device__ sqdd block_dd(sqdd x, sqdd *sh){
+    for(int off = 16; off; off >>= 1) x = x + dd_shfl(x, off);
+    if((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = x;
     __syncthreads();
-    unsigned long long x = pre[t]; for(long j = j0; j < j1; j++){ boff[j] = x; x += bcnt[j]; }
+    if(threadIdx.x < 32){
+        sqdd y = threadIdx.x < T/32 ? sh[threadIdx.x] : sqdd(0.0);
+        for(int off = 16; off; off >>= 1) y = y + dd_shfl(y, off);
+        x = y;
+    }
+    __syncthreads();
+    return x;
 }
-template<class Op>
-__global__ void __launch_bounds__(TG_T) k_scatter(Op op, long n, const unsigned long long *boff){
-    const long t0 = blockIdx.x*(long)TG_TILE + threadIdx.x*(long)TG_I;
-    unsigned mask = 0; int c = 0;
-    for(int j = 0; j < TG_I; j++){ long i = t0 + j; if(i < n && op.pred(i)){ mask |= 1u << j; c++; } }
-    __shared__ int ws[TG_T/32];
-    const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
-    int x = c;
-    for(int off = 1; off < 32; off <<= 1){ int y = __shfl_up_sync(0xffffffffu, x, off); if(l >= off) x += y; }
-    if(l == 31) ws[w] = x;
+template<int T> __device__ u64 block_sum(u64 x, u64 *sh){
+    for(int off = 16; off; off >>= 1) x += __shfl_down_sync(0xffffffffu, x, off);
+    if((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = x;
     __syncthreads();
-    if(threadIdx.x == 0){ int s = 0; for(int q = 0; q < TG_T/32; q++){ int y = ws[q]; ws[q] = s; s += y; } }
+    u64 s = 0;
+    for(int w = 0; w < T/32; w++) s += sh[w];
     __syncthreads();
-    unsigned long long r = boff[blockIdx.x] + (unsigned long long)(ws[w] + x - c);
-    for(int j = 0; j < TG_I; j++) if(mask >> j & 1) op.emit(t0 + j, r++);
+    return s;
+}
+/* exclusive scan of x over the CTA, every partial sum cut off at cap; *total the CTA's sum */
+template<int T> __device__ u64 block_scan(u64 x, u64 cap, u64 *total, u64 *sh){
+    const int l = threadIdx.x & 31, w = threadIdx.x >> 5;
+    u64 inc = x < cap ? x : cap;
+    for(int off = 1; off < 32; off <<= 1){
+        const u64 y = __shfl_up_sync(0xffffffffu, inc, off);
+        if(l >= off){ inc += y; inc = inc < cap ? inc : cap; }
+    }
+    u64 ex = __shfl_up_sync(0xffffffffu, inc, 1);
+    if(l == 0) ex = 0;
+    if(l == 31) sh[w] = inc;
+    __syncthreads();
+    if(w == 0){
+        u64 z = l < T/32 ? sh[l] : 0;
+        for(int off = 1; off < 32; off <<= 1){
+            const u64 y = __shfl_up_sync(0xffffffffu, z, off);
+            if(l >= off){ z += y; z = z < cap ? z : cap; }
+        }
+        if(l < T/32) sh[l] = z;
+    }
+    __syncthreads();
+    if(w > 0){ ex += sh[w - 1]; ex = ex < cap ? ex : cap; }
+    *total = sh[T/32 - 1];
+    __syncthreads();
+    return ex;
+}
+template<int T> __device__ unsigned block_min(unsigned x, unsigned *sh){
+    x = __reduce_min_sync(0xffffffffu, x);
+    if((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = x;
+    __syncthreads();
+    unsigned m = 0xFFFFFFFFu;
+    for(int w = 0; w < T/32; w++) m = min(m, sh[w]);
+    __syncthreads();
+    return m;
 }
 
-struct Scratch { unsigned *bcnt; unsigned long long *boff, *tot; long nbcap; };
+/* ------------------------------ a sequential rounded sum, in parallel --------------------------------- */
+/* For x >= 0 and a in [2^e, 2^(e+1)), u = 2^(e-52): RN(a + x) = a + u RN(x/u) as long as the result stays in the
+ * binade and x/u is not half-way between two integers (there the parity of a/u decides).  So over the elements
+ * up to the first that breaks this, the rounded additions in order are one sum of integers. */
+#define SQ_ONE53 (1ULL << 53)
+#define SQ_ODD (1ULL << 63)      /* the element, or an element of the tile, has to be added by itself */
+__device__ __forceinline__ bool seq_binade(double a, double *inv, double *u){
+    const int ex = (__double2hiint(a) >> 20) & 0x7ff;
+    if(!(a > 0) || ex < 100 || ex > 1900) return false;
+    *u = __hiloint2double((ex - 52) << 20, 0);
+    *inv = __hiloint2double((2046 - (ex - 52)) << 20, 0);
+    return true;
+}
+/* x in units of u: RN(x/u), or SQ_ODD */
+__device__ __forceinline__ u64 seq_units(double x, double inv){
+    const double t = __dmul_rn(x, inv), r = rint(t);
+    return !(t < 0x1p53) || fabs(__dsub_rn(t, r)) == 0.5 ? SQ_ODD : (u64)r;
+}
+struct seq_sh { u64 s[GT/32]; unsigned m[GT/32]; u64 pre; };
+/* a after the additions of |v[i]| pw, i0 <= i < i1, one after another (called by all GT threads) */
+__device__ double seq_sum(double a, const double *v, double pw, long i0, long i1, seq_sh &sh){
+    long i = i0;
+    while(i < i1){
+        if(!(a < INFINITY)) return a;                       /* infinite, and so it stays */
+        double inv = 0, u = 0;
+        const bool ok = seq_binade(a, &inv, &u);
+        const u64 A0 = ok ? (u64)__dmul_rn(a, inv) : 0, room = ok ? SQ_ONE53 - A0 : SQ_ONE53;
+        u64 q[4], s = 0;
+#pragma unroll
+        for(int e = 0; e < 4; e++){
+            const long j = i + threadIdx.x*4L + e;
+            const double w = j < i1 ? __dmul_rn(fabs(v[j]), pw) : 0.0;
+            q[e] = ok ? seq_units(w, inv) : (w == 0 ? 0 : SQ_ODD);   /* outside the range only zeros pass */
+            s += q[e] < room ? q[e] : room; s = s < room ? s : room;
+        }
+        u64 total, pre = block_scan<GT>(s, room, &total, sh.s);
+        unsigned first = 0xFFFFFFFFu; u64 at = 0;
+#pragma unroll
+        for(int e = 0; e < 4; e++){
+            if(first == 0xFFFFFFFFu && (q[e] == SQ_ODD || pre + q[e] >= room)){ first = threadIdx.x*4u + e; at = pre; }
+            if(first == 0xFFFFFFFFu) pre += q[e];
+        }
+        const unsigned f = block_min<GT>(first, sh.m);
+        if(f == 0xFFFFFFFFu){
+            if(ok) a = __dmul_rn((double)(A0 + total), u);
+            i += 4L*GT;
+            continue;
+        }
+        if(first == f) sh.pre = at;
+        __syncthreads();
+        if(ok) a = __dmul_rn((double)(A0 + sh.pre), u);
+        a = __dadd_rn(a, __dmul_rn(fabs(v[i + f]), pw));
+        i += f + 1;
+        __syncthreads();
+    }
+    return a;
+}
+
+/* --------------------------------- ordered compaction ------------------------------------------------- */
+/* An Op has bool pred(long i) and void emit(long i, u64 rank); with DROP, weight(i) of an element that is left
+ * out adds to the grow's dropped sums.  The number of elements is read on the device (*np + nadd); the grid covers
+ * the host's bound on it.  Counting and emitting are two launches; a CTA finds its offset by adding the counts
+ * before it itself, up to OFFS_CTAS CTAs, above that from a scan of the counts. */
+#define OFFS_CTAS 1024
+struct drop_t { double dr[2], gs[2]; u64 n; };
+struct cnt_t { const u64 *np; long mul, max; };          /* min(*np mul, max) elements (np NULL: max) */
+__device__ __forceinline__ long cnt_of(const cnt_t &c){
+    if(!c.np) return c.max;
+    const long n = (long)*c.np*c.mul;
+    return n < c.max ? n : c.max;
+}
+template<class Op, int I>
+__global__ void __launch_bounds__(TG_T) k_count(Op op, cnt_t cn, unsigned *bcnt, drop_t *drop){
+    __shared__ u64 ws[TG_T/32];
+    __shared__ sqdd wd[TG_T/32];
+    const long n = cnt_of(cn), b0 = blockIdx.x*(long)(TG_T*I);
+    u64 c = 0;
+    if(b0 < n){
+        sqdd dr, gs; u64 nd = 0;
+        for(int j = 0; j < I; j++){
+            const long i = b0 + j*TG_T + threadIdx.x;
+            if(i >= n) break;
+            if(op.pred(i)) c++;
+            else if constexpr(Op::DROP){
+                const double w = op.weight(i);
+                dr = sqdd_add_d(dr, fabs(w)); gs = sqdd_add_d(gs, w); nd++;
+            }
+        }
+        if constexpr(Op::DROP){
+            dr = block_dd<TG_T>(dr, wd); gs = block_dd<TG_T>(gs, wd); nd = block_sum<TG_T>(nd, ws);
+            if(threadIdx.x == 0) drop[blockIdx.x] = {{dr.hi, dr.lo}, {gs.hi, gs.lo}, nd};
+        }
+        c = block_sum<TG_T>(c, ws);
+    } else if(Op::DROP && threadIdx.x == 0) drop[blockIdx.x] = {{0, 0}, {0, 0}, 0};
+    if(threadIdx.x == 0) bcnt[blockIdx.x] = (unsigned)c;
+}
+/* one CTA: exclusive scan of nb counts; the total into *tot */
+__global__ void __launch_bounds__(GT) k_scan(const unsigned *bcnt, long nb, u64 *boff, u64 *tot){
+    __shared__ u64 sh[GT/32];
+    u64 carry = 0;
+    for(long b = 0; b < nb; b += 4*GT){
+        const long j = b + threadIdx.x*4L;
+        unsigned c[4]; u64 s = 0, t;
+#pragma unroll
+        for(int e = 0; e < 4; e++){ c[e] = j + e < nb ? bcnt[j + e] : 0; s += c[e]; }
+        u64 x = carry + block_scan<GT>(s, ~0ULL, &t, sh);
+#pragma unroll
+        for(int e = 0; e < 4; e++){ if(j + e < nb) boff[j + e] = x; x += c[e]; }
+        carry += t;
+    }
+    if(threadIdx.x == 0 && tot) *tot = carry;
+}
+/* everything a CTA of an emitting kernel needs: counts, their scan (or NULL), and where the total goes */
+struct emit_t { const unsigned *bcnt; const u64 *boff; long nb; u64 *tot; drop_t *drop; gacc_t *acc, *host; };
+__device__ __forceinline__ void dd_into(double *dst, const sqdd &x){
+    const sqdd z = sqdd(dst[0], dst[1]) + x;
+    dst[0] = z.hi; dst[1] = z.lo;
+}
+/* the grow's record to pinned host memory (one warp) */
+__device__ __forceinline__ void publish(const gacc_t *acc, gacc_t *host){
+    const u64 *s = (const u64*)acc; u64 *d = (u64*)host;
+    for(unsigned w = threadIdx.x; w < sizeof(gacc_t)/8; w += 32) d[w] = s[w];
+}
+template<class Op, int I>
+__global__ void __launch_bounds__(TG_T) k_emit(Op op, cnt_t cn, emit_t e){
+    __shared__ u64 ws[TG_T/32];
+    __shared__ sqdd wd[TG_T/32];
+    const long n = cnt_of(cn), b0 = blockIdx.x*(long)(TG_T*I);
+    const bool last = blockIdx.x == gridDim.x - 1;
+    if(b0 >= n && !last) return;
+    u64 r;
+    if(e.boff) r = e.boff[blockIdx.x];
+    else {
+        u64 s = 0;
+        for(long j = threadIdx.x; j < (long)blockIdx.x; j += TG_T) s += e.bcnt[j];
+        r = block_sum<TG_T>(s, ws);
+    }
+    for(int j = 0; j < I; j++){                     /* TG_T consecutive elements at a time keep the order */
+        const long i = b0 + j*TG_T + threadIdx.x;
+        if(b0 + j*TG_T >= n) break;
+        const int p = i < n && op.pred(i);
+        u64 t;
+        const u64 x = block_scan<TG_T>((u64)p, ~0ULL, &t, ws);
+        if(p) op.emit(i, r + x);
+        r += t;
+    }
+    if(!last) return;
+    if constexpr(Op::DROP){
+        sqdd dr, gs; u64 nd = 0;
+        for(long j = threadIdx.x; j < e.nb; j += TG_T){
+            dr = dr + sqdd(e.drop[j].dr[0], e.drop[j].dr[1]); gs = gs + sqdd(e.drop[j].gs[0], e.drop[j].gs[1]); nd += e.drop[j].n;
+        }
+        dr = block_dd<TG_T>(dr, wd); gs = block_dd<TG_T>(gs, wd); nd = block_sum<TG_T>(nd, ws);
+        if(threadIdx.x == 0){ dd_into(e.acc->dr, dr); dd_into(e.acc->gs, gs); e.acc->ngs += nd; }
+    }
+    if(threadIdx.x == 0){ *e.tot = r; if(Op::DROP) e.acc->nkeep = op.base + r; __threadfence(); }
+    __syncthreads();
+    if(e.host && threadIdx.x < 32) publish(e.acc, e.host);
+}
+
+struct Scratch { unsigned *bcnt; u64 *boff; drop_t *drop; long nbcap; };
 static thread_local Scratch SC;
 static thread_local cudaStream_t TS;
 /* stream-ordered allocation from the device's memory pool: no device-wide synchronisation, and the pool
  * keeps freed memory for the next integral (the runtime sets its release threshold) */
 #define DMALLOC(p, n) cudaMallocAsync((void**)(p), (n), TS)
 #define DFREE(p) cudaFreeAsync((p), TS)
-static thread_local unsigned long long TL;    /* kernels launched by this file */
+static thread_local u64 TL;    /* kernels launched by this file */
 extern "C" unsigned long long sqb_top_launches(void){ return TL; }
 extern "C" void sqb_dev_count_copy(unsigned long long h2d, unsigned long long d2h);
 
-static int scratch(long n){
-    long nb = (n + TG_TILE - 1)/TG_TILE; if(nb < 1) nb = 1;
+static int scratch(long nb){
     if(nb <= SC.nbcap) return 0;
-    if(SC.bcnt){ DFREE(SC.bcnt); DFREE(SC.boff); }
+    if(SC.bcnt){ DFREE(SC.bcnt); DFREE(SC.boff); DFREE(SC.drop); SC.bcnt = NULL; SC.nbcap = 0; }
     long c = 1024; while(c < nb) c <<= 1;
-    TCK(DMALLOC(&SC.bcnt, c*sizeof(unsigned))); TCK(DMALLOC(&SC.boff, c*sizeof(unsigned long long)));
-    if(!SC.tot) TCK(DMALLOC(&SC.tot, sizeof(unsigned long long)));
+    TCK(DMALLOC(&SC.bcnt, c*sizeof(unsigned))); TCK(DMALLOC(&SC.boff, c*sizeof(u64))); TCK(DMALLOC(&SC.drop, c*sizeof(drop_t)));
     SC.nbcap = c;
     return 0;
 }
-/* ordered compaction; returns the count (synchronous) */
-template<class Op>
-static int compact(const Op &op, long n, long *count){
-    *count = 0;
-    if(n <= 0) return 0;
-    if(scratch(n)) return -1;
-    const long nb = (n + TG_TILE - 1)/TG_TILE;
-    k_count<Op><<<(unsigned)nb, TG_T, 0, TS>>>(op, n, SC.bcnt);
-    k_scan<<<1, 256, 0, TS>>>(SC.bcnt, nb, SC.boff, SC.tot);
-    k_scatter<Op><<<(unsigned)nb, TG_T, 0, TS>>>(op, n, SC.boff);
-    TL += 3;
+template<class Op, int I>
+static int compact_i(const Op &op, cnt_t cn, u64 *tot, gacc_t *acc, gacc_t *host){
+    const long nb = (cn.max + TG_T*I - 1)/(TG_T*I);
+    if(scratch(nb)) return -1;
+    k_count<Op, I><<<(unsigned)nb, TG_T, 0, TS>>>(op, cn, SC.bcnt, SC.drop);
+    const bool scan = nb > OFFS_CTAS;
+    if(scan){ k_scan<<<1, GT, 0, TS>>>(SC.bcnt, nb, SC.boff, NULL); TL++; }
+    emit_t e = {SC.bcnt, scan ? SC.boff : NULL, nb, tot, SC.drop, acc, host};
+    k_emit<Op, I><<<(unsigned)nb, TG_T, 0, TS>>>(op, cn, e);
+    TL += 2;
     TCK(cudaGetLastError());
-    unsigned long long t = 0;
-    TCK(cudaMemcpyAsync(&t, SC.tot, sizeof t, cudaMemcpyDeviceToHost, TS));
-    TCK(cudaStreamSynchronize(TS));
-    sqb_dev_count_copy(0, sizeof t);
-    *count = (long)t;
     return 0;
+}
+/* one element per thread while that fills the device in one round, else eight */
+template<class Op>
+static int compact(const Op &op, cnt_t cn, u64 *tot, gacc_t *acc, gacc_t *host){
+    return cn.max <= 1L << 18 ? compact_i<Op, 1>(op, cn, tot, acc, host) : compact_i<Op, 8>(op, cn, tot, acc, host);
 }
 
 /* --------------------------------------------- grow --------------------------------------------- */
+struct gpart_t { u64 q; double S[2], x1[2], x2[2], u[2]; u64 nq, unres; };    /* one tile of a frontier's sums */
 struct Grow {
     geom_t g;
-    unsigned long long *key; unsigned *word; unsigned long long mask; long nseen;   /* seen table */
-    sqb_pt_t *fr, *nx; unsigned char *frsk, *nxsk, *cls; long nfr, frcap;         /* frontier, next */
-    sqb_pt_t *keep; double *kv; long nkeep, keepcap;                              /* kept so far */
-    long *kj; long kjcap;                                                        /* this frontier's kept */
-    long *qs; long qscap;                                                        /* slot per candidate */
-    unsigned long long *err;
-    int gs, abskip;
-    unsigned char *hcls; long hclscap;     /* pinned: the frontier's shell classes, read after the next sync */
-    unsigned long long *herr;              /* pinned: the overflow count, read after the next sync */
+    u64 *key; unsigned *word; u64 mask; long nseen;   /* seen table */
+    sqb_pt_t *fr, *nx; unsigned char *frsk, *nxsk; long nfr, frcap;         /* frontier, next */
+    sqb_pt_t *keep; double *kv; long nkeep, keepcap;                        /* kept so far */
+    long *kj; long kjcap;                                                  /* this frontier's kept */
+    long *qs; long qscap;                                                  /* slot per candidate */
+    gpart_t *part; long partcap;                                           /* sums per tile */
+    gacc_t *acc, *host;                                                    /* device record; its pinned copy */
+    sqb_pt_t *probe;                                                       /* the zero probe's points */
+    int gs, abskip, nfrs;
 };
 static thread_local Grow GR;
 
-__global__ void k_rehash(const unsigned long long *ok, const unsigned *ow, long ocap, unsigned long long *key,
-                         unsigned *word, unsigned long long mask, unsigned long long *err){
+__global__ void k_rehash(const u64 *ok, const unsigned *ow, long ocap, u64 *key, unsigned *word, u64 mask, gacc_t *acc){
     for(long i = blockIdx.x*(long)blockDim.x + threadIdx.x; i < ocap; i += (long)gridDim.x*blockDim.x){
         if(!ok[i]) continue;
         int nw; long q = h_insert(key, mask, ok[i], &nw);
-        if(q < 0){ atomicAdd(err, 1ULL); continue; }
+        if(q < 0){ atomicAdd(&acc->err, 1ULL); continue; }
         word[q] = ow[i];
     }
 }
@@ -181,14 +386,13 @@ static int table_room(long extra){
     long cap = (long)GR.mask + 1;
     if((double)(GR.nseen + extra) <= 0.6*cap) return 0;
     long nc = cap; while((double)(GR.nseen + extra) > 0.6*nc) nc <<= 1;
-    unsigned long long *k2; unsigned *w2;
-    TCK(DMALLOC(&k2, nc*sizeof(unsigned long long))); TCK(DMALLOC(&w2, nc*sizeof(unsigned)));
-    TCK(cudaMemsetAsync(k2, 0, nc*sizeof(unsigned long long), TS)); TCK(cudaMemsetAsync(w2, 0, nc*sizeof(unsigned), TS));
-    k_rehash<<<1184, 256, 0, TS>>>(GR.key, GR.word, cap, k2, w2, (unsigned long long)(nc - 1), GR.err); TL++;
+    u64 *k2; unsigned *w2;
+    TCK(DMALLOC(&k2, nc*sizeof(u64))); TCK(DMALLOC(&w2, nc*sizeof(unsigned)));
+    TCK(cudaMemsetAsync(k2, 0, nc*sizeof(u64), TS)); TCK(cudaMemsetAsync(w2, 0, nc*sizeof(unsigned), TS));
+    k_rehash<<<1184, 256, 0, TS>>>(GR.key, GR.word, cap, k2, w2, (u64)(nc - 1), GR.acc); TL++;
     TCK(cudaGetLastError());
-    TCK(cudaStreamSynchronize(TS));
     DFREE(GR.key); DFREE(GR.word);
-    GR.key = k2; GR.word = w2; GR.mask = (unsigned long long)(nc - 1);
+    GR.key = k2; GR.word = w2; GR.mask = (u64)(nc - 1);
     return 0;
 }
 /* device array of at least n elements, keeping the first keep elements */
@@ -196,7 +400,7 @@ template<class T> static int devbuf(T **p, long *cap, long n, long keep){
     if(n <= *cap && *p) return 0;
     long c = 1L << 16; while(c < n) c <<= 1;
     T *q; TCK(DMALLOC(&q, c*sizeof(T)));
-    if(*p && keep > 0){ TCK(cudaMemcpyAsync(q, *p, keep*sizeof(T), cudaMemcpyDeviceToDevice, TS)); TCK(cudaStreamSynchronize(TS)); }
+    if(*p && keep > 0) TCK(cudaMemcpyAsync(q, *p, keep*sizeof(T), cudaMemcpyDeviceToDevice, TS));
     if(*p) DFREE(*p);
     *p = q; *cap = c;
     return 0;
@@ -205,113 +409,230 @@ template<class T> static int devbuf(T **p, long *cap, long n, long keep){
 static int frontier_room(long n){
     if(n <= GR.frcap && GR.fr) return 0;
     long c = 1L << 16; while(c < n) c <<= 1;
-    sqb_pt_t *a, *b; unsigned char *s1, *s2, *s3;
+    sqb_pt_t *a, *b; unsigned char *s1, *s2;
     TCK(DMALLOC(&a, c*sizeof(sqb_pt_t))); TCK(DMALLOC(&b, c*sizeof(sqb_pt_t)));
-    TCK(DMALLOC(&s1, c)); TCK(DMALLOC(&s2, c)); TCK(DMALLOC(&s3, c));
+    TCK(DMALLOC(&s1, c)); TCK(DMALLOC(&s2, c));
     if(GR.fr){
         TCK(cudaMemcpyAsync(a, GR.fr, GR.nfr*sizeof(sqb_pt_t), cudaMemcpyDeviceToDevice, TS));
         TCK(cudaMemcpyAsync(s1, GR.frsk, GR.nfr, cudaMemcpyDeviceToDevice, TS));
-        TCK(cudaStreamSynchronize(TS));
-        DFREE(GR.fr); DFREE(GR.nx); DFREE(GR.frsk); DFREE(GR.nxsk); DFREE(GR.cls);
+        DFREE(GR.fr); DFREE(GR.nx); DFREE(GR.frsk); DFREE(GR.nxsk);
     }
-    GR.fr = a; GR.nx = b; GR.frsk = s1; GR.nxsk = s2; GR.cls = s3; GR.frcap = c;
+    GR.fr = a; GR.nx = b; GR.frsk = s1; GR.nxsk = s2; GR.frcap = c;
     return 0;
 }
 
-__global__ void k_seed(unsigned long long *key, unsigned *word, unsigned long long mask, unsigned long long y0,
-                       sqb_pt_t *fr, unsigned char *frsk, unsigned long long *err){
-    int nw; long q = h_insert(key, mask, y0, &nw);
-    if(q < 0){ atomicAdd(err, 1ULL); return; }
-    word[q] = SEEN;
-    for(int i = 0; i < SQB_MAXD; i++) fr[0].k[i] = 0;
-    frsk[0] = 0;
+/* z = 0 into the table and the frontier, the record cleared, and the zero probe's nodes (driver/sum.c:346-359): z = 0
+ * and NPROBE nodes from a fixed hash */
+#define NPROBE 4096
+__global__ void k_seed(geom_t g, u64 *key, unsigned *word, u64 mask, u64 y0, sqb_pt_t *fr, unsigned char *frsk, gacc_t *acc,
+                       double eps, double pw, sqb_pt_t *probe){
+    const int j = blockIdx.x*blockDim.x + threadIdx.x;
+    if(j == 0){
+        gacc_t z = {}; z.eps = eps; z.pw = pw;
+        int nw; const long q = h_insert(key, mask, y0, &nw);
+        if(q < 0) z.err = 1; else word[q] = SEEN;
+        for(int i = 0; i < SQB_MAXD; i++) fr[0].k[i] = 0;
+        frsk[0] = 0;
+        *acc = z;
+    }
+    if(j > NPROBE) return;
+    sqb_pt_t p;
+    for(int i = 0; i < SQB_MAXD; i++) p.k[i] = 0;
+    u64 y = 0x9E3779B97F4A7C15ULL*(u64)(j + 1);
+    const int h = g.K/g.st; const u64 W = 2*h + 1;
+    if(j) for(int d = 0; d < g.D; d++){ y ^= y >> 29; y *= 0xBF58476D1CE4E5B9ULL; y ^= y >> 32; p.k[d] = (signed char)(((int)(y % W) - h)*g.st); }
+    probe[j] = p;
+}
+__global__ void __launch_bounds__(GT) k_probe_check(const double *v, const unsigned char *stt, gacc_t *acc){
+    __shared__ u64 sh[GT/32];
+    u64 nz = 0, un = 0;
+    for(int j = threadIdx.x; j <= NPROBE; j += GT){ nz += v[j] != 0; un += (stt[j] & SQB_UNRES) != 0; }
+    nz = block_sum<GT>(nz, sh); un = block_sum<GT>(un, sh);
+    if(threadIdx.x == 0){ acc->nz = nz; acc->punres = un; }
 }
 
-/* a new grow at step st; the frontier is z = 0 */
-extern "C" int sqb_grow_begin(int D, int K, int st, int W, const unsigned long long *P, int gs, int abskip, void *stream){
+/* a new grow at step st with threshold eps times the running sum; the frontier is z = 0.  *probe, *nprobe: the zero
+ * probe's nodes, for the caller to evaluate and hand to sqb_grow_probe */
+extern "C" int sqb_grow_begin(int D, int K, int st, int W, const unsigned long long *P, int gs, int abskip, double eps, double pw,
+                              void *stream, const sqb_pt_t **probe, long *nprobe){
     TS = (cudaStream_t)stream;
     memset(&GR.g, 0, sizeof GR.g);
     GR.g.D = D; GR.g.K = K; GR.g.st = st; GR.g.W = W; for(int i = 0; i < D; i++) GR.g.P[i] = P[i];
-    GR.gs = gs; GR.abskip = abskip; GR.nseen = 1; GR.nkeep = 0; GR.nfr = 0;
-    const long cap = 1L << 22;
+    while((1 << GR.g.sh) < st) GR.g.sh++;
+    GR.gs = gs; GR.abskip = abskip; GR.nseen = 1; GR.nkeep = 0; GR.nfr = 0; GR.nfrs = 0;
+    const long cap = 1L << 20;
     if(GR.key){ DFREE(GR.key); DFREE(GR.word); GR.key = NULL; }
-    TCK(DMALLOC(&GR.key, cap*sizeof(unsigned long long))); TCK(DMALLOC(&GR.word, cap*sizeof(unsigned)));
-    TCK(cudaMemsetAsync(GR.key, 0, cap*sizeof(unsigned long long), TS)); TCK(cudaMemsetAsync(GR.word, 0, cap*sizeof(unsigned), TS));
-    GR.mask = (unsigned long long)(cap - 1);
-    if(!GR.err) TCK(DMALLOC(&GR.err, sizeof(unsigned long long)));
-    TCK(cudaMemsetAsync(GR.err, 0, sizeof(unsigned long long), TS));
+    TCK(DMALLOC(&GR.key, cap*sizeof(u64))); TCK(DMALLOC(&GR.word, cap*sizeof(unsigned)));
+    TCK(cudaMemsetAsync(GR.key, 0, cap*sizeof(u64), TS)); TCK(cudaMemsetAsync(GR.word, 0, cap*sizeof(unsigned), TS));
+    GR.mask = (u64)(cap - 1);
+    if(!GR.acc) TCK(DMALLOC(&GR.acc, sizeof(gacc_t)));
+    if(!GR.host) TCK(cudaMallocHost(&GR.host, sizeof(gacc_t)));
+    if(!GR.probe) TCK(DMALLOC(&GR.probe, (NPROBE + 1)*sizeof(sqb_pt_t)));
     if(frontier_room(1)) return -1;
-    unsigned long long y0 = 1; for(int i = 0; i < D; i++) y0 = y0*W + (unsigned long long)(K/st);
-    k_seed<<<1, 1, 0, TS>>>(GR.key, GR.word, GR.mask, y0, GR.fr, GR.frsk, GR.err); TL++;
+    u64 y0 = 1; for(int i = 0; i < D; i++) y0 = y0*W + (u64)(K/st);
+    k_seed<<<(NPROBE + 256)/256, 256, 0, TS>>>(GR.g, GR.key, GR.word, GR.mask, y0, GR.fr, GR.frsk, GR.acc, eps, pw, GR.probe); TL++;
     TCK(cudaGetLastError());
-    TCK(cudaStreamSynchronize(TS));
     GR.nfr = 1;
+    *probe = GR.probe; *nprobe = NPROBE + 1;
+    return 0;
+}
+extern "C" int sqb_grow_probe(const double *v_dev, const unsigned char *stt_dev){
+    k_probe_check<<<1, GT, 0, TS>>>(v_dev, stt_dev, GR.acc); TL++;
+    TCK(cudaGetLastError());
     return 0;
 }
 extern "C" long sqb_grow_frontier(const sqb_pt_t **pts, const unsigned char **skip){
     *pts = GR.fr; *skip = GR.gs ? GR.frsk : NULL; return GR.nfr;
 }
 
-/* per frontier point: bit 1 mx == K, bit 2 mx == K - st (the outer shells, driver/sumkey.h:236-238) */
-__global__ void k_shell(const sqb_pt_t *fr, long n, geom_t g, unsigned char *cls){
-    for(long i = blockIdx.x*(long)blockDim.x + threadIdx.x; i < n; i += (long)gridDim.x*blockDim.x){
-        int mx = 0; for(int d = 0; d < g.D; d++){ int x = abs((int)fr[i].k[d]); if(x > mx) mx = x; }
-        cls[i] = mx == g.K ? 2 : (mx == g.K - g.st ? 4 : 0);
+/* a frontier point's part of the sums */
+struct fsum_t { sqdd S, x1, x2, u; u64 nq, unres; };
+__device__ __forceinline__ void fsum_add(fsum_t &f, const geom_t &g, const sqb_pt_t *fr, const double *v, const unsigned char *stt,
+                                         const double *uu, double pw, long i){
+    const double x = __dmul_rn(v[i], pw), w = fabs(x);
+    f.S = sqdd_add_d(f.S, x);
+    int mx = 0;                               /* the outer shells, driver/sumkey.h:236-238 */
+    for(int d = 0; d < g.D; d++){ const int y = abs((int)fr[i].k[d]); mx = y > mx ? y : mx; }
+    if(mx == g.K) f.x1 = sqdd_add_d(f.x1, w); else if(mx == g.K - g.st) f.x2 = sqdd_add_d(f.x2, w);
+    const unsigned char s = stt[i];
+    if(s & SQB_FALLBACK){ f.nq++; f.u = sqdd_add_d(f.u, uu[i]); }
+    if(s & SQB_UNRES) f.unres++;
+}
+template<int T> __device__ void fsum_block(fsum_t &f, sqdd *wd, u64 *ws){
+    f.S = block_dd<T>(f.S, wd); f.x1 = block_dd<T>(f.x1, wd); f.x2 = block_dd<T>(f.x2, wd); f.u = block_dd<T>(f.u, wd);
+    f.nq = block_sum<T>(f.nq, ws); f.unres = block_sum<T>(f.unres, ws);
+}
+__device__ __forceinline__ void fsum_into(gacc_t *a, const fsum_t &f){
+    dd_into(a->S, f.S); dd_into(a->x1, f.x1); dd_into(a->x2, f.x2); dd_into(a->u, f.u);
+    a->nq += f.nq; a->unres += f.unres;
+}
+/* per tile of GS_TILE points: the sums, and the running sum's additions in units of its binade */
+__global__ void __launch_bounds__(TG_T) k_gs_tiles(geom_t g, const sqb_pt_t *fr, const double *v, const unsigned char *stt,
+                                                   const double *uu, long n, const gacc_t *acc, gpart_t *part){
+    __shared__ sqdd wd[TG_T/32];
+    __shared__ u64 ws[TG_T/32];
+    const double pw = acc->pw; double inv = 0, u;
+    const bool ok = seq_binade(acc->a, &inv, &u);
+    fsum_t f = {}; u64 q = 0, odd = 0;
+    for(int j = 0; j < GS_TILE/TG_T; j++){
+        const long i = blockIdx.x*(long)GS_TILE + j*TG_T + threadIdx.x;
+        if(i >= n) break;
+        fsum_add(f, g, fr, v, stt, uu, pw, i);
+        const u64 x = ok ? seq_units(__dmul_rn(fabs(v[i]), pw), inv) : SQ_ODD;
+        if(x == SQ_ODD || x >= SQ_ONE53 >> 11) odd = 1; else q += x;      /* GS_TILE = 2^11 terms below 2^53 in all */
+    }
+    fsum_block<TG_T>(f, wd, ws);
+    q = block_sum<TG_T>(q, ws); odd = block_sum<TG_T>(odd, ws);
+    if(threadIdx.x == 0){
+        gpart_t p = {odd ? SQ_ODD : q, {f.S.hi, f.S.lo}, {f.x1.hi, f.x1.lo}, {f.x2.hi, f.x2.lo}, {f.u.hi, f.u.lo}, f.nq, f.unres};
+        part[blockIdx.x] = p;
     }
 }
-/* the frontier's shell classes: the kernel and the copy to pinned memory are queued on the grow's stream
- * without waiting (sqb_grow_shells_async, before the frontier's evaluation, whose results the caller waits
- * for anyway), and sqb_grow_shells_take copies them out after that wait */
-extern "C" int sqb_grow_shells_async(void){
-    if(!GR.nfr) return 0;
-    if(GR.nfr > GR.hclscap){
-        if(GR.hcls) cudaFreeHost(GR.hcls);
-        long c = 1L << 16; while(c < GR.nfr) c <<= 1;
-        TCK(cudaMallocHost(&GR.hcls, c)); GR.hclscap = c;
+/* one CTA: the tiles' sums in order, the running sum and its threshold */
+__global__ void __launch_bounds__(GT) k_gs_total(const double *v, long n, gacc_t *acc, const gpart_t *part, long nb){
+    __shared__ sqdd wd[GT/32];
+    __shared__ u64 ws[GT/32];
+    __shared__ unsigned wm[GT/32];
+    __shared__ seq_sh sh;
+    __shared__ u64 pre_;
+    fsum_t f = {};
+    for(long j = threadIdx.x; j < nb; j += GT){
+        const gpart_t &p = part[j];
+        f.S = f.S + sqdd(p.S[0], p.S[1]); f.x1 = f.x1 + sqdd(p.x1[0], p.x1[1]); f.x2 = f.x2 + sqdd(p.x2[0], p.x2[1]);
+        f.u = f.u + sqdd(p.u[0], p.u[1]); f.nq += p.nq; f.unres += p.unres;
     }
-    k_shell<<<1184, 256, 0, TS>>>(GR.fr, GR.nfr, GR.g, GR.cls); TL++;
-    TCK(cudaGetLastError());
-    TCK(cudaMemcpyAsync(GR.hcls, GR.cls, GR.nfr, cudaMemcpyDeviceToHost, TS));
-    sqb_dev_count_copy(0, GR.nfr);
-    return 0;
-}
-extern "C" void sqb_grow_shells_take(unsigned char *cls_host){
-    if(GR.nfr) memcpy(cls_host, GR.hcls, GR.nfr);
+    fsum_block<GT>(f, wd, ws);
+    const double pw = acc->pw, a0 = acc->a;
+    double a = a0, inv = 0, u = 0;
+    const bool ok = seq_binade(a0, &inv, &u);
+    long tb = 0;
+    while(tb < nb){
+        double i2, u2;
+        if(!ok || !seq_binade(a, &i2, &u2) || u2 != u){ a = seq_sum(a, v, pw, tb*GS_TILE, n, sh); break; }
+        const u64 A0 = (u64)__dmul_rn(a, inv), room = SQ_ONE53 - A0;
+        const long b = tb + threadIdx.x;
+        const u64 q = b < nb ? part[b].q : 0;
+        u64 total, pre = block_scan<GT>(q, room, &total, ws);
+        const bool stop = q == SQ_ODD || pre + q >= room;
+        const unsigned fb = block_min<GT>(stop ? threadIdx.x : 0xFFFFFFFFu, wm);
+        if(fb == 0xFFFFFFFFu){ a = __dmul_rn((double)(A0 + total), u); tb += GT; continue; }
+        if(threadIdx.x == fb) pre_ = pre;
+        __syncthreads();
+        a = __dmul_rn((double)(A0 + pre_), u);
+        const long i0 = (tb + fb)*GS_TILE, i1 = i0 + GS_TILE;
+        a = seq_sum(a, v, pw, i0, i1 < n ? i1 : n, sh);
+        tb += fb + 1;
+        __syncthreads();
+    }
+    if(threadIdx.x == 0){ fsum_into(acc, f); acc->a = a; acc->thr = __dmul_rn(acc->eps, a); }
 }
 
 struct KeepOp {                  /* kept frontier points appended to the keep list, their index to kj */
-    const sqb_pt_t *fr; const double *v; const unsigned char *stt; double thr; int abskip, D;
-    sqb_pt_t *keep; double *kv; long *kj; long base;
-    __device__ bool pred(long i) const { return fabs(v[i]) >= thr; }
-    __device__ void emit(long i, unsigned long long r) const {
+    enum { DROP = 1 };
+    const sqb_pt_t *fr; const double *v; const unsigned char *stt; const gacc_t *acc; int abskip, D;
+    sqb_pt_t *keep; double *kv; long *kj; u64 base;
+    __device__ bool pred(long i) const { return fabs(v[i]) >= acc->thr; }
+    __device__ double weight(long i) const { return __dmul_rn(v[i], acc->pw); }
+    __device__ void emit(long i, u64 r) const {
         sqb_pt_t p; for(int q = 0; q < SQB_MAXD; q++) p.k[q] = 0;
         for(int d = 0; d < D; d++) p.k[d] = fr[i].k[d];
         if(abskip) p.k[SQB_PFLAG] = (stt[i] & SQB_NEAR) ? 0 : 1;
         keep[base + r] = p; kv[base + r] = fabs(v[i]); kj[r] = i;
     }
 };
+/* a small frontier (n <= GS_SMALL) in one CTA: its sums, its threshold, its kept points.  Launch latency bounds a
+ * frontier of this size: five launches a frontier with this kernel, against twelve with the tiles' */
+__global__ void __launch_bounds__(GT) k_gs_small(geom_t g, KeepOp op, const double *uu, long n, gacc_t *acc){
+    __shared__ sqdd wd[GT/32];
+    __shared__ u64 ws[GT/32];
+    __shared__ seq_sh sh;
+    __shared__ double thr_;
+    fsum_t f = {};
+    const double pw = acc->pw;
+    for(int e = 0; e < GS_SMALL/GT; e++){
+        const long i = threadIdx.x + (long)e*GT;
+        if(i < n) fsum_add(f, g, op.fr, op.v, op.stt, uu, pw, i);
+    }
+    fsum_block<GT>(f, wd, ws);
+    const double a = seq_sum(acc->a, op.v, pw, 0, n, sh);
+    if(threadIdx.x == 0){ fsum_into(acc, f); acc->a = a; thr_ = acc->thr = __dmul_rn(acc->eps, a); }
+    __syncthreads();
+    const double thr = thr_;
+    sqdd dr, gs; u64 nd = 0, r = 0;
+    for(int e = 0; e < GS_SMALL/GT && (long)e*GT < n; e++){
+        const long i = threadIdx.x + (long)e*GT;
+        const bool in = i < n, p = in && fabs(op.v[i]) >= thr;
+        if(in && !p){ const double w = op.weight(i); dr = sqdd_add_d(dr, fabs(w)); gs = sqdd_add_d(gs, w); nd++; }
+        u64 t;
+        const u64 x = block_scan<GT>((u64)p, ~0ULL, &t, ws);
+        if(p) op.emit(i, r + x);
+        r += t;
+    }
+    dr = block_dd<GT>(dr, wd); gs = block_dd<GT>(gs, wd); nd = block_sum<GT>(nd, ws);
+    if(threadIdx.x == 0){ dd_into(acc->dr, dr); dd_into(acc->gs, gs); acc->ngs += nd; acc->nk = r; acc->nkeep = op.base + r; }
+}
 
-__global__ void k_claim(geom_t g, const sqb_pt_t *fr, const long *kj, long nk, unsigned long long *key, unsigned *word,
-                        unsigned long long mask, long *qs, unsigned long long *err){
+__global__ void k_claim(geom_t g, const sqb_pt_t *fr, const long *kj, u64 *key, unsigned *word, u64 mask, long *qs, gacc_t *acc){
     const int D2 = 2*g.D;
-    const long nc = nk*D2;
+    const long nc = (long)acc->nk*D2;
     for(long id = blockIdx.x*(long)blockDim.x + threadIdx.x; id < nc; id += (long)gridDim.x*blockDim.x){
         const long j = id/D2; const int c = (int)(id - j*D2), d = c >> 1, sg = (c & 1) ? 1 : -1;
         const signed char *k = fr[kj[j]].k;
         const int kk = k[d] + g.st*sg;
         if(kk > g.K || kk < -g.K){ qs[id] = -1; continue; }
-        const unsigned long long y = key_of(g, k) + (sg > 0 ? g.P[d] : (unsigned long long)0 - g.P[d]);
+        const u64 y = key_of(g, k) + (sg > 0 ? g.P[d] : (u64)0 - g.P[d]);
         int nw; const long q = h_insert(key, mask, y, &nw);
-        if(q < 0){ atomicAdd(err, 1ULL); qs[id] = -1; continue; }
+        if(q < 0){ atomicAdd(&acc->err, 1ULL); qs[id] = -1; continue; }
         qs[id] = q;
         atomicMax(&word[q], CLAIM(id));
     }
 }
 struct WinOp {                   /* winners in id order become the next frontier */
+    enum { DROP = 0 };
     const sqb_pt_t *fr; const long *kj; const long *qs; unsigned *word; const unsigned char *frsk; const unsigned char *stt;
-    sqb_pt_t *nx; unsigned char *nxsk; int D2, st, gs;
+    sqb_pt_t *nx; unsigned char *nxsk; int D2, st, gs; u64 base;
     __device__ bool pred(long id) const { const long q = qs[id]; return q >= 0 && word[q] == CLAIM(id); }
-    __device__ void emit(long id, unsigned long long r) const {
+    __device__ void emit(long id, u64 r) const {
         const long j = id/D2; const int c = (int)(id - j*D2), d = c >> 1, sg = (c & 1) ? 1 : -1;
         const long pi = kj[j];
         sqb_pt_t p = fr[pi];
@@ -325,171 +646,249 @@ struct WinOp {                   /* winners in id order become the next frontier
     }
 };
 
-/* after the host has the frontier's threshold: kept points appended, next frontier built */
-extern "C" int sqb_grow_expand(const double *v_dev, const unsigned char *stt_dev, double thr, long *nkept, long *nnext){
-    const long n = GR.nfr;
+/* the frontier's evaluation (device arrays) in; its sums and kept points added, the next frontier built.  The host
+ * waits once, for the next frontier's size; a frontier with more than 2^22 possible candidates also waits for its
+ * kept count, so that the table and the candidate list grow by what is needed and not by that bound */
+extern "C" int sqb_grow_expand(const double *v_dev, const unsigned char *stt_dev, const double *uu_dev, long *nnext){
+    const long n = GR.nfr; const int D2 = 2*GR.g.D;
     long kc = GR.keepcap, vc = GR.keepcap;
     if(devbuf(&GR.keep, &kc, GR.nkeep + n, GR.nkeep) || devbuf(&GR.kv, &vc, GR.nkeep + n, GR.nkeep)) return -1;
     GR.keepcap = kc;
     if(devbuf(&GR.kj, &GR.kjcap, n, 0)) return -1;
-    KeepOp ko; ko.fr = GR.fr; ko.v = v_dev; ko.stt = stt_dev; ko.thr = thr; ko.abskip = GR.abskip; ko.D = GR.g.D;
-    ko.keep = GR.keep; ko.kv = GR.kv; ko.kj = GR.kj; ko.base = GR.nkeep;
-    long nk = 0;
-    if(compact(ko, n, &nk)) return -1;
-    GR.nkeep += nk; *nkept = nk;
-    const long nc = nk*2*GR.g.D;
+    KeepOp ko; ko.fr = GR.fr; ko.v = v_dev; ko.stt = stt_dev; ko.acc = GR.acc; ko.abskip = GR.abskip; ko.D = GR.g.D;
+    ko.keep = GR.keep; ko.kv = GR.kv; ko.kj = GR.kj; ko.base = (u64)GR.nkeep;
+    if(n <= GS_SMALL){ k_gs_small<<<1, GT, 0, TS>>>(GR.g, ko, uu_dev, n, GR.acc); TL++; }
+    else {
+        const long nb = (n + GS_TILE - 1)/GS_TILE;
+        if(devbuf(&GR.part, &GR.partcap, nb, 0)) return -1;
+        k_gs_tiles<<<(unsigned)nb, TG_T, 0, TS>>>(GR.g, GR.fr, v_dev, stt_dev, uu_dev, n, GR.acc, GR.part);
+        k_gs_total<<<1, GT, 0, TS>>>(v_dev, n, GR.acc, GR.part, nb);
+        TL += 2;
+        if(compact(ko, cnt_t{NULL, 1, n}, &GR.acc->nk, GR.acc, NULL)) return -1;
+    }
+    TCK(cudaGetLastError());
+    long nk = n;
+    if(n*D2 > 1L << 22){
+        TCK(cudaMemcpyAsync(GR.host, GR.acc, sizeof(gacc_t), cudaMemcpyDeviceToHost, TS));
+        TCK(cudaStreamSynchronize(TS));
+        sqb_dev_count_copy(0, sizeof(gacc_t));
+        nk = (long)GR.host->nk;
+    }
+    const long nc = nk*D2;
     if(nc >= 0xFFFFFFF0L){ snprintf(terr, sizeof terr, "grow: %ld candidates exceed the 32-bit claim ids", nc); return -1; }
     if(table_room(nc)) return -1;
     if(devbuf(&GR.qs, &GR.qscap, nc, 0)) return -1;
     if(frontier_room(nc)) return -1;
-    if(nc){ k_claim<<<1184, 256, 0, TS>>>(GR.g, GR.fr, GR.kj, nk, GR.key, GR.word, GR.mask, GR.qs, GR.err); TL++; }
-    TCK(cudaGetLastError());
-    /* the overflow count after the claims (the only writers), read once the next compaction has waited */
-    if(!GR.herr) TCK(cudaMallocHost(&GR.herr, sizeof(unsigned long long)));
-    TCK(cudaMemcpyAsync(GR.herr, GR.err, sizeof(unsigned long long), cudaMemcpyDeviceToHost, TS));
-    WinOp wo; wo.fr = GR.fr; wo.kj = GR.kj; wo.qs = GR.qs; wo.word = GR.word; wo.frsk = GR.frsk; wo.stt = stt_dev;
-    wo.nx = GR.nx; wo.nxsk = GR.nxsk; wo.D2 = 2*GR.g.D; wo.st = GR.g.st; wo.gs = GR.gs;
     long nn = 0;
-    if(compact(wo, nc, &nn)) return -1;
-    GR.nseen += nn;
+    if(nc){
+        const long want = (nc + 255)/256;
+        k_claim<<<(unsigned)(want < 1184 ? want : 1184), 256, 0, TS>>>(GR.g, GR.fr, GR.kj, GR.key, GR.word, GR.mask, GR.qs, GR.acc); TL++;
+        TCK(cudaGetLastError());
+        WinOp wo; wo.fr = GR.fr; wo.kj = GR.kj; wo.qs = GR.qs; wo.word = GR.word; wo.frsk = GR.frsk; wo.stt = stt_dev;
+        wo.nx = GR.nx; wo.nxsk = GR.nxsk; wo.D2 = D2; wo.st = GR.g.st; wo.gs = GR.gs; wo.base = 0;
+        if(compact(wo, cnt_t{&GR.acc->nk, D2, nc}, &GR.acc->nn, GR.acc, GR.host)) return -1;
+        TCK(cudaStreamSynchronize(TS));
+        sqb_dev_count_copy(0, sizeof(gacc_t));
+        nn = (long)GR.host->nn;
+    }
+    GR.nkeep = (long)GR.host->nkeep;
+    GR.nseen += nn; GR.nfrs++;
     { sqb_pt_t *t = GR.fr; GR.fr = GR.nx; GR.nx = t; unsigned char *q = GR.frsk; GR.frsk = GR.nxsk; GR.nxsk = q; }
     GR.nfr = nn; *nnext = nn;
-    if(nc <= 0) TCK(cudaStreamSynchronize(TS));          /* no compaction waited for the copy */
-    if(*GR.herr){ snprintf(terr, sizeof terr, "grow: hash table overflow"); return -1; }
+    if(GR.host->err){ snprintf(terr, sizeof terr, "grow: hash table overflow"); return -1; }
     return 0;
 }
 
-/* kept |f| values in keep order (host), for the final threshold's dropped weight */
-extern "C" int sqb_grow_kv(double *kv_host, long n){
-    TCK(cudaMemcpyAsync(kv_host, GR.kv, n*sizeof(double), cudaMemcpyDeviceToHost, TS));
+/* the running sum on its own (checks): a + |v[0]| pw + |v[1]| pw + ..., each addition rounded, for n values on the
+ * device, through the small frontiers' route (tiles = 0) or the tiles' */
+__global__ void __launch_bounds__(GT) k_seq_check(const double *v, long n, gacc_t *acc){
+    __shared__ seq_sh sh;
+    const double a = seq_sum(acc->a, v, acc->pw, 0, n, sh);
+    if(threadIdx.x == 0) acc->a = a;
+}
+extern "C" int sqb_running_sum(const double *v_dev, long n, double a, double pw, int tiles, void *stream, double *out){
+    TS = (cudaStream_t)stream;
+    const long nb = (n + GS_TILE - 1)/GS_TILE;
+    gacc_t h; memset(&h, 0, sizeof h); h.a = a; h.pw = pw;
+    gacc_t *acc; gpart_t *part; char *pts;
+    const size_t pb = (size_t)(n + 1)*(sizeof(sqb_pt_t) + 1);
+    TCK(DMALLOC(&acc, sizeof h)); TCK(DMALLOC(&part, (nb + 1)*sizeof(gpart_t))); TCK(DMALLOC(&pts, pb));
+    TCK(cudaMemcpyAsync(acc, &h, sizeof h, cudaMemcpyHostToDevice, TS));
+    TCK(cudaMemsetAsync(pts, 0, pb, TS));
+    geom_t g; memset(&g, 0, sizeof g); g.D = 1; g.K = 1; g.st = 1; g.W = 3;
+    if(!tiles) k_seq_check<<<1, GT, 0, TS>>>(v_dev, n, acc);
+    else if(n > 0){
+        k_gs_tiles<<<(unsigned)nb, TG_T, 0, TS>>>(g, (const sqb_pt_t*)pts, v_dev, (const unsigned char*)pts + (n + 1)*sizeof(sqb_pt_t), v_dev, n, acc, part);
+        k_gs_total<<<1, GT, 0, TS>>>(v_dev, n, acc, part, nb);
+    }
+    TCK(cudaGetLastError());
+    TCK(cudaMemcpyAsync(&h, acc, sizeof h, cudaMemcpyDeviceToHost, TS));
     TCK(cudaStreamSynchronize(TS));
-    sqb_dev_count_copy(0, n*sizeof(double));
+    DFREE(acc); DFREE(part); DFREE(pts);
+    *out = h.a;
     return 0;
 }
+
+/* the zero probe's answer (valid after the first frontier's expansion) */
+extern "C" int sqb_grow_probe_zero(long *unres){ *unres = (long)GR.host->punres; return GR.host->nz == 0; }
 
 struct RethOp {
-    const sqb_pt_t *keep; const double *kv; double thr; sqb_pt_t *out; double *okv;
-    __device__ bool pred(long i) const { return kv[i] >= thr; }
-    __device__ void emit(long i, unsigned long long r) const { out[r] = keep[i]; okv[r] = kv[i]; }
+    enum { DROP = 1 };
+    const sqb_pt_t *keep; const double *kv; const gacc_t *acc; sqb_pt_t *out; double *okv; u64 base;
+    __device__ bool pred(long i) const { return kv[i] >= acc->thr; }
+    __device__ double weight(long i) const { return __dmul_rn(kv[i], acc->pw); }
+    __device__ void emit(long i, u64 r) const { out[r] = keep[i]; okv[r] = kv[i]; }
 };
 
-/* shadow tiers: breadth-first from z = 0 through kept points with |f| >= lim (driver/sumkey.h:402-444) */
-__global__ void k_index(geom_t g, const sqb_pt_t *keep, long m, unsigned long long *key, unsigned *word,
-                        unsigned long long mask, unsigned long long *err){
+/* shadow tiers: breadth-first from z = 0 through kept points with |f| >= 10 thr (tier 1) and 100 thr (tier 2)
+ * (driver/sumkey.h:402-444), both at once: a point of tier t raises a neighbour to the highest tier up to t
+ * whose bound the neighbour's value meets, and a raised point goes (again) into the next step's list */
+__global__ void k_index(geom_t g, const sqb_pt_t *keep, const u64 *key, unsigned *word, u64 mask, gacc_t *acc){
+    const long m = (long)acc->m;
     for(long i = blockIdx.x*(long)blockDim.x + threadIdx.x; i < m; i += (long)gridDim.x*blockDim.x){
-        int nw; long q = h_insert(key, mask, key_of(g, keep[i].k), &nw);
-        if(q < 0){ atomicAdd(err, 1ULL); continue; }
+        const long q = h_find(key, mask, key_of(g, keep[i].k));
+        if(q < 0){ atomicAdd(&acc->err, 1ULL); continue; }
         word[q] = (unsigned)i;
     }
 }
-__global__ void k_tier_seed(geom_t g, const unsigned long long *key, const unsigned *word, unsigned long long mask,
-                            const double *kv, double lim, int t, unsigned *tr, long *cu, unsigned long long *ncu){
-    unsigned long long y = 1; for(int i = 0; i < g.D; i++) y = y*g.W + (unsigned long long)(g.K/g.st);
-    long q = h_find(key, mask, y);
-    *ncu = 0;
-    if(q < 0) return;
-    long i = word[q];
-    if(kv[i] >= lim){ atomicMax(&tr[i], (unsigned)t); cu[0] = i; *ncu = 1; }
+__device__ __forceinline__ unsigned tier_of(double f, double thr){ return (f >= 10*thr) + (f >= 100*thr); }
+__global__ void k_tier_seed(geom_t g, const u64 *key, const unsigned *word, u64 mask, const double *kv, const gacc_t *acc,
+                            unsigned *tr, long *cu, u64 *cnt){
+    u64 y = 1; for(int i = 0; i < g.D; i++) y = y*g.W + (u64)(g.K >> g.sh);
+    const long q = h_find(key, mask, y);
+    cnt[0] = cnt[1] = cnt[2] = 0;
+    if(q < 0 || word[q] == SEEN) return;
+    const long i = word[q];
+    const unsigned t = tier_of(kv[i], acc->thr);
+    if(t){ tr[i] = t; cu[0] = i; cnt[0] = 1; }
 }
-__global__ void k_tier_step(geom_t g, const sqb_pt_t *keep, const unsigned long long *key, const unsigned *word,
-                            unsigned long long mask, const double *kv, double lim, int t, unsigned *tr,
-                            const long *cu, const unsigned long long *ncu, long *nw, unsigned long long *nnw){
+__device__ __forceinline__ void tier_edge(const geom_t &g, const sqb_pt_t *keep, const u64 *key, const unsigned *word, u64 mask,
+                                          const double *kv, double thr, unsigned *tr, long i, int c, long *nw, u64 *nnw){
+    const int d = c >> 1, sg = (c & 1) ? 1 : -1;
+    const int kk = keep[i].k[d] + g.st*sg;
+    if(kk > g.K || kk < -g.K) return;
+    const u64 y = key_of(g, keep[i].k) + (sg > 0 ? g.P[d] : (u64)0 - g.P[d]);
+    const long q = h_find(key, mask, y);
+    if(q < 0 || word[q] == SEEN) return;
+    const long j = word[q];
+    const unsigned t = min(*(volatile unsigned*)&tr[i], tier_of(kv[j], thr));
+    if(t && *(volatile unsigned*)&tr[j] < t && atomicMax(&tr[j], t) < t) nw[atomicAdd(nnw, 1ULL)] = j;
+}
+__global__ void k_tier_step(geom_t g, const sqb_pt_t *keep, const u64 *key, const unsigned *word, u64 mask, const double *kv,
+                            const gacc_t *acc, unsigned *tr, const long *cu, long *nw, u64 *cnt, int s){
     const int D2 = 2*g.D;
-    const long nc = (long)*ncu;          /* the frontier's size, written by the step (or seed) before */
-    for(long x = blockIdx.x*(long)blockDim.x + threadIdx.x; x < nc*D2; x += (long)gridDim.x*blockDim.x){
-        const long i = cu[x/D2]; const int c = (int)(x % D2), d = c >> 1, sg = (c & 1) ? 1 : -1;
-        const int kk = keep[i].k[d] + g.st*sg;
-        if(kk > g.K || kk < -g.K) continue;
-        const unsigned long long y = key_of(g, keep[i].k) + (sg > 0 ? g.P[d] : (unsigned long long)0 - g.P[d]);
-        const long q = h_find(key, mask, y);
-        if(q < 0) continue;
-        const long j = word[q];
-        if(kv[j] >= lim && atomicMax(&tr[j], (unsigned)t) < (unsigned)t) nw[atomicAdd(nnw, 1ULL)] = j;
+    const long nc = (long)cnt[s % 3]*D2;      /* this step's list, written by the step (or seed) before */
+    if(blockIdx.x == 0 && threadIdx.x == 0) cnt[(s + 2) % 3] = 0;
+    for(long x = blockIdx.x*(long)blockDim.x + threadIdx.x; x < nc; x += (long)gridDim.x*blockDim.x)
+        tier_edge(g, keep, key, word, mask, kv, acc->thr, tr, cu[x/D2], (int)(x % D2), nw, &cnt[(s + 1) % 3]);
+}
+/* what a long way round leaves after the steps the host launched: one CTA, step after step to the end (every step
+ * raises at least one point, at most twice) */
+__global__ void __launch_bounds__(GT) k_tier_rest(geom_t g, const sqb_pt_t *keep, const u64 *key, const unsigned *word, u64 mask,
+                                                  const double *kv, const gacc_t *acc, unsigned *tr, long *cu, long *nw, u64 *cnt, int s){
+    const int D2 = 2*g.D;
+    const long bound = 2*(long)acc->m + 1;
+    for(long it = 0; it < bound; it++, s++){
+        const long nc = (long)*(volatile u64*)&cnt[s % 3]*D2;
+        if(nc == 0) break;
+        if(threadIdx.x == 0) cnt[(s + 2) % 3] = 0;
+        __syncthreads();
+        for(long x = threadIdx.x; x < nc; x += GT)
+            tier_edge(g, keep, key, word, mask, kv, acc->thr, tr, cu[x/D2], (int)(x % D2), nw, &cnt[(s + 1) % 3]);
+        __threadfence();
+        __syncthreads();
+        long *t = cu; cu = nw; nw = t;
     }
 }
-__global__ void k_tier_apply(sqb_pt_t *keep, const unsigned *tr, long m){
+__global__ void k_tier_apply(sqb_pt_t *keep, const unsigned *tr, const gacc_t *acc){
+    const long m = (long)acc->m;
     for(long i = blockIdx.x*(long)blockDim.x + threadIdx.x; i < m; i += (long)gridDim.x*blockDim.x)
         keep[i].k[SQB_PFLAG] = (signed char)((keep[i].k[SQB_PFLAG] & 1) | (tr[i] << 1));
 }
+/* a grid that covers n items, at most 1184 CTAs of 256 */
+static unsigned grid256(long n){ const long w = (n + 255)/256; return (unsigned)(w < 1 ? 1 : w < 1184 ? w : 1184); }
 
-/* the final threshold and the tiers; *m = kept points left; the keep list stays on the device */
-extern "C" int sqb_grow_finish(double thr, int tiers, long *m_out){
+/* the final threshold (eps times the whole sum) and the tiers; the kept list stays on the device, its length there
+ * too (GR.nkeep bounds it until a wait) */
+extern "C" int sqb_grow_finish(int tiers){
     sqb_pt_t *out; double *okv; const long n = GR.nkeep;
     TCK(DMALLOC(&out, (n ? n : 1)*sizeof(sqb_pt_t))); TCK(DMALLOC(&okv, (n ? n : 1)*sizeof(double)));
-    RethOp ro; ro.keep = GR.keep; ro.kv = GR.kv; ro.thr = thr; ro.out = out; ro.okv = okv;
-    long m = 0;
-    if(compact(ro, n, &m)) return -1;
-    DFREE(GR.keep); DFREE(GR.kv); GR.keep = out; GR.kv = okv; GR.keepcap = n ? n : 1; GR.nkeep = m;
-    *m_out = m;
-    if(!tiers || !m) return 0;
-    long cap = 1L << 20; while(cap < 2*m) cap <<= 1;
-    unsigned long long *key; unsigned *word, *tr; long *cu, *nw; unsigned long long *cnt;
-    TCK(DMALLOC(&key, cap*sizeof(unsigned long long))); TCK(DMALLOC(&word, cap*sizeof(unsigned)));
-    TCK(DMALLOC(&tr, m*sizeof(unsigned))); TCK(DMALLOC(&cu, m*sizeof(long))); TCK(DMALLOC(&nw, m*sizeof(long)));
-    TCK(DMALLOC(&cnt, 2*sizeof(unsigned long long)));
-    TCK(cudaMemsetAsync(key, 0, cap*sizeof(unsigned long long), TS)); TCK(cudaMemsetAsync(tr, 0, m*sizeof(unsigned), TS));
-    k_index<<<1184, 256, 0, TS>>>(GR.g, GR.keep, m, key, word, (unsigned long long)(cap - 1), GR.err); TL++;
-    /* breadth-first steps read the frontier's size on the device, so the host checks for the end only
-     * every TSTEPS steps (steps after the end find an empty frontier and do nothing) */
-    const int TSTEPS = 8;
-    for(int t = 1; t <= 2; t++){
-        const double lim = (t == 1 ? 10 : 100)*thr;
-        unsigned long long *ca = cnt, *cb = cnt + 1;
-        k_tier_seed<<<1, 1, 0, TS>>>(GR.g, key, word, (unsigned long long)(cap - 1), GR.kv, lim, t, tr, cu, ca); TL++;
-        for(;;){
-            for(int s = 0; s < TSTEPS; s++){
-                TCK(cudaMemsetAsync(cb, 0, sizeof(unsigned long long), TS));
-                k_tier_step<<<1184, 256, 0, TS>>>(GR.g, GR.keep, key, word, (unsigned long long)(cap - 1), GR.kv, lim, t, tr,
-                                                  cu, ca, nw, cb); TL++;
-                TCK(cudaGetLastError());
-                long *x = cu; cu = nw; nw = x;
-                unsigned long long *y = ca; ca = cb; cb = y;
-            }
-            unsigned long long nc = 0;
-            TCK(cudaMemcpyAsync(&nc, ca, sizeof nc, cudaMemcpyDeviceToHost, TS)); TCK(cudaStreamSynchronize(TS));
-            if(!nc) break;
-        }
+    if(n){
+        RethOp ro; ro.keep = GR.keep; ro.kv = GR.kv; ro.acc = GR.acc; ro.out = out; ro.okv = okv; ro.base = 0;
+        if(compact(ro, cnt_t{NULL, 1, n}, &GR.acc->m, GR.acc, NULL)) return -1;
     }
-    k_tier_apply<<<1184, 256, 0, TS>>>(GR.keep, tr, m); TL++;
+    DFREE(GR.keep); DFREE(GR.kv); GR.keep = out; GR.kv = okv; GR.keepcap = n ? n : 1;
+    if(!tiers || !n) return 0;
+    unsigned *tr; long *cu, *nw; u64 *cnt;
+    TCK(DMALLOC(&tr, n*sizeof(unsigned))); TCK(DMALLOC(&cu, 2*n*sizeof(long))); TCK(DMALLOC(&nw, 2*n*sizeof(long)));
+    TCK(DMALLOC(&cnt, 3*sizeof(u64)));
+    TCK(cudaMemsetAsync(tr, 0, n*sizeof(unsigned), TS));
+    k_index<<<grid256(n), 256, 0, TS>>>(GR.g, GR.keep, GR.key, GR.word, GR.mask, GR.acc);
+    k_tier_seed<<<1, 1, 0, TS>>>(GR.g, GR.key, GR.word, GR.mask, GR.kv, GR.acc, tr, cu, cnt);
+    TL += 2;
+    /* the points lie within as many steps of z = 0 as the grow had frontiers; a way through the larger values
+     * alone may be longer, and the rest kernel walks it */
+    int s = 0;
+    for(; s < GR.nfrs; s++){
+        k_tier_step<<<grid256(n), 256, 0, TS>>>(GR.g, GR.keep, GR.key, GR.word, GR.mask, GR.kv, GR.acc, tr, cu, nw, cnt, s); TL++;
+        long *x = cu; cu = nw; nw = x;
+    }
+    k_tier_rest<<<1, GT, 0, TS>>>(GR.g, GR.keep, GR.key, GR.word, GR.mask, GR.kv, GR.acc, tr, cu, nw, cnt, s);
+    k_tier_apply<<<grid256(n), 256, 0, TS>>>(GR.keep, tr, GR.acc);
+    TL += 2;
     TCK(cudaGetLastError());
+    DFREE(tr); DFREE(cu); DFREE(nw); DFREE(cnt);
+    return 0;
+}
+/* waits and reads the record: the grow's sums (S, a, x1, x2, dropped weight, signed sum below the threshold) and counts */
+extern "C" int sqb_grow_sums(sqb_grow_sums_t *r){
+    TCK(cudaMemcpyAsync(GR.host, GR.acc, sizeof(gacc_t), cudaMemcpyDeviceToHost, TS));
     TCK(cudaStreamSynchronize(TS));
-    DFREE(key); DFREE(word); DFREE(tr); DFREE(cu); DFREE(nw); DFREE(cnt);
+    sqb_dev_count_copy(0, sizeof(gacc_t));
+    const gacc_t &h = *GR.host;
+    if(h.err){ snprintf(terr, sizeof terr, "grow: %llu table lookups failed", h.err); return -1; }
+    r->S = h.S[0] + h.S[1]; r->a = h.a; r->x1 = h.x1[0] + h.x1[1]; r->x2 = h.x2[0] + h.x2[1]; r->drop = h.dr[0] + h.dr[1];
+    r->gshs = h.gs[0] + h.gs[1]; r->gshn = (long)h.ngs; r->u = h.u[0] + h.u[1]; r->nq = (long)h.nq; r->unres = (long)h.unres;
+    r->kept = (long)h.m; r->cells = (long)h.ncell;
+    GR.nkeep = (long)h.m;
     return 0;
 }
 
 /* ------------------------------------------- dilation -------------------------------------------- */
-__global__ void k_dil_insert(geom_t g, const sqb_pt_t *cur, long n0, unsigned long long *key, unsigned *skb, unsigned *trm,
-                             unsigned long long mask, unsigned long long *cnt, unsigned long long *err){
+/* every kept cell and its in-box axis neighbours marked in the seen table, which holds them all: bit 3 present,
+ * bit 0 some cell does not skip (the skip bits' AND), bits 1 and 2 the tier's maximum in unary (driver/sumkey.h:41-44) */
+__global__ void k_dil_mark(geom_t g, const sqb_pt_t *cur, const u64 *key, unsigned *word, u64 mask, gacc_t *acc){
     const int C = 2*g.D + 1;
-    for(long x = blockIdx.x*(long)blockDim.x + threadIdx.x; x < n0*C; x += (long)gridDim.x*blockDim.x){
+    const long n = (long)acc->m*C;
+    for(long x = blockIdx.x*(long)blockDim.x + threadIdx.x; x < n; x += (long)gridDim.x*blockDim.x){
         const long q0 = x/C; const int c = (int)(x - q0*C);
         const signed char *k = cur[q0].k; const int fl = k[SQB_PFLAG];
-        unsigned long long y = key_of(g, k);
+        u64 y = key_of(g, k);
         if(c > 0){
             const int j = (c - 1) >> 1, sg = ((c - 1) & 1) ? 1 : -1, kk = k[j] + g.st*sg;
             if(kk > g.K || kk < -g.K) continue;
             y = sg > 0 ? y + g.P[j] : y - g.P[j];
         }
-        int nw; const long q = h_insert(key, mask, y, &nw);
-        if(q < 0){ atomicAdd(err, 1ULL); continue; }
-        if(nw) atomicAdd(cnt, 1ULL);
-        if(!(fl & 1)) atomicAnd(&skb[q], 0u);
-        atomicMax(&trm[q], (unsigned)(fl >> 1));
+        const long q = h_find(key, mask, y);
+        if(q < 0){ atomicAdd(&acc->err, 1ULL); continue; }
+        const unsigned b = 8u | ((fl & 1) ? 0 : 1) | (((fl >> 1) & 3) >= 1 ? 2 : 0) | (((fl >> 1) & 3) >= 2 ? 4 : 0);
+        if((*(volatile unsigned*)&word[q] & b) != b) atomicOr(&word[q], b);
     }
 }
 struct SlotOp {
-    const unsigned long long *key; unsigned long long *out;
-    __device__ bool pred(long i) const { return key[i] != 0; }
-    __device__ void emit(long i, unsigned long long r) const { out[r] = key[i]; }
+    enum { DROP = 0 };
+    const u64 *key; const unsigned *word; u64 *out; u64 base;
+    __device__ bool pred(long i) const { return word[i] != 0; }
+    __device__ void emit(long i, u64 r) const { out[r] = key[i]; }
 };
-__global__ void k_dil_decode(geom_t g, const unsigned long long *U, long m, const unsigned long long *key, const unsigned *skb,
-                             const unsigned *trm, unsigned long long mask, sqb_pt_t *out){
+__global__ void k_dil_decode(geom_t g, const u64 *U, const u64 *key, const unsigned *word, u64 mask, sqb_pt_t *out, const gacc_t *acc){
+    const long m = (long)acc->ncell;
     for(long j = blockIdx.x*(long)blockDim.x + threadIdx.x; j < m; j += (long)gridDim.x*blockDim.x){
-        unsigned long long y = U[j]; sqb_pt_t p;
+        u64 y = U[j]; sqb_pt_t p;
         for(int i = 0; i < SQB_MAXD; i++) p.k[i] = 0;
-        for(int i = g.D - 1; i >= 0; i--){ p.k[i] = (signed char)(((int)(y % g.W) - g.K/g.st)*g.st); y /= g.W; }
+        for(int i = g.D - 1; i >= 0; i--){ p.k[i] = (signed char)((int)(y % g.W)*g.st - g.K); y /= g.W; }
         const long q = h_find(key, mask, U[j]);
-        if(q >= 0) p.k[SQB_PFLAG] = (signed char)((skb[q] & 1) | (trm[q] << 1));
+        if(q >= 0){ const unsigned b = word[q]; p.k[SQB_PFLAG] = (signed char)(((b & 1) ? 0 : 1) | ((b & 4) ? 4 : (b & 2))); }
         out[j] = p;
     }
 }
@@ -498,34 +897,36 @@ __global__ void k_dil_decode(geom_t g, const unsigned long long *U, long m, cons
 #define RS_T 256
 #define RS_I 16
 #define RS_TILE (RS_T*RS_I)
-__global__ void __launch_bounds__(RS_T) k_rs_hist(const unsigned long long *a, long n, int sh, unsigned *hist, long nblk){
+__global__ void __launch_bounds__(RS_T) k_rs_hist(const u64 *a, cnt_t cn, int sh, unsigned *hist, long nblk){
     __shared__ unsigned h[256];
+    const long n = cnt_of(cn);
     h[threadIdx.x] = 0; __syncthreads();
     const long t0 = blockIdx.x*(long)RS_TILE;
     for(int j = 0; j < RS_I; j++){ long i = t0 + j*RS_T + threadIdx.x; if(i < n) atomicAdd(&h[(a[i] >> sh) & 255], 1u); }
     __syncthreads();
     hist[(long)threadIdx.x*nblk + blockIdx.x] = h[threadIdx.x];
 }
-__global__ void __launch_bounds__(RS_T) k_rs_scatter(const unsigned long long *a, unsigned long long *b, long n, int sh,
-                                                     const unsigned long long *off, long nblk){
-    __shared__ unsigned long long base[256];
+__global__ void __launch_bounds__(RS_T) k_rs_scatter(const u64 *a, u64 *b, cnt_t cn, int sh, const u64 *off, long nblk){
+    __shared__ u64 base[256];
     __shared__ unsigned wc[RS_T/32][256];
+    const long n = cnt_of(cn);
     base[threadIdx.x] = off[(long)threadIdx.x*nblk + blockIdx.x];
     const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
     const long t0 = blockIdx.x*(long)RS_TILE;
     for(int j = 0; j < RS_I; j++){
+        if(t0 + j*RS_T >= n) break;
         for(int q = 0; q < RS_T/32; q++) wc[q][threadIdx.x] = 0;
         __syncthreads();
         const long i = t0 + j*RS_T + threadIdx.x;
         const bool in = i < n;
-        const unsigned long long x = in ? a[i] : 0;
+        const u64 x = in ? a[i] : 0;
         const unsigned dg = in ? (unsigned)((x >> sh) & 255) : 256u + l;   /* out-of-range lanes never match */
         const unsigned peers = __match_any_sync(0xffffffffu, dg);
         const unsigned lt = peers & ((1u << l) - 1);
         if(in && lt == 0) wc[w][dg] = __popc(peers);
         __syncthreads();
         if(in){
-            unsigned long long o = base[dg] + __popc(lt);
+            u64 o = base[dg] + __popc(lt);
             for(int q = 0; q < w; q++) o += wc[q][dg];
             b[o] = x;
         }
@@ -535,70 +936,54 @@ __global__ void __launch_bounds__(RS_T) k_rs_scatter(const unsigned long long *a
         __syncthreads();
     }
 }
-static int radix_sort(unsigned long long **a, unsigned long long **b, long n, int nbits){
-    if(n <= 1) return 0;
-    const long nblk = (n + RS_TILE - 1)/RS_TILE;
-    unsigned *hist; unsigned long long *off, *tot;
-    TCK(DMALLOC(&hist, 256*nblk*sizeof(unsigned))); TCK(DMALLOC(&off, 256*nblk*sizeof(unsigned long long)));
-    TCK(DMALLOC(&tot, sizeof(unsigned long long)));
+static int radix_sort(u64 **a, u64 **b, cnt_t cn, int nbits){
+    if(cn.max <= 1) return 0;
+    const long nblk = (cn.max + RS_TILE - 1)/RS_TILE;
+    unsigned *hist; u64 *off;
+    TCK(DMALLOC(&hist, 256*nblk*sizeof(unsigned))); TCK(DMALLOC(&off, 256*nblk*sizeof(u64)));
     for(int sh = 0; sh < nbits; sh += 8){
-        k_rs_hist<<<(unsigned)nblk, RS_T, 0, TS>>>(*a, n, sh, hist, nblk); TL++;
-        k_scan<<<1, 256, 0, TS>>>(hist, 256*nblk, off, tot); TL++;
-        k_rs_scatter<<<(unsigned)nblk, RS_T, 0, TS>>>(*a, *b, n, sh, off, nblk); TL++;
+        k_rs_hist<<<(unsigned)nblk, RS_T, 0, TS>>>(*a, cn, sh, hist, nblk);
+        k_scan<<<1, GT, 0, TS>>>(hist, 256*nblk, off, NULL);
+        k_rs_scatter<<<(unsigned)nblk, RS_T, 0, TS>>>(*a, *b, cn, sh, off, nblk);
+        TL += 3;
         TCK(cudaGetLastError());
-        unsigned long long *t = *a; *a = *b; *b = t;
+        u64 *t = *a; *a = *b; *b = t;
     }
-    TCK(cudaStreamSynchronize(TS));
-    DFREE(hist); DFREE(off); DFREE(tot);
+    DFREE(hist); DFREE(off);
     return 0;
 }
 extern "C" int sqb_radix_sort_u64(unsigned long long *keys_dev, long n, int nbits, void *stream){
     TS = (cudaStream_t)stream;
-    unsigned long long *b, *a = keys_dev;
-    TCK(DMALLOC(&b, (n ? n : 1)*sizeof(unsigned long long)));
-    if(radix_sort(&a, &b, n, nbits)) return -1;
-    if(a != keys_dev){ TCK(cudaMemcpy(keys_dev, a, n*sizeof(unsigned long long), cudaMemcpyDeviceToDevice)); DFREE(a); }
+    u64 *b, *a = keys_dev;
+    TCK(DMALLOC(&b, (n ? n : 1)*sizeof(u64)));
+    if(radix_sort(&a, &b, cnt_t{NULL, 1, n}, nbits)) return -1;
+    if(a != keys_dev){ TCK(cudaMemcpyAsync(keys_dev, a, n*sizeof(u64), cudaMemcpyDeviceToDevice, TS)); DFREE(a); }
     else DFREE(b);
+    TCK(cudaStreamSynchronize(TS));
     return 0;
 }
 
-/* the kept list (from sqb_grow_finish) and its axis neighbours at the top step, sorted, flags merged;
- * *out is a device list of *n cells owned by the caller (sqb_dev_free) */
-extern "C" int sqb_grow_dilate(int nbits, sqb_pt_t **out, long *n){
-    const long n0 = GR.nkeep;
-    *out = NULL; *n = 0;
-    if(!n0) return 0;
-    long cap = 1L << 20; while(cap < 4*n0) cap <<= 1;
-    for(;;){
-        unsigned long long *key, *cnt; unsigned *skb, *trm;
-        TCK(DMALLOC(&key, cap*sizeof(unsigned long long))); TCK(DMALLOC(&skb, cap*sizeof(unsigned)));
-        TCK(DMALLOC(&trm, cap*sizeof(unsigned))); TCK(DMALLOC(&cnt, sizeof(unsigned long long)));
-        TCK(cudaMemsetAsync(key, 0, cap*sizeof(unsigned long long), TS)); TCK(cudaMemsetAsync(skb, 0xff, cap*sizeof(unsigned), TS));
-        TCK(cudaMemsetAsync(trm, 0, cap*sizeof(unsigned), TS)); TCK(cudaMemsetAsync(cnt, 0, sizeof(unsigned long long), TS));
-        TCK(cudaMemsetAsync(GR.err, 0, sizeof(unsigned long long), TS));
-        k_dil_insert<<<1184, 256, 0, TS>>>(GR.g, GR.keep, n0, key, skb, trm, (unsigned long long)(cap - 1), cnt, GR.err); TL++;
-        TCK(cudaGetLastError());
-        unsigned long long m = 0, e = 0;
-        TCK(cudaMemcpyAsync(&m, cnt, sizeof m, cudaMemcpyDeviceToHost, TS));
-        TCK(cudaMemcpyAsync(&e, GR.err, sizeof e, cudaMemcpyDeviceToHost, TS));
-        TCK(cudaStreamSynchronize(TS));
-        if(e || (double)m > 0.75*cap){ DFREE(key); DFREE(skb); DFREE(trm); DFREE(cnt); cap *= 2; continue; }
-        unsigned long long *U, *T;
-        TCK(DMALLOC(&U, m*sizeof(unsigned long long))); TCK(DMALLOC(&T, m*sizeof(unsigned long long)));
-        SlotOp so; so.key = key; so.out = U; long mm = 0;
-        if(compact(so, cap, &mm)) return -1;
-        if(radix_sort(&U, &T, mm, nbits)) return -1;
-        sqb_pt_t *o; TCK(DMALLOC(&o, mm*sizeof(sqb_pt_t)));
-        k_dil_decode<<<1184, 256, 0, TS>>>(GR.g, U, mm, key, skb, trm, (unsigned long long)(cap - 1), o); TL++;
-        TCK(cudaGetLastError());
-        TCK(cudaStreamSynchronize(TS));
-        DFREE(U); DFREE(T); DFREE(key); DFREE(skb); DFREE(trm); DFREE(cnt);
-        *out = o; *n = mm;
-        return 0;
-    }
+/* the kept list (from sqb_grow_finish) and its axis neighbours at the top step, sorted, flags merged; *out is a device
+ * list owned by the caller (sqb_dev_free), its length in sqb_grow_sums' record */
+extern "C" int sqb_grow_dilate(int nbits, sqb_pt_t **out){
+    *out = NULL;
+    if(!GR.nkeep) return 0;
+    const long cap = (long)GR.mask + 1, n = GR.nseen;
+    u64 *U, *T; sqb_pt_t *o;
+    TCK(DMALLOC(&U, n*sizeof(u64))); TCK(DMALLOC(&T, n*sizeof(u64))); TCK(DMALLOC(&o, n*sizeof(sqb_pt_t)));
+    TCK(cudaMemsetAsync(GR.word, 0, cap*sizeof(unsigned), TS));
+    k_dil_mark<<<grid256(GR.nkeep*(2*GR.g.D + 1)), 256, 0, TS>>>(GR.g, GR.keep, GR.key, GR.word, GR.mask, GR.acc); TL++;
+    SlotOp so; so.key = GR.key; so.word = GR.word; so.out = U; so.base = 0;
+    if(compact(so, cnt_t{NULL, 1, cap}, &GR.acc->ncell, GR.acc, NULL)) return -1;
+    if(radix_sort(&U, &T, cnt_t{&GR.acc->ncell, 1, n}, nbits)) return -1;
+    k_dil_decode<<<grid256(n), 256, 0, TS>>>(GR.g, U, GR.key, GR.word, GR.mask, o, GR.acc); TL++;
+    TCK(cudaGetLastError());
+    DFREE(U); DFREE(T);
+    *out = o;
+    return 0;
 }
 
-/* the kept list after sqb_grow_finish (tiers in the flag byte), on the device */
+/* the kept list after sqb_grow_finish (tiers in the flag byte), on the device; its length after a wait (sqb_grow_sums) */
 extern "C" void sqb_grow_kept(const sqb_pt_t **keep, long *m){ *keep = GR.keep; *m = GR.nkeep; }
 
 /* top = 0 keeps no list; the kept list is released with the table */
