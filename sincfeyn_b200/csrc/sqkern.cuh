@@ -601,11 +601,12 @@ __global__ void __launch_bounds__(SQB_BLOCK) sqb_k_dd(const __grid_constant__ sq
     extern __shared__ double sqb_sm[];
     __shared__ sqb_inst_t sI[SQB_MAXINST];
     const sqb_eval_t &e = a.e;
-    sqb_tables(e, sqb_sm, sI);
     const bool multi = e.ninst > 0;
     long n;
     if(a.all) n = multi ? e.ntile*SQB_TILE : (e.cells ? (e.n << D) : e.n);
     else { n = (long)*a.nlist; if(n > a.listcap) n = a.listcap; }
+    if(blockIdx.x*(long)blockDim.x >= n) return;      /* the grid is for a full queue: most queues are short */
+    sqb_tables(e, sqb_sm, sI);
     for(long j = blockIdx.x*(long)blockDim.x + threadIdx.x; j < n; j += (long)gridDim.x*blockDim.x){
         const long i = a.all ? j : a.list[j];
         const int k = multi ? sqb_inst_at(e, i) : 0;
