@@ -46,7 +46,10 @@
 #define NA_BO    (NA_BK + NA_UP(4L*NA_TILES))        /* unsigned long long offset per tile */
 #define NA_ACC   (NA_BO + NA_UP(8L*NA_TILES))        /* sqb_acc_t */
 #define NA_MISC  (NA_ACC + NA_UP(sizeof(sqb_acc_t))) /* base, fallback count */
-#define NA_END   (NA_MISC + 256L)
+#define NA_AX    (NA_MISC + 256L)                    /* axis tables (sqb_graph_t axis), FP64 then double-double, where they
+                                                         fit: about 130,000 bytes are left, 2,000 (axis, k) entries of
+                                                         eight doubles */
+#define NA_END   NA_AX
 static_assert(NA_END <= SQB_NOALLOC_BYTES, "the scratch layout must fit the array the header states");
 static_assert(2*255*sizeof(double) <= 4096, "the lattice tables (|k| <= 127) must fit their slot");
 static_assert(sizeof(sqb_acc_t) <= 256 && 2*sizeof(unsigned long long) <= 256, "accumulator slots");
@@ -108,13 +111,21 @@ extern "C" int sqb_level_noalloc(const char *graph, double h, int K, const void 
     for(int k = -K; k <= K; k++){ tab[k + K] = exp(k*h); tab[255 + k + K] = tab[k + K]*h; }
 #define NACK(x) do { cudaError_t e_ = (x); if(e_ != cudaSuccess){ snprintf(msg, sizeof msg, "sqb_level_noalloc: %s", cudaGetErrorString(e_)); sqb_set_error_msg(msg); return (int)e_; } } while(0)
     NACK(cudaMemcpyAsync(X, tab, 2*255*sizeof(double), cudaMemcpyHostToDevice, s));
-    NACK(cudaMemsetAsync(acc, 0, sizeof(sqb_acc_t), s));
-    NACK(cudaMemsetAsync(nfb, 0, sizeof(unsigned long long), s));
+    NACK(cudaMemsetAsync(acc, 0, NA_AX - NA_ACC, s));           /* the accumulator, and with it base and the fallback count */
     if(nch > 0){
         sqb_eval_t a; memset(&a, 0, sizeof a);
         a.pts = cells; a.n = ncell; a.esize = 1; a.stride = SQB_MAXD; a.flag_at = SQB_PFLAG; a.cells = 1; a.st = st;
         a.X = X; a.Wt = Wt; a.K = K; a.raw = 0; a.abskip = abskip; a.abcheck = abcheck;
         a.abserr = abserr; a.near_thr = nearf*abserr; a.ddslack = ddslack;
+        /* the axis form: the functions of one coordinate once per (axis, k) instead of once per child (1000 cells of syn_d8: 208 -> 109 us a call,
+         * three cells of syn_d11: 129 -> 85) */
+        const long ax0 = g->axis ? (long)D*(2*K + 1)*g->axw[0] : 0, ax1 = g->axis ? (long)D*(2*K + 1)*g->axw[1] : 0;
+        if(g->axis && NA_AX + 8*(ax0 + ax1) <= SQB_NOALLOC_BYTES){
+            double *U = (double*)(B + NA_AX);
+            g->axis(0, X, K, U, U + ax0, s);
+            NACK(cudaGetLastError());
+            a.U = U; a.Ud = U + ax0;
+        }
         a.v = (double*)(B + NA_V); a.stt = B + NA_STT; a.fb = (long*)(B + NA_FB); a.nfb = nfb; a.fbcap = NA_CH;
         const size_t smem = 2*(2*K + 1)*sizeof(double);
         sqb_kattr_t at; int per = 2;

@@ -177,10 +177,9 @@ extern "C" long sqb_dev_axis_words(const sqb_graph_t *g, int K){ return axis_wor
 /* fills the tables of the lattice X (device) for the FP64 build fma at T (device), on the thread's stream */
 extern "C" int sqb_dev_axis_fill(const sqb_graph_t *g, int fma, const double *X, int K, double *T){
     if(!g->axis) return 0;
-    g->axis(fma && g->f64_fma ? 2 : 0, X, K, T, G.s);
-    g->axis(1, X, K, T + axis_words(g, K, 0), G.s);
+    g->axis(fma, X, K, T, T + axis_words(g, K, 0), G.s);
     CKR(cudaGetLastError());
-    G.launches += 2;
+    G.launches++;
     return 0;
 }
 /* the axis tables of graph g on the thread's current lattice (sqb_dev_tables), used by the evaluations that
@@ -235,9 +234,10 @@ static long grid_cap(const sqb_graph_t *g, int which, size_t smem, int *fused = 
 
 static int grid_for(const sqb_graph_t *g, int which, long npts, size_t smem){
     sqb_kattr_t at; int per = 2;
+    long want = (npts + 127)/128;
+    if(want <= G.nsm) return want < 1 ? 1 : (int)want;       /* resident whatever the kernel: no occupancy query */
     if(g->attr(which, 128, smem, &at) && at.blocks_per_sm > 0) per = at.blocks_per_sm;
-    long want = (npts + 127)/128, full = (long)G.nsm*per;
-    if(want < 1) want = 1;
+    const long full = (long)G.nsm*per;
     return (int)(want < full ? want : full);
 }
 
@@ -391,6 +391,23 @@ __device__ __forceinline__ void child_of(const lvl_t &a, const lvi_t &L, long il
     const signed char *p = L.cells + c*SQB_MAXD;
     for(int d = 0; d < a.D; d++) k[d] = p[d] - (((b >> d) & 1) ? L.st : 0);
 }
+/* child b of cell p as the three words of its pt_t, flag byte fl, in bytes four at a time: bit d of b spread to byte d
+ * (the product puts bit j of its four-bit factor at bit 8 j) times the step, subtracted per byte; a kept child lies in the
+ * box, so no byte overflows.  Bytes from D on are 0.  Cells that the caller does not keep 4-byte aligned are
+ * read byte by byte */
+__device__ __forceinline__ void child_words(const signed char *p, int D, int st, int b, signed char fl, unsigned *w){
+    if(((size_t)p & 3) == 0){ w[0] = ((const unsigned*)p)[0]; w[1] = ((const unsigned*)p)[1]; w[2] = ((const unsigned*)p)[2]; }
+    else for(int q = 0; q < 3; q++) w[q] = (unsigned char)p[4*q] | (unsigned)(unsigned char)p[4*q + 1] << 8 |
+                                           (unsigned)(unsigned char)p[4*q + 2] << 16 | (unsigned)(unsigned char)p[4*q + 3] << 24;
+#pragma unroll
+    for(int q = 0; q < 3; q++){
+        const unsigned sub = ((((unsigned)b >> (4*q)) & 15u)*0x00204081u & 0x01010101u)*(unsigned)st;
+        const int nb = D - 4*q;                                    /* axes in this word */
+        const unsigned keep = nb >= 4 ? 0xffffffffu : nb <= 0 ? 0u : (1u << (8*nb)) - 1;
+        w[q] = __vsub4(w[q], sub) & keep;
+    }
+    w[2] = (w[2] & 0x00ffffffu) | ((unsigned)(unsigned char)fl << 24);
+}
 /* a present child's multiplicity: its orbit size under a fold, else 1 */
 __device__ __forceinline__ int child_weight(const lvl_t &a, const lvi_t &L, long il){
     if(a.cw) return a.cw[il];
@@ -419,24 +436,37 @@ __global__ void __launch_bounds__(RT) sqb_k_reduce(const __grid_constant__ lvl_t
     sqdd S, b1, b2;
     double A = 0, dr = 0, uu = 0;
     unsigned ne = 0, nq = 0, nu = 0, nsk = 0, keep = 0;
-    for(int j = 0; j < RPT; j++){
-        const long i = t0 + (long)j*RT, il = i - L.child0;
-        if(il >= L.n) break;
-        const unsigned char s = a.stt[i];
-        if(!(s & SQB_PRESENT)) continue;
-        /* a folded point stands for its orbit: (mw v) pw and mw |v| (driver/sum.c:734-745) */
-        const int mw = child_weight(a, L, il);
-        const double m = (double)mw, v = a.v[i], vp = (m*v)*L.pw, av = fabs(v);
-        S = sqdd_add_d(S, vp); A += m*av; ne++;
-        nsk += (s & SQB_SKIPPED) ? 1 : 0;
-        if(s & SQB_FALLBACK){ nq++; uu += a.uu[i]; }
-        if(s & SQB_UNRES) nu++;
-        if(L.last){
-            const int te = parent_tier(a, L, i, il);
-            if(te >= 1) b1 = sqdd_add_d(b1, vp);
-            if(te >= 2) b2 = sqdd_add_d(b2, vp);
-        } else if(av >= L.thr) keep += mw;
-        else dr += (m*av)*L.pw;
+    /* four children's loads at a time, in flight together (a load per child left each waiting for the one before) */
+#pragma unroll 1
+    for(int j0 = 0; j0 < RPT; j0 += 4){
+        unsigned char st_[4]; double v_[4], u_[4];
+#pragma unroll
+        for(int j = 0; j < 4; j++){
+            const long i = t0 + (long)(j0 + j)*RT;
+            const bool in = i - L.child0 < L.n;
+            st_[j] = in ? a.stt[i] : 0; v_[j] = in ? a.v[i] : 0.0;
+        }
+#pragma unroll
+        for(int j = 0; j < 4; j++) u_[j] = (st_[j] & SQB_FALLBACK) ? a.uu[t0 + (long)(j0 + j)*RT] : 0.0;
+#pragma unroll
+        for(int j = 0; j < 4; j++){
+            const long i = t0 + (long)(j0 + j)*RT, il = i - L.child0;
+            const unsigned char s = st_[j];
+            if(!(s & SQB_PRESENT)) continue;
+            /* a folded point stands for its orbit: (mw v) pw and mw |v| (driver/sum.c:734-745) */
+            const int mw = child_weight(a, L, il);
+            const double m = (double)mw, v = v_[j], vp = (m*v)*L.pw, av = fabs(v);
+            S = sqdd_add_d(S, vp); A += m*av; ne++;
+            nsk += (s & SQB_SKIPPED) ? 1 : 0;
+            if(s & SQB_FALLBACK){ nq++; uu += u_[j]; }
+            if(s & SQB_UNRES) nu++;
+            if(L.last){
+                const int te = parent_tier(a, L, i, il);
+                if(te >= 1) b1 = sqdd_add_d(b1, vp);
+                if(te >= 2) b2 = sqdd_add_d(b2, vp);
+            } else if(av >= L.thr) keep += mw;
+            else dr += (m*av)*L.pw;
+        }
     }
     sqdd Ad(A), dd(dr), ud(uu);
     for(int off = 16; off; off >>= 1){
@@ -538,11 +568,21 @@ __global__ void __launch_bounds__(RT) sqb_k_scatter(const __grid_constant__ lvl_
     if(a.ninst > 0){ base = L.base; next = L.next; cap = L.cap; overflow = &L.acc->overflow; }
     const long t0 = blockIdx.x*(long)RTILE + threadIdx.x*(long)RPT;
     unsigned mask = 0; int cnt = 0;
-    for(int j = 0; j < RPT; j++){
-        const long i = t0 + j, il = i - L.child0;
-        if(il >= L.n) break;
-        if((a.stt[i] & SQB_PRESENT) && fabs(a.v[i]) >= L.thr){ mask |= 1u << j; cnt += child_weight(a, L, il); }
+    /* the thread's sixteen statuses in one load and its values in eight, before anything depends on them (the arrays
+     * hold whole tiles, and a tile starts at a multiple of RTILE: the vectors are aligned and in bounds) */
+    static_assert(RPT == 16, "one 16-byte load of statuses per thread");
+    {
+        union { uint4 q; unsigned char c[RPT]; } sv;
+        double2 vv[RPT/2];
+        sv.q = *(const uint4*)(a.stt + t0);
+#pragma unroll
+        for(int j = 0; j < RPT/2; j++) vv[j] = *(const double2*)(a.v + t0 + 2*j);
+#pragma unroll
+        for(int j = 0; j < RPT; j++)
+            if(t0 + j - L.child0 < L.n && (sv.c[j] & SQB_PRESENT) && fabs(j & 1 ? vv[j/2].y : vv[j/2].x) >= L.thr) mask |= 1u << j;
     }
+    if(!a.cw && a.sym.n <= 1) cnt = __popc(mask);
+    else for(unsigned b = mask; b; b &= b - 1) cnt += child_weight(a, L, t0 + __ffs(b) - 1 - L.child0);
     /* block exclusive scan of cnt */
     __shared__ int ws[RT/32];
     const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
@@ -554,9 +594,8 @@ __global__ void __launch_bounds__(RT) sqb_k_scatter(const __grid_constant__ lvl_
     __syncthreads();
     unsigned long long o = *base + boff[blockIdx.x] + (unsigned long long)(ws[w] + x - cnt);
     const double thr10 = 10*L.thr, thr100 = 100*L.thr;
-    for(int j = 0; j < RPT; j++){
-        if(!(mask >> j & 1)) continue;
-        const long i = t0 + j, il = i - L.child0;
+    for(unsigned b = mask; b; b &= b - 1){
+        const long i = t0 + __ffs(b) - 1, il = i - L.child0;
         const long c = il >> a.D;
         const signed char *p = L.cells + c*SQB_MAXD;
         const unsigned char s = a.stt[i];
@@ -564,12 +603,22 @@ __global__ void __launch_bounds__(RT) sqb_k_scatter(const __grid_constant__ lvl_
         const int te = (p[SQB_PFLAG] >> 1) & 3, tv = (av >= thr10) + (av >= thr100);
         const int psk = (s & SQB_SKIPPED) ? 1 : 0, nr = (s & SQB_NEAR) ? 1 : 0;
         const signed char fl = (signed char)((a.abskip && (psk || !nr)) | ((te < tv ? te : tv) << 1));
+        if(a.sym.n <= 1){
+            if((long)o >= cap) atomicAdd(overflow, 1ULL);
+            else {
+                unsigned w3[3];
+                child_words(p, a.D, L.st, (int)(il & ((1L << a.D) - 1)), fl, w3);
+                unsigned *dst = (unsigned*)(next + o);
+                dst[0] = w3[0]; dst[1] = w3[1]; dst[2] = w3[2];
+            }
+            o++;
+            continue;
+        }
         int k[SQB_MAXD];
         child_of(a, L, il, k);
-        /* the child, then (under a fold) the other members of its orbit in group order, each once
+        /* the child, then the other members of its orbit in group order, each once
          * (symorbit(), driver/sum.c:38-46), all with the child's flags (driver/sum.c:741-744) */
-        const int ng = a.sym.n > 1 ? a.sym.n : 1;
-        for(int e = 0; e < ng; e++){
+        for(int e = 0; e < a.sym.n; e++){
             if(!sqb_image_new(a.sym, k, a.D, e)) continue;
             if((long)o >= cap){ atomicAdd(overflow, 1ULL); o++; continue; }
             union { signed char k[SQB_MAXD]; int w[3]; } q;

@@ -178,10 +178,10 @@ typedef struct {
     int (*split_attr)(int P, int fma, int block, size_t smem, sqb_kattr_t *out);
     /* the scaling test on the raw double-double point function ptq; NULL for graphs without one (VP) */
     void (*scale)(const sqb_scale_t *a, int grid, int block, void *stream);
-    /* the axis form (kgen.axis_plan; axis NULL: the integrand has none): fills the table T of one lattice,
-     * D (2K+1) entries of axw[which] doubles, which as attr (0 as written, 1 double-double, 2 contracted) */
-    void (*axis)(int which, const double *X, int K, double *T, void *stream);
-    int axw[3];
+    /* the axis form (kgen.axis_plan; axis NULL: the integrand has none): fills the tables of one lattice, D (2K+1)
+     * entries of axw[0] doubles at T (the FP64 pass, as written or contracted) and of axw[1] at Td (double-double) */
+    void (*axis)(int fma, const double *X, int K, double *T, double *Td, void *stream);
+    int axw[2];
 } sqb_graph_t;
 
 #ifdef __cplusplus

@@ -256,50 +256,59 @@ __device__ __noinline__ sqb_fab sqb_fcall(const sqb_pt<D> p){
  * reciprocals of the NR columns it divides by.  Entries in FP64: u then r; in double-double: (hi, lo) of
  * every column, then r. */
 template<class R> struct sqb_axrow;
+template<int SM> __device__ __forceinline__ double sqb_axld(const double *e){ if constexpr(SM) return *e; else return __ldg(e); }
 template<> struct sqb_axrow<double> {
     static __device__ __forceinline__ void put(double *e, int c, double x){ e[c] = x; }
-    static __device__ __forceinline__ double get(const double *e, int c){ return __ldg(e + c); }
+    template<int SM> static __device__ __forceinline__ double get(const double *e, int c){ return sqb_axld<SM>(e + c); }
     enum { W = 1 };
 };
 template<> struct sqb_axrow<sqdd> {
     static __device__ __forceinline__ void put(double *e, int c, const sqdd &x){ e[2*c] = x.hi; e[2*c + 1] = x.lo; }
-    static __device__ __forceinline__ sqdd get(const double *e, int c){ return sqdd(__ldg(e + 2*c), __ldg(e + 2*c + 1)); }
+    template<int SM> static __device__ __forceinline__ sqdd get(const double *e, int c){
+        return sqdd(sqb_axld<SM>(e + 2*c), sqb_axld<SM>(e + 2*c + 1)); }
     enum { W = 2 };
 };
 template<class A, class R> struct sqb_axw { enum { N = A::NU*sqb_axrow<R>::W + A::NR }; };
 
-/* the table of one lattice: one thread per (axis, k) */
-template<class A, class R, int D>
-__global__ void sqb_k_axis(const double *X, int K, double *T){
-    const int nt = 2*K + 1;
-    for(int j = blockIdx.x*blockDim.x + threadIdx.x; j < D*nt; j += gridDim.x*blockDim.x){
-        R u[A::NU > 0 ? A::NU : 1];
-        A::axis(j/nt, R(X[j % nt]), u);
-        double *e = T + (long)j*sqb_axw<A, R>::N;
-#pragma unroll
-        for(int c = 0; c < A::NU; c++) sqb_axrow<R>::put(e, c, u[c]);
-#pragma unroll
-        for(int n = 0; n < A::NR; n++) e[A::NU*sqb_axrow<R>::W + n] = sqdd_rcp(u[A::rc(n)]);
-    }
-}
-/* one step of the scan from table entry e */
+/* entry j = axis (2K+1) + k + K of the table T over the variables X */
 template<class A, class R>
+__device__ __forceinline__ void sqb_axentry(const double *X, int nt, int j, double *T){
+    R u[A::NU > 0 ? A::NU : 1];
+    A::axis(j/nt, R(X[j % nt]), u);
+    double *e = T + (long)j*sqb_axw<A, R>::N;
+#pragma unroll
+    for(int c = 0; c < A::NU; c++) sqb_axrow<R>::put(e, c, u[c]);
+#pragma unroll
+    for(int n = 0; n < A::NR; n++) e[A::NU*sqb_axrow<R>::W + n] = sqdd_rcp(u[A::rc(n)]);
+}
+/* the tables of one lattice, FP64 at T and double-double at Td: one thread per entry, the double-double ones (the
+ * longer chains) in the first CTAs */
+template<class A, class Ad, int D>
+__global__ void __launch_bounds__(32) sqb_k_axis(const double *X, int K, double *T, double *Td){
+    const int nt = 2*K + 1, n = D*nt, h = (n + 31)/32;
+    const int j = (blockIdx.x % h)*32 + threadIdx.x;
+    if(j >= n) return;
+    if((int)blockIdx.x < h) sqb_axentry<Ad, sqdd>(X, nt, j, Td);
+    else sqb_axentry<A, double>(X, nt, j, T);
+}
+/* one step of the scan from table entry e (SM: in shared memory) */
+template<class A, class R, int SM = 0>
 __device__ __forceinline__ void sqb_axstep(typename A::st &S, double si, const double *e){
     R u[A::NU > 0 ? A::NU : 1]; double r[A::NR > 0 ? A::NR : 1];
 #pragma unroll
-    for(int c = 0; c < A::NU; c++) u[c] = sqb_axrow<R>::get(e, c);
+    for(int c = 0; c < A::NU; c++) u[c] = sqb_axrow<R>::template get<SM>(e, c);
 #pragma unroll
-    for(int n = 0; n < A::NR; n++) r[n] = __ldg(e + A::NU*sqb_axrow<R>::W + n);
+    for(int n = 0; n < A::NR; n++) r[n] = sqb_axld<SM>(e + A::NU*sqb_axrow<R>::W + n);
     A::step(S, R(si), u, r);
 }
 /* the integrand at one point k (inside the box) from its table */
-template<class A, class R, int D>
+template<class A, class R, int D, int SM = 0>
 __device__ __forceinline__ R sqb_axeval(const double *T, int K, const double *sf, const int *k, R *ab){
     typename A::st S;
     A::init(S);
     const int nt = 2*K + 1;
 #pragma unroll
-    for(int d = 0; d < D; d++) sqb_axstep<A, R>(S, sf[d], T + (d*nt + k[d] + K)*(int)sqb_axw<A, R>::N);
+    for(int d = 0; d < D; d++) sqb_axstep<A, R, SM>(S, sf[d], T + (d*nt + k[d] + K)*(int)sqb_axw<A, R>::N);
     return A::fin(S, ab);
 }
 
@@ -369,22 +378,19 @@ __global__ void __launch_bounds__(SQB_BLOCK, SQB_MINB) sqb_k_f64(const __grid_co
         for(int j = 0; j < tl/SQB_BLOCK; j++){
             long il, i; int mw;
             long c; double sf[D], w;
-            [[maybe_unused]] int kk[D];
-            constexpr bool AX = F::template AX<double, 0>::NU > 0;
-            int *const ko = AX ? kk : NULL;
             if(list){
                 const long e_ = tile*tl + (long)j*SQB_BLOCK + t;
                 if(e_ >= nsel) break;
                 const unsigned long long e = a.sel[e_];
                 il = i = (long)(e & ((1ULL << SQB_SEL_SHIFT) - 1));
-                sqb_point<D, false, LV>(a, I, sX, sW, il, i, &c, sf, &w, ko);
+                sqb_point<D, false, LV>(a, I, sX, sW, il, i, &c, sf, &w);
                 mw = (int)(e >> SQB_SEL_SHIFT);
             } else {
                 il = base + (long)j*SQB_BLOCK + t; i = il + off;
                 if(il >= n) break;
                 /* two sweeps: this child only in its cell's sweep (0: skips the |.| sums, 1: the others) */
                 if(NSW > 1 && (sqb_skip<D>(a, I, il >> D) ? 0 : 1) != sweep) continue;
-                mw = sqb_point<D, true, LV>(a, I, sX, sW, il, i, &c, sf, &w, ko);
+                mw = sqb_point<D, true, LV>(a, I, sX, sW, il, i, &c, sf, &w);
             }
             if(!mw){
                 a.v[i] = 0;
@@ -394,14 +400,8 @@ __global__ void __launch_bounds__(SQB_BLOCK, SQB_MINB) sqb_k_f64(const __grid_co
             const int sk = sqb_skip<D>(a, I, c);
             const bool noab = sk && !a.abcheck;
             double ab = 0, f;
-            bool tab = false;
-            if constexpr(AX) if(I.U){
-                tab = true;
-                if(noab) f = sqb_axeval<typename F::template AX<double, 0>, double, D>(I.U, I.K, sf, kk, &ab);
-                else     f = sqb_axeval<typename F::template AX<double, 1>, double, D>(I.U, I.K, sf, kk, &ab);
-            }
 #if SQB_LEVEL_KERNEL
-            if(!AX || !tab){
+            {
                 sqb_pt<D> p;
 #pragma unroll
                 for(int d = 0; d < D; d++) p.s[d] = sf[d];
@@ -409,8 +409,7 @@ __global__ void __launch_bounds__(SQB_BLOCK, SQB_MINB) sqb_k_f64(const __grid_co
                 f = r.f; ab = r.ab;
             }
 #else
-            if(AX && tab);
-            else if(noab) f = F::template f<double, 0>(sf, &ab);
+            if(noab) f = F::template f<double, 0>(sf, &ab);
             else     f = F::template f<double, 1>(sf, &ab);
 #endif
             const double fw = f*w;
@@ -450,6 +449,45 @@ __global__ void __launch_bounds__(SQB_BLOCK, SQB_MINB) sqb_k_f64(const __grid_co
             __syncthreads();
             q = s_tile;
         } else q += gridDim.x;
+    }
+}
+
+/* The axis form's kernel for launches outside the level batches: one batch of nodes or cells, tested or raw.  SM = 0 reads
+ * the table at a.U; SM = 1 (the plug-in's launches, which have no table) fills one in shared memory per CTA first,
+ * which pays from SQB_AX_RAW points on (sqb_ax_points). */
+template<class F, int D, int SM>
+__global__ void __launch_bounds__(SQB_BLOCK) sqb_k_ax(const __grid_constant__ sqb_eval_t a){
+    extern __shared__ double sqb_sm[];
+    __shared__ sqb_inst_t sI[SQB_MAXINST];
+    using A0 = typename F::template AX<double, 0>;
+    using A1 = typename F::template AX<double, 1>;
+    sqb_tables(a, sqb_sm, sI);
+    const sqb_inst_t &I = sI[0];
+    const int nt = 2*a.K + 1;
+    const double *sX = sqb_sm, *sW = sqb_sm + nt;
+    double *T = sqb_sm + 2*nt;
+    if constexpr(SM){
+        for(int j = threadIdx.x; j < D*nt; j += SQB_BLOCK) sqb_axentry<A0, double>(sX, nt, j, T);
+        __syncthreads();
+    }
+    const double *U = SM ? T : a.U;
+    const long n = a.cells ? (a.n << D) : a.n;
+    for(long i = blockIdx.x*(long)SQB_BLOCK + threadIdx.x; i < n; i += (long)gridDim.x*SQB_BLOCK){
+        long c; double sf[D], w; int kk[D];
+        if(!sqb_point<D>(a, I, sX, sW, i, i, &c, sf, &w, kk)){
+            a.v[i] = 0;
+            if(a.raw) a.ab[i] = 0; else a.stt[i] = 0;
+            continue;
+        }
+        const int sk = sqb_skip<D>(a, I, c);
+        const bool noab = sk && !a.abcheck;
+        double ab = 0, f;
+        if(noab) f = sqb_axeval<A0, double, D, SM>(U, a.K, sf, kk, &ab);
+        else     f = sqb_axeval<A1, double, D, SM>(U, a.K, sf, kk, &ab);
+        const double fw = f*w;
+        if(a.raw){ a.v[i] = fw; a.ab[i] = ab*w; continue; }
+        bool fallback;
+        sqb_point_test(a, I, i, sk, noab, fw, ab*w, &fallback);
     }
 }
 
@@ -737,6 +775,21 @@ static bool sqb_ax_level(const sqb_eval_t *a, int grid, int block, size_t smem, 
     }
     return false;
 }
+/* a raw launch of the plug-in fills a table per CTA from this many points on and if it fits beside the lattice
+ * tables in the 48 KB that need no opt-in.  Measured per launch, K = 44: 131,072 children of syn_d5, d8, d11 13.3, 16.5,
+ * 21.0 us -> 10.0, 12.3, 14.4; 65,536 the same either way; 4.1e6 of d8 and d11 390 and 457 us -> 114 and 120 */
+#define SQB_AX_RAW (1L << 17)
+template<class F, int D>
+static bool sqb_ax_points(const sqb_eval_t *a, int grid, int block, size_t smem, cudaStream_t st){
+    if constexpr(F::template AX<double, 0>::NU > 0){
+        if(a->ninst > 0 || a->sfin || a->sel || a->part || a->sym.n > 1 || a->cfl) return false;
+        if(a->U){ sqb_k_ax<F, D, 0><<<grid, block, smem, st>>>(*a); return true; }
+        const size_t sm = smem + (size_t)D*(2*a->K + 1)*sqb_axw<typename F::template AX<double, 0>, double>::N*sizeof(double);
+        if(a->raw && (a->cells ? a->n << D : a->n) >= SQB_AX_RAW && sm <= 48*1024){
+            sqb_k_ax<F, D, 1><<<grid, block, sm, st>>>(*a); return true; }
+    }
+    return false;
+}
 template<class F, int D>
 static bool sqb_ax_attr(int block, size_t smem, sqb_kattr_t *o, int *ok){
     if constexpr(F::template AX<double, 0>::NU > 0){
@@ -746,12 +799,10 @@ static bool sqb_ax_attr(int block, size_t smem, sqb_kattr_t *o, int *ok){
     }
     return false;
 }
-template<class F, class R, int AB, int D>
-static void sqb_ax_table(const double *X, int K, double *T, cudaStream_t st){
-    if constexpr(F::template AX<double, 0>::NU > 0){
-        const int n = D*(2*K + 1);
-        sqb_k_axis<typename F::template AX<R, AB>, R, D><<<(n + 31)/32, 32, 0, st>>>(X, K, T);
-    }
+template<class F, int D>
+static void sqb_ax_table(const double *X, int K, double *T, double *Td, cudaStream_t st){
+    if constexpr(F::template AX<double, 0>::NU > 0)
+        sqb_k_axis<typename F::template AX<double, 0>, typename F::template AX<sqdd, 1>, D><<<2*((D*(2*K + 1) + 31)/32), 32, 0, st>>>(X, K, T, Td);
 }
 template<class F, class R> struct sqb_ax_words { enum { N = F::template AX<R, 0>::NU > 0 ? (int)sqb_axw<typename F::template AX<R, 0>, R>::N : 0 }; };
 
@@ -794,10 +845,11 @@ struct F {                                                                      
         return K<R, AB>::f_##NAME(sf, ab); }                                                       \
 };                                                                                                 \
 }                                                                                                  \
-extern "C" void SQB_##NAME##_axisfma(const double *X, int K, double *T, void *st){                 \
-    sqb_ax_table<SQG_NS(NAME)::F, double, 0, D>(X, K, T, (cudaStream_t)st); }                       \
+extern "C" void SQB_##NAME##_axisfma(const double *X, int K, double *T, double *Td, void *st){     \
+    sqb_ax_table<SQG_NS(NAME)::F, D>(X, K, T, Td, (cudaStream_t)st); }                              \
 extern "C" void SQB_##NAME##_f64fma(const sqb_eval_t *a, int grid, int block, size_t smem, void *st){ \
     if(sqb_ax_level<SQG_NS(NAME)::F, D>(a, grid, block, smem, (cudaStream_t)st)) return;            \
+    if(sqb_ax_points<SQG_NS(NAME)::F, D>(a, grid, block, smem, (cudaStream_t)st)) return;           \
     if(sqb_level_launch(a)) sqb_k_f64<SQG_NS(NAME)::F, D, 1><<<grid, block, smem, (cudaStream_t)st>>>(*a); \
     else sqb_k_f64<SQG_NS(NAME)::F, D, 0><<<grid, block, smem, (cudaStream_t)st>>>(*a); }           \
 extern "C" int SQB_##NAME##_attrfma(int lv, int block, size_t smem, sqb_kattr_t *o){               \
@@ -825,7 +877,7 @@ extern "C" void SQB_##NAME##_scale(const sqb_scale_t *a, int grid, int block, vo
     sqb_k_scale<SQG_NS(NAME)::PT><<<grid, block, 0, (cudaStream_t)st>>>(*a); }
 #define SQ_GRAPH_CORE(NAME, D)                                                                      \
 extern "C" void SQB_##NAME##_f64fma(const sqb_eval_t *, int, int, size_t, void *) __attribute__((weak)); \
-extern "C" void SQB_##NAME##_axisfma(const double *, int, double *, void *) __attribute__((weak)); \
+extern "C" void SQB_##NAME##_axisfma(const double *, int, double *, double *, void *) __attribute__((weak)); \
 extern "C" void SQB_##NAME##_scale(const sqb_scale_t *, int, int, void *) __attribute__((weak));   \
 extern "C" int SQB_##NAME##_attrfma(int, int, size_t, sqb_kattr_t *) __attribute__((weak));        \
 namespace SQG_NS(NAME) {                                                                           \
@@ -838,15 +890,15 @@ template<> __device__ __forceinline__ sqdd F::f<sqdd, 1>(const sqdd *sf, sqdd *a
     return KD<sqdd, 1>::f_##NAME(sf, ab); }                                                        \
 static void f64(const sqb_eval_t *a, int grid, int block, size_t smem, void *st){                  \
     if(sqb_ax_level<F, D>(a, grid, block, smem, (cudaStream_t)st)) return;                         \
+    if(sqb_ax_points<F, D>(a, grid, block, smem, (cudaStream_t)st)) return;                        \
     if(SQB_LEVEL_KERNEL && sqb_level_launch(a))                                                    \
         sqb_k_f64<F, D, SQB_LEVEL_KERNEL><<<grid, block, smem, (cudaStream_t)st>>>(*a);            \
     else sqb_k_f64<F, D, 0><<<grid, block, smem, (cudaStream_t)st>>>(*a); }                        \
 static void dd(const sqb_dd_t *a, int grid, int block, size_t smem, void *st){                     \
     sqb_k_dd<F, D><<<grid, block, smem, (cudaStream_t)st>>>(*a); }                                 \
-static void axis(int which, const double *X, int K, double *T, void *st){                          \
-    if(which == 2){ if(SQB_##NAME##_axisfma) SQB_##NAME##_axisfma(X, K, T, st); }                   \
-    else if(which == 1) sqb_ax_table<F, sqdd, 1, D>(X, K, T, (cudaStream_t)st);                     \
-    else sqb_ax_table<F, double, 0, D>(X, K, T, (cudaStream_t)st); }                               \
+static void axis(int fma, const double *X, int K, double *T, double *Td, void *st){                \
+    if(fma && SQB_##NAME##_axisfma) SQB_##NAME##_axisfma(X, K, T, Td, st);                         \
+    else sqb_ax_table<F, D>(X, K, T, Td, (cudaStream_t)st); }                                      \
 static int attr(int which, int block, size_t smem, sqb_kattr_t *o){                                \
     const int lv = (which & SQB_ATTR_LEVEL) != 0; which &= ~SQB_ATTR_LEVEL;                        \
     if(which == 2) return SQB_##NAME##_attrfma ? SQB_##NAME##_attrfma(lv, block, smem, o) : 0;      \
@@ -856,8 +908,7 @@ static int attr(int which, int block, size_t smem, sqb_kattr_t *o){             
                                   : sqb_f64_attr(sqb_k_f64<F, D, 0>, 0, block, smem, o); }         \
 }
 #define SQ_AXIS_ENTRY(NAME) sqb_ax_words<SQG_NS(NAME)::F, double>::N ? SQG_NS(NAME)::axis : NULL,    \
-    {sqb_ax_words<SQG_NS(NAME)::F, double>::N, sqb_ax_words<SQG_NS(NAME)::F, sqdd>::N,              \
-     sqb_ax_words<SQG_NS(NAME)::F, double>::N}
+    {sqb_ax_words<SQG_NS(NAME)::F, double>::N, sqb_ax_words<SQG_NS(NAME)::F, sqdd>::N}
 #define SQ_GRAPH_AXIS(NAME, VOLKOV, L, D, W, NP, FIX)                                               \
 SQ_GRAPH_CORE(NAME, D)                                                                             \
 extern "C" const sqb_graph_t SQB_##NAME = {#NAME, VOLKOV, L, D, W, NP, FIX, 0,                     \
@@ -881,5 +932,5 @@ static int split_attr(int P, int fma, int block, size_t smem, sqb_kattr_t *o){  
 }                                                                                                  \
 extern "C" const sqb_graph_t SQB_##NAME = {#NAME, VOLKOV, L, D, W, NP, FIX, 0,                     \
     SQG_NS(NAME)::f64, SQG_NS(NAME)::dd, SQG_NS(NAME)::attr, SQB_##NAME##_f64fma, NPARTS,           \
-    SQG_NS(NAME)::split, SQG_NS(NAME)::split_attr, SQB_##NAME##_scale, NULL, {0, 0, 0}};
+    SQG_NS(NAME)::split, SQG_NS(NAME)::split_attr, SQB_##NAME##_scale, NULL, {0, 0}};
 #endif
