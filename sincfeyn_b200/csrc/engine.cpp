@@ -132,7 +132,8 @@ static int grow(Run &R, int lev, double eps_rel, GrowOut *go, sqb_pt_t **dilated
     for(;;){
         n = sqb_grow_frontier(&pts, &skip);
         if(n <= 0) break;
-        if(sqb_dev_eval_resident(R.g, pts, n, skip, &R.t, &vd, &sd, &ud)) FAIL("device: %s", sqb_last_error());
+        /* the first frontier, z = 0, is the probe's first node: its value is there */
+        if(nfr && sqb_dev_eval_resident(R.g, pts, n, skip, &R.t, &vd, &sd, &ud)) FAIL("device: %s", sqb_last_error());
         /* the predictor stores every grow value (driver/sumkey.h:219-222) */
         if(R.vt && (sqb_vtab_reserve(R.vt, n, sqb_dev_stream()) || sqb_vtab_put_nodes(R.vt, pts, vd, n, R.D, sqb_dev_stream())))
             FAIL("predictor: %s", sqb_vtab_error());
