@@ -45,21 +45,21 @@
 #define NA_BK    (NA_BP + NA_UP(sizeof(sqb_part_t)*NA_TILES))   /* unsigned keep count per tile */
 #define NA_BO    (NA_BK + NA_UP(4L*NA_TILES))        /* unsigned long long offset per tile */
 #define NA_ACC   (NA_BO + NA_UP(8L*NA_TILES))        /* sqb_acc_t */
-#define NA_MISC  (NA_ACC + NA_UP(sizeof(sqb_acc_t))) /* base, fallback count */
+#define NA_MISC  (NA_ACC + NA_UP(sizeof(sqb_acc_t))) /* base, fallback count; from byte 64 the finish kernel's */
 #define NA_AX    (NA_MISC + 256L)                    /* axis tables (sqb_graph_t axis), FP64 then double-double, where they
                                                          fit: about 130,000 bytes are left, 2,000 (axis, k) entries of
                                                          eight doubles */
 #define NA_END   NA_AX
 static_assert(NA_END <= SQB_NOALLOC_BYTES, "the scratch layout must fit the array the header states");
 static_assert(2*255*sizeof(double) <= 4096, "the lattice tables (|k| <= 127) must fit their slot");
-static_assert(sizeof(sqb_acc_t) <= 256 && 2*sizeof(unsigned long long) <= 256, "accumulator slots");
+static_assert(sizeof(sqb_acc_t) <= 256 && 64 + SQB_FIN_BYTES <= 256, "accumulator slots");
 
 static __device__ __align__(256) unsigned char sqb_noalloc_scratch[SQB_NOALLOC_BYTES];
 
 extern "C" int sqb_level_tail(const void *cells, long nchildren, int D, int st, int last, int abskip, double pw, double thr,
                               const double *v, const double *uu, const unsigned char *stt,
                               void *bp, unsigned *bkeep, unsigned long long *boff, sqb_acc_t *acc, unsigned long long *base,
-                              void *next, long next_cap, void *stream);
+                              void *fin, void *next, long next_cap, void *stream);
 extern "C" size_t sqb_level_tile_bytes(void);
 extern "C" long sqb_level_tile_children(void);
 extern "C" void sqb_set_error_msg(const char *msg);
@@ -140,7 +140,7 @@ extern "C" int sqb_level_noalloc(const char *graph, double h, int K, const void 
         NACK(cudaGetLastError());
         int rc = sqb_level_tail(cells, nch, D, st, last, abskip, pw, thr, a.v, d.uu, a.stt,
                                 B + NA_BP, (unsigned*)(B + NA_BK), (unsigned long long*)(B + NA_BO), acc, base,
-                                next, next_cap, s);
+                                B + NA_MISC + 64, next, next_cap, s);
         if(rc){ sqb_set_error_msg("sqb_level_noalloc: kernel launch failed"); return rc; }
     }
     sqb_acc_t r;

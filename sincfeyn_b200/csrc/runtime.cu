@@ -9,7 +9,7 @@
  *   3. sqb_k_reduce: per tile of children (in cell order, b ascending), compensated double-double sums of
  *      v*pw, |v|, the dropped weight, the shadow-tier sums and the round column, plus counters and the
  *      number of kept children;
- *   4. sqb_k_finish (one CTA): exclusive scan of the tiles' kept counts and the tiles' sums added in
+ *   4. sqb_k_finish: exclusive scan of the tiles' kept counts and the tiles' sums added in
  *      a fixed order into the level accumulator, so that a run is reproducible;
  *   5. sqb_k_scatter: the kept children written, in order, to the next level's cell list with their
  *      flags (skip bit, shadow tier; driver/sum.c:741-745).
@@ -53,7 +53,7 @@ extern "C" const sqb_graph_t *sqb_graph_at(int i){ return i >= 0 && i < SQB_NALL
 #define RT 256                    /* threads per reduce / scatter CTA */
 #define RPT 16                    /* children per thread (scatter: consecutive; reduce: RT apart) */
 #define RTILE (RT*RPT)
-#define FT 1024                   /* threads of the one-CTA finish kernel (32 warps) */
+#define FT 256                    /* tiles per CTA of the finish kernel, one per thread */
 
 typedef sqb_part_t part_t;
 static_assert(RTILE == SQB_TILE, "the reduce kernel's tiles are the FP64 kernel's");
@@ -82,6 +82,9 @@ typedef struct {
     const unsigned char *cw;      /* list mode: every child's orbit weight from the select pass (0: not evaluated) */
 } lvl_t;
 
+/* the finish kernel's sums of FT tiles: S, |v|, drop, b1, b2, u; evaluated, fallback, unresolved, skipped, kept */
+struct fpart_t { double x[6][2]; unsigned long long c[5]; };
+
 struct Dev {
     int on, dev, nsm;
     cudaEvent_t t0, t1; void *flush; size_t flushn;
@@ -97,6 +100,7 @@ struct Dev {
     double *v, *uu; unsigned char *stt, *cfl, *cw; long *fb; unsigned long long *nfb;
     unsigned long long *sel, *nsel;   /* list mode: the children to evaluate and their number */
     long nbcap; part_t *bp; unsigned *bkeep; unsigned long long *boff; unsigned char *tfb;
+    fpart_t *fp; unsigned long long *coff; unsigned *fcnt;   /* per FT tiles: sums, kept before them; CTAs done per integral */
     long ttcap; double *tt, *ta;   /* split FP64 pass: running sums per point */
     sqb_acc_t *acc; unsigned long long *base;
     sqb_acc_t *accm; unsigned long long *basem, *queue;   /* multi-instance levels: per integral, tile queue */
@@ -152,6 +156,8 @@ extern "C" int sqb_dev_init(int device){
     CKR(cudaMalloc(&G.basem, SQB_MAXINST*sizeof(unsigned long long)));
     CKR(cudaMalloc(&G.queue, sizeof(unsigned long long)));
     CKR(cudaMalloc(&G.nsel, sizeof(unsigned long long)));
+    CKR(cudaMalloc(&G.fcnt, SQB_MAXINST*sizeof(unsigned)));
+    CKR(cudaMemsetAsync(G.fcnt, 0, SQB_MAXINST*sizeof(unsigned), G.s));      /* every finish leaves it 0 */
     G.on = 1;
     return 0;
 }
@@ -204,13 +210,15 @@ static int reserve_points(long n){
     if(n <= G.cap) return 0;
     long c = 1L << 16; while(c < n) c <<= 1;
     if(G.v){ cudaFree(G.v); cudaFree(G.uu); cudaFree(G.stt); cudaFree(G.cfl); cudaFree(G.cw); cudaFree(G.fb); cudaFree(G.sel);
-             cudaFree(G.bp); cudaFree(G.bkeep); cudaFree(G.boff); cudaFree(G.tfb); }
+             cudaFree(G.bp); cudaFree(G.bkeep); cudaFree(G.boff); cudaFree(G.tfb); cudaFree(G.fp); cudaFree(G.coff); }
     CKR(cudaMalloc(&G.v, c*sizeof(double))); CKR(cudaMalloc(&G.uu, c*sizeof(double)));
     CKR(cudaMalloc(&G.stt, c)); CKR(cudaMalloc(&G.cfl, c)); CKR(cudaMalloc(&G.cw, c)); CKR(cudaMalloc(&G.fb, c*sizeof(long)));
     CKR(cudaMalloc(&G.sel, c*sizeof(unsigned long long)));
     long nb = (c + RTILE - 1)/RTILE;
     CKR(cudaMalloc(&G.bp, nb*sizeof(part_t))); CKR(cudaMalloc(&G.bkeep, nb*sizeof(unsigned))); CKR(cudaMalloc(&G.tfb, nb));
     CKR(cudaMalloc(&G.boff, nb*sizeof(unsigned long long)));
+    const long nf = nb/FT + SQB_MAXINST + 1;
+    CKR(cudaMalloc(&G.fp, nf*sizeof(fpart_t))); CKR(cudaMalloc(&G.coff, nf*sizeof(unsigned long long)));
     G.cap = c; G.nbcap = nb;
     return 0;
 }
@@ -374,8 +382,9 @@ __device__ __forceinline__ sqdd shfl_dd(const sqdd &a, int off){
     return sqdd(__shfl_down_sync(0xffffffffu, a.hi, off), __shfl_down_sync(0xffffffffu, a.lo, off));
 }
 /* the integral of tile b of a batch (one batch: the batch itself, with child0 = 0) */
-__device__ __forceinline__ lvi_t lvl_inst(const lvl_t &a, long b){
+__device__ __forceinline__ lvi_t lvl_inst(const lvl_t &a, long b, int *index = NULL){
     lvi_t v;
+    if(index) *index = 0;
     if(a.ninst <= 0){
         v.cells = a.cells; v.n = a.n; v.child0 = 0; v.st = a.st; v.last = a.last; v.pw = a.pw; v.thr = a.thr;
         v.next = NULL; v.cap = 0; v.acc = NULL; v.base = NULL;
@@ -383,8 +392,12 @@ __device__ __forceinline__ lvi_t lvl_inst(const lvl_t &a, long b){
     }
     int k = 0;
     for(int q = 1; q < a.ninst; q++) if(a.inst[q].child0 <= b*(long)RTILE) k = q;
+    if(index) *index = k;
     return a.inst[k];
 }
+/* the finish kernel's slot of tile b (of integral k, whose first tile is tb): FT tiles each, no slot shared by two
+ * integrals */
+__device__ __forceinline__ long fin_slot(long tb, int k, long b){ return tb/FT + k + (b - tb)/FT; }
 /* child il's coordinates k_d - st bit_d(b) (driver/sum.c:407) */
 __device__ __forceinline__ void child_of(const lvl_t &a, const lvi_t &L, long il, int *k){
     const long c = il >> a.D; const int b = (int)(il & ((1L << a.D) - 1));
@@ -423,52 +436,70 @@ __device__ __forceinline__ int parent_tier(const lvl_t &a, const lvi_t &L, long 
     return (L.cells[c*SQB_MAXD + SQB_PFLAG] >> 1) & 3;
 }
 
+/* one child's part of a tile's sums */
+struct rsum_t { sqdd S, b1, b2; double A, dr, uu; unsigned ne, nq, nu, nsk, keep; };
+__device__ __forceinline__ void rsum_add(rsum_t &x, const lvl_t &a, const lvi_t &L, long i, unsigned char s, double v, double u){
+    /* a folded point stands for its orbit: (mw v) pw and mw |v| (driver/sum.c:734-745) */
+    const long il = i - L.child0;
+    const int mw = child_weight(a, L, il);
+    const double m = (double)mw, vp = (m*v)*L.pw, av = fabs(v);
+    x.S = sqdd_add_d(x.S, vp); x.A += m*av; x.ne++;
+    x.nsk += (s & SQB_SKIPPED) ? 1 : 0;
+    if(s & SQB_FALLBACK){ x.nq++; x.uu += u; }
+    if(s & SQB_UNRES) x.nu++;
+    if(L.last){
+        const int te = parent_tier(a, L, i, il);
+        if(te >= 1) x.b1 = sqdd_add_d(x.b1, vp);
+        if(te >= 2) x.b2 = sqdd_add_d(x.b2, vp);
+    } else if(av >= L.thr) x.keep += mw;
+    else x.dr += (m*av)*L.pw;
+}
 /* per tile of RTILE children: S = sum v*pw and the shadow-tier sums in double-double per thread (they
  * can cancel), sum |v|, the dropped weight and the round column (non-negative) in double per thread,
- * then double-double across threads in a fixed tree.  Thread t of the tile takes children t, t + RT,
- * t + 2 RT, ... (each warp reads 256 contiguous bytes of v per step); the order is fixed, so a run is
- * reproducible. */
+ * then double-double across threads in a fixed tree; the order is fixed, so a run is reproducible.  tfb[tile] says
+ * what the FP64 pass left: 0 = nothing; 2 = the tile's fallback points, to be added to its sums (a thread finds them
+ * among sixteen consecutive children by one load of their statuses); 1 (or no tfb) = the whole tile, thread t taking
+ * children t, t + RT, t + 2 RT, ... (each warp reads 256 contiguous bytes of v per step). */
 __global__ void __launch_bounds__(RT) sqb_k_reduce(const __grid_constant__ lvl_t a, part_t *bp, unsigned *bkeep,
                                                    const unsigned char *tfb){
-    if(tfb && !tfb[blockIdx.x]) return;      /* summed by the FP64 pass already (no fallback point in it) */
+    const int mode = tfb ? tfb[blockIdx.x] : 1;
+    if(mode == 0) return;
     const lvi_t L = lvl_inst(a, blockIdx.x);
-    const long t0 = blockIdx.x*(long)RTILE + threadIdx.x;
-    sqdd S, b1, b2;
-    double A = 0, dr = 0, uu = 0;
-    unsigned ne = 0, nq = 0, nu = 0, nsk = 0, keep = 0;
-    /* four children's loads at a time, in flight together (a load per child left each waiting for the one before) */
+    rsum_t rs; rs.A = rs.dr = rs.uu = 0; rs.ne = rs.nq = rs.nu = rs.nsk = rs.keep = 0;
+    if(mode == 2){
+        const long t0 = blockIdx.x*(long)RTILE + threadIdx.x*(long)RPT;
+        const uint4 q = *(const uint4*)(a.stt + t0);
+        const unsigned w[4] = {q.x, q.y, q.z, q.w};
 #pragma unroll 1
-    for(int j0 = 0; j0 < RPT; j0 += 4){
-        unsigned char st_[4]; double v_[4], u_[4];
+        for(int h = 0; h < 4; h++)
+            for(unsigned b = w[h] & (SQB_FALLBACK*0x01010101u); b; b &= b - 1){
+                const int j = 4*h + ((__ffs(b) - 1) >> 3);
+                const long i = t0 + j;
+                if(i - L.child0 < L.n) rsum_add(rs, a, L, i, a.stt[i], a.v[i], a.uu[i]);
+            }
+    } else {
+        const long t0 = blockIdx.x*(long)RTILE + threadIdx.x;
+        /* four children's loads at a time, in flight together (a load per child left each waiting for the one before) */
+#pragma unroll 1
+        for(int j0 = 0; j0 < RPT; j0 += 4){
+            unsigned char st_[4]; double v_[4], u_[4];
 #pragma unroll
-        for(int j = 0; j < 4; j++){
-            const long i = t0 + (long)(j0 + j)*RT;
-            const bool in = i - L.child0 < L.n;
-            st_[j] = in ? a.stt[i] : 0; v_[j] = in ? a.v[i] : 0.0;
-        }
+            for(int j = 0; j < 4; j++){
+                const long i = t0 + (long)(j0 + j)*RT;
+                const bool in = i - L.child0 < L.n;
+                st_[j] = in ? a.stt[i] : 0; v_[j] = in ? a.v[i] : 0.0;
+            }
 #pragma unroll
-        for(int j = 0; j < 4; j++) u_[j] = (st_[j] & SQB_FALLBACK) ? a.uu[t0 + (long)(j0 + j)*RT] : 0.0;
+            for(int j = 0; j < 4; j++) u_[j] = (st_[j] & SQB_FALLBACK) ? a.uu[t0 + (long)(j0 + j)*RT] : 0.0;
 #pragma unroll
-        for(int j = 0; j < 4; j++){
-            const long i = t0 + (long)(j0 + j)*RT, il = i - L.child0;
-            const unsigned char s = st_[j];
-            if(!(s & SQB_PRESENT)) continue;
-            /* a folded point stands for its orbit: (mw v) pw and mw |v| (driver/sum.c:734-745) */
-            const int mw = child_weight(a, L, il);
-            const double m = (double)mw, v = v_[j], vp = (m*v)*L.pw, av = fabs(v);
-            S = sqdd_add_d(S, vp); A += m*av; ne++;
-            nsk += (s & SQB_SKIPPED) ? 1 : 0;
-            if(s & SQB_FALLBACK){ nq++; uu += u_[j]; }
-            if(s & SQB_UNRES) nu++;
-            if(L.last){
-                const int te = parent_tier(a, L, i, il);
-                if(te >= 1) b1 = sqdd_add_d(b1, vp);
-                if(te >= 2) b2 = sqdd_add_d(b2, vp);
-            } else if(av >= L.thr) keep += mw;
-            else dr += (m*av)*L.pw;
+            for(int j = 0; j < 4; j++) if(st_[j] & SQB_PRESENT) rsum_add(rs, a, L, t0 + (long)(j0 + j)*RT, st_[j], v_[j], u_[j]);
         }
     }
+    sqdd S = rs.S, b1 = rs.b1, b2 = rs.b2;
+    unsigned ne = rs.ne, nq = rs.nq, nu = rs.nu, nsk = rs.nsk, keep = rs.keep;
+    const double A = rs.A, dr = rs.dr, uu = rs.uu;
     sqdd Ad(A), dd(dr), ud(uu);
+    if(__any_sync(0xffffffffu, ne))                    /* a warp without a child to add has zeros */
     for(int off = 16; off; off >>= 1){
         S = S + shfl_dd(S, off); Ad = Ad + shfl_dd(Ad, off); dd = dd + shfl_dd(dd, off);
         b1 = b1 + shfl_dd(b1, off); b2 = b2 + shfl_dd(b2, off); ud = ud + shfl_dd(ud, off);
@@ -499,72 +530,130 @@ __global__ void __launch_bounds__(RT) sqb_k_reduce(const __grid_constant__ lvl_t
             p.S[0] = x[0].hi; p.S[1] = x[0].lo; p.A[0] = x[1].hi; p.A[1] = x[1].lo; p.drop[0] = x[2].hi; p.drop[1] = x[2].lo;
             p.b1[0] = x[3].hi; p.b1[1] = x[3].lo; p.b2[0] = x[4].hi; p.b2[1] = x[4].lo; p.u[0] = x[5].hi; p.u[1] = x[5].lo;
             p.ne = c[0]; p.nq = c[1]; p.unres = c[2]; p.skipped = c[3];
+            if(mode == 2){
+                const part_t o = bp[blockIdx.x];
+                const sqdd z[6] = {x[0] + sqdd(o.S[0], o.S[1]), x[1] + sqdd(o.A[0], o.A[1]), x[2] + sqdd(o.drop[0], o.drop[1]),
+                                   x[3] + sqdd(o.b1[0], o.b1[1]), x[4] + sqdd(o.b2[0], o.b2[1]), x[5] + sqdd(o.u[0], o.u[1])};
+                p.S[0] = z[0].hi; p.S[1] = z[0].lo; p.A[0] = z[1].hi; p.A[1] = z[1].lo; p.drop[0] = z[2].hi; p.drop[1] = z[2].lo;
+                p.b1[0] = z[3].hi; p.b1[1] = z[3].lo; p.b2[0] = z[4].hi; p.b2[1] = z[4].lo; p.u[0] = z[5].hi; p.u[1] = z[5].lo;
+                p.ne += o.ne; p.nq += o.nq; p.unres += o.unres; p.skipped += o.skipped;
+                c[4] += bkeep[blockIdx.x];
+            }
             bp[blockIdx.x] = p; bkeep[blockIdx.x] = c[4];
         }
     }
 }
 
-/* one CTA per integral: the tiles' offsets (exclusive scan of their kept counts) and the batch's sums, in
- * a fixed order (each thread a contiguous run of tiles, then a fixed tree), added into the level
- * accumulator; *base = this batch's first slot in the next list.  One batch (a.ninst = 0): its nb tiles
- * into acc and base; a multi-instance batch: CTA k takes integral k's tiles into its own acc and base */
-__global__ void __launch_bounds__(FT) sqb_k_finish(const __grid_constant__ lvl_t a, const part_t *bp, const unsigned *bkeep,
-                                                   long nb, unsigned long long *boff, sqb_acc_t *acc,
-                                                   unsigned long long *base){
-    long tb = 0;
-    if(a.ninst > 0){
-        const lvi_t &L = a.inst[blockIdx.x];
-        tb = L.child0/RTILE; nb = (L.n + RTILE - 1)/RTILE; acc = L.acc; base = L.base;
-    }
-    bp += tb; bkeep += tb; boff += tb;
-    const int t = threadIdx.x, w = t >> 5, l = t & 31;
-    const long ch = (nb + FT - 1)/FT, j0 = t*ch, j1 = j0 + ch < nb ? j0 + ch : nb;
-    sqdd x[6]; unsigned long long c[5] = {0, 0, 0, 0, 0};
-    for(long j = j0; j < j1; j++){
-        const part_t &p = bp[j];
-        x[0] = x[0] + sqdd(p.S[0], p.S[1]); x[1] = x[1] + sqdd(p.A[0], p.A[1]); x[2] = x[2] + sqdd(p.drop[0], p.drop[1]);
-        x[3] = x[3] + sqdd(p.b1[0], p.b1[1]); x[4] = x[4] + sqdd(p.b2[0], p.b2[1]); x[5] = x[5] + sqdd(p.u[0], p.u[1]);
-        c[0] += p.ne; c[1] += p.nq; c[2] += p.unres; c[3] += p.skipped; c[4] += bkeep[j];
-    }
-    /* exclusive scan of the kept counts: warp scan, then across warps */
-    __shared__ unsigned long long wsum[FT/32], wpre[FT/32];
-    unsigned long long inc = c[4];
-    for(int off = 1; off < 32; off <<= 1){ unsigned long long y = __shfl_up_sync(0xffffffffu, inc, off); if(l >= off) inc += y; }
-    if(l == 31) wsum[w] = inc;
-    /* the sums: warp tree, then the warps' results */
+/* the tiles' offsets (exclusive scan of their kept counts) and the batch's sums, in a fixed order, added into the level
+ * accumulator; *base = this batch's first slot in the next list.  One CTA per FT tiles of an integral (blockIdx.y: the
+ * integral of a multi-instance batch, with its own accumulator and base), a tile per thread; the CTA that is
+ * done last adds the CTAs' sums and scans their kept counts (a tile's offset is boff[tile] after coff[its CTA]).  Latency
+ * bounds it: one CTA of 1024 threads, a run of consecutive tiles each, took 79 us for the 8192 tiles of a full batch,
+ * and the reduce kernel 52 us with a fallback point or more in a third of them; together 30 us now (syn_d8, h = 0.7). */
+__device__ __forceinline__ unsigned long long scan256(unsigned long long v, unsigned long long *ws, unsigned long long *total){
+    const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
+    unsigned long long inc = v;
+    for(int off = 1; off < 32; off <<= 1){ const unsigned long long y = __shfl_up_sync(0xffffffffu, inc, off); if(l >= off) inc += y; }
+    if(l == 31) ws[w] = inc;
+    __syncthreads();
+    unsigned long long o = inc - v, t = 0;
+    for(int q = 0; q < FT/32; q++){ if(q < w) o += ws[q]; t += ws[q]; }
+    __syncthreads();
+    *total = t;
+    return o;
+}
+/* the CTA's six sums and four counts, in warp w's lane 0 (sum w of x in warp w < 6, the counts in warp 6) */
+__device__ __forceinline__ void fin_sums(sqdd (&x)[6], unsigned long long (&c)[4], double (*wd)[12], unsigned long long (*wc)[4]){
+    const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
     for(int off = 16; off; off >>= 1){
+#pragma unroll
         for(int q = 0; q < 6; q++) x[q] = x[q] + shfl_dd(x[q], off);
+#pragma unroll
         for(int q = 0; q < 4; q++) c[q] += __shfl_down_sync(0xffffffffu, c[q], off);
     }
+    if(l == 0){
+#pragma unroll
+        for(int q = 0; q < 6; q++){ wd[w][2*q] = x[q].hi; wd[w][2*q + 1] = x[q].lo; }
+#pragma unroll
+        for(int q = 0; q < 4; q++) wc[w][q] = c[q];
+    }
+    __syncthreads();
+    if(w < 6){
+        sqdd y = l < FT/32 ? sqdd(wd[l][2*w], wd[l][2*w + 1]) : sqdd(0.0);
+        for(int off = FT/64; off; off >>= 1) y = y + shfl_dd(y, off);
+        x[0] = y;
+    } else if(w == 6) for(int q = 0; q < 4; q++){ c[q] = 0; for(int j = 0; j < FT/32; j++) c[q] += wc[j][q]; }
+}
+__global__ void __launch_bounds__(FT) sqb_k_finish(const __grid_constant__ lvl_t a, const part_t *bp, const unsigned *bkeep,
+                                                   long nb, unsigned long long *boff, sqb_acc_t *acc, unsigned long long *base,
+                                                   fpart_t *fp, unsigned long long *coff, unsigned *fcnt){
     __shared__ double wd[FT/32][12];
-    __shared__ unsigned long long wc[FT/32][4];
-    if(l == 0){ for(int q = 0; q < 6; q++){ wd[w][2*q] = x[q].hi; wd[w][2*q + 1] = x[q].lo; } for(int q = 0; q < 4; q++) wc[w][q] = c[q]; }
-    __syncthreads();
-    if(t == 0){ unsigned long long s = 0; for(int q = 0; q < FT/32; q++){ wpre[q] = s; s += wsum[q]; } }
-    __syncthreads();
-    { unsigned long long o = wpre[w] + inc - c[4]; for(long j = j0; j < j1; j++){ boff[j] = o; o += bkeep[j]; } }
-    if(w == 0){
-        sqdd y[6]; unsigned long long d[4];
-        for(int q = 0; q < 6; q++) y[q] = sqdd(wd[l][2*q], wd[l][2*q + 1]);
-        for(int q = 0; q < 4; q++) d[q] = wc[l][q];
-        for(int off = 16; off; off >>= 1){
-            for(int q = 0; q < 6; q++) y[q] = y[q] + shfl_dd(y[q], off);
-            for(int q = 0; q < 4; q++) d[q] += __shfl_down_sync(0xffffffffu, d[q], off);
+    __shared__ unsigned long long wc[FT/32][4], ws[FT/32];
+    __shared__ int last_;
+    const int t = threadIdx.x, w = t >> 5, l = t & 31, k = blockIdx.y;
+    long tb = 0;
+    if(a.ninst > 0){
+        const lvi_t &L = a.inst[k];
+        tb = L.child0/RTILE; nb = (L.n + RTILE - 1)/RTILE; acc = L.acc; base = L.base;
+    }
+    const long nch = (nb + FT - 1)/FT, ch = blockIdx.x, j = ch*FT + t;
+    if(ch >= nch) return;
+    const long slot0 = fin_slot(tb, k, tb);
+    sqdd x[6]; unsigned long long c[4] = {0, 0, 0, 0}, kp = 0, total;
+    if(j < nb){
+        const part_t &p = bp[tb + j];
+        x[0] = sqdd(p.S[0], p.S[1]); x[1] = sqdd(p.A[0], p.A[1]); x[2] = sqdd(p.drop[0], p.drop[1]);
+        x[3] = sqdd(p.b1[0], p.b1[1]); x[4] = sqdd(p.b2[0], p.b2[1]); x[5] = sqdd(p.u[0], p.u[1]);
+        c[0] = p.ne; c[1] = p.nq; c[2] = p.unres; c[3] = p.skipped; kp = bkeep[tb + j];
+    }
+    const unsigned long long o = scan256(kp, ws, &total);
+    if(j < nb) boff[tb + j] = o;
+    fin_sums(x, c, wd, wc);
+    if(nch > 1){
+        fpart_t &f = fp[slot0 + ch];
+        if(l == 0 && w < 6){ f.x[w][0] = x[0].hi; f.x[w][1] = x[0].lo; }
+        if(t == 192){ for(int q = 0; q < 4; q++) f.c[q] = c[q]; f.c[4] = total; }
+        __threadfence();
+        __syncthreads();
+        if(t == 0) last_ = atomicAdd(&fcnt[k], 1u) == (unsigned)nch - 1;
+        __syncthreads();
+        if(!last_) return;
+        __threadfence();
+        for(int q = 0; q < 6; q++) x[q] = sqdd(0.0);
+        for(int q = 0; q < 4; q++) c[q] = 0;
+        unsigned long long sum = 0;
+        for(long b = 0; b < nch; b += FT){
+            unsigned long long kc = 0;
+            if(b + t < nch){
+                const fpart_t &g = fp[slot0 + b + t];
+#pragma unroll
+                for(int q = 0; q < 6; q++) x[q] = x[q] + sqdd(__ldcg(&g.x[q][0]), __ldcg(&g.x[q][1]));
+#pragma unroll
+                for(int q = 0; q < 4; q++) c[q] += __ldcg(&g.c[q]);
+                kc = __ldcg(&g.c[4]);
+            }
+            const unsigned long long oc = scan256(kc, ws, &total);
+            if(b + t < nch) coff[slot0 + b + t] = sum + oc;
+            sum += total;
         }
-        if(l == 0){
-            const unsigned long long total = wpre[FT/32 - 1] + wsum[FT/32 - 1];
-            double *dst[6] = {acc->S, acc->A, acc->drop, acc->b1, acc->b2, acc->u};
-            for(int q = 0; q < 6; q++){ sqdd z = sqdd(dst[q][0], dst[q][1]) + y[q]; dst[q][0] = z.hi; dst[q][1] = z.lo; }
-            acc->ne += d[0]; acc->nq += d[1]; acc->unres += d[2]; acc->skipped += d[3];
-            *base = acc->keep; acc->keep += total;
-        }
+        total = sum;
+        fin_sums(x, c, wd, wc);
+        if(t == 0) fcnt[k] = 0;
+    } else if(t == 0) coff[slot0] = 0;
+    double *dst[6] = {acc->S, acc->A, acc->drop, acc->b1, acc->b2, acc->u};
+    if(l == 0 && w < 6){ const sqdd z = sqdd(dst[w][0], dst[w][1]) + x[0]; dst[w][0] = z.hi; dst[w][1] = z.lo; }
+    if(t == 192){
+        acc->ne += c[0]; acc->nq += c[1]; acc->unres += c[2]; acc->skipped += c[3];
+        *base = acc->keep; acc->keep += total;
     }
 }
 
 __global__ void __launch_bounds__(RT) sqb_k_scatter(const __grid_constant__ lvl_t a, const unsigned long long *boff,
-                                                    const unsigned long long *base, sqb_pt_t *next, long cap,
-                                                    unsigned long long *overflow){
-    const lvi_t L = lvl_inst(a, blockIdx.x);
+                                                    const unsigned long long *coff, const unsigned long long *base, sqb_pt_t *next,
+                                                    long cap, unsigned long long *overflow){
+    int ki;
+    const lvi_t L = lvl_inst(a, blockIdx.x, &ki);
+    const long slot = fin_slot(L.child0/RTILE, ki, blockIdx.x);
     if(a.ninst > 0){ base = L.base; next = L.next; cap = L.cap; overflow = &L.acc->overflow; }
     const long t0 = blockIdx.x*(long)RTILE + threadIdx.x*(long)RPT;
     unsigned mask = 0; int cnt = 0;
@@ -592,7 +681,7 @@ __global__ void __launch_bounds__(RT) sqb_k_scatter(const __grid_constant__ lvl_
     __syncthreads();
     if(threadIdx.x == 0){ int s = 0; for(int j = 0; j < RT/32; j++){ int y = ws[j]; ws[j] = s; s += y; } }
     __syncthreads();
-    unsigned long long o = *base + boff[blockIdx.x] + (unsigned long long)(ws[w] + x - cnt);
+    unsigned long long o = *base + coff[slot] + boff[blockIdx.x] + (unsigned long long)(ws[w] + x - cnt);
     const double thr10 = 10*L.thr, thr100 = 100*L.thr;
     for(unsigned b = mask; b; b &= b - 1){
         const long i = t0 + __ffs(b) - 1, il = i - L.child0;
@@ -754,11 +843,11 @@ extern "C" int sqb_dev_level(const sqb_level_t *L, sqb_acc_t *acc, long *next_n,
         }
         sqb_k_reduce<<<(unsigned)nb, RT, 0, G.s>>>(r, G.bp, G.bkeep, fused || queue ? G.tfb : NULL);
         CKR(cudaGetLastError());
-        sqb_k_finish<<<1, FT, 0, G.s>>>(r, G.bp, G.bkeep, nb, G.boff, G.acc, G.base);
+        sqb_k_finish<<<(unsigned)((nb + FT - 1)/FT), FT, 0, G.s>>>(r, G.bp, G.bkeep, nb, G.boff, G.acc, G.base, G.fp, G.coff, G.fcnt);
         CKR(cudaGetLastError());
         G.launches += 2;
         if(!L->last){
-            sqb_k_scatter<<<(unsigned)nb, RT, 0, G.s>>>(r, G.boff, G.base, L->next, L->next_cap, &G.acc->overflow);
+            sqb_k_scatter<<<(unsigned)nb, RT, 0, G.s>>>(r, G.boff, G.coff, G.base, L->next, L->next_cap, &G.acc->overflow);
             CKR(cudaGetLastError());
             G.launches++;
         }
@@ -886,11 +975,11 @@ extern "C" int sqb_dev_level_multi(const sqb_level_t *Ls, int n, sqb_acc_t *accs
         if(eval_batch(g, &a, &Ls[0].t, child0)) return -1;
         sqb_k_reduce<<<(unsigned)a.ntile, RT, 0, G.s>>>(rl, G.bp, G.bkeep, G.tfb);
         CKR(cudaGetLastError());
-        sqb_k_finish<<<(unsigned)m, FT, 0, G.s>>>(rl, G.bp, G.bkeep, 0, G.boff, NULL, NULL);
+        sqb_k_finish<<<dim3((unsigned)((a.ntile + FT - 1)/FT), (unsigned)m), FT, 0, G.s>>>(rl, G.bp, G.bkeep, 0, G.boff, NULL, NULL, G.fp, G.coff, G.fcnt);
         CKR(cudaGetLastError());
         G.launches += 2;
         if(!last){
-            sqb_k_scatter<<<(unsigned)a.ntile, RT, 0, G.s>>>(rl, G.boff, NULL, NULL, 0, NULL);
+            sqb_k_scatter<<<(unsigned)a.ntile, RT, 0, G.s>>>(rl, G.boff, G.coff, NULL, NULL, 0, NULL);
             CKR(cudaGetLastError());
             G.launches++;
         }
@@ -1174,7 +1263,12 @@ extern "C" double sqb_probe_fp64(int fma, long iters){
 extern "C" int sqb_level_tail(const void *cells, long nchildren, int D, int st, int last, int abskip, double pw, double thr,
                               const double *v, const double *uu, const unsigned char *stt,
                               void *bp, unsigned *bkeep, unsigned long long *boff, sqb_acc_t *acc, unsigned long long *base,
-                              void *next, long next_cap, void *stream){
+                              void *fin, void *next, long next_cap, void *stream){
+    /* fin: SQB_FIN_BYTES, zeroed before the first use: the finish kernel's counter, its offsets and its sums, of at most
+     * FT tiles */
+    if((nchildren + RTILE - 1)/RTILE > FT){ snprintf(g_err, sizeof g_err, "level tail: more than %d tiles", FT); return -1; }
+    static_assert(sizeof(fpart_t) + 32 <= SQB_FIN_BYTES, "the caller's room for the finish kernel");
+    unsigned *fcnt = (unsigned*)fin; unsigned long long *coff = (unsigned long long*)fin + 1; fpart_t *fp = (fpart_t*)((char*)fin + 32);
     lvl_t r; memset(&r, 0, sizeof r);        /* no symmetry fold here (r.sym.n = 0) */
     r.cells = (const signed char*)cells; r.n = nchildren; r.D = D; r.st = st; r.last = last;
     r.abskip = abskip; r.pw = pw; r.thr = thr; r.v = v; r.uu = uu; r.stt = stt;
@@ -1182,10 +1276,10 @@ extern "C" int sqb_level_tail(const void *cells, long nchildren, int D, int st, 
     cudaStream_t s = (cudaStream_t)stream;
     sqb_k_reduce<<<(unsigned)nb, RT, 0, s>>>(r, (part_t*)bp, bkeep, NULL);
     CKR(cudaGetLastError());
-    sqb_k_finish<<<1, FT, 0, s>>>(r, (const part_t*)bp, bkeep, nb, boff, acc, base);
+    sqb_k_finish<<<1, FT, 0, s>>>(r, (const part_t*)bp, bkeep, nb, boff, acc, base, fp, coff, fcnt);
     CKR(cudaGetLastError());
     if(!last){
-        sqb_k_scatter<<<(unsigned)nb, RT, 0, s>>>(r, boff, base, (sqb_pt_t*)next, next_cap, &acc->overflow);
+        sqb_k_scatter<<<(unsigned)nb, RT, 0, s>>>(r, boff, coff, base, (sqb_pt_t*)next, next_cap, &acc->overflow);
         CKR(cudaGetLastError());
     }
     return 0;

@@ -85,8 +85,8 @@ typedef struct {
     unsigned long long *nfb;
     long fbcap;
     /* level mode (test mode over cells, part != NULL): the FP64 pass also sums every tile of SQB_TILE
-     * children that needs no fallback (part, tkeep: kept count), and flags the others (tfb = 1) for the
-     * reduce kernel, which sums them after the double-double pass */
+     * children over those that need no fallback (part, tkeep: kept count) and flags the tiles with others (tfb = 2) for the
+     * reduce kernel, which adds them after the double-double pass (tfb = 1: it sums the whole tile) */
     sqb_part_t *part;
     unsigned *tkeep;
     unsigned char *tfb;

@@ -124,6 +124,8 @@ unsigned long long sqb_top_launches(void);
 void sqb_kernel_timing(int on);
 void sqb_kernel_times(double *f64_ms, double *dd_ms, long *f64_launches, int reset);
 
+#define SQB_FIN_BYTES 192              /* sqb_level_tail's scratch for the finish kernel */
+
 /* device memory for level lists */
 void *sqb_dev_alloc(size_t bytes);
 void  sqb_dev_free(void *p);

@@ -99,16 +99,17 @@ SQDD_HD sqdd operator/(const sqdd &a, const sqdd &b){
 }
 #endif
 
-/* a / b with r = RN(1/b) at hand (a table column and its reciprocal): the rounded quotient in five
+/* a / b with r = sqdd_rcp(b) at hand (a table column and its reciprocal): the rounded quotient in five
  * operations instead of a division's ten or more.  a r is within two ulp of a / b; one correction brings it
  * within one ulp, and a second, from its exact remainder, to RN(a / b) (Markstein's theorem: P. Markstein,
- * IBM J. Res. Dev. 34, 1990, 111), as long as nothing leaves the normal range: the quotient and the dividend
- * are checked to lie within 2^+-500, which bounds b and r too; any other (zeros, infinities, NaN) divides. */
-SQDD_HD bool sqdd_mid(double x){
+ * IBM J. Res. Dev. 34, 1990, 111), as long as nothing leaves the normal range.  One test sees to that: r is NaN unless b lies
+ * within 2^+-200, and the quotient is checked to lie within 2^+-700, so that a lies within 2^+-900 and the remainders,
+ * 2^-106 a at the least, are normal; any other operands (zeros, infinities, NaN) divide. */
+SQDD_HD bool sqdd_within(double x, int bits){
 #if defined(__CUDA_ARCH__)
-    return (((unsigned)__double2hiint(x) >> 20) & 0x7ff) - 523u < 1000u;
+    return (((unsigned)__double2hiint(x) >> 20) & 0x7ff) - (1023u - bits) < 2u*bits;
 #else
-    return fabs(x) >= 0x1p-500 && fabs(x) < 0x1p500;
+    return fabs(x) >= ldexp(1.0, -bits) && fabs(x) < ldexp(1.0, bits);
 #endif
 }
 #if defined(__CUDACC__)
@@ -118,9 +119,11 @@ static inline double sqdd_div_any(double a, double b){ return SQ_DIV(a, b); }
 #endif
 SQDD_HD double sq_divu(double a, double b, double r){
     const double q0 = SQ_MUL(a, r), q1 = SQ_FMA(SQ_FMA(-q0, b, a), r, q0), q2 = SQ_FMA(SQ_FMA(-q1, b, a), r, q1);
-    return sqdd_mid(a) && sqdd_mid(q1) ? q2 : sqdd_div_any(a, b);
+    return sqdd_within(q1, 700) ? q2 : sqdd_div_any(a, b);
 }
-/* a / b in double-double (operator/) with r = RN(1/b.hi): its three quotient digits by sq_divu */
+/* what a table keeps of a divisor: RN(1/b), of the high part; NaN if sq_divu is not to use it */
+SQDD_HD double sqdd_rcp(double b){ return sqdd_within(b, 200) ? SQ_DIV(1.0, b) : NAN; }
+/* a / b in double-double (operator/) with r = sqdd_rcp(b): its three quotient digits by sq_divu */
 SQDD_HD sqdd sq_divu(const sqdd &a, const sqdd &b, double r){
     double q1 = sq_divu(a.hi, b.hi, r);
     sqdd t = a - b*sqdd(q1);
@@ -130,9 +133,7 @@ SQDD_HD sqdd sq_divu(const sqdd &a, const sqdd &b, double r){
     sqdd q = sqdd_quick_two_sum(q1, q2);
     return q + sqdd(q3);
 }
-/* what a table keeps of a divisor: RN(1/b), of the high part */
-SQDD_HD double sqdd_rcp(double b){ return SQ_DIV(1.0, b); }
-SQDD_HD double sqdd_rcp(const sqdd &b){ return SQ_DIV(1.0, b.hi); }
+SQDD_HD double sqdd_rcp(const sqdd &b){ return sqdd_rcp(b.hi); }
 #if defined(__CUDA_ARCH__)
 /* the three quotient digits share one reciprocal: the same rounded quotients (sq_divu) for one division and fifteen
  * operations instead of three divisions */

@@ -183,7 +183,8 @@ __device__ __forceinline__ double sqb_point_test(const sqb_eval_t &a, const sqb_
     *fallback = false;
     if(noab) v = isfinite(fw) ? fw : 0.0;
     else {
-        const double bnd = abw*16*DBL_EPSILON/a.ddslack;
+        double bnd = abw*16*DBL_EPSILON;
+        if(a.ddslack != 1.0) bnd = bnd/a.ddslack;      /* x/1 = x: the default divides nothing */
         if(!(bnd <= I.near_thr)) s |= SQB_NEAR;
         if(!(bnd <= I.abserr)){
             s |= SQB_FALLBACK; v = 0.0; *fallback = true;
@@ -231,7 +232,7 @@ __device__ __forceinline__ void sqb_tile_flush(const sqb_eval_t &a, sqb_tile_acc
         p.S[0] = S.hi; p.S[1] = S.lo; p.A[0] = Ad.hi; p.A[1] = Ad.lo; p.drop[0] = dd.hi; p.drop[1] = dd.lo;
         p.b1[0] = b1.hi; p.b1[1] = b1.lo; p.b2[0] = b2.hi; p.b2[1] = b2.lo; p.u[0] = 0; p.u[1] = 0;
         p.ne = ne; p.nq = 0; p.unres = 0; p.skipped = nsk;
-        a.part[tile] = p; a.tkeep[tile] = keep; a.tfb[tile] = 0;
+        a.part[tile] = p; a.tkeep[tile] = keep;
     }
 }
 
@@ -319,8 +320,8 @@ __device__ __forceinline__ R sqb_axeval(const double *T, int K, const double *sf
  * points).
  * In level mode (a.part) each CTA also sums the tiles of its integrals that it is asked to (sqb_inst_t
  * fused): the children that need no fallback add v*pw and the rest into the thread's column of shared
- * memory; a tile with a fallback point, or of an integral the reduce kernel sums, is only flagged (a.tfb),
- * and the reduce kernel sums it after the double-double pass.
+ * memory; a tile with a fallback point is flagged (a.tfb = 2), and the reduce kernel adds those points after the
+ * double-double pass; a tile of an integral that the reduce kernel sums is only flagged (a.tfb = 1).
  * LV = 1 is the level kernel: the same pass compiled for level batches alone (cells of int8 coordinates,
  * tiles from the device queue, no list, no plain-form output), which leaves the other modes' code out of
  * the kernel that runs almost every point (measured 3-4 % faster on the three-loop graphs); with
@@ -437,8 +438,8 @@ __global__ void __launch_bounds__(SQB_BLOCK, SQB_MINB) sqb_k_f64(const __grid_co
 #if SQB_FUSE
         if(tsum){
             __syncthreads();
-            if(ta.fb){ if(t == 0) a.tfb[tile] = 1; }
-            else sqb_tile_flush(a, ta, tile);
+            sqb_tile_flush(a, ta, tile);
+            if(t == 0) a.tfb[tile] = ta.fb ? 2 : 0;
             __syncthreads();
         } else
 #endif
@@ -499,64 +500,97 @@ __global__ void __launch_bounds__(SQB_BLOCK) sqb_k_ax(const __grid_constant__ sq
  * order of (cell, first axes): a warp's writes for one choice of the last axes are 2^(D-3) consecutive
  * children.  The thread's sums stay in registers.  Every child's value is the general kernel's bit for bit; the
  * tile sums add the same values in another fixed order.  Measured on the B200, whole last level against the
- * general kernel: syn_d8 at h = 0.7 (1.18e9 children) 125.4 -> 21.8 ms, syn_d11 at h = 2 (9.2e8) 93.6 -> 16.9 ms,
- * syn_d5 at h = 1 (2.7e6) 0.40 -> 0.12 ms. */
+ * general kernel: syn_d8 at h = 0.7 (1.18e9 children) 125.4 -> 17.0 ms, syn_d11 at h = 2 (9.2e8) 93.6 -> 13.8 ms,
+ * syn_d5 at h = 1 (2.7e6) 0.40 -> 0.12 ms; this kernel 11.7 ps a child of syn_d8, with five CTAs an SM (96 registers, 84 bytes
+ * spilled; four without a spill 12.1, six 12.2).  FP64 dependences bound it: the pipe is half busy. */
 #define SQB_AXG 8
 #ifndef SQB_AX_MINB
 #define SQB_AX_MINB 5
 #endif
-struct sqb_ax_acc { sqdd S, b1, b2; double A, dr; unsigned ne, nsk, keep; bool fb; };
+/* a thread's sums: S, b1, b2 as (hi, running error), normalised at the tile's end */
+struct sqb_ax_acc { double S, Se, b1, b1e, b2, b2e, A, dr; unsigned ne, nsk, keep; bool fb; };
+__device__ __forceinline__ void sqb_ax_add(double &s, double &e, double x){
+    const sqdd z = sqdd_two_sum(s, x);
+    s = z.hi; e = SQ_ADD(e, z.lo);
+}
+/* an integral's fields in registers (in shared memory every store to global memory would have them read again) */
+struct sqb_ax_in { const double *U, *sX, *sW; int K, st, last; bool tsum; double pw, thr, abserr, near_thr, slack; };
 
 template<class F, int D, int AB>
-__device__ __forceinline__ void sqb_ax_group(const sqb_eval_t &a, const sqb_inst_t &I, const double *sX, const double *sW,
-                                             const int *k, int low, int sk, int tier, long i0, bool tsum, sqb_ax_acc &t){
+__device__ __forceinline__ void sqb_ax_group(const sqb_eval_t &a, const sqb_ax_in &I, const int *k, int low, int sk, int tier, long i0,
+                                             sqb_ax_acc &t){
     using A = typename F::template AX<double, AB>;
     constexpr int M = D - 3, EW = sqb_axw<A, double>::N;
     const int K = I.K, st = I.st, nt = 2*K + 1;
-    const double *U = I.U + K*EW;
+    /* the axes along which the lower child lies below the box; its coordinate is clamped, and the children with such a
+     * bit are no points */
+    int out = 0;
+#pragma unroll
+    for(int d = 0; d < D; d++) out |= (k[d] - st < -K) << d;
     typename A::st S0;
     A::init(S0);
-    double w0 = 1.0; bool in0 = true;
+    double w0 = 1.0;
 #pragma unroll
     for(int d = 0; d < M; d++){
         int kd = k[d] - (((low >> d) & 1) ? st : 0);
-        if(kd < -K){ in0 = false; kd = -K; }
-        sqb_axstep<A, double>(S0, sX[kd + K], U + (d*nt + kd)*EW);
-        w0 = w0*sW[kd + K];
+        kd = kd < -K ? 0 : kd + K;
+        sqb_axstep<A, double>(S0, I.sX[kd], I.U + (d*nt + kd)*EW);
+        w0 = w0*I.sW[kd];
     }
+    double *const v = a.v + i0; unsigned char *const stt = a.stt + i0;
+    const unsigned char s0 = SQB_PRESENT | (sk ? SQB_SKIPPED : 0);
+    unsigned added = 0;
+    const int kl = k[D - 1] - st < -K ? 0 : k[D - 1] - st + K, kh = k[D - 1] + K;      /* the last axis' two entries */
 #pragma unroll 1
     for(int h = 0; h < 4; h++){
-        typename A::st S1 = S0; double w1 = w0; bool in1 = in0;
+        typename A::st S1 = S0; double w1 = w0;
 #pragma unroll
         for(int q = 0; q < 2; q++){
             int kd = k[M + q] - (((h >> q) & 1) ? st : 0);
-            if(kd < -K){ in1 = false; kd = -K; }
-            sqb_axstep<A, double>(S1, sX[kd + K], U + ((M + q)*nt + kd)*EW);
-            w1 = w1*sW[kd + K];
+            kd = kd < -K ? 0 : kd + K;
+            sqb_axstep<A, double>(S1, I.sX[kd], I.U + ((M + q)*nt + kd)*EW);
+            w1 = w1*I.sW[kd];
+        }
+        double fw[2], abw[2];
+#pragma unroll
+        for(int b = 0; b < 2; b++){
+            const int kd = b ? kl : kh;
+            typename A::st S2 = S1;
+            sqb_axstep<A, double>(S2, I.sX[kd], I.U + ((D - 1)*nt + kd)*EW);
+            const double w = w1*I.sW[kd];
+            double ab = 0;
+            fw[b] = A::fin(S2, &ab)*w; abw[b] = ab*w;
         }
 #pragma unroll
         for(int b = 0; b < 2; b++){
-            const long i = i0 + ((long)(h + 4*b) << M);
-            int kd = k[D - 1] - (b ? st : 0);
-            if(!in1 || kd < -K){ a.v[i] = 0; a.stt[i] = 0; continue; }
-            typename A::st S2 = S1;
-            sqb_axstep<A, double>(S2, sX[kd + K], U + ((D - 1)*nt + kd)*EW);
-            const double w = w1*sW[kd + K];
-            double ab = 0;
-            const double f = A::fin(S2, &ab);
-            bool fallback;
-            const double v = sqb_point_test(a, I, i, sk, AB == 0, f*w, ab*w, &fallback);
-            if(!tsum) continue;
+            const int o = (h + 4*b) << M;
+            if((low | o) & out){ v[o] = 0; stt[o] = 0; continue; }
+            /* finish()'s tests, as sqb_point_test */
+            unsigned char s = s0; bool fallback = false;
+            double x = isfinite(fw[b]) ? fw[b] : 0.0;
+            if(AB){
+                double bnd = abw[b]*16*DBL_EPSILON;
+                if(I.slack != 1.0) bnd = bnd/I.slack;              /* x/1 = x: the default divides nothing */
+                if(!(bnd <= I.near_thr)) s |= SQB_NEAR;
+                if(!(bnd <= I.abserr)){
+                    s |= SQB_FALLBACK; x = 0.0; fallback = true;
+                    const unsigned long long q = atomicAdd(a.nfb, 1ULL);
+                    if((long)q < a.fbcap) a.fb[q] = i0 + o;
+                }
+            }
+            v[o] = x; stt[o] = s;
+            if(!I.tsum) continue;
             if(fallback){ t.fb = true; continue; }
-            const double vp = v*I.pw, av = fabs(v);
-            t.S = sqdd_add_d(t.S, vp); t.A += av; t.ne++; t.nsk += sk ? 1 : 0;
+            const double vp = x*I.pw, av = fabs(x);
+            sqb_ax_add(t.S, t.Se, vp); t.A += av; added++;
             if(I.last){
-                if(tier >= 1) t.b1 = sqdd_add_d(t.b1, vp);
-                if(tier >= 2) t.b2 = sqdd_add_d(t.b2, vp);
+                if(tier >= 1) sqb_ax_add(t.b1, t.b1e, vp);
+                if(tier >= 2) sqb_ax_add(t.b2, t.b2e, vp);
             } else if(av >= I.thr) t.keep++;
             else t.dr += av*I.pw;
         }
     }
+    t.ne += added; t.nsk += sk ? added : 0;
 }
 
 template<class F, int D>
@@ -581,40 +615,43 @@ __global__ void __launch_bounds__(SQB_BLOCK, SQB_AX_MINB) sqb_k_lvax(const __gri
         const sqb_inst_t &I = sI[ki];
         const double *sX = sqb_sm + I.toff, *sW = sX + (2*I.K + 1);
         const bool tsum = I.fused != 0;
-        const long g0 = (tile*SQB_TILE - I.child0)/SQB_AXG + (item - tile*sub)*gper;
-        sqb_ax_acc ac; ac.A = ac.dr = 0; ac.ne = ac.nsk = ac.keep = 0; ac.fb = false;
+        const sqb_ax_in in = {I.U, sX, sW, I.K, I.st, I.last, tsum, I.pw, I.thr, I.abserr, I.near_thr, a.ddslack};
+        const int *const pts = (const int*)I.pts;
+        const long ncell = I.n, child0 = I.child0;
+        const long g0 = (tile*SQB_TILE - child0)/SQB_AXG + (item - tile*sub)*gper;
+        sqb_ax_acc ac = {0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, false};
         for(int j = t; j < gper; j += SQB_BLOCK){
             const long gi = g0 + j, c = gi >> M;
-            if(c >= I.n) break;
+            if(c >= ncell) break;
             const int low = (int)(gi & ((1 << M) - 1));
-            union { int w[3]; signed char k[12]; } p;
-            const int *src = (const int*)((const signed char*)I.pts + c*12);
-            p.w[0] = src[0]; p.w[1] = src[1]; p.w[2] = src[2];
+            const int *src = pts + c*3;
+            const int w3[3] = {src[0], src[1], src[2]};
             int k[D];
 #pragma unroll
-            for(int d = 0; d < D; d++) k[d] = (int)(signed char)(p.w[d >> 2] >> (8*(d & 3)));
-            const int fl = (int)(signed char)(p.w[2] >> 24);
+            for(int d = 0; d < D; d++) k[d] = (int)(signed char)(w3[d >> 2] >> (8*(d & 3)));
+            const int fl = w3[2] >> 24;
             const int sk = a.abskip && (fl & 1);
-            const long i0 = (c << D) + low + I.child0;
-            if(sk && !a.abcheck) sqb_ax_group<F, D, 0>(a, I, sX, sW, k, low, sk, (fl >> 1) & 3, i0, tsum, ac);
-            else                 sqb_ax_group<F, D, 1>(a, I, sX, sW, k, low, sk, (fl >> 1) & 3, i0, tsum, ac);
+            const long i0 = (c << D) + low + child0;
+            if(sk && !a.abcheck) sqb_ax_group<F, D, 0>(a, in, k, low, sk, (fl >> 1) & 3, i0, ac);
+            else                 sqb_ax_group<F, D, 1>(a, in, k, low, sk, (fl >> 1) & 3, i0, ac);
         }
         const int fb = __syncthreads_or(tsum && ac.fb);
-        if(!tsum || fb){ if(t == 0) a.tfb[tile] = 1; continue; }       /* summed by the reduce kernel */
+        if(!tsum){ if(t == 0) a.tfb[tile] = 1; continue; }             /* summed by the reduce kernel */
+        sqdd S = sqdd_two_sum(ac.S, ac.Se), b1 = sqdd_two_sum(ac.b1, ac.b1e), b2 = sqdd_two_sum(ac.b2, ac.b2e);
         sqdd Ad(ac.A), dd(ac.dr);
         for(int off = 16; off; off >>= 1){
-            ac.S = ac.S + sqdd(__shfl_down_sync(0xffffffffu, ac.S.hi, off), __shfl_down_sync(0xffffffffu, ac.S.lo, off));
+            S = S + sqdd(__shfl_down_sync(0xffffffffu, S.hi, off), __shfl_down_sync(0xffffffffu, S.lo, off));
             Ad = Ad + sqdd(__shfl_down_sync(0xffffffffu, Ad.hi, off), __shfl_down_sync(0xffffffffu, Ad.lo, off));
             dd = dd + sqdd(__shfl_down_sync(0xffffffffu, dd.hi, off), __shfl_down_sync(0xffffffffu, dd.lo, off));
-            ac.b1 = ac.b1 + sqdd(__shfl_down_sync(0xffffffffu, ac.b1.hi, off), __shfl_down_sync(0xffffffffu, ac.b1.lo, off));
-            ac.b2 = ac.b2 + sqdd(__shfl_down_sync(0xffffffffu, ac.b2.hi, off), __shfl_down_sync(0xffffffffu, ac.b2.lo, off));
+            b1 = b1 + sqdd(__shfl_down_sync(0xffffffffu, b1.hi, off), __shfl_down_sync(0xffffffffu, b1.lo, off));
+            b2 = b2 + sqdd(__shfl_down_sync(0xffffffffu, b2.hi, off), __shfl_down_sync(0xffffffffu, b2.lo, off));
             ac.ne += __shfl_down_sync(0xffffffffu, ac.ne, off); ac.nsk += __shfl_down_sync(0xffffffffu, ac.nsk, off);
             ac.keep += __shfl_down_sync(0xffffffffu, ac.keep, off);
         }
         if((t & 31) == 0){
             double *x = wd[t >> 5];
-            x[0] = ac.S.hi; x[1] = ac.S.lo; x[2] = Ad.hi; x[3] = Ad.lo; x[4] = dd.hi; x[5] = dd.lo;
-            x[6] = ac.b1.hi; x[7] = ac.b1.lo; x[8] = ac.b2.hi; x[9] = ac.b2.lo;
+            x[0] = S.hi; x[1] = S.lo; x[2] = Ad.hi; x[3] = Ad.lo; x[4] = dd.hi; x[5] = dd.lo;
+            x[6] = b1.hi; x[7] = b1.lo; x[8] = b2.hi; x[9] = b2.lo;
             wc[t >> 5][0] = ac.ne; wc[t >> 5][1] = ac.nsk; wc[t >> 5][2] = ac.keep;
         }
         __syncthreads();
@@ -629,7 +666,7 @@ __global__ void __launch_bounds__(SQB_BLOCK, SQB_AX_MINB) sqb_k_lvax(const __gri
             for(int w = 0; w < SQB_BLOCK/32; w++){ ne += wc[w][0]; nsk += wc[w][1]; keep += wc[w][2]; }
             sqb_part_t &P = a.part[tile];
             P.u[0] = P.u[1] = 0; P.ne = ne; P.nq = 0; P.unres = 0; P.skipped = nsk;
-            a.tkeep[tile] = keep; a.tfb[tile] = 0;
+            a.tkeep[tile] = keep; a.tfb[tile] = fb ? 2 : 0;
         }
     }
 }

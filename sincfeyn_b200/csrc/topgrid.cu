@@ -392,7 +392,8 @@ struct gpart_t { u64 q; double f[4][2]; u64 nq, unres; };    /* one tile of a fr
 #define CL 8                     /* CTAs of the one-cluster kernels, and their threads */
 #define CT 512
 #define CL_MAX ((long)CL*CT)     /* points of a frontier that one cluster takes: one per thread.  With four per thread
-                                    the grow of d = 5, h = 1 (16 frontiers up to 12,000 points) took 1.24 ms, with one 0.95 */
+                                    the whole sum of d = 5, h = 1 (16 frontiers up to 12,000 points) took 1.76 ms, with one
+                                    1.40, without the cluster 1.67 */
 struct clpart_t { gpart_t s; drop_t d; double a; u64 nk, nw; };                /* one of its CTAs' sums and counts */
 struct Grow {
     geom_t g;
@@ -648,7 +649,7 @@ struct WinOp {                   /* winners in id order become the next frontier
 /* A frontier of up to CL_MAX points in one cluster: sums, threshold, kept points, claims and the next frontier, with
  * a cluster barrier between the steps.  Latency bounds a frontier of this size; as seven launches (sums, kept points in
  * one CTA, claims, winners counted and emitted) the same steps
- * made the grow of d = 5, h = 1.5 0.66 ms (10 frontiers, 8816 points); 0.52 with this.  CTA r takes the r-th eighth of the points
+ * took 0.66 ms for the grow of d = 5, h = 1.5 (10 frontiers, 8816 points); 0.59 with this.  CTA r takes the r-th eighth of the points
  * and of the candidates, a thread a run of consecutive ones, so that one scan per CTA ranks them. */
 __global__ void __cluster_dims__(CL, 1, 1) __launch_bounds__(CT)
 k_frontier(geom_t g, KeepOp ko, WinOp wo, const double *uu, long n, u64 *key, u64 mask, long *qs, gacc_t *acc, gacc_t *host, clpart_t *part){
