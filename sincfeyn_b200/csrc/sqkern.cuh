@@ -507,6 +507,9 @@ __global__ void __launch_bounds__(SQB_BLOCK) sqb_k_ax(const __grid_constant__ sq
 #ifndef SQB_AX_MINB
 #define SQB_AX_MINB 5
 #endif
+#ifndef SQB_AX_UNROLL
+#define SQB_AX_UNROLL 1
+#endif
 /* a thread's sums: S, b1, b2 as (hi, running error), normalised at the tile's end */
 struct sqb_ax_acc { double S, Se, b1, b1e, b2, b2e, A, dr; unsigned ne, nsk, keep; bool fb; };
 __device__ __forceinline__ void sqb_ax_add(double &s, double &e, double x){
@@ -541,7 +544,8 @@ __device__ __forceinline__ void sqb_ax_group(const sqb_eval_t &a, const sqb_ax_i
     const unsigned char s0 = SQB_PRESENT | (sk ? SQB_SKIPPED : 0);
     unsigned added = 0;
     const int kl = k[D - 1] - st < -K ? 0 : k[D - 1] - st + K, kh = k[D - 1] + K;      /* the last axis' two entries */
-#pragma unroll 1
+    constexpr int UN = SQB_AX_UNROLL;
+#pragma unroll UN
     for(int h = 0; h < 4; h++){
         typename A::st S1 = S0; double w1 = w0;
 #pragma unroll

@@ -80,10 +80,34 @@ __device__ long h_find(const u64 *key, u64 mask, u64 y){
 /* sh: log2 of the step */
 struct geom_t { int D, K, st, sh, W; u64 P[SQB_MAXD]; };
 
-__device__ __forceinline__ u64 key_of(const geom_t &g, const signed char *k){
+/* a point of this file's lists as three words (the lists are 4-byte aligned; byte 11 is the flags) */
+struct pt3 { unsigned w[3]; };
+__device__ __forceinline__ pt3 ld_pt(const sqb_pt_t *p){ const unsigned *q = (const unsigned*)p; return {{q[0], q[1], q[2]}}; }
+__device__ __forceinline__ void st_pt(sqb_pt_t *p, const pt3 &x){ unsigned *q = (unsigned*)p; q[0] = x.w[0]; q[1] = x.w[1]; q[2] = x.w[2]; }
+__device__ __forceinline__ int pt_byte(const pt3 &x, int d){
+    const unsigned w = d < 4 ? x.w[0] : d < 8 ? x.w[1] : x.w[2];
+    return (int)(signed char)(w >> (8*(d & 3)));
+}
+__device__ __forceinline__ void pt_add(pt3 &x, int d, int v){            /* k[d] += v (no overflow of the byte) */
+    const unsigned b = ((unsigned)v & 0xffu) << (8*(d & 3));
+    if(d < 4) x.w[0] = __vadd4(x.w[0], b); else if(d < 8) x.w[1] = __vadd4(x.w[1], b); else x.w[2] = __vadd4(x.w[2], b);
+}
+__device__ __forceinline__ void pt_flag(pt3 &x, int f){ x.w[2] = (x.w[2] & 0x00ffffffu) | ((unsigned)(f & 0xff) << 24); }
+/* max |k_d| */
+__device__ __forceinline__ int pt_max(const pt3 &x){
+    unsigned m = __vmaxu4(__vabs4(x.w[0]), __vmaxu4(__vabs4(x.w[1]), __vabs4(x.w[2] & 0x00ffffffu)));
+    m = __vmaxu4(m, m >> 16);
+    return (int)max(m & 0xffu, (m >> 8) & 0xffu);
+}
+__device__ __forceinline__ u64 key_pt(const geom_t &g, const pt3 &x){
     u64 y = 1;
-    for(int i = 0; i < g.D; i++) y = y*g.W + (u64)((k[i] + g.K) >> g.sh);
+    for(int i = 0; i < g.D; i++) y = y*g.W + (u64)((pt_byte(x, i) + g.K) >> g.sh);
     return y;
+}
+/* x = q n + r, in 32 bits where they do */
+__device__ __forceinline__ void split(long x, int n, long *q, int *r){
+    if(x <= 0xFFFFFFFFL){ const unsigned y = (unsigned)x/(unsigned)n; *q = y; *r = (int)((unsigned)x - y*(unsigned)n); }
+    else { *q = x/n; *r = (int)(x - *q*n); }
 }
 
 /* the grow's counters and sums, in device memory and, after each wait, in pinned host memory */
@@ -155,12 +179,13 @@ template<int T, int NQ, int NC> struct sums_sh { double h[NQ][T/32], l[NQ][T/32]
 template<int T, int NQ, int NC> __device__ void block_sums(sqdd (&x)[NQ], u64 (&c)[NC], sums_sh<T, NQ, NC> &sh){
     static_assert(NQ + NC <= T/32, "a warp for each sum");
     const int l = threadIdx.x & 31, w = threadIdx.x >> 5;
-    for(int off = 16; off; off >>= 1){
+    /* a sum that is zero in the whole warp (the shells, the round column mostly) has no tree */
 #pragma unroll
-        for(int q = 0; q < NQ; q++) x[q] = x[q] + dd_shfl(x[q], off);
+    for(int q = 0; q < NQ; q++)
+        if(__any_sync(0xffffffffu, x[q].hi != 0)) for(int off = 16; off; off >>= 1) x[q] = x[q] + dd_shfl(x[q], off);
 #pragma unroll
-        for(int q = 0; q < NC; q++) c[q] += __shfl_down_sync(0xffffffffu, c[q], off);
-    }
+    for(int q = 0; q < NC; q++)
+        if(__any_sync(0xffffffffu, c[q] != 0)) for(int off = 16; off; off >>= 1) c[q] += __shfl_down_sync(0xffffffffu, c[q], off);
     if(l == 0){
 #pragma unroll
         for(int q = 0; q < NQ; q++){ sh.h[q][w] = x[q].hi; sh.l[q][w] = x[q].lo; }
@@ -257,7 +282,7 @@ __device__ __forceinline__ long cnt_of(const cnt_t &c){
     return n < c.max ? n : c.max;
 }
 template<class Op, int I>
-__global__ void __launch_bounds__(TG_T) k_count(Op op, cnt_t cn, unsigned *bcnt, drop_t *drop){
+__global__ void __launch_bounds__(TG_T) k_count(const __grid_constant__ Op op, cnt_t cn, unsigned *bcnt, drop_t *drop){
     __shared__ u64 ws[TG_T/32];
     __shared__ sums_sh<TG_T, 2, 2> wd;
     const long n = cnt_of(cn), b0 = blockIdx.x*(long)(TG_T*I);
@@ -310,7 +335,7 @@ __device__ __forceinline__ void publish(const gacc_t *acc, gacc_t *host){
     for(unsigned w = threadIdx.x; w < sizeof(gacc_t)/8; w += 32) d[w] = s[w];
 }
 template<class Op, int I>
-__global__ void __launch_bounds__(TG_T) k_emit(Op op, cnt_t cn, emit_t e){
+__global__ void __launch_bounds__(TG_T) k_emit(const __grid_constant__ Op op, cnt_t cn, emit_t e){
     __shared__ u64 ws[TG_T/32];
     __shared__ sums_sh<TG_T, 2, 1> wd;
     const long n = cnt_of(cn), b0 = blockIdx.x*(long)(TG_T*I);
@@ -399,7 +424,7 @@ struct Grow {
     geom_t g;
     u64 *key; unsigned *word; u64 mask; long nseen;   /* seen table */
     sqb_pt_t *fr, *nx; unsigned char *frsk, *nxsk; long nfr, frcap;         /* frontier, next */
-    sqb_pt_t *keep; double *kv; long nkeep, keepcap;                        /* kept so far */
+    sqb_pt_t *keep; double *kv; u64 *kk; long nkeep, keepcap;               /* kept so far: points, values, keys */
     long *kj; long kjcap;                                                  /* this frontier's kept */
     long *qs; long qscap;                                                  /* slot per candidate */
     gpart_t *part; long partcap; clpart_t *cpart;                          /* sums per tile; per CTA of a cluster */
@@ -460,7 +485,7 @@ static int frontier_room(long n){
 /* z = 0 into the table and the frontier, the record cleared, and the zero probe's nodes (driver/sum.c:346-359): z = 0
  * and NPROBE nodes from a fixed hash */
 #define NPROBE 4096
-__global__ void k_seed(geom_t g, u64 *key, unsigned *word, u64 mask, u64 y0, sqb_pt_t *fr, unsigned char *frsk, gacc_t *acc,
+__global__ void k_seed(const __grid_constant__ geom_t g, u64 *key, unsigned *word, u64 mask, u64 y0, sqb_pt_t *fr, unsigned char *frsk, gacc_t *acc,
                        double eps, double pw, sqb_pt_t *probe){
     const int j = blockIdx.x*blockDim.x + threadIdx.x;
     if(j == 0){
@@ -527,15 +552,14 @@ __device__ __forceinline__ void fsum_add(sqdd (&f)[4], u64 &nq, u64 &unres, cons
                                          const unsigned char *stt, const double *uu, double pw, long i){
     const double x = __dmul_rn(v[i], pw), w = fabs(x);
     f[0] = sqdd_add_d(f[0], x);
-    int mx = 0;                               /* driver/sumkey.h:236-238 */
-    for(int d = 0; d < g.D; d++){ const int y = abs((int)fr[i].k[d]); mx = y > mx ? y : mx; }
+    const int mx = pt_max(ld_pt(fr + i));     /* driver/sumkey.h:236-238 */
     if(mx == g.K) f[1] = sqdd_add_d(f[1], w); else if(mx == g.K - g.st) f[2] = sqdd_add_d(f[2], w);
     const unsigned char s = stt[i];
     if(s & SQB_FALLBACK){ nq++; f[3] = sqdd_add_d(f[3], uu[i]); }
     if(s & SQB_UNRES) unres++;
 }
 /* per tile of GS_TILE points: the sums, and the running sum's additions in units of its binade */
-__global__ void __launch_bounds__(TG_T) k_gs_tiles(geom_t g, const sqb_pt_t *fr, const double *v, const unsigned char *stt,
+__global__ void __launch_bounds__(TG_T) k_gs_tiles(const __grid_constant__ geom_t g, const sqb_pt_t *fr, const double *v, const unsigned char *stt,
                                                    const double *uu, long n, const gacc_t *acc, gpart_t *part){
     __shared__ sums_sh<TG_T, 4, 4> sh;
     const double pw = acc->pw; double inv = 0, u;
@@ -596,36 +620,35 @@ __global__ void __launch_bounds__(GT) k_gs_total(const double *v, long n, gacc_t
     }
 }
 
-struct KeepOp {                  /* kept frontier points appended to the keep list, their index to kj */
+struct KeepOp {                  /* kept frontier points and their keys appended to the keep list, their index to kj */
     enum { DROP = 1 };
-    const sqb_pt_t *fr; const double *v; const unsigned char *stt; const gacc_t *acc; int abskip, D;
-    sqb_pt_t *keep; double *kv; long *kj; u64 base;
+    geom_t g; const sqb_pt_t *fr; const double *v; const unsigned char *stt; const gacc_t *acc; int abskip;
+    sqb_pt_t *keep; double *kv; u64 *kk; long *kj; u64 base;
     __device__ bool pred(long i) const { return fabs(v[i]) >= acc->thr; }
     __device__ double weight(long i) const { return __dmul_rn(v[i], acc->pw); }
     __device__ void emit(long i, u64 r) const {
-        sqb_pt_t p; for(int q = 0; q < SQB_MAXD; q++) p.k[q] = 0;
-        for(int d = 0; d < D; d++) p.k[d] = fr[i].k[d];
-        if(abskip) p.k[SQB_PFLAG] = (stt[i] & SQB_NEAR) ? 0 : 1;
-        keep[base + r] = p; kv[base + r] = fabs(v[i]); kj[r] = i;
+        pt3 p = ld_pt(fr + i);
+        kk[base + r] = key_pt(g, p);
+        pt_flag(p, abskip && !(stt[i] & SQB_NEAR));
+        st_pt(keep + base + r, p); kv[base + r] = fabs(v[i]); kj[r] = i;
     }
 };
-/* candidate id = (kept point, axis, sign): its slot in the table, and its claim */
-__device__ __forceinline__ void claim_one(const geom_t &g, const sqb_pt_t *fr, const long *kj, u64 *key, unsigned *word, u64 mask,
+/* candidate id = (kept point j of this frontier, axis, sign): its slot in the table, and its claim; keep, kk: the
+ * frontier's part of the keep list */
+__device__ __forceinline__ void claim_one(const geom_t &g, const sqb_pt_t *keep, const u64 *kk, u64 *key, unsigned *word, u64 mask,
                                           long *qs, gacc_t *acc, long id){
-    const int D2 = 2*g.D;
-    const long j = id/D2; const int c = (int)(id - j*D2), d = c >> 1, sg = (c & 1) ? 1 : -1;
-    const signed char *k = fr[kj[j]].k;
-    const int kk = k[d] + g.st*sg;
-    if(kk > g.K || kk < -g.K){ qs[id] = -1; return; }
-    const u64 y = key_of(g, k) + (sg > 0 ? g.P[d] : (u64)0 - g.P[d]);
-    int nw; const long q = h_insert(key, mask, y, &nw);
+    long j; int c;
+    split(id, 2*g.D, &j, &c);
+    const int d = c >> 1, sg = (c & 1) ? 1 : -1, kx = keep[j].k[d] + g.st*sg;
+    if(kx > g.K || kx < -g.K){ qs[id] = -1; return; }
+    int nw; const long q = h_insert(key, mask, kk[j] + (sg > 0 ? g.P[d] : (u64)0 - g.P[d]), &nw);
     qs[id] = q;
     if(q < 0) atomicAdd(&acc->err, 1ULL); else atomicMax(&word[q], CLAIM(id));
 }
-__global__ void k_claim(geom_t g, const sqb_pt_t *fr, const long *kj, u64 *key, unsigned *word, u64 mask, long *qs, gacc_t *acc){
+__global__ void k_claim(const __grid_constant__ geom_t g, const sqb_pt_t *keep, const u64 *kk, u64 *key, unsigned *word, u64 mask, long *qs, gacc_t *acc){
     const long nc = (long)acc->nk*2*g.D;
     for(long id = blockIdx.x*(long)blockDim.x + threadIdx.x; id < nc; id += (long)gridDim.x*blockDim.x)
-        claim_one(g, fr, kj, key, word, mask, qs, acc, id);
+        claim_one(g, keep, kk, key, word, mask, qs, acc, id);
 }
 struct WinOp {                   /* winners in id order become the next frontier */
     enum { DROP = 0 };
@@ -633,15 +656,17 @@ struct WinOp {                   /* winners in id order become the next frontier
     sqb_pt_t *nx; unsigned char *nxsk; int D2, st, gs; u64 base;
     __device__ bool pred(long id) const { const long q = qs[id]; return q >= 0 && word[q] == CLAIM(id); }
     __device__ void emit(long id, u64 r) const {
-        const long j = id/D2; const int c = (int)(id - j*D2), d = c >> 1, sg = (c & 1) ? 1 : -1;
+        long j; int c;
+        split(id, D2, &j, &c);
         const long pi = kj[j];
-        sqb_pt_t p = fr[pi];
-        p.k[d] = (signed char)(p.k[d] + st*sg);
-        if(gs){ const int pg = fr[pi].k[SQB_PFLAG];
-            p.k[SQB_PFLAG] = (signed char)(!frsk[pi] ? ((stt[pi] & SQB_NEAR) ? 0 : 1) : (pg < gs ? pg + 1 : 0));
-            nxsk[r] = p.k[SQB_PFLAG] > 0; }
-        else p.k[SQB_PFLAG] = 0;
-        nx[r] = p;
+        pt3 p = ld_pt(fr + pi);
+        int fl = 0;
+        if(gs){ const int pg = pt_byte(p, SQB_PFLAG);
+            fl = !frsk[pi] ? ((stt[pi] & SQB_NEAR) ? 0 : 1) : (pg < gs ? pg + 1 : 0);
+            nxsk[r] = fl > 0; }
+        pt_add(p, c >> 1, (c & 1) ? st : -st);
+        pt_flag(p, fl);
+        st_pt(nx + r, p);
         word[qs[id]] = SEEN;
     }
 };
@@ -652,11 +677,12 @@ struct WinOp {                   /* winners in id order become the next frontier
  * took 0.66 ms for the grow of d = 5, h = 1.5 (10 frontiers, 8816 points); 0.59 with this.  CTA r takes the r-th eighth of the points
  * and of the candidates, a thread a run of consecutive ones, so that one scan per CTA ranks them. */
 __global__ void __cluster_dims__(CL, 1, 1) __launch_bounds__(CT)
-k_frontier(geom_t g, KeepOp ko, WinOp wo, const double *uu, long n, u64 *key, u64 mask, long *qs, gacc_t *acc, gacc_t *host, clpart_t *part){
+k_frontier(const __grid_constant__ KeepOp ko, const __grid_constant__ WinOp wo, const double *uu, long n, u64 *key, u64 mask, long *qs, gacc_t *acc, gacc_t *host, clpart_t *part){
     __shared__ sums_sh<CT, 4, 4> ss;
     __shared__ sums_sh<CT, 2, 1> sd;
     __shared__ u64 ws[CT/32];
     __shared__ seq_sh<CT> sh;
+    const geom_t &g = ko.g;
     const int r = cl_rank(), t = threadIdx.x, D2 = 2*g.D;
     const double pw = acc->pw, a0 = acc->a;
     double inv = 0, u = 0;
@@ -725,7 +751,7 @@ k_frontier(geom_t g, KeepOp ko, WinOp wo, const double *uu, long n, u64 *key, u6
     cl_sync();
     /* the claims */
     const long nc = (long)nk*D2;
-    for(long id = (long)r*CT + t; id < nc; id += CL*CT) claim_one(g, ko.fr, ko.kj, key, wo.word, mask, qs, acc, id);
+    for(long id = (long)r*CT + t; id < nc; id += CL*CT) claim_one(g, ko.keep + ko.base, ko.kk + ko.base, key, wo.word, mask, qs, acc, id);
     if(r == 0 && t == 0){ acc->a = a; acc->thr = thr; acc->nk = nk; acc->nkeep = ko.base + nk; }
     cl_sync();
     /* the winners */
@@ -750,12 +776,13 @@ k_frontier(geom_t g, KeepOp ko, WinOp wo, const double *uu, long n, u64 *key, u6
  * kept count, so that the table and the candidate list grow by what is needed and not by that bound */
 extern "C" int sqb_grow_expand(const double *v_dev, const unsigned char *stt_dev, const double *uu_dev, long *nnext){
     const long n = GR.nfr; const int D2 = 2*GR.g.D;
-    long kc = GR.keepcap, vc = GR.keepcap;
-    if(devbuf(&GR.keep, &kc, GR.nkeep + n, GR.nkeep) || devbuf(&GR.kv, &vc, GR.nkeep + n, GR.nkeep)) return -1;
+    long kc = GR.keepcap, vc = GR.keepcap, yc = GR.keepcap;
+    if(devbuf(&GR.keep, &kc, GR.nkeep + n, GR.nkeep) || devbuf(&GR.kv, &vc, GR.nkeep + n, GR.nkeep) ||
+       devbuf(&GR.kk, &yc, GR.nkeep + n, GR.nkeep)) return -1;
     GR.keepcap = kc;
     if(devbuf(&GR.kj, &GR.kjcap, n, 0)) return -1;
-    KeepOp ko; ko.fr = GR.fr; ko.v = v_dev; ko.stt = stt_dev; ko.acc = GR.acc; ko.abskip = GR.abskip; ko.D = GR.g.D;
-    ko.keep = GR.keep; ko.kv = GR.kv; ko.kj = GR.kj; ko.base = (u64)GR.nkeep;
+    KeepOp ko; ko.g = GR.g; ko.fr = GR.fr; ko.v = v_dev; ko.stt = stt_dev; ko.acc = GR.acc; ko.abskip = GR.abskip;
+    ko.keep = GR.keep; ko.kv = GR.kv; ko.kk = GR.kk; ko.kj = GR.kj; ko.base = (u64)GR.nkeep;
     const bool one = n <= CL_MAX && n*D2 <= 64L*CL*CT;
     if(!one){
         const long nb = (n + GS_TILE - 1)/GS_TILE;
@@ -784,10 +811,10 @@ extern "C" int sqb_grow_expand(const double *v_dev, const unsigned char *stt_dev
         wo.nx = GR.nx; wo.nxsk = GR.nxsk; wo.D2 = D2; wo.st = GR.g.st; wo.gs = GR.gs; wo.base = 0;
         if(one){
             ko.fr = GR.fr;
-            k_frontier<<<CL, CT, 0, TS>>>(GR.g, ko, wo, uu_dev, n, GR.key, GR.mask, GR.qs, GR.acc, GR.host, GR.cpart); TL++;
+            k_frontier<<<CL, CT, 0, TS>>>(ko, wo, uu_dev, n, GR.key, GR.mask, GR.qs, GR.acc, GR.host, GR.cpart); TL++;
             TCK(cudaGetLastError());
         } else {
-            k_claim<<<grid256(nc), 256, 0, TS>>>(GR.g, GR.fr, GR.kj, GR.key, GR.word, GR.mask, GR.qs, GR.acc); TL++;
+            k_claim<<<grid256(nc), 256, 0, TS>>>(GR.g, GR.keep + GR.nkeep, GR.kk + GR.nkeep, GR.key, GR.word, GR.mask, GR.qs, GR.acc); TL++;
             TCK(cudaGetLastError());
             if(compact(wo, cnt_t{&GR.acc->nk, D2, nc}, &GR.acc->nn, GR.acc, GR.host)) return -1;
         }
@@ -838,19 +865,19 @@ extern "C" int sqb_grow_probe_zero(long *unres){ *unres = (long)GR.host->punres;
 
 struct RethOp {
     enum { DROP = 1 };
-    const sqb_pt_t *keep; const double *kv; const gacc_t *acc; sqb_pt_t *out; double *okv; u64 base;
+    const sqb_pt_t *keep; const double *kv; const u64 *kk; const gacc_t *acc; sqb_pt_t *out; double *okv; u64 *okk; u64 base;
     __device__ bool pred(long i) const { return kv[i] >= acc->thr; }
     __device__ double weight(long i) const { return __dmul_rn(kv[i], acc->pw); }
-    __device__ void emit(long i, u64 r) const { out[r] = keep[i]; okv[r] = kv[i]; }
+    __device__ void emit(long i, u64 r) const { st_pt(out + r, ld_pt(keep + i)); okv[r] = kv[i]; okk[r] = kk[i]; }
 };
 
 /* shadow tiers: breadth-first from z = 0 through kept points with |f| >= 10 thr (tier 1) and 100 thr (tier 2)
  * (driver/sumkey.h:402-444), both at once: a point of tier t raises a neighbour to the highest tier up to t
  * whose bound the neighbour's value meets, and a raised point goes (again) into the next step's list */
-__global__ void k_index(geom_t g, const sqb_pt_t *keep, const u64 *key, unsigned *word, u64 mask, gacc_t *acc){
+__global__ void k_index(const u64 *kk, const u64 *key, unsigned *word, u64 mask, gacc_t *acc){
     const long m = (long)acc->m;
     for(long i = blockIdx.x*(long)blockDim.x + threadIdx.x; i < m; i += (long)gridDim.x*blockDim.x){
-        const long q = h_find(key, mask, key_of(g, keep[i].k));
+        const long q = h_find(key, mask, kk[i]);
         if(q < 0){ atomicAdd(&acc->err, 1ULL); continue; }
         word[q] = (unsigned)i;
     }
@@ -866,33 +893,34 @@ __device__ __forceinline__ void tier_seed(const geom_t &g, const u64 *key, const
     const unsigned t = tier_of(kv[i], thr);
     if(t){ tr[i] = t; cu[0] = i; cnt[0] = 1; }
 }
-__global__ void k_tier_seed(geom_t g, const u64 *key, const unsigned *word, u64 mask, const double *kv, const gacc_t *acc,
+__global__ void k_tier_seed(const __grid_constant__ geom_t g, const u64 *key, const unsigned *word, u64 mask, const double *kv, const gacc_t *acc,
                             unsigned *tr, long *cu, u64 *cnt){
     tier_seed(g, key, word, mask, kv, acc->thr, tr, cu, cnt);
 }
-__device__ __forceinline__ void tier_edge(const geom_t &g, const sqb_pt_t *keep, const u64 *key, const unsigned *word, u64 mask,
-                                          const double *kv, double thr, unsigned *tr, long i, int c, long *nw, u64 *nnw){
-    const int d = c >> 1, sg = (c & 1) ? 1 : -1;
-    const int kk = keep[i].k[d] + g.st*sg;
-    if(kk > g.K || kk < -g.K) return;
-    const u64 y = key_of(g, keep[i].k) + (sg > 0 ? g.P[d] : (u64)0 - g.P[d]);
-    const long q = h_find(key, mask, y);
+__device__ __forceinline__ void tier_edge(const geom_t &g, const sqb_pt_t *keep, const u64 *kk, const u64 *key, const unsigned *word,
+                                          u64 mask, const double *kv, double thr, unsigned *tr, const long *cu, long x, long *nw, u64 *nnw){
+    long p; int c;
+    split(x, 2*g.D, &p, &c);
+    const long i = __ldcg(cu + p);
+    const int d = c >> 1, sg = (c & 1) ? 1 : -1, kx = keep[i].k[d] + g.st*sg;
+    if(kx > g.K || kx < -g.K) return;
+    const long q = h_find(key, mask, kk[i] + (sg > 0 ? g.P[d] : (u64)0 - g.P[d]));
     if(q < 0 || word[q] == SEEN) return;
     const long j = word[q];
     const unsigned t = min(*(volatile unsigned*)&tr[i], tier_of(kv[j], thr));
     if(t && *(volatile unsigned*)&tr[j] < t && atomicMax(&tr[j], t) < t) nw[atomicAdd(nnw, 1ULL)] = j;
 }
-__global__ void k_tier_step(geom_t g, const sqb_pt_t *keep, const u64 *key, const unsigned *word, u64 mask, const double *kv,
+__global__ void k_tier_step(const __grid_constant__ geom_t g, const sqb_pt_t *keep, const u64 *kk, const u64 *key, const unsigned *word, u64 mask, const double *kv,
                             const gacc_t *acc, unsigned *tr, const long *cu, long *nw, u64 *cnt, int s){
     const int D2 = 2*g.D;
     const long nc = (long)cnt[s % 3]*D2;      /* this step's list, written by the step (or seed) before */
     if(blockIdx.x == 0 && threadIdx.x == 0) cnt[(s + 2) % 3] = 0;
     for(long x = blockIdx.x*(long)blockDim.x + threadIdx.x; x < nc; x += (long)gridDim.x*blockDim.x)
-        tier_edge(g, keep, key, word, mask, kv, acc->thr, tr, cu[x/D2], (int)(x % D2), nw, &cnt[(s + 1) % 3]);
+        tier_edge(g, keep, kk, key, word, mask, kv, acc->thr, tr, cu, x, nw, &cnt[(s + 1) % 3]);
 }
 /* what a long way round leaves after the steps the host launched: one CTA, step after step to the end (every step
  * raises at least one point, at most twice) */
-__global__ void __launch_bounds__(GT) k_tier_rest(geom_t g, const sqb_pt_t *keep, const u64 *key, const unsigned *word, u64 mask,
+__global__ void __launch_bounds__(GT) k_tier_rest(const __grid_constant__ geom_t g, const sqb_pt_t *keep, const u64 *kk, const u64 *key, const unsigned *word, u64 mask,
                                                   const double *kv, const gacc_t *acc, unsigned *tr, long *cu, long *nw, u64 *cnt, int s){
     const int D2 = 2*g.D;
     const long bound = 2*(long)acc->m + 1;
@@ -902,7 +930,7 @@ __global__ void __launch_bounds__(GT) k_tier_rest(geom_t g, const sqb_pt_t *keep
         if(threadIdx.x == 0) cnt[(s + 2) % 3] = 0;
         __syncthreads();
         for(long x = threadIdx.x; x < nc; x += GT)
-            tier_edge(g, keep, key, word, mask, kv, acc->thr, tr, cu[x/D2], (int)(x % D2), nw, &cnt[(s + 1) % 3]);
+            tier_edge(g, keep, kk, key, word, mask, kv, acc->thr, tr, cu, x, nw, &cnt[(s + 1) % 3]);
         __threadfence();
         __syncthreads();
         long *t = cu; cu = nw; nw = t;
@@ -913,13 +941,13 @@ __global__ void __launch_bounds__(GT) k_tier_rest(geom_t g, const sqb_pt_t *keep
  * ms; of 47,579 kept points one cluster is the slower one (0.43 against 0.35 ms) */
 #define TIER_CL (1L << 14)
 __global__ void __cluster_dims__(CL, 1, 1) __launch_bounds__(CT)
-k_tiers(geom_t g, sqb_pt_t *keep, const u64 *key, unsigned *word, u64 mask, const double *kv, gacc_t *acc, unsigned *tr,
+k_tiers(const __grid_constant__ geom_t g, sqb_pt_t *keep, const u64 *kk, const u64 *key, unsigned *word, u64 mask, const double *kv, gacc_t *acc, unsigned *tr,
         long *cu, long *nw, u64 *cnt){
     const long m = (long)acc->m; const int D2 = 2*g.D, r = cl_rank();
     const double thr = acc->thr;
     const long x0 = (long)r*CT + threadIdx.x;
     for(long i = x0; i < m; i += CL*CT){
-        const long q = h_find(key, mask, key_of(g, keep[i].k));
+        const long q = h_find(key, mask, kk[i]);
         tr[i] = 0;
         if(q < 0) atomicAdd(&acc->err, 1ULL); else word[q] = (unsigned)i;
     }
@@ -932,7 +960,7 @@ k_tiers(geom_t g, sqb_pt_t *keep, const u64 *key, unsigned *word, u64 mask, cons
         if(nc == 0) break;
         if(x0 == 0) cnt[(s + 2) % 3] = 0;
         for(long x = x0; x < nc; x += CL*CT)
-            tier_edge(g, keep, key, word, mask, kv, thr, tr, __ldcg(&cu[x/D2]), (int)(x % D2), nw, &cnt[(s + 1) % 3]);
+            tier_edge(g, keep, kk, key, word, mask, kv, thr, tr, cu, x, nw, &cnt[(s + 1) % 3]);
         cl_sync();
         long *y = cu; cu = nw; nw = y;
     }
@@ -948,35 +976,35 @@ __global__ void k_tier_apply(sqb_pt_t *keep, const unsigned *tr, const gacc_t *a
 /* the final threshold (eps times the whole sum) and the tiers; the kept list stays on the device, its length there
  * too (GR.nkeep bounds it until a wait) */
 extern "C" int sqb_grow_finish(int tiers){
-    sqb_pt_t *out; double *okv; const long n = GR.nkeep;
-    TCK(DMALLOC(&out, (n ? n : 1)*sizeof(sqb_pt_t))); TCK(DMALLOC(&okv, (n ? n : 1)*sizeof(double)));
+    sqb_pt_t *out; double *okv; u64 *okk; const long n = GR.nkeep;
+    TCK(DMALLOC(&out, (n ? n : 1)*sizeof(sqb_pt_t))); TCK(DMALLOC(&okv, (n ? n : 1)*sizeof(double))); TCK(DMALLOC(&okk, (n ? n : 1)*sizeof(u64)));
     if(n){
-        RethOp ro; ro.keep = GR.keep; ro.kv = GR.kv; ro.acc = GR.acc; ro.out = out; ro.okv = okv; ro.base = 0;
+        RethOp ro; ro.keep = GR.keep; ro.kv = GR.kv; ro.kk = GR.kk; ro.acc = GR.acc; ro.out = out; ro.okv = okv; ro.okk = okk; ro.base = 0;
         if(compact(ro, cnt_t{NULL, 1, n}, &GR.acc->m, GR.acc, NULL)) return -1;
     }
-    DFREE(GR.keep); DFREE(GR.kv); GR.keep = out; GR.kv = okv; GR.keepcap = n ? n : 1;
+    DFREE(GR.keep); DFREE(GR.kv); DFREE(GR.kk); GR.keep = out; GR.kv = okv; GR.kk = okk; GR.keepcap = n ? n : 1;
     if(!tiers || !n) return 0;
     unsigned *tr; long *cu, *nw; u64 *cnt;
     TCK(DMALLOC(&tr, n*sizeof(unsigned))); TCK(DMALLOC(&cu, 2*n*sizeof(long))); TCK(DMALLOC(&nw, 2*n*sizeof(long)));
     TCK(DMALLOC(&cnt, 3*sizeof(u64)));
     if(n <= TIER_CL){
-        k_tiers<<<CL, CT, 0, TS>>>(GR.g, GR.keep, GR.key, GR.word, GR.mask, GR.kv, GR.acc, tr, cu, nw, cnt); TL++;
+        k_tiers<<<CL, CT, 0, TS>>>(GR.g, GR.keep, GR.kk, GR.key, GR.word, GR.mask, GR.kv, GR.acc, tr, cu, nw, cnt); TL++;
         TCK(cudaGetLastError());
         DFREE(tr); DFREE(cu); DFREE(nw); DFREE(cnt);
         return 0;
     }
     TCK(cudaMemsetAsync(tr, 0, n*sizeof(unsigned), TS));
-    k_index<<<grid256(n), 256, 0, TS>>>(GR.g, GR.keep, GR.key, GR.word, GR.mask, GR.acc);
+    k_index<<<grid256(n), 256, 0, TS>>>(GR.kk, GR.key, GR.word, GR.mask, GR.acc);
     k_tier_seed<<<1, 1, 0, TS>>>(GR.g, GR.key, GR.word, GR.mask, GR.kv, GR.acc, tr, cu, cnt);
     TL += 2;
     /* the points lie within as many steps of z = 0 as the grow had frontiers; a way through the larger values
      * alone may be longer, and the rest kernel walks it */
     int s = 0;
     for(; s < GR.nfrs; s++){
-        k_tier_step<<<grid256(n), 256, 0, TS>>>(GR.g, GR.keep, GR.key, GR.word, GR.mask, GR.kv, GR.acc, tr, cu, nw, cnt, s); TL++;
+        k_tier_step<<<grid256(n), 256, 0, TS>>>(GR.g, GR.keep, GR.kk, GR.key, GR.word, GR.mask, GR.kv, GR.acc, tr, cu, nw, cnt, s); TL++;
         long *x = cu; cu = nw; nw = x;
     }
-    k_tier_rest<<<1, GT, 0, TS>>>(GR.g, GR.keep, GR.key, GR.word, GR.mask, GR.kv, GR.acc, tr, cu, nw, cnt, s);
+    k_tier_rest<<<1, GT, 0, TS>>>(GR.g, GR.keep, GR.kk, GR.key, GR.word, GR.mask, GR.kv, GR.acc, tr, cu, nw, cnt, s);
     k_tier_apply<<<grid256(n), 256, 0, TS>>>(GR.keep, tr, GR.acc);
     TL += 2;
     TCK(cudaGetLastError());
@@ -1000,16 +1028,17 @@ extern "C" int sqb_grow_sums(sqb_grow_sums_t *r){
 /* ------------------------------------------- dilation -------------------------------------------- */
 /* every kept cell and its in-box axis neighbours marked in the seen table, which holds them all: bit 3 present,
  * bit 0 some cell does not skip (the skip bits' AND), bits 1 and 2 the tier's maximum in unary (driver/sumkey.h:41-44) */
-__global__ void k_dil_mark(geom_t g, const sqb_pt_t *cur, const u64 *key, unsigned *word, u64 mask, gacc_t *acc, unsigned *bm, u64 base){
+__global__ void k_dil_mark(const __grid_constant__ geom_t g, const sqb_pt_t *cur, const u64 *kk, const u64 *key, unsigned *word, u64 mask, gacc_t *acc, unsigned *bm, u64 base){
     const int C = 2*g.D + 1;
     const long n = (long)acc->m*C;
     for(long x = blockIdx.x*(long)blockDim.x + threadIdx.x; x < n; x += (long)gridDim.x*blockDim.x){
-        const long q0 = x/C; const int c = (int)(x - q0*C);
+        long q0; int c;
+        split(x, C, &q0, &c);
         const signed char *k = cur[q0].k; const int fl = k[SQB_PFLAG];
-        u64 y = key_of(g, k);
+        u64 y = kk[q0];
         if(c > 0){
-            const int j = (c - 1) >> 1, sg = ((c - 1) & 1) ? 1 : -1, kk = k[j] + g.st*sg;
-            if(kk > g.K || kk < -g.K) continue;
+            const int j = (c - 1) >> 1, sg = ((c - 1) & 1) ? 1 : -1, kx = k[j] + g.st*sg;
+            if(kx > g.K || kx < -g.K) continue;
             y = sg > 0 ? y + g.P[j] : y - g.P[j];
         }
         const long q = h_find(key, mask, y);
@@ -1072,7 +1101,7 @@ struct SlotOp {
     __device__ bool pred(long i) const { return word[i] != 0; }
     __device__ void emit(long i, u64 r) const { out[r] = key[i]; }
 };
-__global__ void k_dil_decode(geom_t g, const u64 *U, const u64 *key, const unsigned *word, u64 mask, sqb_pt_t *out, const gacc_t *acc){
+__global__ void k_dil_decode(const __grid_constant__ geom_t g, const u64 *U, const u64 *key, const unsigned *word, u64 mask, sqb_pt_t *out, const gacc_t *acc){
     const long m = (long)acc->ncell;
     for(long j = blockIdx.x*(long)blockDim.x + threadIdx.x; j < m; j += (long)gridDim.x*blockDim.x){
         u64 y = U[j]; sqb_pt_t p;
@@ -1172,7 +1201,7 @@ extern "C" int sqb_grow_dilate(int nbits, sqb_pt_t **out){
         TCK(cudaMemsetAsync(bm, 0, bmb, TS));
     }
     TCK(cudaMemsetAsync(GR.word, 0, cap*sizeof(unsigned), TS));
-    k_dil_mark<<<grid256(GR.nkeep*(2*GR.g.D + 1)), 256, 0, TS>>>(GR.g, GR.keep, GR.key, GR.word, GR.mask, GR.acc, bm, base); TL++;
+    k_dil_mark<<<grid256(GR.nkeep*(2*GR.g.D + 1)), 256, 0, TS>>>(GR.g, GR.keep, GR.kk, GR.key, GR.word, GR.mask, GR.acc, bm, base); TL++;
     if(bm){
         if(base <= 1ULL << 25 ? bm_order<1>(bm, base, base, U, &GR.acc->ncell) : bm_order<8>(bm, base, base, U, &GR.acc->ncell)) return -1;
         DFREE(bm);
@@ -1196,5 +1225,6 @@ extern "C" void sqb_grow_end(void){
     if(GR.key){ DFREE(GR.key); DFREE(GR.word); GR.key = NULL; }
     if(GR.keep){ DFREE(GR.keep); GR.keep = NULL; GR.keepcap = 0; }
     if(GR.kv){ DFREE(GR.kv); GR.kv = NULL; }
+    if(GR.kk){ DFREE(GR.kk); GR.kk = NULL; }
     GR.nkeep = 0;
 }
