@@ -120,32 +120,46 @@ static int grow(Run &R, int lev, double eps_rel, GrowOut *go, sqb_pt_t **dilated
     /* the grow's device tables are released on every return, an error included, so that a failed
      * integral leaves its memory to the next one */
     struct End { ~End(){ sqb_grow_end(); } } end_of_grow;
-    const sqb_pt_t *pts; const unsigned char *skip, *sd; const double *vd, *ud; long n = 0, nfr = 0, nn = 0;
+    const sqb_pt_t *pts; const unsigned char *skip, *sd; const double *vd, *ud; long n = 0;
     if(sqb_grow_begin(R.D, R.K, st, W ? W : 1, (const unsigned long long*)P, gs, R.o.abskip, eps_rel, pow(st, R.D), sqb_dev_stream(), &pts, &n))
         FAIL("device grow: %s", sqb_top_error());
-    if(sqb_dev_eval_resident(R.g, pts, n, NULL, &R.t, &vd, &sd, &ud)) FAIL("device: %s", sqb_last_error());
+    if(sqb_dev_eval_resident(R.g, pts, n, NULL, NULL, &R.t, &vd, &sd, &ud)) FAIL("device: %s", sqb_last_error());
     if(sqb_grow_probe(vd, sd)) FAIL("device grow: %s", sqb_top_error());
     const long nprobe = n;
     sqb_grow_sums_t s;
-    if(!W && (sqb_grow_sums(&s) || !sqb_grow_probe_zero(&nn)))
-        FAIL("lattice too wide for 64-bit grid keys (D=%d, N=%d, step %dh)", R.D, 2*R.K + 1, st);
-    for(;;){
-        n = sqb_grow_frontier(&pts, &skip);
-        if(n <= 0) break;
-        /* the first frontier, z = 0, is the probe's first node: its value is there */
-        if(nfr && sqb_dev_eval_resident(R.g, pts, n, skip, &R.t, &vd, &sd, &ud)) FAIL("device: %s", sqb_last_error());
-        /* the predictor stores every grow value (driver/sumkey.h:219-222) */
-        if(R.vt && (sqb_vtab_reserve(R.vt, n, sqb_dev_stream()) || sqb_vtab_put_nodes(R.vt, pts, vd, n, R.D, sqb_dev_stream())))
-            FAIL("predictor: %s", sqb_vtab_error());
-        if(sqb_grow_expand(vd, sd, ud, &nn)) FAIL("device grow: %s", sqb_top_error());
-        go->nev += n;
-        if(!nfr++){
+    bool first = true;                 /* the first frontier, z = 0, is the probe's first node: its value is there */
+    if(!W){
+        long un = 0;
+        if(sqb_grow_sums(&s) || !sqb_grow_probe_zero(&un))
+            FAIL("lattice too wide for 64-bit grid keys (D=%d, N=%d, step %dh)", R.D, 2*R.K + 1, st);
+        R.unresdrop += un; go->zero = 1; go->nev = nprobe;
+        return 0;
+    }
+    while((n = sqb_grow_frontier(&pts, &skip)) > 0){
+        long nmax; const unsigned long long *np;
+        int links = sqb_grow_chain(&nmax, &np);
+        if(links < 0) FAIL("device grow: %s", sqb_top_error());
+        if(links && R.vt) links = 1;                /* the predictor takes every frontier's values with its size */
+        sqb_grow_frontier(&pts, &skip);             /* the lists may have moved */
+        for(int q = 0; q < (links ? links : 1); q++){
+            if(q) sqb_grow_link(q, &pts, &skip);
+            if(!first && sqb_dev_eval_resident(R.g, pts, q ? nmax : n, q ? np : NULL, skip, &R.t, &vd, &sd, &ud))
+                FAIL("device: %s", sqb_last_error());
+            /* the predictor stores every grow value (driver/sumkey.h:219-222) */
+            if(R.vt && (sqb_vtab_reserve(R.vt, n, sqb_dev_stream()) || sqb_vtab_put_nodes(R.vt, pts, vd, n, R.D, sqb_dev_stream())))
+                FAIL("predictor: %s", sqb_vtab_error());
+            if(links ? sqb_grow_step(q, vd, sd, ud) : sqb_grow_expand(vd, sd, ud)) FAIL("device grow: %s", sqb_top_error());
+            first = false;
+        }
+        if(links && sqb_grow_wait()) FAIL("device grow: %s", sqb_top_error());
+        if(go->nev == 0){
             /* the first wait has brought the probe's answer; its fallback count and round column are its own, its
              * unresolved points are counted, as the global UNRESDROP does */
             long un = 0;
             go->zero = sqb_grow_probe_zero(&un);
             R.unresdrop += un;
-            if(go->zero){ go->nev = nprobe; return 0; }
+            go->nev = nprobe;
+            if(go->zero) return 0;
         }
     }
     const double t1 = now();
@@ -159,12 +173,12 @@ static int grow(Run &R, int lev, double eps_rel, GrowOut *go, sqb_pt_t **dilated
     }
     if(store && sqb_grow_dilate(nbits, dilated)) FAIL("device dilate: %s", sqb_top_error());
     if(sqb_grow_sums(&s)){ sqb_dev_free(*dilated); *dilated = NULL; FAIL("device grow: %s", sqb_top_error()); }
-    *ndil = s.cells;
+    *ndil = s.cells; go->nev = s.seen;
     R.nq += s.nq; R.u += s.u; R.unresdrop += s.unres;
     go->S = s.S; go->A = s.a; go->e1 = s.x1; go->e2 = s.x2; go->drop = s.drop; go->gshs = s.gshs; go->gshn = s.gshn;
     if(R.o.verbose)
         fprintf(stderr, "# %s grow: %ld frontiers, %ld points, %ld kept, %ld dilated cells: frontiers %.2f ms; final threshold, "
-                "tiers and dilation %.2f ms\n", R.g->name, nfr, go->nev, s.kept, s.cells, 1e3*(t1 - t0), 1e3*(now() - t1));
+                "tiers and dilation %.2f ms\n", R.g->name, s.frontiers, go->nev, s.kept, s.cells, 1e3*(t1 - t0), 1e3*(now() - t1));
     return 0;
 }
 

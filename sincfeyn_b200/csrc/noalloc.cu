@@ -131,14 +131,17 @@ extern "C" int sqb_level_noalloc(const char *graph, double h, int K, const void 
         sqb_kattr_t at; int per = 2;
         if(g->attr(0, 128, smem, &at) && at.blocks_per_sm > 0) per = at.blocks_per_sm;
         long want = (nch + 127)/128, full = (long)na_nsm[dev]*per;
+        a.inl = g->axis && sqb_axis_inline(&a, nch); a.dropunres = dropunres; a.uu = (double*)(B + NA_UU);
         g->f64(&a, (int)(want < full ? want : full), 128, smem, s);
         NACK(cudaGetLastError());
-        sqb_dd_t d; memset(&d, 0, sizeof d);
-        d.e = a; d.list = a.fb; d.nlist = nfb; d.listcap = NA_CH; d.all = 0; d.dropunres = dropunres; d.uu = (double*)(B + NA_UU);
-        per = 2; if(g->attr(1, 128, smem, &at) && at.blocks_per_sm > 0) per = at.blocks_per_sm;
-        g->dd(&d, na_nsm[dev]*per, 128, smem, s);
-        NACK(cudaGetLastError());
-        int rc = sqb_level_tail(cells, nch, D, st, last, abskip, pw, thr, a.v, d.uu, a.stt,
+        if(!a.inl){
+            sqb_dd_t d; memset(&d, 0, sizeof d);
+            d.e = a; d.list = a.fb; d.nlist = nfb; d.listcap = NA_CH; d.all = 0; d.dropunres = dropunres; d.uu = a.uu;
+            per = 2; if(g->attr(1, 128, smem, &at) && at.blocks_per_sm > 0) per = at.blocks_per_sm;
+            g->dd(&d, na_nsm[dev]*per, 128, smem, s);
+            NACK(cudaGetLastError());
+        }
+        int rc = sqb_level_tail(cells, nch, D, st, last, abskip, pw, thr, a.v, a.uu, a.stt,
                                 B + NA_BP, (unsigned*)(B + NA_BK), (unsigned long long*)(B + NA_BO), acc, base,
                                 B + NA_MISC + 64, next, next_cap, s);
         if(rc){ sqb_set_error_msg("sqb_level_noalloc: kernel launch failed"); return rc; }

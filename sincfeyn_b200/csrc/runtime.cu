@@ -293,9 +293,18 @@ static int eval_batch(const sqb_graph_t *g, sqb_eval_t *a, const sqb_test_t *t, 
         G.launches++;
         return 0;
     }
-    CKR(cudaMemsetAsync(G.nfb, 0, sizeof(unsigned long long), G.s));
     cudaEvent_t *ev = ktime_slot();
     if(ev) CKR(cudaEventRecord(ev[0], G.s));
+    if(g->axis && !use_split(g, a, t) && sqb_axis_inline(a, npts)){
+        const int w = f64_which(g, t->fma);
+        a->inl = 1; a->dropunres = t->dropunres; a->uu = G.uu;
+        launch_f64(g, w, a, grid_for(g, w, npts, smem), smem, G.s);
+        CKR(cudaGetLastError());
+        G.launches++;
+        if(ev){ CKR(cudaEventRecord(ev[1], G.s)); CKR(cudaEventRecord(ev[2], G.s)); }
+        return 0;
+    }
+    CKR(cudaMemsetAsync(G.nfb, 0, sizeof(unsigned long long), G.s));
     if(use_split(g, a, t)){
         if(npts > G.ttcap){
             if(G.tt){ cudaFree(G.tt); cudaFree(G.ta); }
@@ -333,16 +342,16 @@ static int eval_batch(const sqb_graph_t *g, sqb_eval_t *a, const sqb_test_t *t, 
     return 0;
 }
 
-/* n device-resident nodes (pt_t, flags ignored; skip per node on the device or NULL) evaluated with the tests and the
- * fallback; the values, status and round column stay on the device until the next evaluation.  Queued on the
+/* n device-resident nodes (pt_t, flags ignored; np: their number on the device, at most n, or NULL; skip per node on the
+ * device or NULL) evaluated with the tests and the fallback; the values, status and round column stay on the device until the next evaluation.  Queued on the
  * thread's stream, no wait */
-extern "C" int sqb_dev_eval_resident(const sqb_graph_t *g, const sqb_pt_t *pts, long n, const unsigned char *skip, const sqb_test_t *t,
-                                     const double **v_dev, const unsigned char **stt_dev, const double **uu_dev){
+extern "C" int sqb_dev_eval_resident(const sqb_graph_t *g, const sqb_pt_t *pts, long n, const unsigned long long *np,
+                                     const unsigned char *skip, const sqb_test_t *t, const double **v_dev, const unsigned char **stt_dev, const double **uu_dev){
     *v_dev = *uu_dev = NULL; *stt_dev = NULL;
     if(n <= 0) return 0;
     if(reserve_points(n)) return -1;
     sqb_eval_t a; memset(&a, 0, sizeof a); fill_eval(&a, t);
-    a.pts = pts; a.n = n; a.esize = 1; a.stride = SQB_MAXD; a.flag_at = -1; a.cells = 0; a.st = 0; a.skip = skip;
+    a.pts = pts; a.n = n; a.esize = 1; a.stride = SQB_MAXD; a.flag_at = -1; a.cells = 0; a.st = 0; a.skip = skip; a.np = np;
     if(eval_batch(g, &a, t, n)) return -1;
     *v_dev = G.v; *stt_dev = G.stt; *uu_dev = G.uu;
     return 0;

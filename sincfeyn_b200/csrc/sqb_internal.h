@@ -65,6 +65,7 @@ typedef struct {
 typedef struct {
     const void *pts;
     long n;                       /* nodes, or cells */
+    const unsigned long long *np; /* their number on the device, at most n (NULL: n); launches outside the level kernels */
     int esize, stride, flag_at;
     int cells, st;                /* cells: child b of cell c is k_d - st*bit_d(b) (driver/sum.c:407) */
     const double *X, *Wt;         /* 2K+1 entries: integration variable and weight factor per k;
@@ -107,6 +108,8 @@ typedef struct {
      * others; the FP64 kernel walks the list (tiles of SQB_TILE entries from the queue) and leaves every
      * tile's sums to the reduce kernel */
     const unsigned long long *sel, *nsel;
+    int inl, dropunres;           /* inl: axis form, the fallback inside the FP64 kernel (sqb_axis_inline); then dropunres and */
+    double *uu;                   /* uu as in sqb_dd_t */
     int sub;                      /* level launch of the axis form: work items per tile (1, or 4 when the reduce kernel sums
                                      every tile, so that a small batch fills the device) */
 } sqb_eval_t;
@@ -154,6 +157,15 @@ static inline bool sqb_axis_launch(const sqb_eval_t *a){
     if(!sqb_level_launch(a) || a->sym.n > 1 || a->cfl) return false;
     for(int q = 0; q < a->ninst; q++) if(!a->inst[q].U) return false;
     return true;
+}
+/* a tested launch of npts points outside the level kernel whose fallback the axis form's kernel does itself: up to the
+ * size where the second kernel's balance makes up for its launch (allocation-free batch of syn_d8, 768 children 87 -> 70 us,
+ * 25,600 97 -> 81, 262,144 97 both ways) */
+#ifndef SQB_INLINE_MAX
+#define SQB_INLINE_MAX (1L << 18)
+#endif
+static inline bool sqb_axis_inline(const sqb_eval_t *a, long npts){
+    return a->U && a->Ud && !a->raw && !a->sfin && a->ninst <= 0 && !a->sel && !a->part && a->sym.n <= 1 && !a->cfl && npts <= SQB_INLINE_MAX;
 }
 
 typedef struct {

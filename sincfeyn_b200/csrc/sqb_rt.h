@@ -92,21 +92,28 @@ int  sqb_dev_level(const sqb_level_t *L, sqb_acc_t *acc, long *next_n, double *m
  * or the pass split run one after another through sqb_dev_level. */
 int  sqb_dev_level_multi(const sqb_level_t *L, int n, sqb_acc_t *acc, long *next_n, double *ms);
 
-/* n nodes on the device (pts, skip device pointers) evaluated with the tests and the fallback, queued on the thread's
- * stream; the values, status and round column stay on the device until the next evaluation */
-int  sqb_dev_eval_resident(const sqb_graph_t *g, const sqb_pt_t *pts, long n, const unsigned char *skip, const sqb_test_t *t,
-                           const double **v_dev, const unsigned char **stt_dev, const double **uu_dev);
+/* n nodes on the device (pts, skip device pointers; np: at most n, their number on the device, or NULL) evaluated with the
+ * tests and the fallback, queued on the thread's stream; the values, status and round column stay on the device until the next evaluation */
+int  sqb_dev_eval_resident(const sqb_graph_t *g, const sqb_pt_t *pts, long n, const unsigned long long *np, const unsigned char *skip,
+                           const sqb_test_t *t, const double **v_dev, const unsigned char **stt_dev, const double **uu_dev);
 void *sqb_dev_stream(void);
 
 /* the top level on the device (topgrid.cu): the zero probe, grow frontiers, final threshold, tiers, dilation.  Calls
- * in this order: begin, probe, (frontier, expand)..., finish, dilate, sums, end */
-typedef struct { double S, a, x1, x2, drop, gshs, u; long gshn, nq, unres, kept, cells; } sqb_grow_sums_t;
+ * in this order: begin, probe, (frontier, then chain: link, step..., wait, or expand)..., finish, dilate, sums, end */
+typedef struct { double S, a, x1, x2, drop, gshs, u; long gshn, nq, unres, kept, cells, seen, frontiers; } sqb_grow_sums_t;
 int  sqb_grow_begin(int D, int K, int st, int W, const unsigned long long *P, int gs, int abskip, double eps, double pw, void *stream,
                     const sqb_pt_t **probe, long *nprobe);
 int  sqb_grow_probe(const double *v_dev, const unsigned char *stt_dev);
 int  sqb_grow_probe_zero(long *unres);
 long sqb_grow_frontier(const sqb_pt_t **pts, const unsigned char **skip);
-int  sqb_grow_expand(const double *v_dev, const unsigned char *stt_dev, const double *uu_dev, long *nnext);
+/* the number of frontiers (1 to SQB_GROW_CHAIN, 0: this one is too large) that may be evaluated and stepped without a wait:
+ * frontier s of the chain, its number of points on the device (*np), at most *nmax; then sqb_grow_wait */
+#define SQB_GROW_CHAIN 4
+int  sqb_grow_chain(long *nmax, const unsigned long long **np);
+void sqb_grow_link(int s, const sqb_pt_t **pts, const unsigned char **skip);
+int  sqb_grow_step(int s, const double *v_dev, const unsigned char *stt_dev, const double *uu_dev);
+int  sqb_grow_wait(void);
+int  sqb_grow_expand(const double *v_dev, const unsigned char *stt_dev, const double *uu_dev);
 int  sqb_grow_finish(int tiers);
 int  sqb_grow_dilate(int nbits, sqb_pt_t **out);
 int  sqb_grow_sums(sqb_grow_sums_t *r);

@@ -87,6 +87,8 @@ __device__ __forceinline__ int sqb_inst_at(const sqb_eval_t &a, long i){
     for(int q = 1; q < a.ninst; q++) if(a.inst[q].child0 <= i) k = q;
     return k;
 }
+/* the nodes or cells of a launch over one batch */
+__device__ __forceinline__ long sqb_count(const sqb_eval_t &a){ return a.np ? (long)*a.np : a.n; }
 /* shared-memory words of the tables of a launch: 2(2K+1) per integral */
 __host__ __device__ __forceinline__ int sqb_table_words(const sqb_eval_t &a){
     if(a.ninst <= 0) return 2*(2*a.K + 1);
@@ -344,7 +346,7 @@ __global__ void __launch_bounds__(SQB_BLOCK, SQB_MINB) sqb_k_f64(const __grid_co
     sqb_tables(a, sqb_sm, sI);
     const bool multi = LV || a.ninst > 0;
     const bool list = !LV && a.sel;
-    const long n1 = multi ? 0 : (a.cells ? (a.n << D) : a.n);      /* one batch: its points */
+    const long n1 = multi ? 0 : sqb_count(a) << (a.cells ? D : 0);  /* one batch: its points */
     const long tl = (lvl || multi) ? SQB_TILE : SQB_BLOCK;          /* other modes: one point per thread per step */
     const long nsel = list ? (long)*a.nsel : 0;                     /* list mode (one integral, queue): its entries */
     const long ntiles = list ? (nsel + tl - 1)/tl : multi ? a.ntile : (n1 + tl - 1)/tl;
@@ -453,15 +455,29 @@ __global__ void __launch_bounds__(SQB_BLOCK, SQB_MINB) sqb_k_f64(const __grid_co
     }
 }
 
+/* qvalue() (driver/eval.c:25-30) on a point's double-double value and |.| sum: the value, the round column's e^2 and the
+ * status s with the unresolved bit */
+__device__ __forceinline__ double sqb_dd_value(double vqd, double abqd, double w, double abserr, int dropunres, double *u, unsigned char *s){
+    const double ee = abqd*w*SQB_QEPS;
+    *u = !(ee*16 <= abserr) ? (isfinite(ee) ? ee*ee : 0.0) : 0.0;
+    double v = isfinite(vqd) ? vqd*w : 0.0;
+    if(!(ee <= fabs(v))){ *s |= SQB_UNRES; if(dropunres) v = 0.0; }
+    return v;
+}
+
 /* The axis form's kernel for launches outside the level batches: one batch of nodes or cells, tested or raw.  SM = 0 reads
  * the table at a.U; SM = 1 (the plug-in's launches, which have no table) fills one in shared memory per CTA first,
- * which pays from SQB_AX_RAW points on (sqb_ax_points). */
-template<class F, int D, int SM>
+ * which pays from SQB_AX_RAW points on (sqb_ax_points).  DDI = 1: a point that needs the fallback is recomputed in
+ * double-double at once, by its own thread (a.inl: a small launch, whose time is latency; the queue and the second
+ * kernel would only add to it). */
+template<class F, int D, int SM, int DDI>
 __global__ void __launch_bounds__(SQB_BLOCK) sqb_k_ax(const __grid_constant__ sqb_eval_t a){
     extern __shared__ double sqb_sm[];
     __shared__ sqb_inst_t sI[SQB_MAXINST];
     using A0 = typename F::template AX<double, 0>;
     using A1 = typename F::template AX<double, 1>;
+    const long n = sqb_count(a) << (a.cells ? D : 0);
+    if(blockIdx.x*(long)SQB_BLOCK >= n) return;
     sqb_tables(a, sqb_sm, sI);
     const sqb_inst_t &I = sI[0];
     const int nt = 2*a.K + 1;
@@ -472,7 +488,6 @@ __global__ void __launch_bounds__(SQB_BLOCK) sqb_k_ax(const __grid_constant__ sq
         __syncthreads();
     }
     const double *U = SM ? T : a.U;
-    const long n = a.cells ? (a.n << D) : a.n;
     for(long i = blockIdx.x*(long)SQB_BLOCK + threadIdx.x; i < n; i += (long)gridDim.x*SQB_BLOCK){
         long c; double sf[D], w; int kk[D];
         if(!sqb_point<D>(a, I, sX, sW, i, i, &c, sf, &w, kk)){
@@ -487,8 +502,28 @@ __global__ void __launch_bounds__(SQB_BLOCK) sqb_k_ax(const __grid_constant__ sq
         else     f = sqb_axeval<A1, double, D, SM>(U, a.K, sf, kk, &ab);
         const double fw = f*w;
         if(a.raw){ a.v[i] = fw; a.ab[i] = ab*w; continue; }
-        bool fallback;
-        sqb_point_test(a, I, i, sk, noab, fw, ab*w, &fallback);
+        if constexpr(DDI){
+            /* sqb_point_test with the fallback in place of the queue */
+            unsigned char s = SQB_PRESENT | (sk ? SQB_SKIPPED : 0);
+            double v = isfinite(fw) ? fw : 0.0;
+            if(!noab){
+                double bnd = ab*w*16*DBL_EPSILON;
+                if(a.ddslack != 1.0) bnd = bnd/a.ddslack;
+                if(!(bnd <= I.near_thr)) s |= SQB_NEAR;
+                if(!(bnd <= I.abserr)){
+                    s |= SQB_FALLBACK;
+                    sqdd abq;
+                    const sqdd vq = sqb_axeval<typename F::template AX<sqdd, 1>, sqdd, D>(a.Ud, a.K, sf, kk, &abq);
+                    double u;
+                    v = sqb_dd_value(vq.value(), abq.value(), w, I.abserr, a.dropunres, &u, &s);
+                    a.uu[i] = u;
+                }
+            }
+            a.v[i] = v; a.stt[i] = s;
+        } else {
+            bool fallback;
+            sqb_point_test(a, I, i, sk, noab, fw, ab*w, &fallback);
+        }
     }
 }
 
@@ -506,9 +541,6 @@ __global__ void __launch_bounds__(SQB_BLOCK) sqb_k_ax(const __grid_constant__ sq
 #define SQB_AXG 8
 #ifndef SQB_AX_MINB
 #define SQB_AX_MINB 5
-#endif
-#ifndef SQB_AX_UNROLL
-#define SQB_AX_UNROLL 1
 #endif
 /* a thread's sums: S, b1, b2 as (hi, running error), normalised at the tile's end */
 struct sqb_ax_acc { double S, Se, b1, b1e, b2, b2e, A, dr; unsigned ne, nsk, keep; bool fb; };
@@ -544,8 +576,9 @@ __device__ __forceinline__ void sqb_ax_group(const sqb_eval_t &a, const sqb_ax_i
     const unsigned char s0 = SQB_PRESENT | (sk ? SQB_SKIPPED : 0);
     unsigned added = 0;
     const int kl = k[D - 1] - st < -K ? 0 : k[D - 1] - st + K, kh = k[D - 1] + K;      /* the last axis' two entries */
-    constexpr int UN = SQB_AX_UNROLL;
-#pragma unroll UN
+    /* rolled: with both forms of the leaf in the kernel the instruction caches hold no more (two turns unrolled took 20.4 ms
+     * instead of 14.3 on syn_d8 at h = 0.7, where both run, four 32 ms) */
+#pragma unroll 1
     for(int h = 0; h < 4; h++){
         typename A::st S1 = S0; double w1 = w0;
 #pragma unroll
@@ -682,7 +715,7 @@ __global__ void __launch_bounds__(SQB_BLOCK) sqb_k_dd(const __grid_constant__ sq
     const sqb_eval_t &e = a.e;
     const bool multi = e.ninst > 0;
     long n;
-    if(a.all) n = multi ? e.ntile*SQB_TILE : (e.cells ? (e.n << D) : e.n);
+    if(a.all) n = multi ? e.ntile*SQB_TILE : sqb_count(e) << (e.cells ? D : 0);
     else { n = (long)*a.nlist; if(n > a.listcap) n = a.listcap; }
     if(blockIdx.x*(long)blockDim.x >= n) return;      /* the grid is for a full queue: most queues are short */
     sqb_tables(e, sqb_sm, sI);
@@ -708,17 +741,14 @@ __global__ void __launch_bounds__(SQB_BLOCK) sqb_k_dd(const __grid_constant__ sq
         }
         if(e.raw){ e.v[i] = vq.hi; e.vlo[i] = vq.lo; e.ab[i] = abq.hi; e.ablo[i] = abq.lo; continue; }
         const double vqd = vq.value(), abqd = abq.value();
-        /* qvalue(), driver/eval.c:25-30 */
-        const double ee = abqd*w*SQB_QEPS;
-        const double u = !(ee*16 <= I.abserr) ? (isfinite(ee) ? ee*ee : 0.0) : 0.0;
-        double v = isfinite(vqd) ? vqd*w : 0.0;
         unsigned char s;
         if(a.all){
             /* the all-double-double form: the near flag from the double-double |.| sum */
             s = SQB_PRESENT | SQB_FALLBACK | (sqb_skip<D>(e, I, c) ? SQB_SKIPPED : 0);
             if(!(abqd*w*16*DBL_EPSILON/e.ddslack <= I.near_thr)) s |= SQB_NEAR;
         } else s = e.stt[i];
-        if(!(ee <= fabs(v))){ s |= SQB_UNRES; if(a.dropunres) v = 0.0; }
+        double u;
+        const double v = sqb_dd_value(vqd, abqd, w, I.abserr, a.dropunres, &u, &s);
         e.v[i] = v; e.stt[i] = s; a.uu[i] = u;
     }
 }
@@ -824,10 +854,11 @@ template<class F, int D>
 static bool sqb_ax_points(const sqb_eval_t *a, int grid, int block, size_t smem, cudaStream_t st){
     if constexpr(F::template AX<double, 0>::NU > 0){
         if(a->ninst > 0 || a->sfin || a->sel || a->part || a->sym.n > 1 || a->cfl) return false;
-        if(a->U){ sqb_k_ax<F, D, 0><<<grid, block, smem, st>>>(*a); return true; }
+        if(a->inl){ sqb_k_ax<F, D, 0, 1><<<grid, block, smem, st>>>(*a); return true; }
+        if(a->U){ sqb_k_ax<F, D, 0, 0><<<grid, block, smem, st>>>(*a); return true; }
         const size_t sm = smem + (size_t)D*(2*a->K + 1)*sqb_axw<typename F::template AX<double, 0>, double>::N*sizeof(double);
         if(a->raw && (a->cells ? a->n << D : a->n) >= SQB_AX_RAW && sm <= 48*1024){
-            sqb_k_ax<F, D, 1><<<grid, block, sm, st>>>(*a); return true; }
+            sqb_k_ax<F, D, 1, 0><<<grid, block, sm, st>>>(*a); return true; }
     }
     return false;
 }

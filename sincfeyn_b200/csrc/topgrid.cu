@@ -28,6 +28,7 @@
  * reference's summation order.  Every probe loop is bounded by the table size and reports overflow instead of
  * spinning. */
 #include <cuda_runtime.h>
+#include <stddef.h>
 #include <stdio.h>
 #include <stdlib.h>
 #include <string.h>
@@ -116,6 +117,7 @@ struct gacc_t {
     double S[2], x1[2], x2[2], dr[2], gs[2], u[2];   /* sum f w; outer shells; dropped weight; its signed sum; round column */
     u64 ngs, nq, unres;                     /* points below the threshold; fallback and unresolved points */
     u64 nk, nn, nkeep;                      /* this frontier's kept points, the next frontier, kept so far */
+    u64 nrun, seen, steps;                  /* the next frontier if one cluster takes it, else 0; points and frontiers so far */
     u64 m, ncell, err;                      /* kept after the final threshold; dilated cells; full-table inserts */
     u64 nz, punres;                         /* the zero probe: any value not 0; its unresolved points */
 };
@@ -334,6 +336,16 @@ __device__ __forceinline__ void publish(const gacc_t *acc, gacc_t *host){
     const u64 *s = (const u64*)acc; u64 *d = (u64*)host;
     for(unsigned w = threadIdx.x; w < sizeof(gacc_t)/8; w += 32) d[w] = s[w];
 }
+/* one cluster takes a frontier of up to CL_MAX points, a thread up to 64 of its candidates */
+#define CL 8                     /* CTAs of the one-cluster kernels, and their threads */
+#define CT 512
+#define CL_MAX ((long)CL*CT)     /* points of a frontier that one cluster takes: one per thread.  With four per thread
+                                    the whole sum of d = 5, h = 1 (16 frontiers up to 12,000 points) took 1.76 ms, with one
+                                    1.40, without the cluster 1.67 */
+static __host__ __device__ __forceinline__ bool one_cluster(long n, int D2){ return n <= CL_MAX && n*D2 <= 64L*CL*CT; }
+__device__ __forceinline__ void next_frontier(gacc_t *acc, u64 nn, int D2){
+    acc->nn = nn; acc->seen += nn; acc->steps++; acc->nrun = one_cluster((long)nn, D2) ? nn : 0;
+}
 template<class Op, int I>
 __global__ void __launch_bounds__(TG_T) k_emit(const __grid_constant__ Op op, cnt_t cn, emit_t e){
     __shared__ u64 ws[TG_T/32];
@@ -367,7 +379,12 @@ __global__ void __launch_bounds__(TG_T) k_emit(const __grid_constant__ Op op, cn
         block_sums<TG_T, 2, 1>(d, m, wd);
         if(threadIdx.x == 0){ dd_into(e.acc->dr, d[0]); dd_into(e.acc->gs, d[1]); e.acc->ngs += m[0]; }
     }
-    if(threadIdx.x == 0){ *e.tot = r; if(Op::DROP) e.acc->nkeep = op.base + r; __threadfence(); }
+    if(threadIdx.x == 0){
+        *e.tot = r;
+        if(Op::DROP) e.acc->nkeep = op.base + r;
+        if(e.host) next_frontier(e.acc, r, op.D2);         /* the winners */
+        __threadfence();
+    }
     __syncthreads();
     if(e.host && threadIdx.x < 32) publish(e.acc, e.host);
 }
@@ -414,11 +431,6 @@ static int compact(const Op &op, cnt_t cn, u64 *tot, gacc_t *acc, gacc_t *host){
 
 /* --------------------------------------------- grow --------------------------------------------- */
 struct gpart_t { u64 q; double f[4][2]; u64 nq, unres; };    /* one tile of a frontier's sums */
-#define CL 8                     /* CTAs of the one-cluster kernels, and their threads */
-#define CT 512
-#define CL_MAX ((long)CL*CT)     /* points of a frontier that one cluster takes: one per thread.  With four per thread
-                                    the whole sum of d = 5, h = 1 (16 frontiers up to 12,000 points) took 1.76 ms, with one
-                                    1.40, without the cluster 1.67 */
 struct clpart_t { gpart_t s; drop_t d; double a; u64 nk, nw; };                /* one of its CTAs' sums and counts */
 struct Grow {
     geom_t g;
@@ -489,7 +501,7 @@ __global__ void k_seed(const __grid_constant__ geom_t g, u64 *key, unsigned *wor
                        double eps, double pw, sqb_pt_t *probe){
     const int j = blockIdx.x*blockDim.x + threadIdx.x;
     if(j == 0){
-        gacc_t z = {}; z.eps = eps; z.pw = pw;
+        gacc_t z = {}; z.eps = eps; z.pw = pw; z.nrun = z.seen = 1;
         int nw; const long q = h_insert(key, mask, y0, &nw);
         if(q < 0) z.err = 1; else word[q] = SEEN;
         for(int i = 0; i < SQB_MAXD; i++) fr[0].k[i] = 0;
@@ -621,16 +633,17 @@ __global__ void __launch_bounds__(GT) k_gs_total(const double *v, long n, gacc_t
 }
 
 struct KeepOp {                  /* kept frontier points and their keys appended to the keep list, their index to kj */
-    enum { DROP = 1 };
+    enum { DROP = 1, D2 = 0 };
     geom_t g; const sqb_pt_t *fr; const double *v; const unsigned char *stt; const gacc_t *acc; int abskip;
     sqb_pt_t *keep; double *kv; u64 *kk; long *kj; u64 base;
     __device__ bool pred(long i) const { return fabs(v[i]) >= acc->thr; }
     __device__ double weight(long i) const { return __dmul_rn(v[i], acc->pw); }
-    __device__ void emit(long i, u64 r) const {
+    __device__ void emit(long i, u64 r) const { put(i, base + r, r); }
+    __device__ void put(long i, u64 at, u64 r) const {
         pt3 p = ld_pt(fr + i);
-        kk[base + r] = key_pt(g, p);
+        kk[at] = key_pt(g, p);
         pt_flag(p, abskip && !(stt[i] & SQB_NEAR));
-        st_pt(keep + base + r, p); kv[base + r] = fabs(v[i]); kj[r] = i;
+        st_pt(keep + at, p); kv[at] = fabs(v[i]); kj[r] = i;
     }
 };
 /* candidate id = (kept point j of this frontier, axis, sign): its slot in the table, and its claim; keep, kk: the
@@ -677,18 +690,20 @@ struct WinOp {                   /* winners in id order become the next frontier
  * took 0.66 ms for the grow of d = 5, h = 1.5 (10 frontiers, 8816 points); 0.59 with this.  CTA r takes the r-th eighth of the points
  * and of the candidates, a thread a run of consecutive ones, so that one scan per CTA ranks them. */
 __global__ void __cluster_dims__(CL, 1, 1) __launch_bounds__(CT)
-k_frontier(const __grid_constant__ KeepOp ko, const __grid_constant__ WinOp wo, const double *uu, long n, u64 *key, u64 mask, long *qs, gacc_t *acc, gacc_t *host, clpart_t *part){
+k_frontier(const __grid_constant__ KeepOp ko, const __grid_constant__ WinOp wo, const double *uu, u64 *key, u64 mask, long *qs, gacc_t *acc, gacc_t *host, clpart_t *part){
     __shared__ sums_sh<CT, 4, 4> ss;
     __shared__ sums_sh<CT, 2, 1> sd;
     __shared__ u64 ws[CT/32];
     __shared__ seq_sh<CT> sh;
     const geom_t &g = ko.g;
     const int r = cl_rank(), t = threadIdx.x, D2 = 2*g.D;
+    const long n = (long)acc->nrun; const u64 base = acc->nkeep;
+    if(n == 0) return;                                         /* the chain has ended, or its next frontier is larger */
     const double pw = acc->pw, a0 = acc->a;
     double inv = 0, u = 0;
     const bool ok = seq_binade(a0, &inv, &u);
     /* the sums */
-    const int E = (int)((n + CL*CT - 1)/(CL*CT));              /* points per thread, at most 4 */
+    const int E = (int)((n + CL*CT - 1)/(CL*CT));              /* points per thread: 1 */
     const long i0 = ((long)r*CT + t)*E;
     {
         sqdd f[4]; u64 c[4] = {0, 0, 0, 0};
@@ -732,7 +747,7 @@ k_frontier(const __grid_constant__ KeepOp ko, const __grid_constant__ WinOp wo, 
     cl_sync();
     u64 nk = 0;
     for(int q = 0; q < CL; q++){ const u64 x = __ldcg(&part[q].nk); if(q < r) rank += x; nk += x; }
-    for(unsigned b = km; b; b &= b - 1) ko.emit(i0 + __ffs(b) - 1, rank++);
+    for(unsigned b = km; b; b &= b - 1, rank++) ko.put(i0 + __ffs(b) - 1, base + rank, rank);
     if(r == CL - 1 && t < 7*32){
         /* the CTAs' parts into the record: warp w adds sum w, the last one the counts */
         const int w = t >> 5, l = t & 31;
@@ -751,8 +766,8 @@ k_frontier(const __grid_constant__ KeepOp ko, const __grid_constant__ WinOp wo, 
     cl_sync();
     /* the claims */
     const long nc = (long)nk*D2;
-    for(long id = (long)r*CT + t; id < nc; id += CL*CT) claim_one(g, ko.keep + ko.base, ko.kk + ko.base, key, wo.word, mask, qs, acc, id);
-    if(r == 0 && t == 0){ acc->a = a; acc->thr = thr; acc->nk = nk; acc->nkeep = ko.base + nk; }
+    for(long id = (long)r*CT + t; id < nc; id += CL*CT) claim_one(g, ko.keep + base, ko.kk + base, key, wo.word, mask, qs, acc, id);
+    if(r == 0 && t == 0){ acc->a = a; acc->thr = thr; acc->nk = nk; acc->nkeep = base + nk; }
     cl_sync();
     /* the winners */
     const long m = (nc + CL*CT - 1)/(CL*CT), id0 = ((long)r*CT + t)*m;
@@ -765,34 +780,83 @@ k_frontier(const __grid_constant__ KeepOp ko, const __grid_constant__ WinOp wo, 
     for(int q = 0; q < CL; q++){ const u64 x = __ldcg(&part[q].nw); if(q < r) rank += x; nn += x; }
     for(u64 b = wm; b; b &= b - 1) wo.emit(id0 + __ffsll((long long)b) - 1, rank++);
     if(r == 0 && t < 32){
-        if(t == 0) acc->nn = nn;
+        if(t == 0) next_frontier(acc, nn, D2);
         __syncwarp();
         publish(acc, host);
     }
 }
 
-/* the frontier's evaluation (device arrays) in; its sums and kept points added, the next frontier built.  The host
- * waits once, for the next frontier's size; a frontier with more than 2^22 possible candidates also waits for its
- * kept count, so that the table and the candidate list grow by what is needed and not by that bound */
-extern "C" int sqb_grow_expand(const double *v_dev, const unsigned char *stt_dev, const double *uu_dev, long *nnext){
-    const long n = GR.nfr; const int D2 = 2*GR.g.D;
+/* the lists' part of the launch arguments, for the frontier in fr and its successor in nx */
+static void frontier_ops(KeepOp *ko, WinOp *wo, sqb_pt_t *fr, sqb_pt_t *nx, unsigned char *frsk, unsigned char *nxsk, const double *v_dev,
+                         const unsigned char *stt_dev){
+    ko->g = GR.g; ko->fr = fr; ko->v = v_dev; ko->stt = stt_dev; ko->acc = GR.acc; ko->abskip = GR.abskip;
+    ko->keep = GR.keep; ko->kv = GR.kv; ko->kk = GR.kk; ko->kj = GR.kj; ko->base = (u64)GR.nkeep;
+    wo->fr = fr; wo->kj = GR.kj; wo->qs = GR.qs; wo->word = GR.word; wo->frsk = frsk; wo->stt = stt_dev;
+    wo->nx = nx; wo->nxsk = nxsk; wo->D2 = 2*GR.g.D; wo->st = GR.g.st; wo->gs = GR.gs; wo->base = 0;
+}
+/* room for the points of n more frontier points and nc more candidates */
+static int keep_room(long n){
     long kc = GR.keepcap, vc = GR.keepcap, yc = GR.keepcap;
     if(devbuf(&GR.keep, &kc, GR.nkeep + n, GR.nkeep) || devbuf(&GR.kv, &vc, GR.nkeep + n, GR.nkeep) ||
        devbuf(&GR.kk, &yc, GR.nkeep + n, GR.nkeep)) return -1;
     GR.keepcap = kc;
-    if(devbuf(&GR.kj, &GR.kjcap, n, 0)) return -1;
-    KeepOp ko; ko.g = GR.g; ko.fr = GR.fr; ko.v = v_dev; ko.stt = stt_dev; ko.acc = GR.acc; ko.abskip = GR.abskip;
-    ko.keep = GR.keep; ko.kv = GR.kv; ko.kk = GR.kk; ko.kj = GR.kj; ko.base = (u64)GR.nkeep;
-    const bool one = n <= CL_MAX && n*D2 <= 64L*CL*CT;
-    if(!one){
-        const long nb = (n + GS_TILE - 1)/GS_TILE;
-        if(devbuf(&GR.part, &GR.partcap, nb, 0)) return -1;
-        k_gs_tiles<<<(unsigned)nb, TG_T, 0, TS>>>(GR.g, GR.fr, v_dev, stt_dev, uu_dev, n, GR.acc, GR.part);
-        k_gs_total<<<1, GT, 0, TS>>>(v_dev, n, GR.acc, GR.part, nb);
-        TL += 2;
-        if(compact(ko, cnt_t{NULL, 1, n}, &GR.acc->nk, GR.acc, NULL)) return -1;
-    }
+    return devbuf(&GR.kj, &GR.kjcap, n, 0);
+}
+static int cand_room(long nc, long frontiers){
+    if(table_room(nc*frontiers)) return -1;
+    if(devbuf(&GR.qs, &GR.qscap, nc, 0)) return -1;
+    return frontier_room(nc);
+}
+/* after the host's wait: the counts, and err */
+static int grow_counts(void){
+    sqb_dev_count_copy(0, sizeof(gacc_t));
+    GR.nkeep = (long)GR.host->nkeep; GR.nseen = (long)GR.host->seen; GR.nfr = (long)GR.host->nn;
+    const int done = (int)((long)GR.host->steps - GR.nfrs);
+    GR.nfrs = (int)GR.host->steps;
+    if(done & 1){ sqb_pt_t *t = GR.fr; GR.fr = GR.nx; GR.nx = t; unsigned char *q = GR.frsk; GR.frsk = GR.nxsk; GR.nxsk = q; }
+    if(GR.host->err){ snprintf(terr, sizeof terr, "grow: hash table overflow"); return -1; }
+    return 0;
+}
+/* Frontiers that one cluster takes run in a chain: their sizes stay on the device (acc->nrun), the host queues the
+ * evaluation and the step of SQB_GROW_CHAIN of them and waits once.  A frontier that turns out larger, or empty, ends the
+ * chain: nrun is 0, and what is queued behind it does nothing.  (With the fallback inside the axis form's kernel, two launches a frontier and a
+ * wait for four of them: whole sum of d = 5, h = 1.5, ten frontiers, 0.66 -> 0.56 ms.) */
+extern "C" int sqb_grow_chain(long *nmax, const unsigned long long **np){
+    const int D2 = 2*GR.g.D;
+    *nmax = CL_MAX; *np = (const unsigned long long*)((char*)GR.acc + offsetof(gacc_t, nrun));
+    if(!one_cluster(GR.nfr, D2)) return 0;
+    if(keep_room(SQB_GROW_CHAIN*CL_MAX) || cand_room(CL_MAX*D2, SQB_GROW_CHAIN)) return -1;
+    return SQB_GROW_CHAIN;
+}
+extern "C" void sqb_grow_link(int s, const sqb_pt_t **pts, const unsigned char **skip){
+    *pts = s & 1 ? GR.nx : GR.fr; *skip = !GR.gs ? NULL : s & 1 ? GR.nxsk : GR.frsk;
+}
+extern "C" int sqb_grow_step(int s, const double *v_dev, const unsigned char *stt_dev, const double *uu_dev){
+    KeepOp ko; WinOp wo;
+    if(s & 1) frontier_ops(&ko, &wo, GR.nx, GR.fr, GR.nxsk, GR.frsk, v_dev, stt_dev);
+    else frontier_ops(&ko, &wo, GR.fr, GR.nx, GR.frsk, GR.nxsk, v_dev, stt_dev);
+    k_frontier<<<CL, CT, 0, TS>>>(ko, wo, uu_dev, GR.key, GR.mask, GR.qs, GR.acc, GR.host, GR.cpart); TL++;
     TCK(cudaGetLastError());
+    return 0;
+}
+extern "C" int sqb_grow_wait(void){
+    TCK(cudaStreamSynchronize(TS));
+    return grow_counts();
+}
+/* a larger frontier: its evaluation (device arrays) in; its sums and kept points added, the next frontier built.  The host
+ * waits once, for the next frontier's size; a frontier with more than 2^22 possible candidates also waits for its
+ * kept count, so that the table and the candidate list grow by what is needed and not by that bound */
+extern "C" int sqb_grow_expand(const double *v_dev, const unsigned char *stt_dev, const double *uu_dev){
+    const long n = GR.nfr; const int D2 = 2*GR.g.D;
+    if(keep_room(n)) return -1;
+    KeepOp ko; WinOp wo;
+    frontier_ops(&ko, &wo, GR.fr, GR.nx, GR.frsk, GR.nxsk, v_dev, stt_dev);
+    const long nb = (n + GS_TILE - 1)/GS_TILE;
+    if(devbuf(&GR.part, &GR.partcap, nb, 0)) return -1;
+    k_gs_tiles<<<(unsigned)nb, TG_T, 0, TS>>>(GR.g, GR.fr, v_dev, stt_dev, uu_dev, n, GR.acc, GR.part);
+    k_gs_total<<<1, GT, 0, TS>>>(v_dev, n, GR.acc, GR.part, nb);
+    TL += 2;
+    if(compact(ko, cnt_t{NULL, 1, n}, &GR.acc->nk, GR.acc, NULL)) return -1;
     long nk = n;
     if(n*D2 > 1L << 22){
         TCK(cudaMemcpyAsync(GR.host, GR.acc, sizeof(gacc_t), cudaMemcpyDeviceToHost, TS));
@@ -802,32 +866,15 @@ extern "C" int sqb_grow_expand(const double *v_dev, const unsigned char *stt_dev
     }
     const long nc = nk*D2;
     if(nc >= 0xFFFFFFF0L){ snprintf(terr, sizeof terr, "grow: %ld candidates exceed the 32-bit claim ids", nc); return -1; }
-    if(table_room(nc)) return -1;
-    if(devbuf(&GR.qs, &GR.qscap, nc, 0)) return -1;
-    if(frontier_room(nc)) return -1;
-    long nn = 0;
+    if(cand_room(nc > 0 ? nc : 1, 1)) return -1;
+    frontier_ops(&ko, &wo, GR.fr, GR.nx, GR.frsk, GR.nxsk, v_dev, stt_dev);      /* the lists may have moved */
     if(nc){
-        WinOp wo; wo.fr = GR.fr; wo.kj = GR.kj; wo.qs = GR.qs; wo.word = GR.word; wo.frsk = GR.frsk; wo.stt = stt_dev;
-        wo.nx = GR.nx; wo.nxsk = GR.nxsk; wo.D2 = D2; wo.st = GR.g.st; wo.gs = GR.gs; wo.base = 0;
-        if(one){
-            ko.fr = GR.fr;
-            k_frontier<<<CL, CT, 0, TS>>>(ko, wo, uu_dev, n, GR.key, GR.mask, GR.qs, GR.acc, GR.host, GR.cpart); TL++;
-            TCK(cudaGetLastError());
-        } else {
-            k_claim<<<grid256(nc), 256, 0, TS>>>(GR.g, GR.keep + GR.nkeep, GR.kk + GR.nkeep, GR.key, GR.word, GR.mask, GR.qs, GR.acc); TL++;
-            TCK(cudaGetLastError());
-            if(compact(wo, cnt_t{&GR.acc->nk, D2, nc}, &GR.acc->nn, GR.acc, GR.host)) return -1;
-        }
-        TCK(cudaStreamSynchronize(TS));
-        sqb_dev_count_copy(0, sizeof(gacc_t));
-        nn = (long)GR.host->nn;
+        k_claim<<<grid256(nc), 256, 0, TS>>>(GR.g, GR.keep + GR.nkeep, GR.kk + GR.nkeep, GR.key, GR.word, GR.mask, GR.qs, GR.acc); TL++;
+        TCK(cudaGetLastError());
     }
-    GR.nkeep = (long)GR.host->nkeep;
-    GR.nseen += nn; GR.nfrs++;
-    { sqb_pt_t *t = GR.fr; GR.fr = GR.nx; GR.nx = t; unsigned char *q = GR.frsk; GR.frsk = GR.nxsk; GR.nxsk = q; }
-    GR.nfr = nn; *nnext = nn;
-    if(GR.host->err){ snprintf(terr, sizeof terr, "grow: hash table overflow"); return -1; }
-    return 0;
+    if(compact(wo, cnt_t{&GR.acc->nk, D2, nc > 0 ? nc : 1}, &GR.acc->nn, GR.acc, GR.host)) return -1;
+    TCK(cudaStreamSynchronize(TS));
+    return grow_counts();
 }
 
 /* the running sum on its own (checks): a + |v[0]| pw + |v[1]| pw + ..., each addition rounded, for n values on the
@@ -864,7 +911,7 @@ extern "C" int sqb_running_sum(const double *v_dev, long n, double a, double pw,
 extern "C" int sqb_grow_probe_zero(long *unres){ *unres = (long)GR.host->punres; return GR.host->nz == 0; }
 
 struct RethOp {
-    enum { DROP = 1 };
+    enum { DROP = 1, D2 = 0 };
     const sqb_pt_t *keep; const double *kv; const u64 *kk; const gacc_t *acc; sqb_pt_t *out; double *okv; u64 *okk; u64 base;
     __device__ bool pred(long i) const { return kv[i] >= acc->thr; }
     __device__ double weight(long i) const { return __dmul_rn(kv[i], acc->pw); }
@@ -1020,7 +1067,7 @@ extern "C" int sqb_grow_sums(sqb_grow_sums_t *r){
     if(h.err){ snprintf(terr, sizeof terr, "grow: %llu table lookups failed", h.err); return -1; }
     r->S = h.S[0] + h.S[1]; r->a = h.a; r->x1 = h.x1[0] + h.x1[1]; r->x2 = h.x2[0] + h.x2[1]; r->drop = h.dr[0] + h.dr[1];
     r->gshs = h.gs[0] + h.gs[1]; r->gshn = (long)h.ngs; r->u = h.u[0] + h.u[1]; r->nq = (long)h.nq; r->unres = (long)h.unres;
-    r->kept = (long)h.m; r->cells = (long)h.ncell;
+    r->kept = (long)h.m; r->cells = (long)h.ncell; r->seen = (long)h.seen; r->frontiers = (long)h.steps;
     GR.nkeep = (long)h.m;
     return 0;
 }
@@ -1096,7 +1143,7 @@ template<int I> static int bm_order(const unsigned *bm, u64 bits, u64 base, u64 
     return 0;
 }
 struct SlotOp {
-    enum { DROP = 0 };
+    enum { DROP = 0, D2 = 0 };
     const u64 *key; const unsigned *word; u64 *out; u64 base;
     __device__ bool pred(long i) const { return word[i] != 0; }
     __device__ void emit(long i, u64 r) const { out[r] = key[i]; }
