@@ -270,6 +270,47 @@ def _parse(text):
 _LOOP = re.compile(r'^\s*REAL ([^;]*);\s*for\(int i=0;i<(\d+);i\+\+\)\{(.*?)\n  \}\n(.*)$', re.S)
 
 
+def _shared_divisors(tail, carried):
+    """The tail with its divisions by an accumulator that divides more than once (f and the |.| sum by the same
+    factor) made to share one reciprocal: the same rounded quotients (sq_divu).  Returns (tail, those accumulators);
+    the tail as it is if a statement is outside the parsed subset."""
+    out, shared, trees = [], [], []
+    for stmt in [x.strip() for x in tail.split(';') if x.strip()]:
+        m = re.match(r'^(const REAL [A-Za-z_]\w*=|\*ab=|return )(.*)$', stmt, re.S)
+        try:
+            trees.append((m.group(1), _parse(m.group(2))))
+        except (ValueError, AttributeError):
+            return tail, []
+
+    def walk(e, f):
+        f(e)
+        for a in e.args:
+            if isinstance(a, _Expr):
+                walk(a, f)
+    count = {}
+    for _, e in trees:
+        walk(e, lambda x: count.__setitem__(x.args[1].text, count.get(x.args[1].text, 0) + 1)
+             if x.op == '/' and x.args[1].text in carried else None)
+    shared = [c for c in carried if count.get(c, 0) > 1]
+
+    def text(e):
+        if e.op in ('num', 'id', 'idx'):
+            return e.text
+        if e.op == 'neg':
+            return '-' + text(e.args[0])
+        if e.op == 'par':
+            return '(' + text(e.args[0]) + ')'
+        if e.op == 'call':
+            return '%s(%s)' % (e.args[0], ','.join(text(a) for a in e.args[1:]))
+        a, b = e.args
+        if e.op == '/' and b.text in shared:
+            return 'sq_divu(%s,%s,r_%s)' % (text(a), b.text, b.text)
+        return text(a) + e.op + text(b)
+    for head, e in trees:
+        out.append('    %s%s;' % (head, text(e)))
+    return ('\n'.join(out), shared) if shared else (tail, [])
+
+
 def axis_plan(k):
     """The axis form of f_<g>, or None.
 
@@ -370,6 +411,7 @@ def axis_plan(k):
         return None
     if not any(re.search(r'SQ_(EXP|LOG)|/', c) for c in cols + consts):
         return None
+    tail, divisors = _shared_divisors(tail, carried)
     out = ['template<class SqReal_, int SQ_AB> struct KA {',
            '  enum { NU = %d, NR = %d };' % (len(cols), len(recip)),
            '  static SQ_FUNC constexpr int rc(int n){ const int c[%d]={%s}; return c[n]; }'
@@ -380,7 +422,8 @@ def axis_plan(k):
     out += ['    u[%d]=%s;' % (n, re.sub(r'\bsf\[i\]', 'si', c)) for n, c in enumerate(cols)]
     out += ['  }', '  static SQ_FUNC_K void step(st &S, const REAL si, const REAL *u, const double *r){'] + steps
     out += ['  }', '  static SQ_FUNC_K REAL fin(const st &S, REAL *ab){',
-            '    const REAL %s;' % ', '.join('%s=S.%s' % (c, c) for c in carried), tail.rstrip(), '  }', '};']
+            '    const REAL %s;' % ', '.join('%s=S.%s' % (c, c) for c in carried)]
+    out += ['    const double r_%s=sqdd_rcp(%s);' % (c, c) for c in divisors] + [tail.rstrip(), '  }', '};']
     return '\n'.join(out)
 
 

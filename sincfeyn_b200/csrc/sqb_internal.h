@@ -74,7 +74,7 @@ typedef struct {
                                      pass and the double-double pass (sqb_graph_t axis); NULL: evaluate them */
     int K;
     double H;
-    int raw;                      /* 1: plain form, v = f w and ab = ab w, no tests */
+    int raw;                      /* 1: plain form, v = f w and ab = ab w, no tests; the double-double pass: value i at raw*i */
     const unsigned char *skip;    /* per node or cell: evaluate without the |.| sums (may be NULL) */
     int abskip, abcheck;          /* with flag_at >= 0: skip = abskip && (flags & 1) */
     double abserr, near_thr, ddslack;
@@ -93,7 +93,6 @@ typedef struct {
     unsigned char *tfb;
     double pw, thr;               /* the level's weight step^D and keep threshold */
     int last;                     /* the last level: shadow-tier sums, no kept children */
-    sqb_sym_t sym;                /* cells only: the symmetry fold (sym.n <= 1: off) */
     const unsigned char *cfl;     /* cells only, the predictor at the last level (NULL: off): per child, bit 0 =
                                      not evaluated, bits 1-2 = its shadow tier */
     /* multi-instance level launch (ninst >= 1, cells, level mode): the instances' own fields above are
@@ -102,7 +101,6 @@ typedef struct {
     int ninst;
     long ntile;
     unsigned long long *queue;
-    sqb_inst_t inst[SQB_MAXINST];
     /* list mode (one integral's level batch under a fold or the predictor): the children to evaluate, as
      * child index | orbit weight << 56, *nsel of them, written by the select pass, which also zeroed the
      * others; the FP64 kernel walks the list (tiles of SQB_TILE entries from the queue) and leaves every
@@ -112,6 +110,9 @@ typedef struct {
     double *uu;                   /* uu as in sqb_dd_t */
     int sub;                      /* level launch of the axis form: work items per tile (1, or 4 when the reduce kernel sums
                                      every tile, so that a small batch fills the device) */
+    /* the large members last: what every launch reads stays together in its arguments */
+    sqb_sym_t sym;                /* cells only: the symmetry fold (sym.n <= 1: off) */
+    sqb_inst_t inst[SQB_MAXINST]; /* multi-instance level launch */
 } sqb_eval_t;
 #define SQB_SEL_SHIFT 56
 

@@ -103,7 +103,7 @@ SQDD_HD sqdd operator/(const sqdd &a, const sqdd &b){
  * operations instead of a division's ten or more.  a r is within two ulp of a / b; one correction brings it
  * within one ulp, and a second, from its exact remainder, to RN(a / b) (Markstein's theorem: P. Markstein,
  * IBM J. Res. Dev. 34, 1990, 111), as long as nothing leaves the normal range.  One test sees to that: r is NaN unless b lies
- * within 2^+-200, and the quotient is checked to lie within 2^+-700, so that a lies within 2^+-900 and the remainders,
+ * within 2^+-400, and the quotient is checked to lie within 2^+-500, so that a lies within 2^+-900 and the remainders,
  * 2^-106 a at the least, are normal; any other operands (zeros, infinities, NaN) divide. */
 SQDD_HD bool sqdd_within(double x, int bits){
 #if defined(__CUDA_ARCH__)
@@ -119,10 +119,10 @@ static inline double sqdd_div_any(double a, double b){ return SQ_DIV(a, b); }
 #endif
 SQDD_HD double sq_divu(double a, double b, double r){
     const double q0 = SQ_MUL(a, r), q1 = SQ_FMA(SQ_FMA(-q0, b, a), r, q0), q2 = SQ_FMA(SQ_FMA(-q1, b, a), r, q1);
-    return sqdd_within(q1, 700) ? q2 : sqdd_div_any(a, b);
+    return sqdd_within(q1, 500) ? q2 : sqdd_div_any(a, b);
 }
 /* what a table keeps of a divisor: RN(1/b), of the high part; NaN if sq_divu is not to use it */
-SQDD_HD double sqdd_rcp(double b){ return sqdd_within(b, 200) ? SQ_DIV(1.0, b) : NAN; }
+SQDD_HD double sqdd_rcp(double b){ return sqdd_within(b, 400) ? SQ_DIV(1.0, b) : NAN; }
 /* a / b in double-double (operator/) with r = sqdd_rcp(b): its three quotient digits by sq_divu */
 SQDD_HD sqdd sq_divu(const sqdd &a, const sqdd &b, double r){
     double q1 = sq_divu(a.hi, b.hi, r);

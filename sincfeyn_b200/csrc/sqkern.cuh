@@ -533,27 +533,23 @@ __global__ void __launch_bounds__(SQB_BLOCK) sqb_k_ax(const __grid_constant__ sq
  * the first D - 3 axes: it scans those axes once, then the last three as a binary tree, so that a child costs
  * under two and a half steps of the scan instead of D.  Thread t of a tile takes groups t, t + SQB_BLOCK, ... in
  * order of (cell, first axes): a warp's writes for one choice of the last axes are 2^(D-3) consecutive
- * children.  The thread's sums stay in registers.  Every child's value is the general kernel's bit for bit; the
+ * children.  A group's sums stay in registers and are added to the thread's column in shared memory.  Every child's value is the general kernel's bit for bit; the
  * tile sums add the same values in another fixed order.  Measured on the B200, whole last level against the
  * general kernel: syn_d8 at h = 0.7 (1.18e9 children) 125.4 -> 17.0 ms, syn_d11 at h = 2 (9.2e8) 93.6 -> 13.8 ms,
- * syn_d5 at h = 1 (2.7e6) 0.40 -> 0.12 ms; this kernel 11.7 ps a child of syn_d8, with five CTAs an SM (96 registers, 84 bytes
- * spilled; four without a spill 12.1, six 12.2).  FP64 dependences bound it: the pipe is half busy. */
+ * syn_d5 at h = 1 (2.7e6) 0.40 -> 0.12 ms; this kernel 11.5 ps a child of syn_d8, with six CTAs an SM (80 registers, 52 bytes
+ * spilled; four without a spill 13.0, five 11.8, seven 11.6; with the sums in registers and the divisors of fin apart it
+ * took five CTAs, 96 registers and 12.1).  FP64 dependences bound it: the pipe is a little more than half busy. */
 #define SQB_AXG 8
 #ifndef SQB_AX_MINB
-#define SQB_AX_MINB 5
+#define SQB_AX_MINB 6
 #endif
-/* a thread's sums: S, b1, b2 as (hi, running error), normalised at the tile's end */
-struct sqb_ax_acc { double S, Se, b1, b1e, b2, b2e, A, dr; unsigned ne, nsk, keep; bool fb; };
-__device__ __forceinline__ void sqb_ax_add(double &s, double &e, double x){
-    const sqdd z = sqdd_two_sum(s, x);
-    s = z.hi; e = SQ_ADD(e, z.lo);
-}
-/* an integral's fields in registers (in shared memory every store to global memory would have them read again) */
-struct sqb_ax_in { const double *U, *sX, *sW; int K, st, last; bool tsum; double pw, thr, abserr, near_thr, slack; };
+/* an integral's fields: of the launch's arguments (one integral: constant memory, no registers), or read once per tile (in
+ * shared memory every store to global memory would have them read again) */
+struct sqb_ax_in { const double *U, *sX, *sW; int K, st; bool tsum; double pw, thr, abserr, near_thr, slack; };
 
-template<class F, int D, int AB>
+template<class F, int D, int AB, int LAST>
 __device__ __forceinline__ void sqb_ax_group(const sqb_eval_t &a, const sqb_ax_in &I, const int *k, int low, int sk, int tier, long i0,
-                                             sqb_ax_acc &t){
+                                             sqb_tile_acc &ta, bool &fb){
     using A = typename F::template AX<double, AB>;
     constexpr int M = D - 3, EW = sqb_axw<A, double>::N;
     const int K = I.K, st = I.st, nt = 2*K + 1;
@@ -574,7 +570,8 @@ __device__ __forceinline__ void sqb_ax_group(const sqb_eval_t &a, const sqb_ax_i
     }
     double *const v = a.v + i0; unsigned char *const stt = a.stt + i0;
     const unsigned char s0 = SQB_PRESENT | (sk ? SQB_SKIPPED : 0);
-    unsigned added = 0;
+    /* the group's sums: S as (hi, running error), |v|, the dropped weight; its children added and kept */
+    double S = 0, Se = 0, Ag = 0, dr = 0; unsigned added = 0, kept = 0;
     const int kl = k[D - 1] - st < -K ? 0 : k[D - 1] - st + K, kh = k[D - 1] + K;      /* the last axis' two entries */
     /* rolled: with both forms of the leaf in the kernel the instruction caches hold no more (two turns unrolled took 20.4 ms
      * instead of 14.3 on syn_d8 at h = 0.7, where both run, four 32 ms) */
@@ -617,20 +614,27 @@ __device__ __forceinline__ void sqb_ax_group(const sqb_eval_t &a, const sqb_ax_i
             }
             v[o] = x; stt[o] = s;
             if(!I.tsum) continue;
-            if(fallback){ t.fb = true; continue; }
+            if(fallback){ fb = true; continue; }
             const double vp = x*I.pw, av = fabs(x);
-            sqb_ax_add(t.S, t.Se, vp); t.A += av; added++;
-            if(I.last){
-                if(tier >= 1) sqb_ax_add(t.b1, t.b1e, vp);
-                if(tier >= 2) sqb_ax_add(t.b2, t.b2e, vp);
-            } else if(av >= I.thr) t.keep++;
-            else t.dr += av*I.pw;
+            const sqdd z = sqdd_two_sum(S, vp);
+            S = z.hi; Se = SQ_ADD(Se, z.lo); Ag += av; added++;
+            if(!LAST){ if(av >= I.thr) kept++; else dr += av*I.pw; }
         }
     }
-    t.ne += added; t.nsk += sk ? added : 0;
+    if(!I.tsum) return;
+    /* into the thread's column; a cell's children share its shadow tier */
+    const int t = threadIdx.x;
+    const sqdd z = sqdd_two_sum(S, Se);
+    const auto add = [&](double (*c)[SQB_TILE_THREADS]){
+        const sqdd y = sqdd(c[0][t], c[1][t]) + z;
+        c[0][t] = y.hi; c[1][t] = y.lo; };
+    add(ta.S);
+    ta.A[t] += Ag; ta.ne[t] += added; ta.nsk[t] += sk ? added : 0;
+    if(LAST){ if(tier >= 1) add(ta.b1); if(tier >= 2) add(ta.b2); }
+    else { ta.dr[t] += dr; ta.keep[t] += kept; }
 }
 
-template<class F, int D>
+template<class F, int D, int LAST, int MULTI>
 __global__ void __launch_bounds__(SQB_BLOCK, SQB_AX_MINB) sqb_k_lvax(const __grid_constant__ sqb_eval_t a){
     extern __shared__ double sqb_sm[];
     __shared__ sqb_inst_t sI[SQB_MAXINST];
@@ -638,6 +642,7 @@ __global__ void __launch_bounds__(SQB_BLOCK, SQB_AX_MINB) sqb_k_lvax(const __gri
     __shared__ double wd[SQB_BLOCK/32][10];
     __shared__ unsigned wc[SQB_BLOCK/32][3];
     constexpr int M = D - 3;
+    sqb_tile_acc &ta = *(sqb_tile_acc*)(sqb_sm + sqb_table_words(a));      /* the tile sums' columns follow the tables */
     sqb_tables(a, sqb_sm, sI);
     const int t = threadIdx.x, sub = a.sub > 1 ? a.sub : 1;
     const int gper = SQB_TILE/SQB_AXG/sub;                     /* groups per work item */
@@ -648,15 +653,18 @@ __global__ void __launch_bounds__(SQB_BLOCK, SQB_AX_MINB) sqb_k_lvax(const __gri
         const long item = s_item;
         if(item >= a.ntile*sub) break;
         const long tile = item/sub;
-        const int ki = sqb_inst_at(a, tile*SQB_TILE);
-        const sqb_inst_t &I = sI[ki];
+        const sqb_inst_t &I = MULTI ? sI[sqb_inst_at(a, tile*SQB_TILE)] : a.inst[0];
         const double *sX = sqb_sm + I.toff, *sW = sX + (2*I.K + 1);
         const bool tsum = I.fused != 0;
-        const sqb_ax_in in = {I.U, sX, sW, I.K, I.st, I.last, tsum, I.pw, I.thr, I.abserr, I.near_thr, a.ddslack};
+        const sqb_ax_in in = {I.U, sX, sW, I.K, I.st, tsum, I.pw, I.thr, I.abserr, I.near_thr, a.ddslack};
         const int *const pts = (const int*)I.pts;
         const long ncell = I.n, child0 = I.child0;
         const long g0 = (tile*SQB_TILE - child0)/SQB_AXG + (item - tile*sub)*gper;
-        sqb_ax_acc ac = {0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, false};
+        bool fbt = false;
+        if(tsum){
+            ta.S[0][t] = ta.S[1][t] = ta.A[t] = ta.dr[t] = ta.b1[0][t] = ta.b1[1][t] = ta.b2[0][t] = ta.b2[1][t] = 0;
+            ta.ne[t] = ta.nsk[t] = ta.keep[t] = 0;
+        }
         for(int j = t; j < gper; j += SQB_BLOCK){
             const long gi = g0 + j, c = gi >> M;
             if(c >= ncell) break;
@@ -669,27 +677,27 @@ __global__ void __launch_bounds__(SQB_BLOCK, SQB_AX_MINB) sqb_k_lvax(const __gri
             const int fl = w3[2] >> 24;
             const int sk = a.abskip && (fl & 1);
             const long i0 = (c << D) + low + child0;
-            if(sk && !a.abcheck) sqb_ax_group<F, D, 0>(a, in, k, low, sk, (fl >> 1) & 3, i0, ac);
-            else                 sqb_ax_group<F, D, 1>(a, in, k, low, sk, (fl >> 1) & 3, i0, ac);
+            if(sk && !a.abcheck) sqb_ax_group<F, D, 0, LAST>(a, in, k, low, sk, (fl >> 1) & 3, i0, ta, fbt);
+            else                 sqb_ax_group<F, D, 1, LAST>(a, in, k, low, sk, (fl >> 1) & 3, i0, ta, fbt);
         }
-        const int fb = __syncthreads_or(tsum && ac.fb);
+        const int fb = __syncthreads_or(tsum && fbt);
         if(!tsum){ if(t == 0) a.tfb[tile] = 1; continue; }             /* summed by the reduce kernel */
-        sqdd S = sqdd_two_sum(ac.S, ac.Se), b1 = sqdd_two_sum(ac.b1, ac.b1e), b2 = sqdd_two_sum(ac.b2, ac.b2e);
-        sqdd Ad(ac.A), dd(ac.dr);
+        sqdd S(ta.S[0][t], ta.S[1][t]), b1(ta.b1[0][t], ta.b1[1][t]), b2(ta.b2[0][t], ta.b2[1][t]), Ad(ta.A[t]), dd(ta.dr[t]);
+        unsigned ne = ta.ne[t], nsk = ta.nsk[t], keep = ta.keep[t];
         for(int off = 16; off; off >>= 1){
             S = S + sqdd(__shfl_down_sync(0xffffffffu, S.hi, off), __shfl_down_sync(0xffffffffu, S.lo, off));
             Ad = Ad + sqdd(__shfl_down_sync(0xffffffffu, Ad.hi, off), __shfl_down_sync(0xffffffffu, Ad.lo, off));
             dd = dd + sqdd(__shfl_down_sync(0xffffffffu, dd.hi, off), __shfl_down_sync(0xffffffffu, dd.lo, off));
             b1 = b1 + sqdd(__shfl_down_sync(0xffffffffu, b1.hi, off), __shfl_down_sync(0xffffffffu, b1.lo, off));
             b2 = b2 + sqdd(__shfl_down_sync(0xffffffffu, b2.hi, off), __shfl_down_sync(0xffffffffu, b2.lo, off));
-            ac.ne += __shfl_down_sync(0xffffffffu, ac.ne, off); ac.nsk += __shfl_down_sync(0xffffffffu, ac.nsk, off);
-            ac.keep += __shfl_down_sync(0xffffffffu, ac.keep, off);
+            ne += __shfl_down_sync(0xffffffffu, ne, off); nsk += __shfl_down_sync(0xffffffffu, nsk, off);
+            keep += __shfl_down_sync(0xffffffffu, keep, off);
         }
         if((t & 31) == 0){
             double *x = wd[t >> 5];
             x[0] = S.hi; x[1] = S.lo; x[2] = Ad.hi; x[3] = Ad.lo; x[4] = dd.hi; x[5] = dd.lo;
             x[6] = b1.hi; x[7] = b1.lo; x[8] = b2.hi; x[9] = b2.lo;
-            wc[t >> 5][0] = ac.ne; wc[t >> 5][1] = ac.nsk; wc[t >> 5][2] = ac.keep;
+            wc[t >> 5][0] = ne; wc[t >> 5][1] = nsk; wc[t >> 5][2] = keep;
         }
         __syncthreads();
         if(t < 5){                                              /* sum t of the five over the warps, in warp order */
@@ -739,7 +747,7 @@ __global__ void __launch_bounds__(SQB_BLOCK) sqb_k_dd(const __grid_constant__ sq
             for(int d = 0; d < D; d++) sq[d] = sqdd(sf[d]);
             vq = F::template f<sqdd, 1>(sq, &abq);
         }
-        if(e.raw){ e.v[i] = vq.hi; e.vlo[i] = vq.lo; e.ab[i] = abq.hi; e.ablo[i] = abq.lo; continue; }
+        if(e.raw){ const long o = i*e.raw; e.v[o] = vq.hi; e.vlo[o] = vq.lo; e.ab[o] = abq.hi; e.ablo[o] = abq.lo; continue; }
         const double vqd = vq.value(), abqd = abq.value();
         unsigned char s;
         if(a.all){
@@ -841,7 +849,11 @@ template<class R, int AB> struct sqb_noaxis { enum { NU = 0, NR = 0 }; };
 template<class F, int D>
 static bool sqb_ax_level(const sqb_eval_t *a, int grid, int block, size_t smem, cudaStream_t st){
     if constexpr(F::template AX<double, 0>::NU > 0) if(sqb_axis_launch(a)){
-        sqb_k_lvax<F, D><<<grid, block, smem, st>>>(*a);
+        if(a->ninst == 1){
+            if(a->inst[0].last) sqb_k_lvax<F, D, 1, 0><<<grid, block, smem, st>>>(*a);
+            else sqb_k_lvax<F, D, 0, 0><<<grid, block, smem, st>>>(*a);
+        } else if(a->inst[0].last) sqb_k_lvax<F, D, 1, 1><<<grid, block, smem, st>>>(*a);      /* the same level of every integral */
+        else sqb_k_lvax<F, D, 0, 1><<<grid, block, smem, st>>>(*a);
         return true;
     }
     return false;
@@ -865,7 +877,7 @@ static bool sqb_ax_points(const sqb_eval_t *a, int grid, int block, size_t smem,
 template<class F, int D>
 static bool sqb_ax_attr(int block, size_t smem, sqb_kattr_t *o, int *ok){
     if constexpr(F::template AX<double, 0>::NU > 0){
-        *ok = sqb_attr_of(sqb_k_lvax<F, D>, block, smem, o);
+        *ok = sqb_attr_of(sqb_k_lvax<F, D, 1, 0>, block, smem, o);
         o->fused = 1; o->sweeps = 1;
         return true;
     }
