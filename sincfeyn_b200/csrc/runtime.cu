@@ -243,7 +243,8 @@ static long grid_cap(const sqb_graph_t *g, int which, size_t smem, int *fused = 
 static int grid_for(const sqb_graph_t *g, int which, long npts, size_t smem){
     sqb_kattr_t at; int per = 2;
     long want = (npts + 127)/128;
-    if(want <= G.nsm) return want < 1 ? 1 : (int)want;       /* resident whatever the kernel: no occupancy query */
+    if(want <= 4*G.nsm) return want < 1 ? 1 : (int)want;     /* two waves at most whatever the kernel: no occupancy query, which
+                                                                costs a small launch a tenth of its time */
     if(g->attr(which, 128, smem, &at) && at.blocks_per_sm > 0) per = at.blocks_per_sm;
     const long full = (long)G.nsm*per;
     return (int)(want < full ? want : full);
@@ -1163,47 +1164,95 @@ extern "C" int sqb_plugin_launch(const char *graph, int form, cudaStream_t st, l
     return 0;
 }
 
+/* Copies of a caller's pageable arrays through the thread's pinned buffers, two halves of PIN_HALF bytes in turn: the host
+ * fills or empties one half (four threads for a large piece) while the device copies the other.  The driver's own staging
+ * of pageable memory took about 170 us of the 342 of 20,001 points of syn_d11 in double-double (1.8 MB in, 0.6 out); 175 in all now.
+ * pin_to_device returns with the last pieces still under way on the stream, pin_to_host when everything has arrived. */
+#define PIN_HALF (512UL << 10)
+struct Pin {
+    char *p; cudaEvent_t ev[2];
+    ~Pin(){ if(p) cudaFreeHost(p); for(cudaEvent_t e : ev) if(e) cudaEventDestroy(e); }      /* given back when the thread ends */
+};
+static thread_local Pin P = {NULL, {NULL, NULL}};
+static int pin_room(void){
+    for(cudaEvent_t &e : P.ev) if(!e) CKR(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+    if(!P.p) CKR(cudaMallocHost(&P.p, 2*PIN_HALF));
+    return 0;
+}
+static void piece_copy(char *dst, const char *src, size_t n){
+    if(n < (128UL << 10)){ memcpy(dst, src, n); return; }
+    const size_t q = (n/4 + 63)/64*64;
+    #pragma omp parallel for num_threads(4) schedule(static, 1)
+    for(int j = 0; j < 4; j++){ const size_t o = j*q; if(o < n) memcpy(dst + o, src + o, n - o < q ? n - o : q); }
+}
+static int pin_to_device(void *dst, const void *src, size_t n){
+    for(size_t o = 0; o < n; o += PIN_HALF){
+        const int h = (o/PIN_HALF) & 1; const size_t m = n - o < PIN_HALF ? n - o : PIN_HALF;
+        CKR(cudaEventSynchronize(P.ev[h]));                /* the half's last copy (a new event is complete) */
+        piece_copy(P.p + h*PIN_HALF, (const char*)src + o, m);
+        CKR(cudaMemcpyAsync((char*)dst + o, P.p + h*PIN_HALF, m, cudaMemcpyHostToDevice, G.s));
+        CKR(cudaEventRecord(P.ev[h], G.s));
+    }
+    return 0;
+}
+static int pin_to_host(void *dst, const void *src, size_t n){
+    const size_t np = (n + PIN_HALF - 1)/PIN_HALF;
+    for(size_t p = 0; p <= np; p++){
+        if(p < np){                                         /* the half's earlier use has ended: on the stream, or below */
+            const size_t o = p*PIN_HALF, m = n - o < PIN_HALF ? n - o : PIN_HALF;
+            CKR(cudaMemcpyAsync(P.p + (p & 1)*PIN_HALF, (const char*)src + o, m, cudaMemcpyDeviceToHost, G.s));
+            CKR(cudaEventRecord(P.ev[p & 1], G.s));
+        }
+        if(p > 0){
+            const size_t o = (p - 1)*PIN_HALF, m = n - o < PIN_HALF ? n - o : PIN_HALF;
+            CKR(cudaEventSynchronize(P.ev[(p - 1) & 1]));
+            piece_copy((char*)dst + o, P.p + ((p - 1) & 1)*PIN_HALF, m);
+        }
+    }
+    return 0;
+}
+
 /* pointwise evaluation (parity checks): n points given by their variables, FP64 (SQ_AB = ab) or
  * double-double; f, abs_ hold n values (FP64) or n (hi, lo) pairs (double-double) */
 extern "C" int sqb_eval_points_impl(const sqb_graph_t *g, long n, const double *sf, int prec, int ab, double *f, double *abs_){
     if(n <= 0) return 0;
     const int D = g->D;
-    /* one stream-ordered block (no device-wide synchronisation, so other threads' work runs on):
-     * sf[n D], v, ab, vlo, ablo [n each], X = 1, skip[n] */
-    const size_t nd = (size_t)n*D + 4*(size_t)n + 1;
-    char *blk = NULL;
-    CKR(cudaMallocAsync((void**)&blk, nd*sizeof(double) + (size_t)n, G.s));
-    double *dsf = (double*)blk, *dv = dsf + (size_t)n*D, *dab = dv + n, *dvl = dab + n, *dabl = dvl + n, *dX = dabl + n;
-    unsigned char *dsk = (unsigned char*)(dX + 1);
-    const double one = 1.0;
-    CKR(cudaMemcpyAsync(dsf, sf, (size_t)n*D*sizeof(double), cudaMemcpyHostToDevice, G.s));
-    CKR(cudaMemcpyAsync(dX, &one, sizeof one, cudaMemcpyHostToDevice, G.s));
-    CKR(cudaMemsetAsync(dsk, ab ? 0 : 1, n, G.s));
+    /* one stream-ordered block (no device-wide synchronisation, so other threads' work runs on): sf[n D], the values and
+     * the |.| sums (n each, or n pairs), skip[n] */
+    const bool dd = !(prec == 0 || prec == 2);
+    const int w = dd ? 1 : f64_which(g, prec == 2);
+    if(prec == 2 && w != 2){ snprintf(g_err, sizeof g_err, "%s: no contracted FP64 kernel in this library", g->name); return -1; }
+    const size_t nv = (dd ? 2 : 1)*(size_t)n, nd = (size_t)n*D + 2*nv, nin = (size_t)n*D*sizeof(double), nout = nv*sizeof(double);
+    if(pin_room()) return -1;
+    struct Block { char *p = NULL; ~Block(){ if(p) cudaFreeAsync(p, G.s); } } blk;       /* released on every return */
+    CKR(cudaMallocAsync((void**)&blk.p, nd*sizeof(double) + (size_t)n, G.s));
+    double *dsf = (double*)blk.p, *dv = dsf + (size_t)n*D, *dab = dv + nv;
+    unsigned char *dsk = (unsigned char*)(dab + nv);
+    const bool small = nin <= PIN_HALF && 2*nout <= PIN_HALF;       /* one piece each way */
+    if(small){
+        memcpy(P.p, sf, nin);
+        CKR(cudaMemcpyAsync(dsf, P.p, nin, cudaMemcpyHostToDevice, G.s));
+    } else if(pin_to_device(dsf, sf, nin)) return -1;
+    if(!ab) CKR(cudaMemsetAsync(dsk, 1, n, G.s));
     sqb_eval_t a; memset(&a, 0, sizeof a);
     a.pts = NULL; a.n = n; a.esize = 1; a.stride = D; a.flag_at = -1; a.cells = 0;
-    a.X = dX; a.Wt = dX; a.K = 0; a.raw = 1; a.skip = dsk; a.v = dv; a.ab = dab; a.sfin = dsf; a.vlo = dvl; a.ablo = dabl;
-    size_t smem = 2*sizeof(double);
-    int rc = 0;
-    if(prec == 0 || prec == 2){
-        const int w = f64_which(g, prec == 2);
-        if(prec == 2 && w != 2){ snprintf(g_err, sizeof g_err, "%s: no contracted FP64 kernel in this library", g->name); rc = -1; }
-        else launch_f64(g, w, &a, grid_for(g, w, n, smem), smem, G.s);
-    } else { sqb_dd_t d; memset(&d, 0, sizeof d); d.e = a; d.all = 1; d.uu = dvl; g->dd(&d, grid_for(g, 1, n, smem), 128, smem, G.s); }
-    if(!rc){
-        CKR(cudaGetLastError());
-        if(prec == 0 || prec == 2){
-            CKR(cudaMemcpyAsync(f, dv, n*sizeof(double), cudaMemcpyDeviceToHost, G.s));
-            CKR(cudaMemcpyAsync(abs_, dab, n*sizeof(double), cudaMemcpyDeviceToHost, G.s));
-            CKR(cudaStreamSynchronize(G.s));
-        } else {
-            std::vector<double> h(4*(size_t)n);
-            CKR(cudaMemcpyAsync(h.data(), dv, 4*n*sizeof(double), cudaMemcpyDeviceToHost, G.s));   /* v, ab, vlo, ablo */
-            CKR(cudaStreamSynchronize(G.s));
-            for(long i = 0; i < n; i++){ f[2*i] = h[i]; f[2*i + 1] = h[2*n + i]; abs_[2*i] = h[n + i]; abs_[2*i + 1] = h[3*n + i]; }
-        }
+    /* no lattice: the one-entry tables are loaded and not used */
+    a.X = dsf; a.Wt = dsf; a.K = 0; a.raw = 1; a.skip = ab ? NULL : dsk; a.v = dv; a.ab = dab; a.sfin = dsf;
+    const size_t smem = 2*sizeof(double);
+    if(!dd) launch_f64(g, w, &a, grid_for(g, w, n, smem), smem, G.s);
+    else {                                           /* raw = 2: (hi, lo) pairs, as the caller's arrays hold them */
+        a.raw = 2; a.vlo = dv + 1; a.ablo = dab + 1;
+        sqb_dd_t d; memset(&d, 0, sizeof d); d.e = a; d.all = 1;
+        g->dd(&d, grid_for(g, 1, n, smem), 128, smem, G.s);
     }
-    cudaFreeAsync(blk, G.s);
-    return rc;
+    CKR(cudaGetLastError());
+    if(small){
+        CKR(cudaMemcpyAsync(P.p + PIN_HALF, dv, 2*nout, cudaMemcpyDeviceToHost, G.s));
+        CKR(cudaStreamSynchronize(G.s));
+        memcpy(f, P.p + PIN_HALF, nout); memcpy(abs_, P.p + PIN_HALF + nout, nout);
+        return 0;
+    }
+    return pin_to_host(f, dv, nout) || pin_to_host(abs_, dab, nout) ? -1 : 0;
 }
 
 /* the scaling test's device part: a->g[3 ndir] for the directions of a, with the factor table xs
