@@ -304,7 +304,7 @@ def _shared_divisors(tail, carried):
             return '%s(%s)' % (e.args[0], ','.join(text(a) for a in e.args[1:]))
         a, b = e.args
         if e.op == '/' and b.text in shared:
-            return 'sq_divu(%s,%s,r_%s)' % (text(a), b.text, b.text)
+            return 'sq_divc<CK>(%s,%s,r_%s,sq_bad)' % (text(a), b.text, b.text)
         return text(a) + e.op + text(b)
     for head, e in trees:
         out.append('    %s%s;' % (head, text(e)))
@@ -391,7 +391,7 @@ def axis_plan(k):
             if c is not None:
                 if c not in recip:
                     recip.append(c)
-                return 'sq_divu(%s,%s,r[%d])' % (rewrite(a), name, recip.index(c))
+                return 'sq_divc<CK>(%s,%s,r[%d],sq_bad)' % (rewrite(a), name, recip.index(c))
         return rewrite(a, e.op in '+-') + e.op + rewrite(b, e.op in '+-')
 
     try:
@@ -420,10 +420,10 @@ def axis_plan(k):
            '  static SQ_FUNC_K void init(st &S){ %s }' % ' '.join('S.%s=%s;' % c for c in carried.items()),
            '  static SQ_FUNC_K void axis(int i, const REAL si, REAL *u){'] + consts
     out += ['    u[%d]=%s;' % (n, re.sub(r'\bsf\[i\]', 'si', c)) for n, c in enumerate(cols)]
-    out += ['  }', '  static SQ_FUNC_K void step(st &S, const REAL si, const REAL *u, const double *r){'] + steps
-    out += ['  }', '  static SQ_FUNC_K REAL fin(const st &S, REAL *ab){',
+    out += ['  }', '  template<int CK=1> static SQ_FUNC_K void step(st &S, const REAL si, const REAL *u, const double *r, unsigned *sq_bad=0){'] + steps
+    out += ['  }', '  template<int CK=1> static SQ_FUNC_K REAL fin(const st &S, REAL *ab, unsigned *sq_bad=0){',
             '    const REAL %s;' % ', '.join('%s=S.%s' % (c, c) for c in carried)]
-    out += ['    const double r_%s=sqdd_rcp(%s);' % (c, c) for c in divisors] + [tail.rstrip(), '  }', '};']
+    out += ['    const double r_%s=sq_rcpc<CK>(%s,sq_bad);' % (c, c) for c in divisors] + [tail.rstrip(), '  }', '};']
     return '\n'.join(out)
 
 

@@ -103,8 +103,9 @@ SQDD_HD sqdd operator/(const sqdd &a, const sqdd &b){
  * operations instead of a division's ten or more.  a r is within two ulp of a / b; one correction brings it
  * within one ulp, and a second, from its exact remainder, to RN(a / b) (Markstein's theorem: P. Markstein,
  * IBM J. Res. Dev. 34, 1990, 111), as long as nothing leaves the normal range.  One test sees to that: r is NaN unless b lies
- * within 2^+-400, and the quotient is checked to lie within 2^+-500, so that a lies within 2^+-900 and the remainders,
+ * within 2^+-SQDD_DIVR, and the quotient is checked to lie there too, so that a lies within 2^+-900 and the remainders,
  * 2^-106 a at the least, are normal; any other operands (zeros, infinities, NaN) divide. */
+#define SQDD_DIVR 450
 SQDD_HD bool sqdd_within(double x, int bits){
 #if defined(__CUDA_ARCH__)
     return (((unsigned)__double2hiint(x) >> 20) & 0x7ff) - (1023u - bits) < 2u*bits;
@@ -119,10 +120,10 @@ static inline double sqdd_div_any(double a, double b){ return SQ_DIV(a, b); }
 #endif
 SQDD_HD double sq_divu(double a, double b, double r){
     const double q0 = SQ_MUL(a, r), q1 = SQ_FMA(SQ_FMA(-q0, b, a), r, q0), q2 = SQ_FMA(SQ_FMA(-q1, b, a), r, q1);
-    return sqdd_within(q1, 500) ? q2 : sqdd_div_any(a, b);
+    return sqdd_within(q1, SQDD_DIVR) ? q2 : sqdd_div_any(a, b);
 }
 /* what a table keeps of a divisor: RN(1/b), of the high part; NaN if sq_divu is not to use it */
-SQDD_HD double sqdd_rcp(double b){ return sqdd_within(b, 400) ? SQ_DIV(1.0, b) : NAN; }
+SQDD_HD double sqdd_rcp(double b){ return sqdd_within(b, SQDD_DIVR) ? SQ_DIV(1.0, b) : NAN; }
 /* a / b in double-double (operator/) with r = sqdd_rcp(b): its three quotient digits by sq_divu */
 SQDD_HD sqdd sq_divu(const sqdd &a, const sqdd &b, double r){
     double q1 = sq_divu(a.hi, b.hi, r);
@@ -134,6 +135,31 @@ SQDD_HD sqdd sq_divu(const sqdd &a, const sqdd &b, double r){
     return q + sqdd(q3);
 }
 SQDD_HD double sqdd_rcp(const sqdd &b){ return sqdd_rcp(b.hi); }
+/* sq_divu and sqdd_rcp with the tests put off (CK = 0): several quotients in a row raise *bad, and one test of it, by
+ * sqdd_bad, tells whether any lay outside the window; the caller then computes the whole again with CK = 1, which
+ * divides where it must.  In double-double every quotient is tested. */
+#define SQDD_DIVLIM ((2u*SQDD_DIVR) << 21)
+SQDD_HD void sqdd_flag(unsigned *bad, double x){
+#if defined(__CUDA_ARCH__)
+    *bad = max(*bad, 2u*(unsigned)__double2hiint(x) - ((1023u - SQDD_DIVR) << 21));     /* without the sign; wraps below */
+#else
+    if(!sqdd_within(x, SQDD_DIVR)) *bad = ~0u;
+#endif
+}
+SQDD_HD bool sqdd_bad(unsigned bad){ return bad >= SQDD_DIVLIM; }
+template<int CK> SQDD_HD double sq_divc(double a, double b, double r, unsigned *bad){
+    if(CK) return sq_divu(a, b, r);
+    const double q0 = SQ_MUL(a, r), q1 = SQ_FMA(SQ_FMA(-q0, b, a), r, q0);
+    sqdd_flag(bad, q1);
+    return SQ_FMA(SQ_FMA(-q1, b, a), r, q1);
+}
+template<int CK> SQDD_HD double sq_rcpc(double b, unsigned *bad){
+    if(CK) return sqdd_rcp(b);
+    sqdd_flag(bad, b);
+    return SQ_DIV(1.0, b);
+}
+template<int CK> SQDD_HD sqdd sq_divc(const sqdd &a, const sqdd &b, double r, unsigned *){ return sq_divu(a, b, r); }
+template<int CK> SQDD_HD double sq_rcpc(const sqdd &b, unsigned *){ return sqdd_rcp(b); }
 #if defined(__CUDA_ARCH__)
 /* the three quotient digits share one reciprocal: the same rounded quotients (sq_divu) for one division and fifteen
  * operations instead of three divisions */

@@ -256,8 +256,9 @@ __device__ __noinline__ sqb_fab sqb_fcall(const sqb_pt<D> p){
 /* ------------------------------------- the axis form --------------------------------------------------
  * An integrand that is a scan over its axes (kgen.axis_plan: class template KA) reads its functions of one
  * coordinate from a table over (axis, k) instead of evaluating them at every point: NU columns and the
- * reciprocals of the NR columns it divides by.  Entries in FP64: u then r; in double-double: (hi, lo) of
- * every column, then r. */
+ * reciprocals of the NR columns it divides by.  Entries in FP64: u then r, and in the lattice's table (PAD) the variable
+ * and a word of padding if need be, so that the level kernel reads an entry by 16-byte loads; in double-double: (hi, lo)
+ * of every column, then r. */
 template<class R> struct sqb_axrow;
 template<int SM> __device__ __forceinline__ double sqb_axld(const double *e){ if constexpr(SM) return *e; else return __ldg(e); }
 template<> struct sqb_axrow<double> {
@@ -271,14 +272,17 @@ template<> struct sqb_axrow<sqdd> {
         return sqdd(sqb_axld<SM>(e + 2*c), sqb_axld<SM>(e + 2*c + 1)); }
     enum { W = 2 };
 };
-template<class A, class R> struct sqb_axw { enum { N = A::NU*sqb_axrow<R>::W + A::NR }; };
+template<class A, class R, int PAD = 0> struct sqb_axw {
+    enum { E = A::NU*sqb_axrow<R>::W + A::NR, N = PAD && sqb_axrow<R>::W == 1 ? (E + 2)/2*2 : E };
+};
 
 /* entry j = axis (2K+1) + k + K of the table T over the variables X */
-template<class A, class R>
+template<class A, class R, int PAD = 0>
 __device__ __forceinline__ void sqb_axentry(const double *X, int nt, int j, double *T){
     R u[A::NU > 0 ? A::NU : 1];
     A::axis(j/nt, R(X[j % nt]), u);
-    double *e = T + (long)j*sqb_axw<A, R>::N;
+    double *e = T + (long)j*sqb_axw<A, R, PAD>::N;
+    if(PAD && sqb_axrow<R>::W == 1) e[sqb_axw<A, R>::E] = X[j % nt];
 #pragma unroll
     for(int c = 0; c < A::NU; c++) sqb_axrow<R>::put(e, c, u[c]);
 #pragma unroll
@@ -291,8 +295,8 @@ __global__ void __launch_bounds__(32) sqb_k_axis(const double *X, int K, double 
     const int nt = 2*K + 1, n = D*nt, h = (n + 31)/32;
     const int j = (blockIdx.x % h)*32 + threadIdx.x;
     if(j >= n) return;
-    if((int)blockIdx.x < h) sqb_axentry<Ad, sqdd>(X, nt, j, Td);
-    else sqb_axentry<A, double>(X, nt, j, T);
+    if((int)blockIdx.x < h) sqb_axentry<Ad, sqdd, 1>(X, nt, j, Td);
+    else sqb_axentry<A, double, 1>(X, nt, j, T);
 }
 /* one step of the scan from table entry e (SM: in shared memory) */
 template<class A, class R, int SM = 0>
@@ -311,8 +315,33 @@ __device__ __forceinline__ R sqb_axeval(const double *T, int K, const double *sf
     A::init(S);
     const int nt = 2*K + 1;
 #pragma unroll
-    for(int d = 0; d < D; d++) sqb_axstep<A, R, SM>(S, sf[d], T + (d*nt + k[d] + K)*(int)sqb_axw<A, R>::N);
+    for(int d = 0; d < D; d++) sqb_axstep<A, R, SM>(S, sf[d], T + (d*nt + k[d] + K)*(int)sqb_axw<A, R, !SM>::N);
     return A::fin(S, ab);
+}
+/* one step by the 16-byte loads of a padded entry, its quotients' tests put off (sqdd_flag) */
+template<class A>
+__device__ __forceinline__ void sqb_axstep_wide(typename A::st &S, const double *e, unsigned *bad){
+    constexpr int E = sqb_axw<A, double, 1>::E;
+    double x[E + 2];
+#pragma unroll
+    for(int c = 0; c <= E; c += 2){ const double2 y = __ldg((const double2*)(e + c)); x[c] = y.x; x[c + 1] = y.y; }
+    A::template step<0>(S, x[E], x, x + A::NU, bad);
+}
+/* the point of cell w (a packed point) whose lower bits are low, with every quotient tested */
+template<class A, int D>
+__device__ __noinline__ sqb_fab sqb_ax_redo(const double *U, int K, int st, int w0, int w1, int w2, int low){
+    constexpr int EW = sqb_axw<A, double, 1>::N;
+    const int w[3] = {w0, w1, w2};
+    typename A::st S;
+    A::init(S);
+#pragma unroll 1
+    for(int d = 0; d < D; d++){
+        const int k = (int)(signed char)(w[d >> 2] >> (8*(d & 3))) - (((low >> d) & 1) ? st : 0);
+        const double *e = U + (d*(2*K + 1) + k + K)*EW;
+        sqb_axstep<A, double>(S, e[sqb_axw<A, double>::E], e);
+    }
+    sqb_fab r; r.ab = 0; r.f = A::fin(S, &r.ab);
+    return r;
 }
 
 /* The FP64 pass.  The CTAs take tiles of consecutive points in turn: tile b, b + gridDim.x, ... of one
@@ -533,25 +562,29 @@ __global__ void __launch_bounds__(SQB_BLOCK) sqb_k_ax(const __grid_constant__ sq
  * the first D - 3 axes: it scans those axes once, then the last three as a binary tree, so that a child costs
  * under two and a half steps of the scan instead of D.  Thread t of a tile takes groups t, t + SQB_BLOCK, ... in
  * order of (cell, first axes): a warp's writes for one choice of the last axes are 2^(D-3) consecutive
- * children.  A group's sums stay in registers and are added to the thread's column in shared memory.  Every child's value is the general kernel's bit for bit; the
- * tile sums add the same values in another fixed order.  Measured on the B200, whole last level against the
- * general kernel: syn_d8 at h = 0.7 (1.18e9 children) 125.4 -> 17.0 ms, syn_d11 at h = 2 (9.2e8) 93.6 -> 13.8 ms,
- * syn_d5 at h = 1 (2.7e6) 0.40 -> 0.12 ms; this kernel 11.5 ps a child of syn_d8, with six CTAs an SM (80 registers, 52 bytes
- * spilled; four without a spill 13.0, five 11.8, seven 11.6; with the sums in registers and the divisors of fin apart it
- * took five CTAs, 96 registers and 12.1).  FP64 dependences bound it: the pipe is a little more than half busy. */
+ * children.  A group's sums stay in registers and are added to the thread's column in shared memory.  Every child's
+ * value is the general kernel's bit for bit; the tile sums add the same values in another fixed order.
+ * Measured on the B200, whole last level against the general kernel: syn_d8 at h = 0.7 (1.18e9 children) 125.4 -> 14.0 ms,
+ * syn_d11 at h = 2 (9.2e8) 93.6 -> 10.6 ms, syn_d5 at h = 1 (2.7e6) 0.40 -> 0.11 ms; this kernel 9.5 ps a child of syn_d8.
+ * What bounds it is the number of instructions, two thirds of them not FP64, and the code's size (46 KB: 61 KB ran 1 ms
+ * longer, 137 KB took 32 ms where both forms of the leaf run).  So the quotients' tests are put off to one per
+ * child (sqdd_flag; 13.6 -> 11.9 ms of kernel with the wide table loads and rolled tile sums), a warp adds up one sum of the
+ * tile instead of every thread all of them (11.9 -> 11.4), and the groups count in 32 bits (11.3 -> 11.25).  Five CTAs an SM
+ * (96 registers, 24 bytes spilled); six 0.2 ms more, seven the same as six.  Sharing the step along axis D - 3 between
+ * two turns of the loop took 11.8, the first axes' loop rolled 11.8. */
 #define SQB_AXG 8
 #ifndef SQB_AX_MINB
-#define SQB_AX_MINB 6
+#define SQB_AX_MINB 5
 #endif
 /* an integral's fields: of the launch's arguments (one integral: constant memory, no registers), or read once per tile (in
  * shared memory every store to global memory would have them read again) */
 struct sqb_ax_in { const double *U, *sX, *sW; int K, st; bool tsum; double pw, thr, abserr, near_thr, slack; };
 
 template<class F, int D, int AB, int LAST>
-__device__ __forceinline__ void sqb_ax_group(const sqb_eval_t &a, const sqb_ax_in &I, const int *k, int low, int sk, int tier, long i0,
+__device__ __forceinline__ void sqb_ax_group(const sqb_eval_t &a, const sqb_ax_in &I, const int *w3, const int *k, int low, int sk, int tier, long i0,
                                              sqb_tile_acc &ta, bool &fb){
     using A = typename F::template AX<double, AB>;
-    constexpr int M = D - 3, EW = sqb_axw<A, double>::N;
+    constexpr int M = D - 3, EW = sqb_axw<A, double, 1>::N;
     const int K = I.K, st = I.st, nt = 2*K + 1;
     /* the axes along which the lower child lies below the box; its coordinate is clamped, and the children with such a
      * bit are no points */
@@ -560,40 +593,46 @@ __device__ __forceinline__ void sqb_ax_group(const sqb_eval_t &a, const sqb_ax_i
     for(int d = 0; d < D; d++) out |= (k[d] - st < -K) << d;
     typename A::st S0;
     A::init(S0);
-    double w0 = 1.0;
+    double w0 = 1.0; unsigned bad0 = 0;
 #pragma unroll
     for(int d = 0; d < M; d++){
-        int kd = k[d] - (((low >> d) & 1) ? st : 0);
-        kd = kd < -K ? 0 : kd + K;
-        sqb_axstep<A, double>(S0, I.sX[kd], I.U + (d*nt + kd)*EW);
+        const int kd = max(k[d] + K - ((low >> d) & 1)*st, 0);
+        sqb_axstep_wide<A>(S0, I.U + (d*nt + kd)*EW, &bad0);
         w0 = w0*I.sW[kd];
     }
     double *const v = a.v + i0; unsigned char *const stt = a.stt + i0;
     const unsigned char s0 = SQB_PRESENT | (sk ? SQB_SKIPPED : 0);
     /* the group's sums: S as (hi, running error), |v|, the dropped weight; its children added and kept */
     double S = 0, Se = 0, Ag = 0, dr = 0; unsigned added = 0, kept = 0;
-    const int kl = k[D - 1] - st < -K ? 0 : k[D - 1] - st + K, kh = k[D - 1] + K;      /* the last axis' two entries */
-    /* rolled: with both forms of the leaf in the kernel the instruction caches hold no more (two turns unrolled took 20.4 ms
-     * instead of 14.3 on syn_d8 at h = 0.7, where both run, four 32 ms) */
+    int kx[3], dx[3];                                          /* the last axes' upper entries and the steps to the lower */
+#pragma unroll
+    for(int q = 0; q < 3; q++){ kx[q] = k[M + q] + K; dx[q] = min(kx[q], st); }
+    /* rolled, for the code's size */
 #pragma unroll 1
     for(int h = 0; h < 4; h++){
-        typename A::st S1 = S0; double w1 = w0;
+        typename A::st S1 = S0; double w1 = w0; unsigned bad1 = bad0;
 #pragma unroll
         for(int q = 0; q < 2; q++){
-            int kd = k[M + q] - (((h >> q) & 1) ? st : 0);
-            kd = kd < -K ? 0 : kd + K;
-            sqb_axstep<A, double>(S1, I.sX[kd], I.U + ((M + q)*nt + kd)*EW);
+            const int kd = kx[q] - ((h >> q) & 1)*dx[q];
+            sqb_axstep_wide<A>(S1, I.U + ((M + q)*nt + kd)*EW, &bad1);
             w1 = w1*I.sW[kd];
         }
         double fw[2], abw[2];
 #pragma unroll
         for(int b = 0; b < 2; b++){
-            const int kd = b ? kl : kh;
-            typename A::st S2 = S1;
-            sqb_axstep<A, double>(S2, I.sX[kd], I.U + ((D - 1)*nt + kd)*EW);
+            const int kd = b ? kx[2] - dx[2] : kx[2];
+            typename A::st S2 = S1; unsigned bad = bad1;
+            sqb_axstep_wide<A>(S2, I.U + ((D - 1)*nt + kd)*EW, &bad);
             const double w = w1*I.sW[kd];
-            double ab = 0;
-            fw[b] = A::fin(S2, &ab)*w; abw[b] = ab*w;
+            double ab = 0, f = A::template fin<0>(S2, &ab, &bad);
+            if(sqdd_bad(bad)){
+                const int lo = low | (h + 4*b) << M;
+                if(!(lo & out)){
+                    const sqb_fab r = sqb_ax_redo<A, D>(I.U, K, st, w3[0], w3[1], w3[2], lo);
+                    f = r.f; ab = r.ab;
+                }
+            }
+            fw[b] = f*w; abw[b] = ab*w;
         }
 #pragma unroll
         for(int b = 0; b < 2; b++){
@@ -624,10 +663,9 @@ __device__ __forceinline__ void sqb_ax_group(const sqb_eval_t &a, const sqb_ax_i
     if(!I.tsum) return;
     /* into the thread's column; a cell's children share its shadow tier */
     const int t = threadIdx.x;
-    const sqdd z = sqdd_two_sum(S, Se);
-    const auto add = [&](double (*c)[SQB_TILE_THREADS]){
-        const sqdd y = sqdd(c[0][t], c[1][t]) + z;
-        c[0][t] = y.hi; c[1][t] = y.lo; };
+    const auto add = [&](double (*c)[SQB_TILE_THREADS]){        /* (hi, running error) again, normalised at the tile's end */
+        const sqdd y = sqdd_two_sum(c[0][t], S);
+        c[0][t] = y.hi; c[1][t] = SQ_ADD(c[1][t], SQ_ADD(y.lo, Se)); };
     add(ta.S);
     ta.A[t] += Ag; ta.ne[t] += added; ta.nsk[t] += sk ? added : 0;
     if(LAST){ if(tier >= 1) add(ta.b1); if(tier >= 2) add(ta.b2); }
@@ -639,15 +677,13 @@ __global__ void __launch_bounds__(SQB_BLOCK, SQB_AX_MINB) sqb_k_lvax(const __gri
     extern __shared__ double sqb_sm[];
     __shared__ sqb_inst_t sI[SQB_MAXINST];
     __shared__ long s_item;
-    __shared__ double wd[SQB_BLOCK/32][10];
-    __shared__ unsigned wc[SQB_BLOCK/32][3];
     constexpr int M = D - 3;
     sqb_tile_acc &ta = *(sqb_tile_acc*)(sqb_sm + sqb_table_words(a));      /* the tile sums' columns follow the tables */
     sqb_tables(a, sqb_sm, sI);
     const int t = threadIdx.x, sub = a.sub > 1 ? a.sub : 1;
     const int gper = SQB_TILE/SQB_AXG/sub;                     /* groups per work item */
     for(;;){
-        __syncthreads();                                       /* every thread has read s_item, wd, wc */
+        __syncthreads();                                       /* every thread has read s_item and the columns */
         if(t == 0) s_item = (long)atomicAdd(a.queue, 1ULL);
         __syncthreads();
         const long item = s_item;
@@ -659,62 +695,63 @@ __global__ void __launch_bounds__(SQB_BLOCK, SQB_AX_MINB) sqb_k_lvax(const __gri
         const sqb_ax_in in = {I.U, sX, sW, I.K, I.st, tsum, I.pw, I.thr, I.abserr, I.near_thr, a.ddslack};
         const int *const pts = (const int*)I.pts;
         const long ncell = I.n, child0 = I.child0;
-        const long g0 = (tile*SQB_TILE - child0)/SQB_AXG + (item - tile*sub)*gper;
+        const long g0 = (tile*SQB_TILE - child0)/SQB_AXG + (item - tile*sub)*gper, c0 = g0 >> M;
+        /* the item's first cell and, from there on, the groups in 32 bits */
+        const int f0 = (int)(g0 & ((1 << M) - 1)), left = (int)min(ncell - c0, (long)SQB_TILE);
+        const int *const src0 = pts + c0*3;
+        const long at0 = (c0 << D) + child0;
         bool fbt = false;
         if(tsum){
             ta.S[0][t] = ta.S[1][t] = ta.A[t] = ta.dr[t] = ta.b1[0][t] = ta.b1[1][t] = ta.b2[0][t] = ta.b2[1][t] = 0;
             ta.ne[t] = ta.nsk[t] = ta.keep[t] = 0;
         }
         for(int j = t; j < gper; j += SQB_BLOCK){
-            const long gi = g0 + j, c = gi >> M;
-            if(c >= ncell) break;
-            const int low = (int)(gi & ((1 << M) - 1));
-            const int *src = pts + c*3;
+            const int c = (f0 + j) >> M;
+            if(c >= left) break;
+            const int low = (f0 + j) & ((1 << M) - 1);
+            const int *src = src0 + c*3;
             const int w3[3] = {src[0], src[1], src[2]};
             int k[D];
 #pragma unroll
             for(int d = 0; d < D; d++) k[d] = (int)(signed char)(w3[d >> 2] >> (8*(d & 3)));
             const int fl = w3[2] >> 24;
             const int sk = a.abskip && (fl & 1);
-            const long i0 = (c << D) + low + child0;
-            if(sk && !a.abcheck) sqb_ax_group<F, D, 0, LAST>(a, in, k, low, sk, (fl >> 1) & 3, i0, ta, fbt);
-            else                 sqb_ax_group<F, D, 1, LAST>(a, in, k, low, sk, (fl >> 1) & 3, i0, ta, fbt);
+            const long i0 = at0 + (((long)c << D) + low);
+            if(sk && !a.abcheck) sqb_ax_group<F, D, 0, LAST>(a, in, w3, k, low, sk, (fl >> 1) & 3, i0, ta, fbt);
+            else                 sqb_ax_group<F, D, 1, LAST>(a, in, w3, k, low, sk, (fl >> 1) & 3, i0, ta, fbt);
         }
         const int fb = __syncthreads_or(tsum && fbt);
         if(!tsum){ if(t == 0) a.tfb[tile] = 1; continue; }             /* summed by the reduce kernel */
-        sqdd S(ta.S[0][t], ta.S[1][t]), b1(ta.b1[0][t], ta.b1[1][t]), b2(ta.b2[0][t], ta.b2[1][t]), Ad(ta.A[t]), dd(ta.dr[t]);
-        unsigned ne = ta.ne[t], nsk = ta.nsk[t], keep = ta.keep[t];
-        for(int off = 16; off; off >>= 1){
-            S = S + sqdd(__shfl_down_sync(0xffffffffu, S.hi, off), __shfl_down_sync(0xffffffffu, S.lo, off));
-            Ad = Ad + sqdd(__shfl_down_sync(0xffffffffu, Ad.hi, off), __shfl_down_sync(0xffffffffu, Ad.lo, off));
-            dd = dd + sqdd(__shfl_down_sync(0xffffffffu, dd.hi, off), __shfl_down_sync(0xffffffffu, dd.lo, off));
-            b1 = b1 + sqdd(__shfl_down_sync(0xffffffffu, b1.hi, off), __shfl_down_sync(0xffffffffu, b1.lo, off));
-            b2 = b2 + sqdd(__shfl_down_sync(0xffffffffu, b2.hi, off), __shfl_down_sync(0xffffffffu, b2.lo, off));
-            ne += __shfl_down_sync(0xffffffffu, ne, off); nsk += __shfl_down_sync(0xffffffffu, nsk, off);
-            keep += __shfl_down_sync(0xffffffffu, keep, off);
+        /* warp q sums the columns of the q-th sum and count; small code, which matters here (32 children a thread and tile) */
+        const int q = t >> 5, l = t & 31;
+        sqb_part_t &P = a.part[tile];
+        {
+            const double *hi = q == 0 ? ta.S[0] : q == 1 ? ta.A : q == 2 ? (LAST ? ta.b1[0] : ta.dr) : ta.b2[0];
+            const double *lo = q == 0 ? ta.S[1] : q == 2 ? ta.b1[1] : ta.b2[1];
+            const bool one = q == 1 || (!LAST && q == 2);          /* |v| and the dropped weight: plain sums */
+            sqdd z;
+#pragma unroll 1
+            for(int c = l; c < SQB_BLOCK; c += 32) z = z + sqdd_two_sum(hi[c], one ? 0.0 : lo[c]);
+#pragma unroll 1
+            for(int off = 16; off; off >>= 1) z = z + sqdd(__shfl_down_sync(0xffffffffu, z.hi, off), __shfl_down_sync(0xffffffffu, z.lo, off));
+            if(l == 0){
+                double *dst = q == 0 ? P.S : q == 1 ? P.A : q == 2 ? (LAST ? P.b1 : P.drop) : P.b2;
+                dst[0] = z.hi; dst[1] = z.lo;
+            }
         }
-        if((t & 31) == 0){
-            double *x = wd[t >> 5];
-            x[0] = S.hi; x[1] = S.lo; x[2] = Ad.hi; x[3] = Ad.lo; x[4] = dd.hi; x[5] = dd.lo;
-            x[6] = b1.hi; x[7] = b1.lo; x[8] = b2.hi; x[9] = b2.lo;
-            wc[t >> 5][0] = ne; wc[t >> 5][1] = nsk; wc[t >> 5][2] = keep;
-        }
-        __syncthreads();
-        if(t < 5){                                              /* sum t of the five over the warps, in warp order */
-            sqdd z(wd[0][2*t], wd[0][2*t + 1]);
-            for(int w = 1; w < SQB_BLOCK/32; w++) z = z + sqdd(wd[w][2*t], wd[w][2*t + 1]);
-            sqb_part_t &P = a.part[tile];
-            double *dst = t == 0 ? P.S : t == 1 ? P.A : t == 2 ? P.drop : t == 3 ? P.b1 : P.b2;
-            dst[0] = z.hi; dst[1] = z.lo;
-        } else if(t == 5){
-            unsigned ne = 0, nsk = 0, keep = 0;
-            for(int w = 0; w < SQB_BLOCK/32; w++){ ne += wc[w][0]; nsk += wc[w][1]; keep += wc[w][2]; }
-            sqb_part_t &P = a.part[tile];
-            P.u[0] = P.u[1] = 0; P.ne = ne; P.nq = 0; P.unres = 0; P.skipped = nsk;
-            a.tkeep[tile] = keep; a.tfb[tile] = fb ? 2 : 0;
+        if(q < 3){
+            const unsigned *col = q == 0 ? ta.ne : q == 1 ? ta.nsk : ta.keep;
+            const unsigned n = __reduce_add_sync(0xffffffffu, col[l] + col[l + 32] + col[l + 64] + col[l + 96]);
+            if(l == 0){
+                if(q == 0) P.ne = n; else if(q == 1) P.skipped = n; else a.tkeep[tile] = n;
+            }
+        } else if(l == 0){
+            double *none = LAST ? P.drop : P.b1;
+            none[0] = none[1] = P.u[0] = P.u[1] = 0; P.nq = 0; P.unres = 0; a.tfb[tile] = fb ? 2 : 0;
         }
     }
 }
+static_assert(SQB_BLOCK == 128, "the tile sums of sqb_k_lvax: four warps");
 
 template<class F, int D>
 __global__ void __launch_bounds__(SQB_BLOCK) sqb_k_dd(const __grid_constant__ sqb_dd_t a){
@@ -888,7 +925,7 @@ static void sqb_ax_table(const double *X, int K, double *T, double *Td, cudaStre
     if constexpr(F::template AX<double, 0>::NU > 0)
         sqb_k_axis<typename F::template AX<double, 0>, typename F::template AX<sqdd, 1>, D><<<2*((D*(2*K + 1) + 31)/32), 32, 0, st>>>(X, K, T, Td);
 }
-template<class F, class R> struct sqb_ax_words { enum { N = F::template AX<R, 0>::NU > 0 ? (int)sqb_axw<typename F::template AX<R, 0>, R>::N : 0 }; };
+template<class F, class R> struct sqb_ax_words { enum { N = F::template AX<R, 0>::NU > 0 ? (int)sqb_axw<typename F::template AX<R, 0>, R, 1>::N : 0 }; };
 
 /* the scaling test (sqb_scale_t): one thread per (direction, q); P::pt is the graph's raw double-double
  * point function (pt_<name> of the QREAL half, SQ_AB = 1 as the reference's default) */

@@ -52,6 +52,12 @@ extern "C" void ax_##NAME(long n, const double *s, int dd, double *o){ \
     else both<decltype(&sqg_##NAME::K<double, 1>::f_##NAME), sqg_##NAME::KA<double, 1>, double, D>(&sqg_##NAME::K<double, 1>::f_##NAME, n, s, o); }
 extern "C" void divu(long n, const double *a, const double *b, double *o){
     for(long i = 0; i < n; i++) o[i] = sq_divu(a[i], b[i], sqdd_rcp(b[i])); }
+extern "C" void divc(long n, const double *a, const double *b, double *o, int *bad){
+    for(long i = 0; i < n; i++){
+        unsigned f = 0;
+        const double r = sq_rcpc<0>(b[i], &f);
+        o[i] = sq_divc<0>(a[i], b[i], r, &f); bad[i] = sqdd_bad(f);
+    } }
 '''
 
 
@@ -131,3 +137,20 @@ def test_an_added_product_keeps_its_factors_apart(tmp_path):
     src.write_text(text)
     plan = kgen.axis_plan(kgen.KernelSource(str(src)))
     assert 'S.x=S.x+u[1]*u[2];' in plan and 'u[1]=e;' in plan and 'u[2]=SQ_EXP(z);' in plan
+
+
+def test_put_off_tests_of_a_division(lib):
+    # either the rounded quotient or flagged, and flagged only outside 2^+-450
+    rng = np.random.default_rng(3)
+    n = 200000
+    a, b = (rng.choice([-1, 1], n)*(1 + rng.integers(0, 1 << 52, n)*2.0**-52)*2.0**rng.integers(-1000, 1000, n) for _ in range(2))
+    b[n//2:] = b[n//2:]/2.0**(2*np.frexp(b[n//2:])[1]//3)
+    a[:7], b[:7] = [0, 1, np.inf, np.nan, 1, 1, 0], [1, 0, 1, 1, np.inf, np.nan, 0]
+    o, bad = np.empty(n), np.empty(n, dtype=np.intc)
+    lib.divc(C.c_long(n), a.ctypes.data_as(C.c_void_p), b.ctypes.data_as(C.c_void_p), o.ctypes.data_as(C.c_void_p), bad.ctypes.data_as(C.c_void_p))
+    with np.errstate(all='ignore'):
+        q = a/b
+        inside = (np.abs(q) >= 2.0**-449) & (np.abs(q) < 2.0**449) & (np.abs(b) >= 2.0**-450) & (np.abs(b) < 2.0**450)
+    assert not np.any(bad[inside]) and np.all(bad[:7] != 0)
+    good = bad == 0
+    assert good.sum() > n//10 and np.array_equal(o[good], q[good])

@@ -150,6 +150,21 @@ def test_level_batch_equals_the_general_kernels(graph, last):
                 assert np.all(np.abs((s1 - s)[0::2] + (s1 - s)[1::2]) <= 64*EPS*s[2]), (n, route, alldd)
 
 
+@pytest.mark.parametrize('graph', ['syn_d5', 'syn_d8', 'syn_d11'])
+def test_level_batch_beyond_the_window_of_shared_reciprocals(graph):
+    # |z| to 300: table entries to 2^700, quotients and products of variables beyond 2^+-450, to zero and infinity
+    d, K, h, n = int(graph[5:]), 120, 2.5, 300
+    g = np.random.default_rng(d)
+    k = np.where(g.random((n, d)) < 0.4, K*g.choice([-1, 1], (n, d)), nodes(d, K, n, 2, d))
+    k[::3] = 2*g.integers(-K//2, K//2 + 1, k[::3].shape)
+    flags = g.random(n) < 0.5
+    for last in (False, True):
+        s, c, nxt = level('general', graph, k, flags, K, h, last, 1e-30)
+        s1, c1, nxt1 = level('axis', graph, k, flags, K, h, last, 1e-30)
+        assert c1 == c and np.array_equal(nxt1, nxt) and np.all(np.isfinite(s))
+        assert np.all(np.abs((s1 - s)[0::2] + (s1 - s)[1::2]) <= 64*EPS*s[2])
+
+
 def same(a, b):
     return all(x == y or (x != x and y != y) for x, y in zip(np.ravel(a), np.ravel(b)))
 
