@@ -309,10 +309,11 @@ __global__ void __launch_bounds__(TG_T) k_count(const __grid_constant__ Op op, c
     } else if(Op::DROP && threadIdx.x == 0) drop[blockIdx.x] = {{0, 0}, {0, 0}, 0};
     if(threadIdx.x == 0) bcnt[blockIdx.x] = (unsigned)c;
 }
-/* one CTA: exclusive scan of nb counts; the total into *tot */
+/* a CTA: exclusive scan of nb counts; the total into *tot.  CTA c scans the c-th nb counts */
 __global__ void __launch_bounds__(GT) k_scan(const unsigned *bcnt, long nb, u64 *boff, u64 *tot){
     __shared__ u64 sh[GT/32];
     u64 carry = 0;
+    bcnt += blockIdx.x*nb; boff += blockIdx.x*nb;
     for(long b = 0; b < nb; b += 4*GT){
         const long j = b + threadIdx.x*4L;
         unsigned c[4]; u64 s = 0, t;
@@ -323,7 +324,7 @@ __global__ void __launch_bounds__(GT) k_scan(const unsigned *bcnt, long nb, u64 
         for(int e = 0; e < 4; e++){ if(j + e < nb) boff[j + e] = x; x += c[e]; }
         carry += t;
     }
-    if(threadIdx.x == 0 && tot) *tot = carry;
+    if(threadIdx.x == 0 && tot) tot[blockIdx.x] = carry;
 }
 /* everything a CTA of an emitting kernel needs: counts, their scan (or NULL), and where the total goes */
 struct emit_t { const unsigned *bcnt; const u64 *boff; long nb; u64 *tot; drop_t *drop; gacc_t *acc, *host; };
@@ -1173,11 +1174,15 @@ __global__ void __launch_bounds__(RS_T) k_rs_hist(const u64 *a, cnt_t cn, int sh
     __syncthreads();
     hist[(long)threadIdx.x*nblk + blockIdx.x] = h[threadIdx.x];
 }
-__global__ void __launch_bounds__(RS_T) k_rs_scatter(const u64 *a, u64 *b, cnt_t cn, int sh, const u64 *off, long nblk){
-    __shared__ u64 base[256];
+/* off: the counts' offsets within their digit, tot: the digits' counts.  One CTA that scanned all 256 nblk counts took 208 us
+ * a pass for 4e6 keys, five times the scatter; a CTA per digit takes 5 */
+__global__ void __launch_bounds__(RS_T) k_rs_scatter(const u64 *a, u64 *b, cnt_t cn, int sh, const u64 *off, const u64 *tot, long nblk){
+    __shared__ u64 base[256], ws[RS_T/32];
+    u64 all;
     __shared__ unsigned wc[RS_T/32][256];
     const long n = cnt_of(cn);
-    base[threadIdx.x] = off[(long)threadIdx.x*nblk + blockIdx.x];
+    static_assert(RS_T == 256, "a thread per digit");
+    base[threadIdx.x] = off[(long)threadIdx.x*nblk + blockIdx.x] + block_scan<RS_T>(tot[threadIdx.x], ~0ULL, &all, ws);
     const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
     const long t0 = blockIdx.x*(long)RS_TILE;
     for(int j = 0; j < RS_I; j++){
@@ -1207,11 +1212,11 @@ static int radix_sort(u64 **a, u64 **b, cnt_t cn, int nbits){
     if(cn.max <= 1) return 0;
     const long nblk = (cn.max + RS_TILE - 1)/RS_TILE;
     unsigned *hist; u64 *off;
-    TCK(DMALLOC(&hist, 256*nblk*sizeof(unsigned))); TCK(DMALLOC(&off, 256*nblk*sizeof(u64)));
+    TCK(DMALLOC(&hist, 256*nblk*sizeof(unsigned))); TCK(DMALLOC(&off, 256*(nblk + 1)*sizeof(u64)));
     for(int sh = 0; sh < nbits; sh += 8){
         k_rs_hist<<<(unsigned)nblk, RS_T, 0, TS>>>(*a, cn, sh, hist, nblk);
-        k_scan<<<1, GT, 0, TS>>>(hist, 256*nblk, off, NULL);
-        k_rs_scatter<<<(unsigned)nblk, RS_T, 0, TS>>>(*a, *b, cn, sh, off, nblk);
+        k_scan<<<256, GT, 0, TS>>>(hist, nblk, off, off + 256*nblk);
+        k_rs_scatter<<<(unsigned)nblk, RS_T, 0, TS>>>(*a, *b, cn, sh, off, off + 256*nblk, nblk);
         TL += 3;
         TCK(cudaGetLastError());
         u64 *t = *a; *a = *b; *b = t;
@@ -1239,7 +1244,7 @@ extern "C" int sqb_grow_dilate(int nbits, sqb_pt_t **out){
     u64 *U, *T; sqb_pt_t *o;
     TCK(DMALLOC(&U, n*sizeof(u64))); TCK(DMALLOC(&T, n*sizeof(u64))); TCK(DMALLOC(&o, n*sizeof(sqb_pt_t)));
     /* the keys are base ... 2 base - 1, base = W^D.  In key order by a bitmap where the grid is small (D = 5: every
-     * lattice up to W = 55; 83,362 cells of 31^5: 33 us), else by a sort (about 35 us a pass of eight bits) */
+     * lattice up to W = 55; 83,362 cells of 31^5: 33 us), else by a sort (about 60 us a pass of eight bits for 4e6 cells) */
     const u64 base = GR.g.P[0]*(u64)GR.g.W;
     unsigned *bm = NULL;
     const size_t bmb = (size_t)((base + 127)/128)*16;
