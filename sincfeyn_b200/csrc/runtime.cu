@@ -206,21 +206,42 @@ extern "C" int sqb_dev_axis(const sqb_graph_t *g, int fma){
     return 0;
 }
 
-static int reserve_points(long n){
-    if(n <= G.cap) return 0;
-    long c = 1L << 16; while(c < n) c <<= 1;
-    if(G.v){ cudaFree(G.v); cudaFree(G.uu); cudaFree(G.stt); cudaFree(G.cfl); cudaFree(G.cw); cudaFree(G.fb); cudaFree(G.sel);
-             cudaFree(G.bp); cudaFree(G.bkeep); cudaFree(G.boff); cudaFree(G.tfb); cudaFree(G.fp); cudaFree(G.coff); }
+static void free_points(void){
+    void *p[] = {G.v, G.uu, G.stt, G.cfl, G.cw, G.fb, G.sel, G.bp, G.bkeep, G.boff, G.tfb, G.fp, G.coff};
+    for(void *q : p) if(q) cudaFree(q);
+    G.v = G.uu = NULL; G.stt = G.cfl = G.cw = G.tfb = NULL; G.fb = NULL; G.sel = G.boff = G.coff = NULL;
+    G.bp = NULL; G.bkeep = NULL; G.fp = NULL; G.cap = G.nbcap = 0;
+}
+static int alloc_points(long c){
     CKR(cudaMalloc(&G.v, c*sizeof(double))); CKR(cudaMalloc(&G.uu, c*sizeof(double)));
     CKR(cudaMalloc(&G.stt, c)); CKR(cudaMalloc(&G.cfl, c)); CKR(cudaMalloc(&G.cw, c)); CKR(cudaMalloc(&G.fb, c*sizeof(long)));
     CKR(cudaMalloc(&G.sel, c*sizeof(unsigned long long)));
-    long nb = (c + RTILE - 1)/RTILE;
+    const long nb = (c + RTILE - 1)/RTILE;
     CKR(cudaMalloc(&G.bp, nb*sizeof(part_t))); CKR(cudaMalloc(&G.bkeep, nb*sizeof(unsigned))); CKR(cudaMalloc(&G.tfb, nb));
     CKR(cudaMalloc(&G.boff, nb*sizeof(unsigned long long)));
     const long nf = nb/FT + SQB_MAXINST + 1;
     CKR(cudaMalloc(&G.fp, nf*sizeof(fpart_t))); CKR(cudaMalloc(&G.coff, nf*sizeof(unsigned long long)));
     G.cap = c; G.nbcap = nb;
     return 0;
+}
+/* room for n points; without it none is left */
+static int reserve_points(long n){
+    if(n <= G.cap) return 0;
+    long c = 1L << 16; while(c < n) c <<= 1;
+    free_points();
+    if(!alloc_points(c)) return 0;
+    free_points();
+    cudaGetLastError();
+    return -1;
+}
+/* children per batch unless the caller says: each batch costs about 80 us beside its children (the tails of its kernels, the
+ * double-double pass's longest chain), and 43 bytes a child are held.  syn_d8 at h = 0.7 with 2^24, 2^25, 2^26, 2^27: 19.7, 16.6,
+ * 15.3, 14.7 ms; 2.9 GB at 2^26.  The split pass holds its running sums as well: 2^25; so does a thread that finds no
+ * room for more. */
+#define CHILDREN (1L << 26)
+#define CHILDREN_LOW (1L << 25)
+static long batch_children(const sqb_graph_t *g, const sqb_level_t *L){
+    return L->max_children > 0 ? L->max_children : L->t.split && g->nparts > 0 ? CHILDREN_LOW : CHILDREN;
 }
 
 /* the FP64 kernel to run: the contracted one (which 2) when asked for and built, else the exact one */
@@ -764,9 +785,10 @@ __global__ void __launch_bounds__(RT) sqb_k_select(const __grid_constant__ lvl_t
 
 extern "C" int sqb_dev_level(const sqb_level_t *L, sqb_acc_t *acc, long *next_n, double *ms){
     const sqb_graph_t *g = L->g; const int D = g->D;
-    long maxch = L->max_children > 0 ? L->max_children : (1L << 25);
+    long maxch = batch_children(g, L), ncb;
+again:
     if(maxch < (1L << D)) maxch = 1L << D;
-    long ncb = maxch >> D;
+    ncb = maxch >> D;
     /* full batches hold whole rounds of tiles: the FP64 kernel's cap resident CTAs take tiles b, b + cap,
      * ..., so with a multiple of cap tiles every CTA takes the same number and none idles while others
      * finish one more */
@@ -776,7 +798,13 @@ extern "C" int sqb_dev_level(const sqb_level_t *L, sqb_acc_t *acc, long *next_n,
         const long round = (cap0*SQB_TILE) >> D;            /* cells per round (SQB_TILE >= 2^D) */
         if(!L->t.alldd && can0 && round > 0 && ncb >= 2*round) ncb = (ncb/round)*round;
     }
-    if(reserve_points(ncb << D)) return -1;
+    /* a small level reserves the lower size, so that the next ones find it */
+    const long low = CHILDREN_LOW >> D, need = L->ncell > low ? L->ncell : low;
+    if(reserve_points((need < ncb ? need : ncb) << D)){
+        if(L->max_children > 0 || maxch <= CHILDREN_LOW) return -1;
+        maxch = CHILDREN_LOW;
+        goto again;
+    }
     /* the predictor runs at the last level when its table holds values (driver/sum.c:385) */
     bool pon = false;
     if(L->last && L->predict > 0 && L->vt && L->vt->tab){
@@ -899,6 +927,7 @@ extern "C" int sqb_dev_level_multi(const sqb_level_t *Ls, int n, sqb_acc_t *accs
                      (L.sym && Ls[0].sym && L.sym->n > 1 && memcmp(L.sym, Ls[0].sym, sizeof(sqb_sym_t)));
     }
     if(one_by_one){
+one_by_one:
         /* each integral on its own tables: the thread's current ones are lent the integral's device copy */
         double tot = 0; int rc = 0;
         double *sx = G.X, *sw = G.Wt; const int sk = G.K; const double *su = G.U, *sd = G.Ud;
@@ -926,7 +955,7 @@ extern "C" int sqb_dev_level_multi(const sqb_level_t *Ls, int n, sqb_acc_t *accs
     const int which = f64_which(g, L0.t.fma);
     for(int k = 0; k < n; k++){
         const sqb_level_t &L = Ls[k];
-        long maxch = L.max_children > 0 ? L.max_children : (1L << 25);
+        long maxch = batch_children(g, &L);
         if(maxch < (1L << D)) maxch = 1L << D;
         long c = maxch >> D;
         const size_t sm1 = 2*(2*(size_t)L.K + 1)*sizeof(double);
@@ -948,7 +977,7 @@ extern "C" int sqb_dev_level_multi(const sqb_level_t *Ls, int n, sqb_acc_t *accs
         }
         if(tot > maxtot) maxtot = tot;
     }
-    if(reserve_points(maxtot)) return -1;
+    if(reserve_points(maxtot)) goto one_by_one;               /* no room for all at once */
     CKR(cudaMemsetAsync(G.accm, 0, n*sizeof(sqb_acc_t), G.s));
     CKR(cudaEventRecord(G.e0, G.s));
     for(long r = 0; r < rounds; r++){
