@@ -564,12 +564,12 @@ __global__ void __launch_bounds__(SQB_BLOCK) sqb_k_ax(const __grid_constant__ sq
  * order of (cell, first axes): a warp's writes for one choice of the last axes are 2^(D-3) consecutive
  * children.  A group's sums stay in registers and are added to the thread's column in shared memory.  Every child's
  * value is the general kernel's bit for bit; the tile sums add the same values in another fixed order.
- * Measured on the B200, whole last level against the general kernel: syn_d8 at h = 0.7 (1.18e9 children) 125.4 -> 14.0 ms,
- * syn_d11 at h = 2 (9.2e8) 93.6 -> 10.6 ms, syn_d5 at h = 1 (2.7e6) 0.40 -> 0.11 ms; this kernel 9.5 ps a child of syn_d8.
- * What bounds it is the number of instructions, two thirds of them not FP64, and the code's size (46 KB: 61 KB ran 1 ms
- * longer, 137 KB took 32 ms where both forms of the leaf run).  So the quotients' tests are put off to one per
- * child (sqdd_flag; 13.6 -> 11.9 ms of kernel with the wide table loads and rolled tile sums), a warp adds up one sum of the
- * tile instead of every thread all of them (11.9 -> 11.4), and the groups count in 32 bits (11.3 -> 11.25).  Five CTAs an SM
+ * Measured on the B200, whole last level against the general kernel: syn_d8 at h = 0.7 (1.18e9 children) 125.4 -> 12.8 ms,
+ * syn_d11 at h = 2 (9.2e8) 93.6 -> 9.7 ms, syn_d5 at h = 1 (2.7e6) 0.40 -> 0.11 ms; this kernel 8.7 ps a child of syn_d8.
+ * What bounds it is the number of instructions, two thirds of them not FP64, and the code's size (46 KB; 52 KB ran 5 %
+ * longer, 137 KB 2.8 times as long where both forms of the leaf run).  In batches of 2^25 children, syn_d8 at h = 0.7: the
+ * quotients' tests put off to one per child (sqdd_flag), wide table loads and rolled tile sums took 13.6 -> 11.9 ms, a warp per sum at the tile's end
+ * instead of every thread for all of them 11.9 -> 11.4, groups counted in 32 bits 11.3 -> 11.25.  Five CTAs an SM
  * (96 registers, 24 bytes spilled); six 0.2 ms more, seven the same as six.  Sharing the step along axis D - 3 between
  * two turns of the loop took 11.8, the first axes' loop rolled 11.8. */
 #define SQB_AXG 8
