@@ -137,12 +137,13 @@ def level(route, graph, k, flags, K, h, last, thr, alldd=0):
 def test_level_batch_equals_the_general_kernels(graph, last):
     d, K, h = int(graph[5:]), 32, 1.0
     g = np.random.default_rng(d)
-    for n in (1, 2, 37, 1 << 18 - d, (1 << 18 - d) + 1, (1 << 20 - d) - 3):
+    # the last: tiles summed by the FP64 pass, their fallback points added by a warp per tile
+    for n in (1, 2, 37, 1 << 18 - d, (1 << 18 - d) + 1, (1 << 20 - d) - 3, ((13 << 20) >> d) + 3):
         k = nodes(d, K, n, 2, n)
         flags = (g.random(n) < 0.5) + 2*g.integers(0, 3, n)
         for alldd in (0, 1) if n < 1000 else (0,):
             s, c, nxt = level('general', graph, k, flags, K, h, last, 1e-9, alldd)
-            assert c[0] > 0
+            assert c[0] > 0 and (n < 1000 or c[2] > 0)
             for route in ('axis', 'noalloc') if n << d <= 1 << 18 and not alldd else ('axis',):
                 s1, c1, nxt1 = level(route, graph, k, flags, K, h, last, 1e-9, alldd)
                 assert c1 == c and np.array_equal(nxt1, nxt), (n, route, alldd)
