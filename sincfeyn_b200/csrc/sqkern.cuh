@@ -564,8 +564,8 @@ __global__ void __launch_bounds__(SQB_BLOCK) sqb_k_ax(const __grid_constant__ sq
  * order of (cell, first axes): a warp's writes for one choice of the last axes are 2^(D-3) consecutive
  * children.  A group's sums stay in registers and are added to the thread's column in shared memory.  Every child's
  * value is the general kernel's bit for bit; the tile sums add the same values in another fixed order.
- * Measured on the B200, whole last level against the general kernel: syn_d8 at h = 0.7 (1.18e9 children) 125.4 -> 12.8 ms,
- * syn_d11 at h = 2 (9.2e8) 93.6 -> 9.7 ms, syn_d5 at h = 1 (2.7e6) 0.40 -> 0.11 ms; this kernel 8.7 ps a child of syn_d8.
+ * Measured on the B200, whole last level against the general kernel: syn_d8 at h = 0.7 (1.18e9 children) 125.4 -> 12.6 ms,
+ * syn_d11 at h = 2 (9.2e8) 93.6 -> 9.5 ms, syn_d5 at h = 1 (2.7e6) 0.40 -> 0.11 ms; this kernel 8.5 ps a child of syn_d8.
  * What bounds it is the number of instructions, two thirds of them not FP64, and the code's size (46 KB; 52 KB ran 5 %
  * longer, 137 KB 2.8 times as long where both forms of the leaf run).  In batches of 2^25 children, syn_d8 at h = 0.7: the
  * quotients' tests put off to one per child (sqdd_flag), wide table loads and rolled tile sums took 13.6 -> 11.9 ms, a warp per sum at the tile's end
@@ -600,6 +600,8 @@ __device__ __forceinline__ void sqb_ax_group(const sqb_eval_t &a, const sqb_ax_i
         sqb_axstep_wide<A>(S0, I.U + (d*nt + kd)*EW, &bad0);
         w0 = w0*I.sW[kd];
     }
+    const bool keepv = !LAST || !I.tsum;         /* the last level's summed tiles need no values but the fallback's, which the
+                                                    double-double pass writes: 9.7 -> 9.5 ms of syn_d11's last level at h = 2 */
     double *const v = a.v + i0; unsigned char *const stt = a.stt + i0;
     const unsigned char s0 = SQB_PRESENT | (sk ? SQB_SKIPPED : 0);
     /* the group's sums: S as (hi, running error), |v|, the dropped weight; its children added and kept */
@@ -637,7 +639,7 @@ __device__ __forceinline__ void sqb_ax_group(const sqb_eval_t &a, const sqb_ax_i
 #pragma unroll
         for(int b = 0; b < 2; b++){
             const int o = (h + 4*b) << M;
-            if((low | o) & out){ v[o] = 0; stt[o] = 0; continue; }
+            if((low | o) & out){ if(keepv) v[o] = 0; stt[o] = 0; continue; }
             /* finish()'s tests, as sqb_point_test */
             unsigned char s = s0; bool fallback = false;
             double x = isfinite(fw[b]) ? fw[b] : 0.0;
@@ -651,7 +653,8 @@ __device__ __forceinline__ void sqb_ax_group(const sqb_eval_t &a, const sqb_ax_i
                     if((long)q < a.fbcap) a.fb[q] = i0 + o;
                 }
             }
-            v[o] = x; stt[o] = s;
+            if(keepv) v[o] = x;
+            stt[o] = s;
             if(!I.tsum) continue;
             if(fallback){ fb = true; continue; }
             const double vp = x*I.pw, av = fabs(x);
