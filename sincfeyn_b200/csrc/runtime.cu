@@ -977,7 +977,8 @@ one_by_one:
         }
         if(tot > maxtot) maxtot = tot;
     }
-    if(reserve_points(maxtot)) goto one_by_one;               /* no room for all at once */
+    /* too large to gain by sharing (eight batches of the lower size: 11.5 GB), or no room for all at once */
+    if(maxtot > SQB_MAXINST*CHILDREN_LOW || reserve_points(maxtot)) goto one_by_one;
     CKR(cudaMemsetAsync(G.accm, 0, n*sizeof(sqb_acc_t), G.s));
     CKR(cudaEventRecord(G.e0, G.s));
     for(long r = 0; r < rounds; r++){
