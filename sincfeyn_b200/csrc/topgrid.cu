@@ -271,8 +271,10 @@ template<int T> __device__ double seq_sum(double a, const double *v, double pw, 
 }
 
 /* --------------------------------- ordered compaction ------------------------------------------------- */
-/* An Op has bool pred(long i) and void emit(long i, u64 rank); with DROP, weight(i) of an element that is left
- * out adds to the grow's dropped sums.  The number of elements is read on the device (*np + nadd); the grid covers
+/* An Op has bool pred(long i) and void emit(long i, u64 rank); with DROP, the |weight(i)| of an element that is left
+ * out adds to the grow's dropped weight, and with DROP = 2 its weight(i) to the signed sum and its number to the
+ * count as well (the frontiers' points; the final threshold has |f| alone and adds to the dropped weight only,
+ * driver/sumkey.h:399-401).  The number of elements is read on the device (*np + nadd); the grid covers
  * the host's bound on it.  Counting and emitting are two launches; a CTA finds its offset by adding the counts
  * before it itself, up to OFFS_CTAS CTAs, above that from a scan of the counts. */
 #define OFFS_CTAS 1024
@@ -378,7 +380,10 @@ __global__ void __launch_bounds__(TG_T) k_emit(const __grid_constant__ Op op, cn
             d[0] = d[0] + sqdd(p.dr[0], p.dr[1]); d[1] = d[1] + sqdd(p.gs[0], p.gs[1]); m[0] += p.n;
         }
         block_sums<TG_T, 2, 1>(d, m, wd);
-        if(threadIdx.x == 0){ dd_into(e.acc->dr, d[0]); dd_into(e.acc->gs, d[1]); e.acc->ngs += m[0]; }
+        if(threadIdx.x == 0){
+            dd_into(e.acc->dr, d[0]);
+            if(Op::DROP == 2){ dd_into(e.acc->gs, d[1]); e.acc->ngs += m[0]; }
+        }
     }
     if(threadIdx.x == 0){
         *e.tot = r;
@@ -634,7 +639,7 @@ __global__ void __launch_bounds__(GT) k_gs_total(const double *v, long n, gacc_t
 }
 
 struct KeepOp {                  /* kept frontier points and their keys appended to the keep list, their index to kj */
-    enum { DROP = 1, D2 = 0 };
+    enum { DROP = 2, D2 = 0 };
     geom_t g; const sqb_pt_t *fr; const double *v; const unsigned char *stt; const gacc_t *acc; int abskip;
     sqb_pt_t *keep; double *kv; u64 *kk; long *kj; u64 base;
     __device__ bool pred(long i) const { return fabs(v[i]) >= acc->thr; }
