@@ -898,10 +898,12 @@ static bool sqb_ax_level(const sqb_eval_t *a, int grid, int block, size_t smem, 
     }
     return false;
 }
-/* a raw launch of the plug-in fills a table per CTA from this many points on and if it fits beside the lattice
- * tables in the 48 KB that need no opt-in.  Measured per launch, K = 44: 131,072 children of syn_d5, d8, d11 13.3, 16.5,
+/* a raw launch of the plug-in fills a table per CTA from this many points on and if it fits, beside the lattice
+ * tables and the kernel's own sI, in the 48 KB that need no opt-in (static and dynamic together): syn_d8 up to K = 115,
+ * syn_d11 to 85, syn_d5 at every K.  Measured per launch, K = 44: 131,072 children of syn_d5, d8, d11 13.3, 16.5,
  * 21.0 us -> 10.0, 12.3, 14.4; 65,536 the same either way; 4.1e6 of d8 and d11 390 and 457 us -> 114 and 120 */
 #define SQB_AX_RAW (1L << 17)
+#define SQB_AX_ROOM (48*1024 - SQB_MAXINST*sizeof(sqb_inst_t))
 template<class F, int D>
 static bool sqb_ax_points(const sqb_eval_t *a, int grid, int block, size_t smem, cudaStream_t st){
     if constexpr(F::template AX<double, 0>::NU > 0){
@@ -909,7 +911,7 @@ static bool sqb_ax_points(const sqb_eval_t *a, int grid, int block, size_t smem,
         if(a->inl){ sqb_k_ax<F, D, 0, 1><<<grid, block, smem, st>>>(*a); return true; }
         if(a->U){ sqb_k_ax<F, D, 0, 0><<<grid, block, smem, st>>>(*a); return true; }
         const size_t sm = smem + (size_t)D*(2*a->K + 1)*sqb_axw<typename F::template AX<double, 0>, double>::N*sizeof(double);
-        if(a->raw && (a->cells ? a->n << D : a->n) >= SQB_AX_RAW && sm <= 48*1024){
+        if(a->raw && (a->cells ? a->n << D : a->n) >= SQB_AX_RAW && sm <= SQB_AX_ROOM){
             sqb_k_ax<F, D, 1, 0><<<grid, block, sm, st>>>(*a); return true; }
     }
     return false;
