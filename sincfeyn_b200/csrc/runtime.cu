@@ -1159,7 +1159,8 @@ extern "C" void gpu_wait(int slot, const double **fw, const double **abw){
 }
 
 /* the reference's per-graph launcher (sq_gpu_launch_t, driver/gpu.h:18-19) on device buffers: int16
- * coordinates, stride D, n points (cells: n = nc << D) */
+ * coordinates, stride D, n points (cells: n = nc << D).  It has no return value, and the caller's own CUDA runtime
+ * does not see this library's errors: a launch that fails prints and exits, as the rest of the plain form */
 extern "C" void sqb_gg_launch(const sqb_graph_t *g, void *st, long n, const short *k, const unsigned char *skip,
                               const double *EX, int K, double H, double *of, double *oab, int cmode, int cst){
     if(n <= 0) return;
@@ -1168,7 +1169,10 @@ extern "C" void sqb_gg_launch(const sqb_graph_t *g, void *st, long n, const shor
     a.pts = k; a.n = cmode ? (n >> g->D) : n; a.esize = 2; a.stride = g->D; a.flag_at = -1; a.cells = cmode; a.st = cst;
     a.X = EX; a.Wt = NULL; a.K = K; a.H = H; a.raw = 1; a.skip = skip; a.v = of; a.ab = oab;
     size_t smem = 2*(2*K + 1)*sizeof(double);
-    g->f64(&a, grid_for(g, 0, n, smem), 128, smem, st);
+    const int grid = grid_for(g, 0, n, smem);
+    cudaGetLastError();                                 /* an earlier call's error is not this launch's */
+    g->f64(&a, grid, 128, smem, st);
+    CKX(cudaGetLastError());
 }
 
 /* GG_<graph>'s launcher with the FP64 build chosen (0 as written, 2 contracted) */
