@@ -408,11 +408,26 @@ static thread_local u64 TL;    /* kernels launched by this file */
 extern "C" unsigned long long sqb_top_launches(void){ return TL; }
 extern "C" void sqb_dev_count_copy(unsigned long long h2d, unsigned long long d2h);
 
+/* device memory of one function: released on every return, an error's included, unless it is handed on (keep) */
+template<class T> struct Tmp {
+    T *p = NULL;
+    Tmp(){}
+    Tmp(const Tmp &) = delete;
+    Tmp &operator=(const Tmp &) = delete;
+    ~Tmp(){ drop(); }
+    int get(long n){ TCK(DMALLOC(&p, n*sizeof(T))); return 0; }
+    T *keep(){ T *q = p; p = NULL; return q; }
+    void drop(){ if(p) DFREE(p); p = NULL; }
+};
+/* a held pointer replaced */
+template<class T> static void hold(T *&dst, T *p){ if(dst) DFREE(dst); dst = p; }
+
 static int scratch(long nb){
     if(nb <= SC.nbcap) return 0;
-    if(SC.bcnt){ DFREE(SC.bcnt); DFREE(SC.boff); DFREE(SC.drop); SC.bcnt = NULL; SC.nbcap = 0; }
     long c = 1024; while(c < nb) c <<= 1;
-    TCK(DMALLOC(&SC.bcnt, c*sizeof(unsigned))); TCK(DMALLOC(&SC.boff, c*sizeof(u64))); TCK(DMALLOC(&SC.drop, c*sizeof(drop_t)));
+    Tmp<unsigned> a; Tmp<u64> b; Tmp<drop_t> d;
+    if(a.get(c) || b.get(c) || d.get(c)) return -1;
+    hold(SC.bcnt, a.keep()); hold(SC.boff, b.keep()); hold(SC.drop, d.keep());
     SC.nbcap = c;
     return 0;
 }
@@ -465,38 +480,35 @@ static int table_room(long extra){
     long cap = (long)GR.mask + 1;
     if((double)(GR.nseen + extra) <= 0.6*cap) return 0;
     long nc = cap; while((double)(GR.nseen + extra) > 0.6*nc) nc <<= 1;
-    u64 *k2; unsigned *w2;
-    TCK(DMALLOC(&k2, nc*sizeof(u64))); TCK(DMALLOC(&w2, nc*sizeof(unsigned)));
-    TCK(cudaMemsetAsync(k2, 0, nc*sizeof(u64), TS)); TCK(cudaMemsetAsync(w2, 0, nc*sizeof(unsigned), TS));
-    k_rehash<<<1184, 256, 0, TS>>>(GR.key, GR.word, cap, k2, w2, (u64)(nc - 1), GR.acc); TL++;
+    Tmp<u64> k2; Tmp<unsigned> w2;
+    if(k2.get(nc) || w2.get(nc)) return -1;
+    TCK(cudaMemsetAsync(k2.p, 0, nc*sizeof(u64), TS)); TCK(cudaMemsetAsync(w2.p, 0, nc*sizeof(unsigned), TS));
+    k_rehash<<<1184, 256, 0, TS>>>(GR.key, GR.word, cap, k2.p, w2.p, (u64)(nc - 1), GR.acc); TL++;
     TCK(cudaGetLastError());
-    DFREE(GR.key); DFREE(GR.word);
-    GR.key = k2; GR.word = w2; GR.mask = (u64)(nc - 1);
+    hold(GR.key, k2.keep()); hold(GR.word, w2.keep()); GR.mask = (u64)(nc - 1);
     return 0;
 }
 /* device array of at least n elements, keeping the first keep elements */
 template<class T> static int devbuf(T **p, long *cap, long n, long keep){
     if(n <= *cap && *p) return 0;
     long c = 1L << 16; while(c < n) c <<= 1;
-    T *q; TCK(DMALLOC(&q, c*sizeof(T)));
-    if(*p && keep > 0) TCK(cudaMemcpyAsync(q, *p, keep*sizeof(T), cudaMemcpyDeviceToDevice, TS));
-    if(*p) DFREE(*p);
-    *p = q; *cap = c;
+    Tmp<T> q;
+    if(q.get(c)) return -1;
+    if(*p && keep > 0) TCK(cudaMemcpyAsync(q.p, *p, keep*sizeof(T), cudaMemcpyDeviceToDevice, TS));
+    hold(*p, q.keep()); *cap = c;
     return 0;
 }
 /* frontier buffers for n points, the current frontier kept */
 static int frontier_room(long n){
     if(n <= GR.frcap && GR.fr) return 0;
     long c = 1L << 16; while(c < n) c <<= 1;
-    sqb_pt_t *a, *b; unsigned char *s1, *s2;
-    TCK(DMALLOC(&a, c*sizeof(sqb_pt_t))); TCK(DMALLOC(&b, c*sizeof(sqb_pt_t)));
-    TCK(DMALLOC(&s1, c)); TCK(DMALLOC(&s2, c));
+    Tmp<sqb_pt_t> a, b; Tmp<unsigned char> s1, s2;
+    if(a.get(c) || b.get(c) || s1.get(c) || s2.get(c)) return -1;
     if(GR.fr){
-        TCK(cudaMemcpyAsync(a, GR.fr, GR.nfr*sizeof(sqb_pt_t), cudaMemcpyDeviceToDevice, TS));
-        TCK(cudaMemcpyAsync(s1, GR.frsk, GR.nfr, cudaMemcpyDeviceToDevice, TS));
-        DFREE(GR.fr); DFREE(GR.nx); DFREE(GR.frsk); DFREE(GR.nxsk);
+        TCK(cudaMemcpyAsync(a.p, GR.fr, GR.nfr*sizeof(sqb_pt_t), cudaMemcpyDeviceToDevice, TS));
+        TCK(cudaMemcpyAsync(s1.p, GR.frsk, GR.nfr, cudaMemcpyDeviceToDevice, TS));
     }
-    GR.fr = a; GR.nx = b; GR.frsk = s1; GR.nxsk = s2; GR.frcap = c;
+    hold(GR.fr, a.keep()); hold(GR.nx, b.keep()); hold(GR.frsk, s1.keep()); hold(GR.nxsk, s2.keep()); GR.frcap = c;
     return 0;
 }
 
@@ -540,8 +552,9 @@ extern "C" int sqb_grow_begin(int D, int K, int st, int W, const unsigned long l
     while((1 << GR.g.sh) < st) GR.g.sh++;
     GR.gs = gs; GR.abskip = abskip; GR.nseen = 1; GR.nkeep = 0; GR.nfr = 0; GR.nfrs = 0;
     const long cap = 1L << 20;
-    if(GR.key){ DFREE(GR.key); DFREE(GR.word); GR.key = NULL; }
-    TCK(DMALLOC(&GR.key, cap*sizeof(u64))); TCK(DMALLOC(&GR.word, cap*sizeof(unsigned)));
+    Tmp<u64> key; Tmp<unsigned> word;
+    if(key.get(cap) || word.get(cap)) return -1;
+    hold(GR.key, key.keep()); hold(GR.word, word.keep());
     TCK(cudaMemsetAsync(GR.key, 0, cap*sizeof(u64), TS)); TCK(cudaMemsetAsync(GR.word, 0, cap*sizeof(unsigned), TS));
     GR.mask = (u64)(cap - 1);
     if(!GR.acc) TCK(DMALLOC(&GR.acc, sizeof(gacc_t)));
@@ -894,9 +907,10 @@ extern "C" int sqb_running_sum(const double *v_dev, long n, double a, double pw,
     TS = (cudaStream_t)stream;
     const long nb = (n + GS_TILE - 1)/GS_TILE;
     gacc_t h; memset(&h, 0, sizeof h); h.a = a; h.pw = pw;
-    gacc_t *acc; gpart_t *part; char *pts;
     const size_t pb = (size_t)(n + 1)*(sizeof(sqb_pt_t) + 1);
-    TCK(DMALLOC(&acc, sizeof h)); TCK(DMALLOC(&part, (nb + 1)*sizeof(gpart_t))); TCK(DMALLOC(&pts, pb));
+    Tmp<gacc_t> acc_; Tmp<gpart_t> part_; Tmp<char> pts_;
+    if(acc_.get(1) || part_.get(nb + 1) || pts_.get((long)pb)) return -1;
+    gacc_t *const acc = acc_.p; gpart_t *const part = part_.p; char *const pts = pts_.p;
     TCK(cudaMemcpyAsync(acc, &h, sizeof h, cudaMemcpyHostToDevice, TS));
     TCK(cudaMemsetAsync(pts, 0, pb, TS));
     geom_t g; memset(&g, 0, sizeof g); g.D = 1; g.K = 1; g.st = 1; g.W = 3;
@@ -908,7 +922,6 @@ extern "C" int sqb_running_sum(const double *v_dev, long n, double a, double pw,
     TCK(cudaGetLastError());
     TCK(cudaMemcpyAsync(&h, acc, sizeof h, cudaMemcpyDeviceToHost, TS));
     TCK(cudaStreamSynchronize(TS));
-    DFREE(acc); DFREE(part); DFREE(pts);
     *out = h.a;
     return 0;
 }
@@ -1029,21 +1042,23 @@ __global__ void k_tier_apply(sqb_pt_t *keep, const unsigned *tr, const gacc_t *a
 /* the final threshold (eps times the whole sum) and the tiers; the kept list stays on the device, its length there
  * too (GR.nkeep bounds it until a wait) */
 extern "C" int sqb_grow_finish(int tiers){
-    sqb_pt_t *out; double *okv; u64 *okk; const long n = GR.nkeep;
-    TCK(DMALLOC(&out, (n ? n : 1)*sizeof(sqb_pt_t))); TCK(DMALLOC(&okv, (n ? n : 1)*sizeof(double))); TCK(DMALLOC(&okk, (n ? n : 1)*sizeof(u64)));
-    if(n){
-        RethOp ro; ro.keep = GR.keep; ro.kv = GR.kv; ro.kk = GR.kk; ro.acc = GR.acc; ro.out = out; ro.okv = okv; ro.okk = okk; ro.base = 0;
-        if(compact(ro, cnt_t{NULL, 1, n}, &GR.acc->m, GR.acc, NULL)) return -1;
+    const long n = GR.nkeep;
+    {
+        Tmp<sqb_pt_t> out; Tmp<double> okv; Tmp<u64> okk;
+        if(out.get(n ? n : 1) || okv.get(n ? n : 1) || okk.get(n ? n : 1)) return -1;
+        if(n){
+            RethOp ro; ro.keep = GR.keep; ro.kv = GR.kv; ro.kk = GR.kk; ro.acc = GR.acc; ro.out = out.p; ro.okv = okv.p; ro.okk = okk.p; ro.base = 0;
+            if(compact(ro, cnt_t{NULL, 1, n}, &GR.acc->m, GR.acc, NULL)) return -1;
+        }
+        hold(GR.keep, out.keep()); hold(GR.kv, okv.keep()); hold(GR.kk, okk.keep()); GR.keepcap = n ? n : 1;
     }
-    DFREE(GR.keep); DFREE(GR.kv); DFREE(GR.kk); GR.keep = out; GR.kv = okv; GR.kk = okk; GR.keepcap = n ? n : 1;
     if(!tiers || !n) return 0;
-    unsigned *tr; long *cu, *nw; u64 *cnt;
-    TCK(DMALLOC(&tr, n*sizeof(unsigned))); TCK(DMALLOC(&cu, 2*n*sizeof(long))); TCK(DMALLOC(&nw, 2*n*sizeof(long)));
-    TCK(DMALLOC(&cnt, 3*sizeof(u64)));
+    Tmp<unsigned> tr_; Tmp<long> cu_, nw_; Tmp<u64> cnt_;
+    if(tr_.get(n) || cu_.get(2*n) || nw_.get(2*n) || cnt_.get(3)) return -1;
+    unsigned *const tr = tr_.p; long *cu = cu_.p, *nw = nw_.p; u64 *const cnt = cnt_.p;
     if(n <= TIER_CL){
         k_tiers<<<CL, CT, 0, TS>>>(GR.g, GR.keep, GR.kk, GR.key, GR.word, GR.mask, GR.kv, GR.acc, tr, cu, nw, cnt); TL++;
         TCK(cudaGetLastError());
-        DFREE(tr); DFREE(cu); DFREE(nw); DFREE(cnt);
         return 0;
     }
     TCK(cudaMemsetAsync(tr, 0, n*sizeof(unsigned), TS));
@@ -1061,7 +1076,6 @@ extern "C" int sqb_grow_finish(int tiers){
     k_tier_apply<<<grid256(n), 256, 0, TS>>>(GR.keep, tr, GR.acc);
     TL += 2;
     TCK(cudaGetLastError());
-    DFREE(tr); DFREE(cu); DFREE(nw); DFREE(cnt);
     return 0;
 }
 /* waits and reads the record: the grow's sums (S, a, x1, x2, dropped weight, signed sum below the threshold) and counts */
@@ -1216,8 +1230,9 @@ __global__ void __launch_bounds__(RS_T) k_rs_scatter(const u64 *a, u64 *b, cnt_t
 static int radix_sort(u64 **a, u64 **b, cnt_t cn, int nbits){
     if(cn.max <= 1) return 0;
     const long nblk = (cn.max + RS_TILE - 1)/RS_TILE;
-    unsigned *hist; u64 *off;
-    TCK(DMALLOC(&hist, 256*nblk*sizeof(unsigned))); TCK(DMALLOC(&off, 256*(nblk + 1)*sizeof(u64)));
+    Tmp<unsigned> hist_; Tmp<u64> off_;
+    if(hist_.get(256*nblk) || off_.get(256*(nblk + 1))) return -1;
+    unsigned *const hist = hist_.p; u64 *const off = off_.p;
     for(int sh = 0; sh < nbits; sh += 8){
         k_rs_hist<<<(unsigned)nblk, RS_T, 0, TS>>>(*a, cn, sh, hist, nblk);
         k_scan<<<256, GT, 0, TS>>>(hist, nblk, off, off + 256*nblk);
@@ -1226,16 +1241,15 @@ static int radix_sort(u64 **a, u64 **b, cnt_t cn, int nbits){
         TCK(cudaGetLastError());
         u64 *t = *a; *a = *b; *b = t;
     }
-    DFREE(hist); DFREE(off);
     return 0;
 }
 extern "C" int sqb_radix_sort_u64(unsigned long long *keys_dev, long n, int nbits, void *stream){
     TS = (cudaStream_t)stream;
-    u64 *b, *a = keys_dev;
-    TCK(DMALLOC(&b, (n ? n : 1)*sizeof(u64)));
+    Tmp<u64> tmp;
+    if(tmp.get(n ? n : 1)) return -1;
+    u64 *b = tmp.p, *a = keys_dev;
     if(radix_sort(&a, &b, cnt_t{NULL, 1, n}, nbits)) return -1;
-    if(a != keys_dev){ TCK(cudaMemcpyAsync(keys_dev, a, n*sizeof(u64), cudaMemcpyDeviceToDevice, TS)); DFREE(a); }
-    else DFREE(b);
+    if(a != keys_dev) TCK(cudaMemcpyAsync(keys_dev, a, n*sizeof(u64), cudaMemcpyDeviceToDevice, TS));
     TCK(cudaStreamSynchronize(TS));
     return 0;
 }
@@ -1246,31 +1260,31 @@ extern "C" int sqb_grow_dilate(int nbits, sqb_pt_t **out){
     *out = NULL;
     if(!GR.nkeep) return 0;
     const long cap = (long)GR.mask + 1, n = GR.nseen;
-    u64 *U, *T; sqb_pt_t *o;
-    TCK(DMALLOC(&U, n*sizeof(u64))); TCK(DMALLOC(&T, n*sizeof(u64))); TCK(DMALLOC(&o, n*sizeof(sqb_pt_t)));
+    Tmp<u64> U_, T_; Tmp<sqb_pt_t> o; Tmp<char> bm_;
+    if(U_.get(n) || T_.get(n) || o.get(n)) return -1;
+    u64 *U = U_.p, *T = T_.p;
     /* the keys are base ... 2 base - 1, base = W^D.  In key order by a bitmap where the grid is small (D = 5: every
      * lattice up to W = 55; 83,362 cells of 31^5: 33 us), else by a sort (about 60 us a pass of eight bits for 4e6 cells) */
     const u64 base = GR.g.P[0]*(u64)GR.g.W;
     unsigned *bm = NULL;
     const size_t bmb = (size_t)((base + 127)/128)*16;
     if(base <= BM_BITS){
-        TCK(DMALLOC(&bm, bmb));
+        if(bm_.get((long)bmb)) return -1;
+        bm = (unsigned*)bm_.p;
         TCK(cudaMemsetAsync(bm, 0, bmb, TS));
     }
     TCK(cudaMemsetAsync(GR.word, 0, cap*sizeof(unsigned), TS));
     k_dil_mark<<<grid256(GR.nkeep*(2*GR.g.D + 1)), 256, 0, TS>>>(GR.g, GR.keep, GR.kk, GR.key, GR.word, GR.mask, GR.acc, bm, base); TL++;
     if(bm){
         if(base <= 1ULL << 25 ? bm_order<1>(bm, base, base, U, &GR.acc->ncell) : bm_order<8>(bm, base, base, U, &GR.acc->ncell)) return -1;
-        DFREE(bm);
     } else {
         SlotOp so; so.key = GR.key; so.word = GR.word; so.out = U; so.base = 0;
         if(compact(so, cnt_t{NULL, 1, cap}, &GR.acc->ncell, GR.acc, NULL)) return -1;
         if(radix_sort(&U, &T, cnt_t{&GR.acc->ncell, 1, n}, nbits)) return -1;
     }
-    k_dil_decode<<<grid256(n), 256, 0, TS>>>(GR.g, U, GR.key, GR.word, GR.mask, o, GR.acc); TL++;
+    k_dil_decode<<<grid256(n), 256, 0, TS>>>(GR.g, U, GR.key, GR.word, GR.mask, o.p, GR.acc); TL++;
     TCK(cudaGetLastError());
-    DFREE(U); DFREE(T);
-    *out = o;
+    *out = o.keep();
     return 0;
 }
 
@@ -1279,9 +1293,7 @@ extern "C" void sqb_grow_kept(const sqb_pt_t **keep, long *m){ *keep = GR.keep; 
 
 /* top = 0 keeps no list; the kept list is released with the table */
 extern "C" void sqb_grow_end(void){
-    if(GR.key){ DFREE(GR.key); DFREE(GR.word); GR.key = NULL; }
-    if(GR.keep){ DFREE(GR.keep); GR.keep = NULL; GR.keepcap = 0; }
-    if(GR.kv){ DFREE(GR.kv); GR.kv = NULL; }
-    if(GR.kk){ DFREE(GR.kk); GR.kk = NULL; }
-    GR.nkeep = 0;
+    hold(GR.key, (u64*)NULL); hold(GR.word, (unsigned*)NULL);
+    hold(GR.keep, (sqb_pt_t*)NULL); hold(GR.kv, (double*)NULL); hold(GR.kk, (u64*)NULL);
+    GR.nkeep = GR.keepcap = 0;
 }
