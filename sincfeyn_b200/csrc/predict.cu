@@ -29,7 +29,8 @@ static_assert(sizeof(VSlot) == 16, "one slot is 16 bytes, as the checkpoint stor
 
 static thread_local char perr[256];
 extern "C" const char *sqb_vtab_error(void){ return perr; }
-#define PCK(x) do { cudaError_t e_ = (x); if(e_ != cudaSuccess){ snprintf(perr, sizeof perr, "%s: %s", #x, cudaGetErrorString(e_)); return -1; } } while(0)
+#define PCK(x) do { cudaError_t e_ = (x); if(e_ != cudaSuccess){ snprintf(perr, sizeof perr, "%s: %s", #x, cudaGetErrorString(e_)); \
+    cudaGetLastError(); return -1; } } while(0)
 
 __device__ __forceinline__ unsigned long long v_hash(const int *k, int D){
     unsigned long long y = 0x9E3779B97F4A7C15ULL;

@@ -37,6 +37,7 @@ extern "C" const int SQB_NALL;
 static thread_local char g_err[512];
 #define CKR(x) do { cudaError_t e_ = (x); if(e_ != cudaSuccess){                                    \
     snprintf(g_err, sizeof g_err, "%s at %s:%d: %s", #x, __FILE__, __LINE__, cudaGetErrorString(e_)); \
+    cudaGetLastError();              /* reported here: not the next call's error */                  \
     return (int)e_; } } while(0)
 
 extern "C" const char *sqb_last_error(void){ return g_err; }

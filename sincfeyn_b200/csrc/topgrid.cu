@@ -44,6 +44,7 @@
 static thread_local char terr[512];   /* the state of this file is per host thread, like the runtime's */
 #define TCK(x) do { cudaError_t e_ = (x); if(e_ != cudaSuccess){                                    \
     snprintf(terr, sizeof terr, "%s at %s:%d: %s", #x, __FILE__, __LINE__, cudaGetErrorString(e_));   \
+    cudaGetLastError();              /* reported here: not the next call's error */                  \
     return (int)e_; } } while(0)
 extern "C" const char *sqb_top_error(void){ return terr; }
 

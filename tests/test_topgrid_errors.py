@@ -1,7 +1,8 @@
 """The grow's device memory when an allocation fails (CPU, against a stand-in for the CUDA runtime that counts
 allocations and refuses the n-th): whichever allocation of a grow, its final threshold, its tiers and its dilation is
 refused, the call returns an error, nothing is released twice, and after sqb_grow_end only the buffers that the thread
-keeps for its next grow are held; the next grow on the thread runs.  Kernels do not run: the stand-in launches nothing,
+keeps for its next grow are held; the next grow on the thread runs, and does not meet the reported error again as the
+runtime's last one.  Kernels do not run: the stand-in launches nothing,
 and the sizes that the host would read back are set by the test."""
 import ctypes as C
 import os
@@ -32,7 +33,7 @@ int cudaHostAlloc(void **p, size_t n, unsigned f){ *p = calloc(1, n); return 0; 
 int cudaMemcpyAsync(void *d, const void *s, size_t n, int k, void *st){ memmove(d, s, n); return 0; }
 int cudaMemsetAsync(void *d, int v, size_t n, void *st){ memset(d, v, n); return 0; }
 int cudaStreamSynchronize(void *s){ return 0; }
-int cudaGetLastError(void){ return 0; }
+int cudaGetLastError(void){ const int e = fake_last; fake_last = 0; return e; }
 const char *cudaGetErrorString(int e){ return e == 2 ? "out of memory" : "error"; }
 int cudaLaunchKernel(){ return 0; }
 int cudaLaunchKernelExC(){ return 0; }
