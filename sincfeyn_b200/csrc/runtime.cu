@@ -241,6 +241,9 @@ static int reserve_points(long n){
  * room for more. */
 #define CHILDREN (1L << 26)
 #define CHILDREN_LOW (1L << 25)
+/* children per launch of a group's round: a launch takes the batches of as many of its integrals as fit (eight of the lower
+ * size, four of the full one; a batch is never split, so that every integral keeps the batches it has alone) */
+#define GROUP_CHILDREN (SQB_MAXINST*CHILDREN_LOW)
 static long batch_children(const sqb_graph_t *g, const sqb_level_t *L){
     return L->max_children > 0 ? L->max_children : L->t.split && g->nparts > 0 ? CHILDREN_LOW : CHILDREN;
 }
@@ -913,7 +916,8 @@ static const double *level_axis(const sqb_level_t &L, int dd){
 
 /* A level of several integrals of one graph at once (see sqb_rt.h).  Each integral keeps the batches,
  * tiles and fused/unfused choice that sqb_dev_level would give it alone; round r launches batch r of every
- * integral that has one, its children numbered integral after integral from tile boundaries. */
+ * integral that has one, its children numbered integral after integral from tile boundaries, in as few launches of up
+ * to GROUP_CHILDREN as hold them. */
 extern "C" int sqb_dev_level_multi(const sqb_level_t *Ls, int n, sqb_acc_t *accs, long *next_n, double *ms){
     if(n <= 0) return 0;
     bool one_by_one = n == 1 || n > SQB_MAXINST;
@@ -968,31 +972,38 @@ one_by_one:
         nbat[k] = (L.ncell + c - 1)/c;
         if(nbat[k] > rounds) rounds = nbat[k];
     }
-    /* the largest round's children, each integral's batch from a tile boundary */
+    /* the children of integral k's batch r, from a tile boundary; the largest launch's children */
+    const auto batch_tiles = [&](int k, long r){
+        const long nc = Ls[k].ncell - r*ncb[k] < ncb[k] ? Ls[k].ncell - r*ncb[k] : ncb[k];
+        return ((nc << D) + SQB_TILE - 1)/SQB_TILE*SQB_TILE;
+    };
     long maxtot = 0;
     for(long r = 0; r < rounds; r++){
         long tot = 0;
         for(int k = 0; k < n; k++) if(r < nbat[k]){
-            const long nc = Ls[k].ncell - r*ncb[k] < ncb[k] ? Ls[k].ncell - r*ncb[k] : ncb[k];
-            tot += ((nc << D) + SQB_TILE - 1)/SQB_TILE*SQB_TILE;
+            const long b = batch_tiles(k, r);
+            if(tot > 0 && tot + b > GROUP_CHILDREN) tot = 0;
+            tot += b;
+            if(tot > maxtot) maxtot = tot;
         }
-        if(tot > maxtot) maxtot = tot;
     }
-    /* too large to gain by sharing (eight batches of the lower size: 11.5 GB), or no room for all at once */
-    if(maxtot > SQB_MAXINST*CHILDREN_LOW || reserve_points(maxtot)) goto one_by_one;
+    if(reserve_points(maxtot)) goto one_by_one;                /* no room for all at once */
     CKR(cudaMemsetAsync(G.accm, 0, n*sizeof(sqb_acc_t), G.s));
     CKR(cudaEventRecord(G.e0, G.s));
-    for(long r = 0; r < rounds; r++){
+    for(long r = 0; r < rounds; r++) for(int k0 = 0; k0 < n;){
         sqb_eval_t a; memset(&a, 0, sizeof a); fill_eval(&a, &L0.t);
         a.esize = 1; a.stride = SQB_MAXD; a.flag_at = SQB_PFLAG; a.cells = 1;
         if(L0.sym && L0.sym->n > 1) a.sym = *L0.sym;
         a.part = G.bp; a.tkeep = G.bkeep; a.tfb = G.tfb; a.queue = G.queue;
         lvl_t rl; memset(&rl, 0, sizeof rl);
         rl.D = D; rl.abskip = L0.t.abskip; rl.v = G.v; rl.uu = G.uu; rl.stt = G.stt; rl.sym = a.sym;
-        long child0 = 0; int m = 0, toff = 0, last = 0, kof[SQB_MAXINST];
+        long child0 = 0; int m = 0, toff = 0, last = 0;
         a.sub = SQB_SUB;
-        for(int k = 0; k < n; k++){
+        /* the round's integrals in order, as many as a launch takes */
+        for(; k0 < n; k0++){
+            const int k = k0;
             if(r >= nbat[k]) continue;
+            if(m > 0 && child0 + batch_tiles(k, r) > GROUP_CHILDREN) break;
             const sqb_level_t &L = Ls[k];
             const long c0 = r*ncb[k], nc = L.ncell - c0 < ncb[k] ? L.ncell - c0 : ncb[k], nch = nc << D;
             sqb_inst_t &I = a.inst[m];
@@ -1004,12 +1015,12 @@ one_by_one:
             lvi_t &V = rl.inst[m];
             V.cells = (const signed char*)(L.cells + c0); V.n = nch; V.child0 = child0; V.st = L.st; V.last = L.last;
             V.pw = L.pw; V.thr = L.thr; V.next = L.next; V.cap = L.next_cap; V.acc = G.accm + k; V.base = G.basem + k;
-            last = L.last; kof[m] = k;
+            last = L.last;
             toff += 2*(2*L.K + 1);
             child0 += (nch + SQB_TILE - 1)/SQB_TILE*SQB_TILE;
             m++;
         }
-        (void)kof;
+        if(!m) break;
         a.ninst = m; a.ntile = child0/SQB_TILE; rl.ninst = m;
         /* the per-point thresholds of the first integral stand in the launch's own fields (unused by the
          * kernels in a multi-instance launch) */
