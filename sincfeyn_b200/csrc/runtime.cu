@@ -241,6 +241,10 @@ static int reserve_points(long n){
  * room for more. */
 #define CHILDREN (1L << 26)
 #define CHILDREN_LOW (1L << 25)
+/* whether the FP64 pass sums a level's tiles itself: where a batch gives every one of the cap resident CTAs two tiles or more.
+ * One answer for the whole level, a last short batch included: the two ways round |v| differently, and a level's sums
+ * do not depend on the size of its batches (a thread short of memory runs smaller ones) */
+static bool fuses(long ncell, long ncb, int D, long cap){ return ((ncell < ncb ? ncell : ncb) << D) >= 2*SQB_TILE*cap; }
 /* children per launch of a group's round: a launch takes the batches of as many of its integrals as fit (eight of the lower
  * size, four of the full one; a batch is never split, so that every integral keeps the batches it has alone) */
 #define GROUP_CHILDREN (SQB_MAXINST*CHILDREN_LOW)
@@ -843,7 +847,7 @@ again:
         int can = 0;
         const long cap = grid_cap(g, f64_which(g, L->t.fma) | (queue && !listm ? SQB_ATTR_LEVEL : 0),
                                   2*(2*G.K + 1)*sizeof(double), &can);
-        const bool fused = tile_sums() && !L->t.alldd && can && !use_split(g, &a, &L->t) && !listm && nch >= 2*SQB_TILE*cap;
+        const bool fused = tile_sums() && !L->t.alldd && can && !use_split(g, &a, &L->t) && !listm && fuses(L->ncell, ncb, D, cap);
         /* the predictor at the last level: which children to leave out, and their tiers */
         if(pon){
             if(sqb_vtab_predict(L->vt, cells, nc, D, L->st, G.K, L->thr, L->predict, L->esok, L->sym, G.cfl,
@@ -1008,7 +1012,7 @@ one_by_one:
             const long c0 = r*ncb[k], nc = L.ncell - c0 < ncb[k] ? L.ncell - c0 : ncb[k], nch = nc << D;
             sqb_inst_t &I = a.inst[m];
             I.pts = L.cells + c0; I.n = nc; I.child0 = child0; I.st = L.st; I.K = L.K; I.toff = toff;
-            I.fused = tile_sums() && cank[k] && nch >= 2*SQB_TILE*capk[k];
+            I.fused = tile_sums() && cank[k] && fuses(L.ncell, ncb[k], D, capk[k]);
             I.last = L.last; I.pw = L.pw; I.thr = L.thr; I.abserr = L.t.abserr; I.near_thr = L.t.nearf*L.t.abserr;
             I.X = L.X; I.Wt = L.Wt; I.U = level_axis(L, 0); I.Ud = level_axis(L, 1);
             if(I.fused) a.sub = 1;
