@@ -68,7 +68,8 @@ typedef struct {
     int growskip;          /* SINCQED_GROWSKIP, top = 0 only (2) */
     int alldd;             /* 1: every point in double-double (the plain all-dd form); 0: FP64 + fallback */
     int device;            /* CUDA device (0) */
-    long max_children;     /* children per device batch, 0 = default (2^26) */
+    long max_children;     /* children per device batch (35 bytes each), 0 = default: 2^26; 2^25 in a batch of more
+                              than sixteen workers, or where memory is short */
     int verbose;           /* 1: timing lines on stderr */
     double ckpt_every;     /* SINCQED_CKPT: > 0 writes a checkpoint at the end of every refinement level but the
                               last and resumes from a matching one (driver/checkpoint.c:1-6); 0 = off (the

@@ -33,8 +33,9 @@
 #include "sincfeyn_b200.h"
 
 static thread_local char E_[512];
-static thread_local double MEMSHARE = 1.0;    /* share of device memory for this thread's cell lists */
+static thread_local double MEMSHARE = 1.0;    /* share of device memory for this thread's cell lists and work buffers */
 extern "C" void sqb_set_mem_share(double f){ MEMSHARE = f > 0 && f <= 1 ? f : 1.0; }
+extern "C" double sqb_mem_share(void){ return MEMSHARE; }
 extern "C" const char *sqb_error(void){ return E_; }
 extern "C" void sqb_set_error_msg(const char *msg){ snprintf(E_, sizeof E_, "%s", msg); }
 #define FAIL(...) do { snprintf(E_, sizeof E_, __VA_ARGS__); return -1; } while(0)

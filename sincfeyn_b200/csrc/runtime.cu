@@ -236,11 +236,16 @@ static int reserve_points(long n){
     return -1;
 }
 /* children per batch unless the caller says: each batch costs about 80 us beside its children (the tails of its kernels, the
- * double-double pass's longest chain), and 43 bytes a child are held.  syn_d8 at h = 0.7 with 2^24, 2^25, 2^26, 2^27: 19.7, 16.6,
- * 15.3, 14.7 ms; 2.9 GB at 2^26.  The split pass holds its running sums as well: 2^25; so does a thread that finds no
- * room for more. */
+ * double-double pass's longest chain), and 35 bytes a child are held (alloc_points).  syn_d8 at h = 0.7 with 2^24, 2^25, 2^26,
+ * 2^27: 19.7, 16.6, 15.3, 14.7 ms; 2.35 GB at 2^26.  2^25 for the split pass, which holds its running sums as well; for a
+ * thread that finds no room for more; and for one of more than sixteen workers of a batch, so that together they take no
+ * more than the most workers (32) do with the lower size: 37.6 GB, which their cell lists, and an integral run again
+ * alone beside the workers' buffers, leave. */
 #define CHILDREN (1L << 26)
 #define CHILDREN_LOW (1L << 25)
+#define CHILDREN_SHARE (1.0/16)
+extern "C" double sqb_mem_share(void);
+extern "C" long sqb_share_children(double share){ return share >= CHILDREN_SHARE ? CHILDREN : CHILDREN_LOW; }
 /* whether the FP64 pass sums a level's tiles itself: where a batch gives every one of the cap resident CTAs two tiles or more.
  * One answer for the whole level, a last short batch included: the two ways round |v| differently, and a level's sums
  * do not depend on the size of its batches (a thread short of memory runs smaller ones) */
@@ -249,7 +254,7 @@ static bool fuses(long ncell, long ncb, int D, long cap){ return ((ncell < ncb ?
  * size, four of the full one; a batch is never split, so that every integral keeps the batches it has alone) */
 #define GROUP_CHILDREN (SQB_MAXINST*CHILDREN_LOW)
 static long batch_children(const sqb_graph_t *g, const sqb_level_t *L){
-    return L->max_children > 0 ? L->max_children : L->t.split && g->nparts > 0 ? CHILDREN_LOW : CHILDREN;
+    return L->max_children > 0 ? L->max_children : L->t.split && g->nparts > 0 ? CHILDREN_LOW : sqb_share_children(sqb_mem_share());
 }
 
 /* the FP64 kernel to run: the contracted one (which 2) when asked for and built, else the exact one */
