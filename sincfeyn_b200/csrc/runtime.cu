@@ -405,6 +405,7 @@ extern "C" int sqb_preload(const char *graph){
         if(graph && strcmp(graph, g->name)) continue;
         sqb_kattr_t at;
         for(int which = 0; which < 3; which++) if(g->attr(which, 128, 4096, &at)) n++;
+        for(int which = 0; which < 3; which += 2) n += g->attr(which | SQB_ATTR_REST, 128, 4096, &at);
         for(int P = 0; P <= g->nparts && g->nparts > 0; P++)
             for(int fma = 0; fma < 2; fma++) if(g->split_attr(P, fma, 128, 4096, &at)) n++;
     }

@@ -147,6 +147,8 @@ typedef struct {
     int sweeps;                   /* level kernel: passes over a batch's tiles (1, or 2: see SQB_SWEEPS) */
 } sqb_kattr_t;
 #define SQB_ATTR_LEVEL 4          /* attr(which | SQB_ATTR_LEVEL, ...): the FP64 level kernel's attributes */
+#define SQB_ATTR_REST 8           /* attr(which | SQB_ATTR_REST, ...): the FP64 build's other kernels (level kernel, axis form) are
+                                     loaded; returns their number */
 /* a launch that the FP64 level kernel runs: a level batch of cells (int8 coordinates) whose tiles come from
  * the device queue, not in list mode */
 static inline bool sqb_level_launch(const sqb_eval_t *a){

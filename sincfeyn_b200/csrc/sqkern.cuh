@@ -925,6 +925,19 @@ static bool sqb_ax_attr(int block, size_t smem, sqb_kattr_t *o, int *ok){
     }
     return false;
 }
+/* SQB_ATTR_REST: a build's level kernel and its axis form's kernels, loaded by asking for their attributes; their number */
+template<class K_>
+static int sqb_load(K_ kernel){ cudaFuncAttributes fa; return cudaFuncGetAttributes(&fa, kernel) == cudaSuccess; }
+template<class F, int D, int LV>
+static int sqb_load_rest(){
+    int n = 0;
+    if constexpr(LV > 0) n += sqb_load(sqb_k_f64<F, D, LV>);
+    if constexpr(F::template AX<double, 0>::NU > 0)
+        n += sqb_load(sqb_k_lvax<F, D, 0, 0>) + sqb_load(sqb_k_lvax<F, D, 1, 0>) + sqb_load(sqb_k_lvax<F, D, 0, 1>) +
+             sqb_load(sqb_k_lvax<F, D, 1, 1>) + sqb_load(sqb_k_ax<F, D, 0, 0>) + sqb_load(sqb_k_ax<F, D, 0, 1>) + sqb_load(sqb_k_ax<F, D, 1, 0>) +
+             sqb_load(sqb_k_axis<typename F::template AX<double, 0>, typename F::template AX<sqdd, 1>, D>);
+    return n;
+}
 template<class F, int D>
 static void sqb_ax_table(const double *X, int K, double *T, double *Td, cudaStream_t st){
     if constexpr(F::template AX<double, 0>::NU > 0)
@@ -979,6 +992,7 @@ extern "C" void SQB_##NAME##_f64fma(const sqb_eval_t *a, int grid, int block, si
     if(sqb_level_launch(a)) sqb_k_f64<SQG_NS(NAME)::F, D, 1><<<grid, block, smem, (cudaStream_t)st>>>(*a); \
     else sqb_k_f64<SQG_NS(NAME)::F, D, 0><<<grid, block, smem, (cudaStream_t)st>>>(*a); }           \
 extern "C" int SQB_##NAME##_attrfma(int lv, int block, size_t smem, sqb_kattr_t *o){               \
+    if(lv == SQB_ATTR_REST) return sqb_load_rest<SQG_NS(NAME)::F, D, 1>();                          \
     int ok; if(lv && sqb_ax_attr<SQG_NS(NAME)::F, D>(block, smem, o, &ok)) return ok;               \
     return lv ? sqb_f64_attr(sqb_k_f64<SQG_NS(NAME)::F, D, 1>, 1, block, smem, o)                  \
               : sqb_f64_attr(sqb_k_f64<SQG_NS(NAME)::F, D, 0>, 0, block, smem, o); }
@@ -1026,9 +1040,10 @@ static void axis(int fma, const double *X, int K, double *T, double *Td, void *s
     if(fma && SQB_##NAME##_axisfma) SQB_##NAME##_axisfma(X, K, T, Td, st);                         \
     else sqb_ax_table<F, D>(X, K, T, Td, (cudaStream_t)st); }                                      \
 static int attr(int which, int block, size_t smem, sqb_kattr_t *o){                                \
-    const int lv = (which & SQB_ATTR_LEVEL) != 0; which &= ~SQB_ATTR_LEVEL;                        \
+    const int lv = which & (SQB_ATTR_LEVEL | SQB_ATTR_REST); which &= ~lv;                         \
     if(which == 2) return SQB_##NAME##_attrfma ? SQB_##NAME##_attrfma(lv, block, smem, o) : 0;      \
     if(which == 1) return sqb_f64_attr(sqb_k_dd<F, D>, 0, block, smem, o);                         \
+    if(lv == SQB_ATTR_REST) return sqb_load_rest<F, D, SQB_LEVEL_KERNEL>();                         \
     int ok; if(lv && sqb_ax_attr<F, D>(block, smem, o, &ok)) return ok;                             \
     return SQB_LEVEL_KERNEL && lv ? sqb_f64_attr(sqb_k_f64<F, D, SQB_LEVEL_KERNEL>, 1, block, smem, o) \
                                   : sqb_f64_attr(sqb_k_f64<F, D, 0>, 0, block, smem, o); }         \
