@@ -197,6 +197,11 @@ class _Expr:
         self.op, self.text, self.args = op, text, args
 
 
+def _glue(op, right):
+    """op followed by right; a sign after a sign stays two signs."""
+    return op + (' ' if op == right[0] else '') + right
+
+
 def _parse(text):
     """The expression's tree, left-associative as C reads it; ValueError outside the subset."""
     toks, p = [], 0
@@ -223,7 +228,7 @@ def _parse(text):
         t = take()
         if t == '-':
             e = atom()
-            return _Expr('neg', '-' + e.text, (e,))
+            return _Expr('neg', _glue('-', e.text), (e,))
         if t == '(':
             e = add()
             take(')')
@@ -252,7 +257,7 @@ def _parse(text):
         while peek() in ops:
             o = take()
             f = sub()
-            e = _Expr(o, e.text + o + f.text, (e, f))
+            e = _Expr(o, e.text + _glue(o, f.text), (e, f))
         return e
 
     def mul():
@@ -297,7 +302,7 @@ def _shared_divisors(tail, carried):
         if e.op in ('num', 'id', 'idx'):
             return e.text
         if e.op == 'neg':
-            return '-' + text(e.args[0])
+            return _glue('-', text(e.args[0]))
         if e.op == 'par':
             return '(' + text(e.args[0]) + ')'
         if e.op == 'call':
@@ -305,7 +310,7 @@ def _shared_divisors(tail, carried):
         a, b = e.args
         if e.op == '/' and b.text in shared:
             return 'sq_divc<CK>(%s,%s,r_%s,sq_bad)' % (text(a), b.text, b.text)
-        return text(a) + e.op + text(b)
+        return text(a) + _glue(e.op, text(b))
     for head, e in trees:
         out.append('    %s%s;' % (head, text(e)))
     return ('\n'.join(out), shared) if shared else (tail, [])
@@ -328,6 +333,9 @@ def axis_plan(k):
     if not lm or int(lm.group(2)) != k.D or k.D < 4:
         return None
     decl, body, tail = lm.group(1), lm.group(3), lm.group(4)
+    # names that the class declares around the text
+    if any(n in ('S', 'CK', 'sq_bad') or n.startswith('r_') for n in re.findall(r'[A-Za-z_]\w*', m.group(1))):
+        return None
     carried = {}
     for d in decl.split(','):
         dm = re.match(r'^\s*([A-Za-z_]\w*)\s*=\s*(\d+(?:\.\d*)?)\s*$', d)
@@ -375,12 +383,12 @@ def axis_plan(k):
             if term and e.op == '*':
                 return rewrite(e.args[0]) + '*' + rewrite(e.args[1])
             if term and e.op in ('par', 'neg'):
-                return ('(%s)' if e.op == 'par' else '-%s') % rewrite(e.args[0], True)
+                return '(%s)' % rewrite(e.args[0], True) if e.op == 'par' else _glue('-', rewrite(e.args[0], True))
             return column(e)[0]
         if e.op == 'id':
             return 'S.' + e.text
         if e.op == 'neg':
-            return '-' + rewrite(e.args[0])
+            return _glue('-', rewrite(e.args[0]))
         if e.op == 'par':
             return '(' + rewrite(e.args[0]) + ')'
         if e.op == 'call':
@@ -392,7 +400,7 @@ def axis_plan(k):
                 if c not in recip:
                     recip.append(c)
                 return 'sq_divc<CK>(%s,%s,r[%d],sq_bad)' % (rewrite(a), name, recip.index(c))
-        return rewrite(a, e.op in '+-') + e.op + rewrite(b, e.op in '+-')
+        return rewrite(a, e.op in '+-') + _glue(e.op, rewrite(b, e.op in '+-'))
 
     try:
         for stmt in [x.strip() for x in body.split(';') if x.strip()]:
