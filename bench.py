@@ -146,12 +146,24 @@ def cpu_reference(graphs, threads):
     return ev, sec, rows
 
 
+def unavailable(args, why):
+    """The one line of an arm that cannot run here."""
+    metric = 'integrand points/s (time-to-sum) of the three-loop set at h=0.7' if args.workload == 'all3' else args.workload
+    print(json.dumps({'impl': args.impl, 'metric': metric, 'value': None, 'unit': 'points/s', 'n_gpus': args.gpus,
+                      'unavailable': why}), flush=True)
+
+
 def run_reference(args, rank):
     """--impl reference: the reference's CPU implementation of the path (oracle/_ref/sincqed, its OpenMP build,
     all host threads), same metric.  A step of ours is the whole set (minutes of CPU time per integral of
     D = 7, an hour or more for the set); a step here is one integral of the CPU sample in turn, which keeps
     the run to minutes: the warm-up steps run its cheapest integral."""
     if rank != 0:
+        return
+    sys.path.insert(0, os.path.join(ROOT, 'oracle'))
+    import refpy
+    if not refpy.available():
+        unavailable(args, 'oracle/_ref/sincqed (the reference\'s CPU build) is not built: it needs the reference\'s sources')
         return
     threads = os.cpu_count() or 1
     seq = [CPU_SAMPLE[i % len(CPU_SAMPLE)] for i in range(args.steps)]
@@ -417,6 +429,14 @@ def main():
     args = ap.parse_args()
     args.warmup = max(3, args.warmup)
     rank, world, local = env_rank()
+    if args.impl == 'ours':
+        from sincfeyn_b200 import sq
+        need = {'all3': [SET], 'mixed': MIX_SETS, 'vp4': ['vp4'], 'synth': ['synth']}.get(args.workload, [args.graph])
+        gone = [x for x in need if not sq.select([x])]
+        if gone:
+            if rank == 0:
+                unavailable(args, 'this library holds no graph of %s: it was built without the reference\'s kernels' % ', '.join(gone))
+            return
     if args.workload != 'all3':
         if rank == 0 and args.impl == 'ours':
             from sincfeyn_b200 import sq
