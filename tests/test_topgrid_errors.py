@@ -95,7 +95,7 @@ def lib(tmp_path_factory):
     (d / 'fake.c').write_text(FAKE)
     (d / 'harness.cu').write_text(HARNESS)
     subprocess.run(['gcc', '-w', '-std=gnu11', '-fPIC', '-c', str(d / 'fake.c'), '-o', str(d / 'fake.o')], check=True)
-    subprocess.run([NVCC, '-gencode', 'arch=compute_100a,code=sm_100a', '-O1', '-std=c++17', '-cudart', 'none', '-shared', '-Xcompiler', '-fPIC',
+    subprocess.run([NVCC, '-gencode', 'arch=compute_100a,code=sm_100a', '-O1', '-std=c++17', '-cudart', 'none', '-shared', '-Xlinker', '-Bsymbolic', '-Xcompiler', '-fPIC',
                     '-diag-suppress', '177,550', '-I' + CSRC, '-I' + os.path.join(ROOT, 'include'), '-o', str(d / 'topgrid.so'),
                     str(d / 'harness.cu'), str(d / 'fake.o')], check=True)
     L = C.CDLL(str(d / 'topgrid.so'))
