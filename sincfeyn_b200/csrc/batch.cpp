@@ -5,8 +5,8 @@
  * runs them concurrently from a pool of host worker threads.  Every worker owns a CUDA stream, its
  * buffers and its share of device memory (the runtime's state is per thread), and pulls the next
  * integral from a shared queue, largest estimated cost first (longest-processing-time order), so that
- * the latency-bound parts of one integral (the top-level grow, which waits for every frontier's sums
- * on the host) overlap the FP64-bound level passes of others and small integrals fill the gaps
+ * the latency-bound parts of one integral (the top-level grow: a chain of frontiers, each after the sums of
+ * the one before) overlap the FP64-bound level passes of others and small integrals fill the gaps
  * that a single integral's launches leave on the device.
  *
  * Device time: the caller's stream records a start event that every worker stream waits on before its

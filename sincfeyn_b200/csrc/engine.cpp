@@ -3,7 +3,7 @@
  *
  *   lattice      K rounded up to a multiple of 2^(top+1); EX[k+K] = e^{kh}, weight factor EX*h
  *                (driver/lattice.c:13-34);
- *   box_zero     4097 fixed probe nodes; an integrand that is 0 at all of them is reported as zero
+ *   zero probe   (box_zero) 4097 fixed nodes, made and tested on the device (topgrid.cu); an integrand that is 0 at all of them is reported as zero
  *                (driver/sum.c:346-359);
  *   grow         the support-following top level (driver/sumkey.h:126-461): breadth-first from z = 0
  *                over axis neighbours at step 2^top h; a frontier is evaluated as one device batch and
@@ -196,7 +196,7 @@ static int sym_nodes(void *ctx, long n, const int *k, double *f, double *ab){
     return sqb_eval_points_impl(R.g, n, sf.data(), 0, 1, f, ab);
 }
 
-/* One integral's run, in phases: begin() (lattice, symmetry group, checkpoint, box_zero, grow and dilate,
+/* One integral's run, in phases: begin() (lattice, symmetry group, checkpoint, zero probe, grow and dilate,
  * or the resumed state), then per refinement level prep() (the level's sqb_level_t and next list) and
  * done() (the level's sums, its checkpoint, the lists swapped), then end() (the result).  sqb_hsum runs
  * them for one integral; sqb_hsum_group runs several integrals of one graph with their levels in shared

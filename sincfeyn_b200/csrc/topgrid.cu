@@ -602,7 +602,9 @@ __global__ void __launch_bounds__(TG_T) k_gs_tiles(const __grid_constant__ geom_
         if(i >= n) break;
         fsum_add(f, c[0], c[1], g, fr, v, stt, uu, pw, i);
         const u64 x = ok ? seq_units(__dmul_rn(fabs(v[i]), pw), inv) : SQ_ODD;
-        if(x == SQ_ODD || x >= SQ_ONE53 >> 11) c[2] = 1; else c[3] += x;      /* GS_TILE = 2^11 terms below 2^53 in all */
+        /* GS_TILE = 2^11 terms below 2^42 cannot overflow the tile's sum (nor would 2^52: what the sums may not pass is
+         * tested where they are added up); a tile with a larger one goes element by element */
+        if(x == SQ_ODD || x >= SQ_ONE53 >> 11) c[2] = 1; else c[3] += x;
     }
     block_sums<TG_T, 4, 4>(f, c, sh);
     if(threadIdx.x == 0) part[blockIdx.x] = gpart_t{c[2] ? SQ_ODD : c[3], {{f[0].hi, f[0].lo}, {f[1].hi, f[1].lo}, {f[2].hi, f[2].lo},
